@@ -56,8 +56,10 @@ struct RunDesc {
     uint32_t pbase;      // first particle
     uint32_t np;         // particles
     uint32_t tile_base;  // first CTA of the run in the tiled deposit
-    uint32_t en_base;    // first block of the run in the energy sums
-    uint32_t en_blocks;  // blocks of the run in the energy sums
+    uint32_t en_base;    // first block of the run in the kinetic sums
+    uint32_t en_blocks;  // blocks of the run in the kinetic sums
+    uint32_t fe_base;    // the same of the field sums
+    uint32_t fe_blocks;
     int N;
     int tile_w, tile_h, tiles_x;
     float maxq;          // |q| of the run's particles
@@ -612,79 +614,106 @@ __global__ void ens_scale_efield(const RunDesc* __restrict__ runs, int nruns, ui
 // Per-run energies of the step into hist[step*nruns + r]: field energy
 // 0.5*sum(Ex^2+Ey^2) (FP64) and kinetic 0.5*m*sum(vx^2+vy^2), summed in FP32
 // per thread (a few thousand particles) and in FP64 across threads (FP64
-// arithmetic per particle would cost more than the step's particle work). Blocks are given to runs in
-// proportion to their particles (EN_CHUNK per block); a run's blocks are added
-// in index order, so the result does not depend on the launch.
+// arithmetic per particle would cost more than the step's particle work).
+//
+// Kinetic: a run's particles are cut into blocks of about EN_CHUNK, a block
+// into 256 chains (chain t: every 256th particle from t), each one FP32 sum in
+// index order. One warp owns 32 chains and is a CTA of its own, so a small
+// ensemble's few blocks spread over the SMs: a chain is serial, and the time is
+// the latency of its loads, hidden by EN_UNROLL of them per lane in flight.
+// (Eight warps per CTA, one load in flight: 966 us for 16.6 M particles in 23
+// blocks, 23 SMs busy; bound now by the chain's loads and adds.)
+// Field: one warp per FE_CELLS cells. A run's partial sums depend on the run
+// alone and are added in a fixed order.
 constexpr size_t EN_CHUNK = 1 << 20;
-__global__ void ens_energy_partials(const RunDesc* __restrict__ runs, int nruns, const double* __restrict__ Ex,
-                                    const double* __restrict__ Ey, const float* __restrict__ vx,
-                                    const float* __restrict__ vy, double* __restrict__ partial) {
-    __shared__ uint32_t ebase[MAX_RUNS];
-    __shared__ double ws[2][ENS_THREADS / 32];
-    for (int i = threadIdx.x; i < nruns; i += ENS_THREADS) ebase[i] = runs[i].en_base;
-    __syncthreads();
-    const int r = find_run(ebase, nruns, blockIdx.x);
-    const RunDesc& R = runs[r];
-    const int b = (int)(blockIdx.x - R.en_base), nb = (int)R.en_blocks;
-    double fe = 0.0, ke = 0.0;
-    {
-        const size_t n = R.cells, chunk = (n + nb - 1) / nb;
-        const size_t s = (size_t)b * chunk, e = s + chunk < n ? s + chunk : n;
-        for (size_t i = s + threadIdx.x; i < e; i += ENS_THREADS) {
-            const double ex = Ex[R.cell_base + i], ey = Ey[R.cell_base + i];
-            fe = __dadd_rn(fe, __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
-        }
-    }
-    {
-        const size_t n = R.np, chunk = (n + nb - 1) / nb;
-        const size_t s = (size_t)b * chunk, e = s + chunk < n ? s + chunk : n;
-        float kf = 0.0f;
-        for (size_t i = s + threadIdx.x; i < e; i += ENS_THREADS) {
-            const float a = vx[R.pbase + i], c = vy[R.pbase + i];
-            kf += a * a + c * c;
-        }
-        ke = (double)kf;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+constexpr int EN_CHAINS = 8;  // warps (32 chains each) of a kinetic block
+constexpr int EN_UNROLL = 32;
+constexpr uint32_t FE_CELLS = 4096;
+
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        fe = __dadd_rn(fe, __shfl_down_sync(FULLM, fe, o));
-        ke = __dadd_rn(ke, __shfl_down_sync(FULLM, ke, o));
-    }
-    if (lane == 0) {
-        ws[0][warp] = fe;
-        ws[1][warp] = ke;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, c = 0.0;
-        for (int w = 0; w < ENS_THREADS / 32; ++w) {
-            a = __dadd_rn(a, ws[0][w]);
-            c = __dadd_rn(c, ws[1][w]);
-        }
-        partial[2 * blockIdx.x] = a;
-        partial[2 * blockIdx.x + 1] = c;
-    }
+    for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(FULLM, v, o));
+    return v;
 }
 
-__global__ void ens_energy_final(const RunDesc* __restrict__ runs, const float* __restrict__ mass,
-                                 const double* __restrict__ partial, int nruns, const int* __restrict__ step,
-                                 int max_steps, double* __restrict__ fe_hist, double* __restrict__ ke_hist) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32) ens_energy_partials(const RunDesc* __restrict__ runs, int nruns,
+                                                          uint32_t ke_warps, const double* __restrict__ Ex,
+                                                          const double* __restrict__ Ey, const float* __restrict__ vx,
+                                                          const float* __restrict__ vy, double* __restrict__ partial) {
+    __shared__ uint32_t base[MAX_RUNS];
+    const int lane = threadIdx.x;
+    const bool kinetic = blockIdx.x < ke_warps;
+    for (int i = lane; i < nruns; i += 32) base[i] = kinetic ? runs[i].en_base : runs[i].fe_base;
+    __syncwarp();
+    double v = 0.0;
+    if (kinetic) {
+        const uint32_t blk = blockIdx.x / EN_CHAINS, w = blockIdx.x % EN_CHAINS;
+        const RunDesc& R = runs[find_run(base, nruns, blk)];
+        const size_t n = R.np, nb = R.en_blocks, chunk = (n + nb - 1) / nb;
+        const size_t s = (size_t)(blk - R.en_base) * chunk, e = s + chunk < n ? s + chunk : n;
+        const float *px = vx + R.pbase, *py = vy + R.pbase;
+        constexpr int STEP = EN_CHAINS * 32;
+        float a[EN_UNROLL], c[EN_UNROLL];
+        size_t i = s + w * 32 + lane;
+        auto load = [&](size_t i0) {
+#pragma unroll
+            for (int k = 0; k < EN_UNROLL; ++k) {
+                const bool in = i0 + (size_t)k * STEP < e;  // past the end: zeros, which leave the sum as it is
+                a[k] = in ? __ldcs(px + i0 + k * STEP) : 0.0f;
+                c[k] = in ? __ldcs(py + i0 + k * STEP) : 0.0f;
+            }
+        };
+        float kf = 0.0f;
+        load(i);
+        for (; i < e; i += (size_t)EN_UNROLL * STEP) {
+            float t[EN_UNROLL];
+#pragma unroll
+            for (int k = 0; k < EN_UNROLL; ++k) t[k] = a[k] * a[k] + c[k] * c[k];
+            load(i + (size_t)EN_UNROLL * STEP);
+#pragma unroll
+            for (int k = 0; k < EN_UNROLL; ++k) kf += t[k];
+        }
+        v = warp_sum((double)kf);
+    } else {
+        const uint32_t blk = blockIdx.x - ke_warps;
+        const RunDesc& R = runs[find_run(base, nruns, blk)];
+        const uint32_t s = (blk - R.fe_base) * FE_CELLS, e = min(s + FE_CELLS, R.cells);
+#pragma unroll 4
+        for (uint32_t i = s + lane; i < e; i += 32) {
+            const double ex = Ex[R.cell_base + i], ey = Ey[R.cell_base + i];
+            v = __dadd_rn(v, __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
+        }
+        v = warp_sum(v);
+    }
+    if (lane == 0) partial[blockIdx.x] = v;
+}
+
+// One warp per run at a time, one block; then the step counter.
+__global__ void __launch_bounds__(1024) ens_energy_final(const RunDesc* __restrict__ runs,
+                                                         const float* __restrict__ mass,
+                                                         const double* __restrict__ partial, uint32_t ke_warps,
+                                                         int nruns, int* __restrict__ step, int max_steps,
+                                                         double* __restrict__ fe_hist, double* __restrict__ ke_hist) {
+    const int lane = threadIdx.x & 31;
     const int s = *step;
-    if (r < nruns && s < max_steps) {
-        const RunDesc& R = runs[r];
-        double a = 0.0, c = 0.0;
-        for (uint32_t b = R.en_base; b < R.en_base + R.en_blocks; ++b) {
-            a = __dadd_rn(a, partial[2 * b]);
-            c = __dadd_rn(c, partial[2 * b + 1]);
+    if (s < max_steps)
+        for (int r = threadIdx.x >> 5; r < nruns; r += 32) {
+            const RunDesc& R = runs[r];
+            double c = 0.0, a = 0.0;
+            for (uint32_t b = R.en_base * EN_CHAINS + lane; b < (R.en_base + R.en_blocks) * EN_CHAINS; b += 32)
+                c = __dadd_rn(c, partial[b]);
+            for (uint32_t b = R.fe_base + lane; b < R.fe_base + R.fe_blocks; b += 32)
+                a = __dadd_rn(a, partial[ke_warps + b]);
+            c = warp_sum(c);
+            a = warp_sum(a);
+            if (lane == 0) {
+                fe_hist[(size_t)s * nruns + r] = __dmul_rn(0.5, a);
+                ke_hist[(size_t)s * nruns + r] = __dmul_rn(__dmul_rn(0.5, (double)mass[r]), c);
+            }
         }
-        fe_hist[(size_t)s * nruns + r] = __dmul_rn(0.5, a);
-        ke_hist[(size_t)s * nruns + r] = __dmul_rn(__dmul_rn(0.5, (double)mass[r]), c);
-    }
+    __syncthreads();
+    if (threadIdx.x == 0) *step = s + 1;
 }
-
-__global__ void bump_step(int* step) { *step += 1; }
 
 // ring[step] = the order breaks the step's kernel counted; the counter restarts
 __global__ void take_breaks(unsigned long long* counter, unsigned long long* ring, const int* step, int cap) {
@@ -721,7 +750,8 @@ struct pic_ens {
     long long sorts = 0;
     long long steps_done = 0;
     int coop_blocks = 0;
-    uint32_t en_blocks = 0;  // blocks of the energy sums (all runs)
+    uint32_t en_blocks = 0;  // blocks of the kinetic sums (all runs)
+    uint32_t fe_blocks = 0;  // and of the field sums
     bool tuned = false;
     // batched FFT per grid size
     struct Batch {
@@ -849,15 +879,13 @@ int poisson(pic_ens* e) {
 int energies(pic_ens* e) {
     pic_ctx* c = e->c;
     const int nr = (int)e->runs.size();
-    ens_energy_partials<<<e->en_blocks, ENS_THREADS, 0, c->stream>>>(e->druns, nr, c->Ex, c->Ey, c->vx, c->vy,
-                                                                    e->en_partial);
+    const uint32_t ke_warps = e->en_blocks * EN_CHAINS;
+    ens_energy_partials<<<ke_warps + e->fe_blocks, 32, 0, c->stream>>>(e->druns, nr, ke_warps, c->Ex, c->Ey, c->vx,
+                                                                       c->vy, e->en_partial);
     PIC_TRY(check_launch(c, "ens_energy_partials"));
-    ens_energy_final<<<(nr + 127) / 128, 128, 0, c->stream>>>(e->druns, e->dmass, e->en_partial, nr, e->step_ctr,
-                                                              e->hist_cap, e->fe_hist, e->ke_hist);
-    PIC_TRY(check_launch(c, "ens_energy_final"));
-    bump_step<<<1, 1, 0, c->stream>>>(e->step_ctr);
-    c->launches += 3;
-    return check_launch(c, "bump_step");
+    ens_energy_final<<<1, 1024, 0, c->stream>>>(e->druns, e->dmass, e->en_partial, ke_warps, nr, e->step_ctr,
+                                                e->hist_cap, e->fe_hist, e->ke_hist);
+    return check_launch(c, "ens_energy_final");
 }
 
 // The step without a sort: persistent kernel, Poisson, energies.
@@ -1037,6 +1065,9 @@ int pic_ens_create(const pic_ens_member* runs_in, int nruns, const pic_ens_confi
         r.en_base = e->en_blocks;
         r.en_blocks = (uint32_t)std::max<size_t>(1, (r.np + EN_CHUNK - 1) / EN_CHUNK);
         e->en_blocks += r.en_blocks;
+        r.fe_base = e->fe_blocks;
+        r.fe_blocks = (r.cells + FE_CELLS - 1) / FE_CELLS;
+        e->fe_blocks += r.fe_blocks;
     }
     int out_rc = PIC_OK;
     auto A = [&](size_t bytes) { return out_rc ? nullptr : dalloc(bytes, &out_rc); };
@@ -1046,7 +1077,7 @@ int pic_ens_create(const pic_ens_member* runs_in, int nruns, const pic_ens_confi
     e->err = (int*)A(sizeof(int));
     e->step_ctr = (int*)A(sizeof(int));
     e->breaks = (unsigned long long*)A(sizeof(unsigned long long));
-    e->en_partial = (double*)A(sizeof(double) * 2 * e->en_blocks);
+    e->en_partial = (double*)A(sizeof(double) * ((size_t)e->en_blocks * EN_CHAINS + e->fe_blocks));
     if (out_rc == PIC_OK) out_rc = ensure_fields(c);
     if (out_rc == PIC_OK) out_rc = upload_runs(e);
     if (out_rc == PIC_OK && (cudaMemcpyAsync(e->dmass, mass.data(), sizeof(float) * nruns, cudaMemcpyHostToDevice,

@@ -187,39 +187,57 @@ static int rb_finish(pic_ctx* c) {
 }
 
 // ---- one cooperative launch per solve ---------------------------------------
-// Each CTA owns a tw x th tile of phi and keeps it, with a halo of PS_HALO
-// cells and the matching piece of b, in shared memory. Between two exchanges it
-// performs PS_HALO half-sweeps (two full red-black sweeps) on its extended
-// tile, the updated region shrinking by one cell per half-sweep, so the owned
-// cells end with exactly the values the one-launch-per-colour path computes
-// (same update, same operation order, same colour order). Then it writes its
-// owned cells back, waits at a grid-wide barrier and reloads its halo. The
-// residual is checked every check_every sweeps: per-CTA sums of r^2 and b^2,
-// a barrier, and every CTA adds the partials in index order and takes the
-// same decision. Barriers give up after about one second (PIC_ERR_TIMEOUT).
-constexpr int PS_THREADS = RB_THREADS;
-constexpr int PS_HALO = 4;
+// The grid is cut into ntx x nty tiles (sizes differ by at most one cell), one
+// CTA each, as many as fill the SMs. A CTA keeps its tile of phi, a halo of
+// `halo` cells around it and the matching piece of b in shared memory for the
+// whole solve, the two colours in separate arrays (neighbouring lanes touch
+// neighbouring words). Between two exchanges it performs `halo` half-sweeps
+// (halo / 2 full red-black sweeps) on the extended tile, the updated region
+// shrinking by one cell per half-sweep, so the owned cells end with exactly the
+// values the one-launch-per-colour path computes (same update, same operation
+// order, same colour order). It then publishes the cells near its edge through
+// one of two exchange buffers in turn and loads its halo from its neighbours'. Each
+// 32-bit word travels with the exchange's number in one 64-bit word, so a value
+// says itself whether it has arrived: no flag, no fence and no grid barrier between
+// its store and its load. (A neighbour can be one exchange ahead at most, hence
+// two buffers.) The residual is checked every check_every
+// sweeps: per-CTA sums of r^2 and b^2, a grid-wide barrier, and every CTA adds
+// the partials in the same order and takes the same decision. Waits give up
+// after about one second (PIC_ERR_TIMEOUT).
+//
+// Bound by FP64 arithmetic (a warp's FP64 instruction takes the SM 16 cycles) and
+// by the exchange's latency, a store and a load through L2.
+// rb_tiling picks tile counts and halo for the smallest sum of the two. With
+// equal spacings that are powers of two (unit cells, say) an update is four FP64
+// instructions instead of seven, with the same bits: the products are exact, so
+// (we*s + sn*s + b)*inv is one fused multiply-add of we + sn and b*inv.
+// 256^2, tol 1e-8, 57,920 sweeps from phi = 0: 102 ms in FP64 (1.8 us a sweep), 54 ms
+// mixed; 515 and 208 ms with 64 x 32 tiles (32 CTAs), seven instructions, an index
+// division per update and a grid-wide barrier per exchange. 64^2, 3,648 sweeps: 3.5
+// ms, from 31. Flags with release and acquire instead of numbered words: 160 ms.
 constexpr int PS_MAX_BLOCKS = 4096;
+constexpr size_t PS_MAX_SMEM = 225 * 1024;
 constexpr unsigned long long PS_WAIT_NS = 1000000000ull;
-
-struct PsArgs {
-    RbArgs a;
-    int tw, th, tiles_x, ew, eh;
-    double tol;
-    int max_iters, check_every;
-    double* partial;  // [2 * blocks]
-    unsigned* bar;    // [0] arrivals, [1] generation
-    int* err;
-    double* out;      // [0] sweeps, [1] residual, [2] first residual
-    int absent_block; // -1, or a CTA that leaves at once (the timeout test hook)
-    unsigned long long wait_ns;  // limit of one barrier wait
-};
 
 __device__ __forceinline__ uint64_t ps_time_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+
+// Limits a spin: true once wait_ns have passed since the first look at the clock.
+// %globaltimer is slow to read (about a microsecond, as much as the whole wait), so
+// only every 256th poll looks.
+struct PsLimit {
+    unsigned polls = 0;
+    uint64_t t0 = 0;
+    __device__ __forceinline__ bool over(unsigned long long wait_ns) {
+        if ((++polls & 255u) != 0) return false;
+        const uint64_t t = ps_time_ns();
+        if (t0 == 0) t0 = t;
+        return t - t0 > wait_ns;
+    }
+};
 
 __device__ bool ps_barrier(unsigned* bar, int* err, unsigned long long wait_ns = PS_WAIT_NS) {
     __syncthreads();
@@ -234,9 +252,9 @@ __device__ bool ps_barrier(unsigned* bar, int* err, unsigned long long wait_ns =
             __threadfence();
             atomicAdd(bar + 1, 1u);
         } else {
-            const uint64_t t0 = ps_time_ns();
+            PsLimit limit;
             while (*vgen == gen)
-                if (ps_time_ns() - t0 > wait_ns) {
+                if (limit.over(wait_ns)) {
                     atomicExch(err, 1);
                     ok = 0;
                     break;
@@ -253,92 +271,241 @@ __device__ __forceinline__ int ps_wrap(int i, int n) {
     return r < 0 ? r + n : r;
 }
 
-__global__ void __launch_bounds__(PS_THREADS) rbgs_persistent(PsArgs p) {
-    extern __shared__ double psm[];
-    const int E = p.ew * p.eh;
-    double* sphi = psm;
-    double* sb = psm + E;
+// A value and its exchange's number: one 64-bit word, stored and loaded whole, per
+// 32 bits of the value.
+__device__ __forceinline__ unsigned long long ps_pack(unsigned word, unsigned epoch) {
+    return (unsigned long long)epoch << 32 | word;
+}
+__device__ __forceinline__ void ps_publish(unsigned long long* x, size_t i, float v, unsigned epoch) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(x + i), "l"(ps_pack(__float_as_uint(v), epoch)) : "memory");
+}
+__device__ __forceinline__ void ps_publish(unsigned long long* x, size_t i, double v, unsigned epoch) {
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(x + 2 * i),
+                 "l"(ps_pack((unsigned)__double2loint(v), epoch)), "l"(ps_pack((unsigned)__double2hiint(v), epoch))
+                 : "memory");
+}
+__device__ __forceinline__ bool ps_receive(const unsigned long long* x, size_t i, unsigned epoch, float& v) {
+    unsigned long long a;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(a) : "l"(x + i) : "memory");
+    v = __uint_as_float((unsigned)a);
+    return (unsigned)(a >> 32) == epoch;
+}
+__device__ __forceinline__ bool ps_receive(const unsigned long long* x, size_t i, unsigned epoch, double& v) {
+    unsigned long long lo, hi;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(x + 2 * i) : "memory");
+    v = __hiloint2double((int)(unsigned)hi, (int)(unsigned)lo);
+    return (unsigned)(lo >> 32) == epoch && (unsigned)(hi >> 32) == epoch;
+}
+
+template <typename T>
+struct PsArgs {
+    T* x;         // phi (FP64), or the correction (FP32); read at the start, written at the end
+    const T* b;   // right-hand side
+    unsigned long long* xb;  // exchange buffers, 2 * Nx * Ny values of sizeof(T) / 4 words (ps_pack); zeroed
+    int Nx, Ny, ntx, nty;
+    T ix2, iy2, inv_denom, denom;
+    double tol;
+    int max_iters, check_every;
+    double* partial;  // [2][2 * PS_MAX_BLOCKS]
+    unsigned* bar;    // [0] arrivals, [1] generation
+    int* err;
+    double* out;      // [0] sweeps, [1] residual, [2] first residual
+    int absent_block; // -1, or a CTA that leaves at once (the timeout test hook)
+    unsigned long long wait_ns;  // limit of one wait
+};
+
+// Sum over the block in a fixed order, the same value in every thread.
+__device__ __forceinline__ double ps_block_sum(double v) {
+    __shared__ double ws[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
+    if (lane == 0) ws[warp] = v;
+    __syncthreads();
+    double s = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s = __dadd_rn(s, ws[w]);
+    __syncthreads();
+    return s;
+}
+
+__device__ __forceinline__ double ps_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float ps_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// t / d for 0 <= t < 2^20, d < 2^10, with inv = 1 / d: the quotient of t + 0.5 is at
+// least 1 / (2 d) away from an integer, far more than the rounding of the product.
+__device__ __forceinline__ int ps_div(int t, float inv) { return (int)(((float)t + 0.5f) * inv); }
+
+// POW2: equal spacings, a power of two; sb holds b * inv_denom (exact).
+// The FP32 correction solve also stops when rounding stalls it.
+// H: the halo. NPT: the updates of a thread in a half-sweep at most; their places
+// are worked out once and kept in registers (a division, address arithmetic and a
+// second round of latency per update otherwise, most of a half-sweep's time).
+template <typename T, bool POW2, int H, int NPT>
+__global__ void __launch_bounds__(1024) rbgs_persistent(PsArgs<T> p) {
+    constexpr bool STALL = sizeof(T) == 4;
+    extern __shared__ __align__(16) unsigned char psm[];
     __shared__ double tot[2];
-    const RbArgs& a = p.a;
+    __shared__ int s_nh, s_nb, s_ok;
     if ((int)blockIdx.x == p.absent_block) return;
-    const int tx = blockIdx.x % p.tiles_x, ty = blockIdx.x / p.tiles_x;
-    const int ox = tx * p.tw - PS_HALO, oy = ty * p.th - PS_HALO;
-    for (int i = threadIdx.x; i < E; i += PS_THREADS) {
-        const int ly = i / p.ew, lx = i - ly * p.ew;
-        const size_t g = (size_t)ps_wrap(oy + ly, a.Ny) * a.Nx + ps_wrap(ox + lx, a.Nx);
-        sb[i] = a.b[g];
-        sphi[i] = a.phi[g];
+    const int nthr = blockDim.x;
+    const int tx = blockIdx.x % p.ntx, ty = blockIdx.x / p.ntx;
+    // tile t of n tiles over N cells starts at t * N / n
+    const int xs = (int)((long long)tx * p.Nx / p.ntx), xe = (int)((long long)(tx + 1) * p.Nx / p.ntx);
+    const int ys = (int)((long long)ty * p.Ny / p.nty), ye = (int)((long long)(ty + 1) * p.Ny / p.nty);
+    const int tw = xe - xs, th = ye - ys, ew = tw + 2 * H, eh = th + 2 * H;
+    const int ox = xs - H, oy = ys - H;
+    const int hw = (ew + 1) >> 1, plane = hw * eh;  // one colour: eh rows of hw cells
+    T* sx = reinterpret_cast<T*>(psm);              // [2 colours][plane]
+    T* sb = sx + 2 * plane;
+    uint2* list = reinterpret_cast<uint2*>(sb + 2 * plane);  // (shared index, global index): halo, then edge cells
+    if (threadIdx.x == 0) s_nh = s_nb = 0;
+    __syncthreads();
+    // colour of the extended tile's cell (lx, ly), global parity of ox + lx + oy + ly
+    const int par0 = (ox + oy) & 1;
+    auto at = [&](int lx, int ly) { return (((par0 + lx + ly) & 1) ? plane : 0) + ly * hw + (lx >> 1); };
+    const float inv_ew = 1.0f / (float)ew;
+    const int E = ew * eh, nown = tw * th;
+    auto in_halo = [&](int lx, int ly) { return lx < H || lx >= H + tw || ly < H || ly >= H + th; };
+    for (int i = threadIdx.x; i < E; i += nthr) {
+        const int ly = ps_div(i, inv_ew), lx = i - ly * ew;
+        const size_t g = (size_t)ps_wrap(oy + ly, p.Ny) * p.Nx + ps_wrap(ox + lx, p.Nx);
+        const int k = at(lx, ly);
+        sb[k] = POW2 ? p.b[g] * p.inv_denom : p.b[g];
+        sx[k] = p.x[g];
+        if (in_halo(lx, ly)) list[atomicAdd(&s_nh, 1)] = make_uint2((unsigned)k, (unsigned)g);
     }
     __syncthreads();
-    const int nown = p.tw * p.th;
-    double bb = 0.0;
-    for (int t = threadIdx.x; t < nown; t += PS_THREADS) {
-        const int i = (PS_HALO + t / p.tw) * p.ew + PS_HALO + t % p.tw;
-        bb = __dadd_rn(bb, __dmul_rn(sb[i], sb[i]));
+    const int nh = s_nh;
+    for (int i = threadIdx.x; i < E; i += nthr) {  // owned cells within H of the tile's edge
+        const int ly = ps_div(i, inv_ew), lx = i - ly * ew;
+        if (in_halo(lx, ly) || !(lx < 2 * H || lx >= tw || ly < 2 * H || ly >= th)) continue;
+        const unsigned g = (unsigned)((oy + ly) * p.Nx + ox + lx);
+        list[nh + atomicAdd(&s_nb, 1)] = make_uint2((unsigned)at(lx, ly), g);
     }
-    bb = rb_block_sum(bb);
-    if (threadIdx.x == 0) p.partial[2 * blockIdx.x + 1] = bb;
+    __syncthreads();
+    const int nb = s_nb;
+    const uint2* edge = list + nh;
+    const size_t G = (size_t)p.Nx * p.Ny;
+    const float inv_tw = 1.0f / (float)tw;
+    auto own_b = [&](int k) { return POW2 ? sb[k] * p.denom : sb[k]; };  // exact
+    double bb = 0.0;
+    for (int t = threadIdx.x; t < nown; t += nthr) {
+        const int r = ps_div(t, inv_tw);
+        const double v = (double)own_b(at(H + t - r * tw, H + r));
+        bb = __dadd_rn(bb, __dmul_rn(v, v));
+    }
+    bb = ps_block_sum(bb);
+    // half-sweep k updates colour k & 1 in rows and columns k + 1 .. of the extended
+    // tile: (index << 1 | column parity), or -1
+    int place[H][NPT];
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+        const int lo = k + 1, rows = eh - 2 * lo, half = (ew - 2 * lo + 1) >> 1;
+        const float inv_half = 1.0f / (float)half;
+#pragma unroll
+        for (int n = 0; n < NPT; ++n) {
+            const int t = threadIdx.x + n * nthr;
+            const int r = ps_div(t, inv_half), ly = lo + r;
+            const int lx = lo + ((par0 + lo + ly + (k & 1)) & 1) + 2 * (t - r * half);
+            place[k][n] = t < rows * half && lx < ew - lo ? ((ly * hw + (lx >> 1)) << 1) | (lx & 1) : -1;
+        }
+    }
     int it = 0;
-    double res = 0.0, res0 = -1.0;
+    unsigned epoch = 0, check = 0;
+    double res = 0.0, res0 = -1.0, prev = 1e300;
+    const T c4 = p.ix2 * p.inv_denom;  // POW2: exact
+    bool failed = false;
     for (;;) {
         if (it % p.check_every == 0 || it >= p.max_iters) {
             double rr = 0.0;
-            for (int t = threadIdx.x; t < nown; t += PS_THREADS) {
-                const int i = (PS_HALO + t / p.tw) * p.ew + PS_HALO + t % p.tw;
-                const double we = __dadd_rn(sphi[i - 1], sphi[i + 1]);
-                const double sn = __dadd_rn(sphi[i - p.ew], sphi[i + p.ew]);
-                const double ap = __dsub_rn(__dsub_rn(__dmul_rn(a.denom, sphi[i]), __dmul_rn(we, a.ix2)),
-                                            __dmul_rn(sn, a.iy2));
-                const double r = __dsub_rn(sb[i], ap);
-                rr = __dadd_rn(rr, __dmul_rn(r, r));
+            for (int t = threadIdx.x; t < nown; t += nthr) {
+                const int r = ps_div(t, inv_tw);
+                const int ly = H + r, lx = H + t - r * tw, k = at(lx, ly), odd = lx & 1;
+                const int o = (k < plane ? plane : 0) + ly * hw + (lx >> 1);  // the other colour, same row and pair
+                const T we = sx[o - 1 + odd] + sx[o + odd], sn = sx[o - hw] + sx[o + hw];
+                const T ap = p.denom * sx[k] - we * p.ix2 - sn * p.iy2;
+                const double q = (double)(own_b(k) - ap);
+                rr = __dadd_rn(rr, __dmul_rn(q, q));
             }
-            rr = rb_block_sum(rr);
-            if (threadIdx.x == 0) p.partial[2 * blockIdx.x] = rr;
-            if (!ps_barrier(p.bar, p.err, p.wait_ns)) break;
+            rr = ps_block_sum(rr);
+            // two sets in turn: a CTA far away can reach its next check before this
+            // one has read the set of this check, but not the one after
+            double* partial = p.partial + (check++ & 1u) * 2 * PS_MAX_BLOCKS;
             if (threadIdx.x == 0) {
+                partial[2 * blockIdx.x] = rr;
+                partial[2 * blockIdx.x + 1] = bb;
+            }
+            if (!ps_barrier(p.bar, p.err, p.wait_ns)) {
+                failed = true;
+                break;
+            }
+            if (threadIdx.x < 32) {
                 double s1 = 0.0, s2 = 0.0;
-                for (unsigned k = 0; k < gridDim.x; ++k) {
-                    s1 = __dadd_rn(s1, p.partial[2 * k]);
-                    s2 = __dadd_rn(s2, p.partial[2 * k + 1]);
+                for (unsigned k = threadIdx.x; k < gridDim.x; k += 32) {
+                    s1 = __dadd_rn(s1, __ldcg(partial + 2 * k));
+                    s2 = __dadd_rn(s2, __ldcg(partial + 2 * k + 1));
                 }
-                tot[0] = s1;
-                tot[1] = s2;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    s1 = __dadd_rn(s1, __shfl_down_sync(0xffffffffu, s1, o));
+                    s2 = __dadd_rn(s2, __shfl_down_sync(0xffffffffu, s2, o));
+                }
+                if (threadIdx.x == 0) {
+                    tot[0] = s1;
+                    tot[1] = s2;
+                }
             }
             __syncthreads();
-            res = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : sqrt(tot[0]);
+            res = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : STALL ? 0.0 : sqrt(tot[0]);
             if (res0 < 0.0) res0 = res;
-            if (res <= p.tol || it >= p.max_iters) break;
+            if (res <= p.tol || it >= p.max_iters || (STALL && res > 0.999 * prev)) break;
+            prev = res;
         }
-        for (int k = 0; k < PS_HALO; ++k) {
-            const int color = k & 1;
-            const int lo = k + 1;
-            const int rows = p.eh - 2 * lo, cols = p.ew - 2 * lo;
-            const int half = (cols + 1) >> 1;
-            for (int t = threadIdx.x; t < rows * half; t += PS_THREADS) {
-                const int r = t / half, m = t - r * half;
-                const int ly = lo + r;
-                const int lx = lo + (((ox + lo + oy + ly) & 1) ^ color) + 2 * m;
-                if (lx >= p.ew - lo) continue;
-                const int i = ly * p.ew + lx;
-                const double we = __dadd_rn(sphi[i - 1], sphi[i + 1]);
-                const double sn = __dadd_rn(sphi[i - p.ew], sphi[i + p.ew]);
-                sphi[i] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(we, a.ix2), __dmul_rn(sn, a.iy2)), sb[i]),
-                                    a.inv_denom);
+#pragma unroll
+        for (int k = 0; k < H; ++k) {
+            T* own = sx + ((k & 1) ? plane : 0);
+            const T* oth = sx + ((k & 1) ? 0 : plane);
+            const T* rhs = sb + ((k & 1) ? plane : 0);
+#pragma unroll
+            for (int n = 0; n < NPT; ++n) {
+                const int e = place[k][n];
+                if (e >= 0) {
+                    const int o = e >> 1, w = o - 1 + (e & 1);
+                    const T we = oth[w] + oth[w + 1], sn = oth[o - hw] + oth[o + hw];
+                    own[o] = POW2 ? ps_fma(we + sn, c4, rhs[o]) : (we * p.ix2 + sn * p.iy2 + rhs[o]) * p.inv_denom;
+                }
             }
             __syncthreads();
         }
-        it += PS_HALO / 2;
-        for (int t = threadIdx.x; t < nown; t += PS_THREADS) {
-            const int ly = PS_HALO + t / p.tw, lx = PS_HALO + t % p.tw;
-            a.phi[(size_t)(oy + ly) * a.Nx + (ox + lx)] = sphi[ly * p.ew + lx];
-        }
-        if (!ps_barrier(p.bar, p.err, p.wait_ns)) break;
-        for (int i = threadIdx.x; i < E; i += PS_THREADS) {
-            const int ly = i / p.ew, lx = i - ly * p.ew;
-            if (ly >= PS_HALO && ly < PS_HALO + p.th && lx >= PS_HALO && lx < PS_HALO + p.tw) continue;
-            sphi[i] = a.phi[(size_t)ps_wrap(oy + ly, a.Ny) * a.Nx + ps_wrap(ox + lx, a.Nx)];
+        it += H / 2;
+        unsigned long long* xb = p.xb + (epoch & 1u) * G * (sizeof(T) / 4);
+        ++epoch;
+        if (threadIdx.x == 0) s_ok = 1;
+        for (int i = threadIdx.x; i < nb; i += nthr) ps_publish(xb, edge[i].y, sx[edge[i].x], epoch);
+        __syncthreads();  // the edge cells are read, s_ok is set
+        PsLimit limit;
+        for (int i = threadIdx.x; i < nh; i += nthr) {
+            const uint2 h = list[i];
+            T v;
+            while (!ps_receive(xb, h.y, epoch, v))
+                if (limit.over(p.wait_ns)) {
+                    atomicExch(p.err, 1);
+                    s_ok = 0;
+                    break;
+                }
+            sx[h.x] = v;
+            if (!s_ok) break;
         }
         __syncthreads();
+        if (!s_ok) {
+            failed = true;
+            break;
+        }
+    }
+    if (failed) return;
+    for (int t = threadIdx.x; t < nown; t += nthr) {
+        const int r = ps_div(t, inv_tw), c = t - r * tw;
+        p.x[(size_t)(ys + r) * p.Nx + xs + c] = sx[at(H + c, H + r)];
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         p.out[0] = (double)it;
@@ -347,55 +514,141 @@ __global__ void __launch_bounds__(PS_THREADS) rbgs_persistent(PsArgs p) {
     }
 }
 
+// How the one-launch solve cuts the grid.
+struct RbTiling {
+    int ntx = 0, nty = 0, halo = 0, npt = 0, threads = 0;
+    size_t smem = 0;
+};
+constexpr int PS_MAX_NPT = 8;
+
+// Tile counts and halo for the least estimated time per sweep: the half-sweeps'
+// updates at `op_cycles` per warp (never below `min_cycles`, the latency of one
+// update and its barrier) and one exchange per halo / 2 sweeps. A tile is at
+// least as wide as the halo (or the whole grid), so that only the eight
+// neighbours' cells are needed; `step`: the sweeps between checks are a multiple
+// of it, so halo / 2 must divide it.
+static RbTiling rb_tiling(int Nx, int Ny, int max_blocks, int step, size_t bytes, double op_cycles, double min_cycles) {
+    constexpr double EXCHANGE = 2000.0;
+    RbTiling best;
+    double best_cost = 1e300;
+    for (int H = 4; H <= 8; H += 4) {
+        if (step % (H / 2)) continue;
+        for (int nx = 1; nx <= max_blocks && nx <= Nx; ++nx) {
+            if (nx > 1 && Nx / nx < H) break;
+            for (int ny = 1; ny <= max_blocks / nx && ny <= Ny; ++ny) {
+                if (ny > 1 && Ny / ny < H) break;
+                const int w = (Nx + nx - 1) / nx, h = (Ny + ny - 1) / ny;
+                const size_t ew = w + 2 * H, eh = h + 2 * H;
+                const size_t plane = (ew + 1) / 2 * eh;
+                const size_t inner = (size_t)(w > 2 * H ? w - 2 * H : 0) * (h > 2 * H ? h - 2 * H : 0);
+                const size_t need = 4 * plane * bytes + (ew * eh - inner) * sizeof(uint2);
+                const size_t most = (ew - 1) / 2 * (eh - 2);  // updates of the first half-sweep, at most
+                if (need > PS_MAX_SMEM || ew >= 1024 || most > (size_t)1024 * PS_MAX_NPT) continue;
+                double cost = EXCHANGE;
+                for (int k = 0; k < H; ++k) {
+                    const double upd = 0.5 * (w + 2 * (H - 1 - k)) * (h + 2 * (H - 1 - k));
+                    const double c = (double)(long long)((upd + 31.0) / 32.0) * op_cycles;
+                    cost += c > min_cycles ? c : min_cycles;
+                }
+                cost /= H / 2;
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best.ntx = nx;
+                    best.nty = ny;
+                    best.halo = H;
+                    best.smem = need;
+                    best.npt = 1;
+                    while (most > (size_t)512 * best.npt && best.npt < PS_MAX_NPT) best.npt *= 2;
+                    best.threads = (int)((most + best.npt - 1) / best.npt + 31) / 32 * 32;
+                    if (best.threads < 64) best.threads = 64;
+                }
+            }
+        }
+    }
+    return best;
+}
+
+// Whether 2^k * 2^k = x for the operator's coefficients: equal spacings, powers of two.
+static bool rb_pow2(const RbArgs& a) {
+    return a.ix2 == a.iy2 && exact_reciprocal(a.ix2) != 0.0 && exact_reciprocal(a.denom) != 0.0 && a.ix2 > 1e-30 && a.ix2 < 1e30;
+}
+
+template <typename T, bool POW2, int H>
+static const void* rb_kernel_npt(int npt) {
+    switch (npt) {
+        case 1:
+            return (const void*)rbgs_persistent<T, POW2, H, 1>;
+        case 2:
+            return (const void*)rbgs_persistent<T, POW2, H, 2>;
+        case 4:
+            return (const void*)rbgs_persistent<T, POW2, H, 4>;
+        default:
+            return (const void*)rbgs_persistent<T, POW2, H, 8>;
+    }
+}
+template <typename T>
+static const void* rb_kernel(bool pow2, int halo, int npt) {
+    return pow2 ? (halo == 4 ? rb_kernel_npt<T, true, 4>(npt) : rb_kernel_npt<T, true, 8>(npt))
+                : (halo == 4 ? rb_kernel_npt<T, false, 4>(npt) : rb_kernel_npt<T, false, 8>(npt));
+}
+
+template <typename T>
+static int rb_launch(pic_ctx* c, const RbTiling& t, const PsArgs<T>& p, bool pow2) {
+    const void* k = rb_kernel<T>(pow2, t.halo, t.npt);
+    PIC_TRY(opt_in_dynamic_smem(k, t.smem));
+    // exchange numbers start again from 1
+    PIC_CUDA_TRY(cudaMemsetAsync(p.xb, 0, 2 * c->G * 2 * sizeof(T), c->stream));
+    PsArgs<T> q = p;
+    void* args[] = {&q};
+    PIC_CUDA_TRY(cudaLaunchCooperativeKernel(k, dim3(t.ntx * t.nty), dim3(t.threads), args, t.smem, c->stream));
+    c->launches++;
+    return PIC_OK;
+}
+
+// Device words of the one-launch solves: partial sums, then out[0..3], the
+// barrier and the error flag.
+static int ensure_ps(pic_ctx* c) {
+    int rc = PIC_OK;
+    if (!c->rb_ps) c->rb_ps = (double*)dalloc((4 * PS_MAX_BLOCKS + 8) * sizeof(double), &rc);
+    return rc;
+}
+
+static int sm_count(pic_ctx* c) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    return sms > PS_MAX_BLOCKS ? PS_MAX_BLOCKS : sms;
+}
+
 static int largest_divisor_tile(int n, const int* cand, int ncand) {
     for (int k = 0; k < ncand; ++k)
         if (cand[k] <= n && n % cand[k] == 0) return cand[k];
     return 0;
 }
 
-// Solves in one cooperative launch when the grid tiles evenly and every CTA can
-// be resident; returns PIC_ERR_UNSUPPORTED (nothing queued) otherwise.
+// Solves in one cooperative launch when the tiles fit the SMs' shared memory;
+// returns PIC_ERR_UNSUPPORTED (nothing queued) otherwise.
 // absent_block >= 0 makes that CTA leave before its first barrier, so that every
 // other CTA's wait runs out after wait_ns (the timeout test hook; -1 in solves).
 static int rbgs_solve_persistent(pic_ctx* c, const RbArgs& a, double tol, int max_iters, int check_every, int* it,
                                  double* res, int absent_block = -1, unsigned long long wait_ns = PS_WAIT_NS) {
     if ((check_every & 1) || (max_iters & 1)) return PIC_ERR_UNSUPPORTED;
-    static const int cw[] = {64, 32, 16, 8, 4, 2};
-    static const int ch[] = {32, 16, 8, 4, 2};
-    const int tw = largest_divisor_tile(c->Nx, cw, 6), th = largest_divisor_tile(c->Ny, ch, 5);
-    if (!tw || !th) return PIC_ERR_UNSUPPORTED;
-    const int tiles_x = c->Nx / tw, blocks = tiles_x * (c->Ny / th);
-    const int ew = tw + 2 * PS_HALO, eh = th + 2 * PS_HALO;
-    const size_t smem = (size_t)2 * ew * eh * sizeof(double);
-    if (blocks > PS_MAX_BLOCKS || smem > 200 * 1024) return PIC_ERR_UNSUPPORTED;
-    if (smem > 48 * 1024 && opt_in_dynamic_smem((const void*)rbgs_persistent, smem) != PIC_OK)
-        return PIC_ERR_UNSUPPORTED;
-    int per_sm = 0, sms = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rbgs_persistent, PS_THREADS, smem);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    if (per_sm * sms < blocks) return PIC_ERR_UNSUPPORTED;
+    const bool pow2 = rb_pow2(a);
+    const int step = (check_every % 4 == 0 && max_iters % 4 == 0) ? 4 : 2;
+    const RbTiling t = rb_tiling(c->Nx, c->Ny, sm_count(c), step, sizeof(double), pow2 ? 64.0 : 112.0, 400.0);
+    if (!t.ntx) return PIC_ERR_UNSUPPORTED;
+    PIC_TRY(ensure_ps(c));
     int rc = PIC_OK;
-    if (!c->rb_ps) c->rb_ps = (double*)dalloc((2 * PS_MAX_BLOCKS + 8) * sizeof(double), &rc);
+    if (!c->rb_xb) c->rb_xb = dalloc(2 * c->G * 2 * sizeof(double), &rc);
     if (rc) return rc;
-    double* out = c->rb_ps + 2 * PS_MAX_BLOCKS;
+    double* out = c->rb_ps + 4 * PS_MAX_BLOCKS;
     unsigned* bar = reinterpret_cast<unsigned*>(out + 4);
     int* err = reinterpret_cast<int*>(out + 5);
     PIC_CUDA_TRY(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), c->stream));
     PIC_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), c->stream));
-    PsArgs p{a,   tw,  th,  tiles_x, ew,  eh,           tol,    max_iters,
-             check_every, c->rb_ps, bar, err,     out, absent_block, wait_ns};
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(blocks);
-    lc.blockDim = dim3(PS_THREADS);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = c->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    PIC_CUDA_TRY(cudaLaunchKernelEx(&lc, rbgs_persistent, p));
-    c->launches++;
+    const PsArgs<double> p{c->phi, c->rb_b, static_cast<unsigned long long*>(c->rb_xb), c->Nx, c->Ny, t.ntx, t.nty, a.ix2, a.iy2,
+                           a.inv_denom, a.denom, tol, max_iters, check_every, c->rb_ps, bar, err, out,
+                           absent_block, wait_ns};
+    PIC_TRY(rb_launch<double>(c, t, p, pow2));
     double h[6];
     PIC_CUDA_TRY(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
     PIC_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -410,110 +663,10 @@ static int rbgs_solve_persistent(pic_ctx* c, const RbArgs& a, double tol, int ma
 
 // ---- mixed precision: FP32 sweeps on the correction, FP64 residual --------
 // Iterative refinement: r = b - A phi in FP64; A e = r is relaxed in FP32 by the
-// same red-black sweeps (one cooperative launch, 8-cell halo, 4 sweeps per grid
-// barrier) until ||r - A e|| <= itol ||r||; phi += e in FP64; repeat until the
+// same red-black sweeps (one cooperative launch) until ||r - A e|| <= itol ||r||; phi += e in FP64; repeat until the
 // FP64 relative residual meets tol. The answer meets the same FP64 test as the
 // FP64 solve; sweeps are counted over all corrections.
-constexpr int PF_HALO = 8;
-
 __global__ void rb_residual_field(RbArgs a, const double* __restrict__ phi, double* __restrict__ r);
-
-struct PsArgsF {
-    float* e;        // correction (in/out)
-    const float* r;  // right-hand side of the correction
-    int Nx, Ny;
-    float ix2, iy2, inv_denom, denom;
-    int tw, th, tiles_x, ew, eh;
-    float itol;
-    int max_sweeps, check_every;
-    double* partial;
-    unsigned* bar;
-    int* err;
-    double* out;  // [0] sweeps
-};
-
-__global__ void __launch_bounds__(PS_THREADS) rbgs_persistent_f32(PsArgsF p) {
-    extern __shared__ float pfm[];
-    const int E = p.ew * p.eh;
-    float* se = pfm;
-    float* sr = pfm + E;
-    __shared__ double tot[2];
-    const int tx = blockIdx.x % p.tiles_x, ty = blockIdx.x / p.tiles_x;
-    const int ox = tx * p.tw - PF_HALO, oy = ty * p.th - PF_HALO;
-    for (int i = threadIdx.x; i < E; i += PS_THREADS) {
-        const int ly = i / p.ew, lx = i - ly * p.ew;
-        const size_t g = (size_t)ps_wrap(oy + ly, p.Ny) * p.Nx + ps_wrap(ox + lx, p.Nx);
-        sr[i] = p.r[g];
-        se[i] = p.e[g];
-    }
-    __syncthreads();
-    const int nown = p.tw * p.th;
-    double rr0 = 0.0;
-    for (int t = threadIdx.x; t < nown; t += PS_THREADS) {
-        const int i = (PF_HALO + t / p.tw) * p.ew + PF_HALO + t % p.tw;
-        rr0 += (double)sr[i] * (double)sr[i];
-    }
-    rr0 = rb_block_sum(rr0);
-    if (threadIdx.x == 0) p.partial[2 * blockIdx.x + 1] = rr0;
-    int it = 0;
-    double prev = 1e300;
-    for (;;) {
-        if (it % p.check_every == 0 || it >= p.max_sweeps) {
-            double rr = 0.0;
-            for (int t = threadIdx.x; t < nown; t += PS_THREADS) {
-                const int i = (PF_HALO + t / p.tw) * p.ew + PF_HALO + t % p.tw;
-                const float ae = p.denom * se[i] - p.ix2 * (se[i - 1] + se[i + 1]) - p.iy2 * (se[i - p.ew] + se[i + p.ew]);
-                const double q = (double)(sr[i] - ae);
-                rr += q * q;
-            }
-            rr = rb_block_sum(rr);
-            if (threadIdx.x == 0) p.partial[2 * blockIdx.x] = rr;
-            if (!ps_barrier(p.bar, p.err)) break;
-            if (threadIdx.x == 0) {
-                double s1 = 0.0, s2 = 0.0;
-                for (unsigned k = 0; k < gridDim.x; ++k) {
-                    s1 += p.partial[2 * k];
-                    s2 += p.partial[2 * k + 1];
-                }
-                tot[0] = s1;
-                tot[1] = s2;
-            }
-            __syncthreads();
-            const double res = tot[1] > 0.0 ? sqrt(tot[0] / tot[1]) : 0.0;
-            // stop at the tolerance, the sweep limit, or when FP32 rounding stalls the residual
-            if (res <= (double)p.itol || it >= p.max_sweeps || res > 0.999 * prev) break;
-            prev = res;
-        }
-        for (int k = 0; k < PF_HALO; ++k) {
-            const int color = k & 1;
-            const int lo = k + 1;
-            const int rows = p.eh - 2 * lo, cols = p.ew - 2 * lo;
-            const int half = (cols + 1) >> 1;
-            for (int t = threadIdx.x; t < rows * half; t += PS_THREADS) {
-                const int rw = t / half, m = t - rw * half;
-                const int ly = lo + rw;
-                const int lx = lo + (((ox + lo + oy + ly) & 1) ^ color) + 2 * m;
-                if (lx >= p.ew - lo) continue;
-                const int i = ly * p.ew + lx;
-                se[i] = ((se[i - 1] + se[i + 1]) * p.ix2 + (se[i - p.ew] + se[i + p.ew]) * p.iy2 + sr[i]) * p.inv_denom;
-            }
-            __syncthreads();
-        }
-        it += PF_HALO / 2;
-        for (int t = threadIdx.x; t < nown; t += PS_THREADS) {
-            const int ly = PF_HALO + t / p.tw, lx = PF_HALO + t % p.tw;
-            p.e[(size_t)(oy + ly) * p.Nx + (ox + lx)] = se[ly * p.ew + lx];
-        }
-        if (!ps_barrier(p.bar, p.err)) break;
-        for (int i = threadIdx.x; i < E; i += PS_THREADS) {
-            const int ly = i / p.ew, lx = i - ly * p.ew;
-            if (ly >= PF_HALO && ly < PF_HALO + p.th && lx >= PF_HALO && lx < PF_HALO + p.tw) continue;
-            se[i] = p.e[(size_t)ps_wrap(oy + ly, p.Ny) * p.Nx + ps_wrap(ox + lx, p.Nx)];
-        }
-        __syncthreads();
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) p.out[0] = (double)it;
-}
 
 __global__ void rb_to_f32(const double* __restrict__ r, size_t n, float* __restrict__ r32, float* __restrict__ e) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -532,27 +685,29 @@ __global__ void rb_add_correction(double* __restrict__ phi, const float* __restr
 // grid does not tile evenly or the tiles cannot all be resident.
 static int rbgs_solve_mixed(pic_ctx* c, const RbArgs& a, double tol, int max_iters, int check_every, int* it_out,
                             double* res_out) {
+    // Which grids refine in FP32 is part of the results (the two modes agree to the
+    // tolerance, not bit for bit): those that divide into 64 x 32 or smaller
+    // power-of-two tiles, few enough of them, as pic_gpu_set_rbgs_precision states.
     static const int cw[] = {64, 32, 16, 8, 4, 2};
     static const int ch[] = {32, 16, 8, 4, 2};
-    const int tw = largest_divisor_tile(c->Nx, cw, 6), th = largest_divisor_tile(c->Ny, ch, 5);
-    if (!tw || !th) return PIC_ERR_UNSUPPORTED;
-    const int tiles_x = c->Nx / tw, blocks = tiles_x * (c->Ny / th);
-    const int ew = tw + 2 * PF_HALO, eh = th + 2 * PF_HALO;
-    const size_t smem = (size_t)2 * ew * eh * sizeof(float);
-    if (blocks > PS_MAX_BLOCKS || smem > 48 * 1024) return PIC_ERR_UNSUPPORTED;
-    int per_sm = 0, sms = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rbgs_persistent_f32, PS_THREADS, smem);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    if (per_sm * sms < blocks) return PIC_ERR_UNSUPPORTED;
+    const int dw = largest_divisor_tile(c->Nx, cw, 6), dh = largest_divisor_tile(c->Ny, ch, 5);
+    if (!dw || !dh) return PIC_ERR_UNSUPPORTED;
+    const long long blocks = (long long)(c->Nx / dw) * (c->Ny / dh);
+    if (blocks > PS_MAX_BLOCKS || blocks > (long long)(dw * dh == 2048 ? 7 : 8) * sm_count(c)) return PIC_ERR_UNSUPPORTED;
+    const bool pow2 = rb_pow2(a);
+    const RbTiling t = rb_tiling(c->Nx, c->Ny, sm_count(c), 4, sizeof(float), 14.0, 200.0);
+    if (!t.ntx) return PIC_ERR_UNSUPPORTED;
+    PIC_TRY(ensure_ps(c));
     int rc = PIC_OK;
-    if (!c->rb_ps) c->rb_ps = (double*)dalloc((2 * PS_MAX_BLOCKS + 8) * sizeof(double), &rc);
-    if (rc) return rc;
     if (!c->rb_mix) c->rb_mix = (double*)dalloc(c->G * (8 + 4 + 4), &rc);
+    if (rc) return rc;
+    if (!c->rb_xb) c->rb_xb = dalloc(2 * c->G * 2 * sizeof(double), &rc);
     if (rc) return rc;
     double* r64 = c->rb_mix;
     float* r32 = reinterpret_cast<float*>(r64 + c->G);
     float* e32 = r32 + c->G;
-    double* out = c->rb_ps + 2 * PS_MAX_BLOCKS;
+    unsigned long long* xb32 = static_cast<unsigned long long*>(c->rb_xb);
+    double* out = c->rb_ps + 4 * PS_MAX_BLOCKS;
     unsigned* bar = reinterpret_cast<unsigned*>(out + 4);
     int* err = reinterpret_cast<int*>(out + 5);
     PIC_CUDA_TRY(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), c->stream));
@@ -594,20 +749,11 @@ static int rbgs_solve_mixed(pic_ctx* c, const RbArgs& a, double tol, int max_ite
             if (prc != PIC_ERR_UNSUPPORTED) return prc;
         }
         prev_res = res;
-        PsArgsF p{e32, r32, c->Nx, c->Ny, (float)a.ix2, (float)a.iy2, (float)a.inv_denom, (float)a.denom,
-                  tw, th, tiles_x, ew, eh, (float)itol, max_iters - it, ce, c->rb_ps, bar, err, out};
-        cudaLaunchConfig_t lc{};
-        lc.gridDim = dim3(blocks);
-        lc.blockDim = dim3(PS_THREADS);
-        lc.dynamicSmemBytes = smem;
-        lc.stream = c->stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-        lc.attrs = at;
-        lc.numAttrs = 1;
-        PIC_CUDA_TRY(cudaLaunchKernelEx(&lc, rbgs_persistent_f32, p));
-        c->launches += 3;
+        // sweeps come in fours, as the check interval does
+        const PsArgs<float> p{e32, r32, xb32, c->Nx, c->Ny, t.ntx, t.nty, (float)a.ix2, (float)a.iy2,
+                              (float)a.inv_denom, (float)a.denom, (double)(float)itol, (max_iters - it + 3) & ~3, ce,
+                              c->rb_ps, bar, err, out, -1, PS_WAIT_NS};
+        PIC_TRY(rb_launch<float>(c, t, p, pow2));
         rb_add_correction<<<gb, 256, 0, c->stream>>>(c->phi, e32, c->G);
         PIC_TRY(check_launch(c, "rb_add_correction"));
         double h[6];
@@ -705,6 +851,7 @@ int rbgs_solve_async(pic_ctx* c, double tol, int max_iters, int check_every) {
 
 void release_rbgs(pic_ctx* c) {
     dfree(c->rb_mix);
+    dfree(c->rb_xb);
     dfree(c->rb_ps);
     dfree(c->rb_b);
     dfree(c->rb_partial);

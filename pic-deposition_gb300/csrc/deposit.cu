@@ -1475,17 +1475,46 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
     }
 }
 
-// One unit of the int64 grid (FP64): max|q| * inv_vol * 2^-24, or, for the
-// exact integer TSC form, max|q| * inv_vol * (qn * 2^-30) (scale != 0).
-__global__ void fixed_unit(double inv_vol, double scale, const DevStats* st, double* unit_out) {
-    *unit_out = scale == 0.0 ? charge_unit(st, inv_vol) : __dmul_rn(__dmul_rn((double)load_maxq(st), inv_vol), scale);
+// After a deposit between sorts whose kernel was chosen on the device: once the
+// cell kernel has found more than `limit` particles outside their sorted cell,
+// the any-order kernel takes the following deposits (it is faster when most
+// particles have moved: every mover is a separate frame of atomics in the cell
+// kernel) until the next sort clears the flag. A deposit made in any order
+// counts every particle as moved, so a sort triggered by the moved fraction
+// still follows.
+__device__ void choose_any_order(DevStats* st, unsigned long long limit, unsigned long long n) {
+    if (st->any_order)
+        st->moved += n;
+    else if (st->moved_dep > limit)
+        st->any_order = 1u;
+    st->moved_dep = 0;
 }
 
-__global__ void fixed_to_rho(const long long* __restrict__ acc, size_t g, double background,
-                             const double* __restrict__ unitp, double* __restrict__ rho) {
-    const double unit = *unitp;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < g) rho[i] = __dadd_rn(__dmul_rn((double)acc[i], unit), background);
+// The int64 grid as FP64 rho, four cells per thread. One unit (FP64) is max|q| *
+// inv_vol * 2^-24, or, for the exact integer TSC form, max|q| * inv_vol * (qn *
+// 2^-30) (scale != 0); each thread forms it, and the first also stores it and,
+// with n > 0, takes the any-order decision of a deposit between sorts: two
+// launches fewer per deposit.
+__global__ void fixed_to_rho(const long long* __restrict__ acc, size_t g, double background, double inv_vol,
+                             double scale, DevStats* st, double* __restrict__ unit_out, double* __restrict__ rho,
+                             unsigned long long limit, unsigned long long n) {
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const double unit = scale == 0.0 ? charge_unit(st, inv_vol)
+                                     : __dmul_rn(__dmul_rn((double)load_maxq(st), inv_vol), scale);
+    if (i == 0) {
+        *unit_out = unit;
+        if (n) choose_any_order(st, limit, n);
+    }
+    if (i + 3 < g) {  // 32-byte aligned: the grids start on 256 bytes
+        const longlong2 a = *reinterpret_cast<const longlong2*>(acc + i);
+        const longlong2 b = *reinterpret_cast<const longlong2*>(acc + i + 2);
+        *reinterpret_cast<double2*>(rho + i) = make_double2(__dadd_rn(__dmul_rn((double)a.x, unit), background),
+                                                            __dadd_rn(__dmul_rn((double)a.y, unit), background));
+        *reinterpret_cast<double2*>(rho + i + 2) = make_double2(__dadd_rn(__dmul_rn((double)b.x, unit), background),
+                                                                __dadd_rn(__dmul_rn((double)b.y, unit), background));
+    } else {
+        for (size_t k = i; k < g; ++k) rho[k] = __dadd_rn(__dmul_rn((double)acc[k], unit), background);
+    }
 }
 
 #ifndef CELLS_LPP
@@ -1507,21 +1536,6 @@ static int launch_cells(pic_ctx* c, const DepArgs& a, unsigned tiles) {
     if (rc != PIC_OK) return rc;
     deposit_cells<S, LPP, NW, MINB, QC, KEYS, NBUF><<<tiles, NW * 32, smem, c->stream>>>(a);
     return PIC_OK;
-}
-
-// After a deposit between sorts whose kernel was chosen on the device: once the
-// cell kernel has found more than `limit` particles outside their sorted cell,
-// the any-order kernel takes the following deposits (it is faster when most
-// particles have moved: every mover is a separate frame of atomics in the cell
-// kernel) until the next sort clears the flag. A deposit made in any order
-// counts every particle as moved, so a sort triggered by the moved fraction
-// still follows.
-__global__ void choose_any_order(DevStats* st, unsigned long long limit, unsigned long long n) {
-    if (st->any_order)
-        st->moved += n;
-    else if (st->moved_dep > limit)
-        st->any_order = 1u;
-    st->moved_dep = 0;
 }
 
 // The fraction of the particles above which deposits between sorts switch to
@@ -1562,13 +1576,7 @@ static int launch_deposit(pic_ctx* c, const DepArgs& a, int kind, bool adaptive)
         int rc = a.qc != 0.0f ? launch_cells<S, CELLS_LPP, 4, 4, true, true>(c, ak, tiles)
                               : launch_cells<S, CELLS_LPP, 4, 4, false, true>(c, ak, tiles);
         if (rc == PIC_OK) rc = check_launch(c, "deposit_cells");
-        if (rc == PIC_OK) rc = launch_runs<S>(c, ar);
-        if (rc == PIC_OK) {
-            choose_any_order<<<1, 1, 0, c->stream>>>(c->dstats,
-                                                     (unsigned long long)(ANY_ORDER_FRACTION * (double)a.n),
-                                                     (unsigned long long)a.n);
-            rc = check_launch(c, "choose_any_order");
-        }
+        if (rc == PIC_OK) rc = launch_runs<S>(c, ar);  // fixed_to_rho takes the decision for the next deposit
         prof_end(c);
         return rc;
     }
@@ -1645,13 +1653,16 @@ int deposit_rho(pic_ctx* c, int scheme, double dt, double background) {
     a.dtdx = (float)(dt / c->dx);
     a.dtdy = (float)(dt / c->dy);
     if (!c->tile_user) {
-        // rows of 32 cells (one per lane) and about 8K particles per tile, at
-        // least as many rows as the 4 warps of a CTA
+        // rows of 32 cells and about 8K particles per tile; a grid too small to
+        // give every SM two such tiles takes lower ones (64^2: 8 tiles of 32 rows
+        // kept 8 SMs busy)
         const double ppc = (double)c->n / (double)c->G;
         const double cells = ppc > 0.0 ? 8192.0 / ppc : 2048.0;
         c->tile_w = 32;
         int h = 4;
         while (h < 32 && (double)(c->tile_w * h * 2) <= cells) h *= 2;
+        const long long cols = (c->Nx + c->tile_w - 1) / c->tile_w;
+        while (h > 1 && cols * ((c->Ny + h - 1) / h) < 300) h /= 2;
         c->tile_h = h;
     }
     a.tile_w = c->tile_w;
@@ -1683,11 +1694,12 @@ int deposit_rho(pic_ctx* c, int scheme, double dt, double background) {
     const double scale = (scheme == PIC_SCHEME_TSC && c->n > 0 && c->qn_uniform != 0.0f)
                              ? (double)c->qn_uniform * 0x1p-30
                              : 0.0;
-    fixed_unit<<<1, 1, 0, c->stream>>>(inv_vol, scale, c->dstats, c->unitbuf);
-    PIC_TRY(check_launch(c, "fixed_unit"));
-    fixed_to_rho<<<(unsigned)((c->G + 255) / 256), 256, 0, c->stream>>>(c->acc, c->G, background, c->unitbuf,
-                                                                         c->rho);
+    const bool decide = c->n > 0 && tiled == 0 && adaptive && !c->sorted;
+    fixed_to_rho<<<(unsigned)((c->G + 1023) / 1024), 256, 0, c->stream>>>(
+        c->acc, c->G, background, inv_vol, scale, c->dstats, c->unitbuf, c->rho,
+        (unsigned long long)(ANY_ORDER_FRACTION * (double)c->n), decide ? (unsigned long long)c->n : 0ull);
     PIC_TRY(check_launch(c, "fixed_to_rho"));
+    c->grid_sums_ready = 0;
     c->last_scheme = scheme;
     return PIC_OK;
 }

@@ -41,8 +41,6 @@ __device__ __forceinline__ double block_sum(double v) {
 
 // Per-item quantities summed by the diagnostics.
 enum SumKind : int {
-    SUM_GRID = 0,      // sum x[i]
-    SUM_GRID_SQ2 = 1,  // sum x[i]^2 + y[i]^2
     SUM_Q = 2,         // sum qn[i]*maxq
     SUM_ABS_Q = 3,     // sum |qn[i]*maxq|
     SUM_KE = 4,        // sum 0.5*m*(vx^2+vy^2)
@@ -50,8 +48,6 @@ enum SumKind : int {
 
 struct SumArgs {
     int kind;
-    const double* x;
-    const double* y;
     const float* q;
     const float* vx;
     const float* vy;
@@ -62,10 +58,6 @@ struct SumArgs {
 
 __device__ __forceinline__ double sum_item(const SumArgs& a, size_t i) {
     switch (a.kind) {
-        case SUM_GRID:
-            return a.x[i];
-        case SUM_GRID_SQ2:
-            return __dadd_rn(__dmul_rn(a.x[i], a.x[i]), __dmul_rn(a.y[i], a.y[i]));
         case SUM_Q:
             return (double)(a.q[i] * load_maxq(a.st));
         case SUM_ABS_Q:
@@ -126,58 +118,146 @@ int device_sum(pic_ctx* c, const SumArgs& a, double* out, double scale) {
 }
 int device_sum(pic_ctx* c, const SumArgs& a, double* out) { return device_sum(c, a, out, 1.0); }
 
-__global__ void copy_charge_sums(double* r) {
+// The last stage of the diagnostics in one block: up to three partial sums
+// (kinetic, rho, E^2; rho and E^2 interleaved), the particle set's charge sums,
+// and, with a history, the step's pic_diag from them (the formulas of
+// read_diagnostics) and the step counter.
+struct FinalArgs {
+    const double* ke;    // null: r[3] already holds the kinetic energy
+    const double* grid;  // pairs (sum rho, sum E^2)
+    int ke_count, grid_count;
+    double* r;           // red_out
+    double vol;
+    double* hist;
+    int* step;
+    int steps;
+};
+
+__global__ void __launch_bounds__(RED_THREADS) diag_final(FinalArgs a) {
+    double ke = 0.0, rho = 0.0, ee = 0.0;
+    if (a.ke)
+        for (int i = threadIdx.x; i < a.ke_count; i += RED_THREADS) ke = __dadd_rn(ke, a.ke[i]);
+    for (int i = threadIdx.x; i < a.grid_count; i += RED_THREADS) {
+        const double2 g = reinterpret_cast<const double2*>(a.grid)[i];
+        rho = __dadd_rn(rho, g.x);
+        ee = __dadd_rn(ee, g.y);
+    }
+    ke = block_sum(ke);
+    rho = block_sum(rho);
+    ee = block_sum(ee);
+    if (threadIdx.x != 0) return;
+    double* r = a.r;
     r[1] = r[8];
     r[6] = r[9];
+    r[2] = rho;
+    if (a.ke) r[3] = __dmul_rn(0.5, ke);
+    r[4] = ee;
+    if (!a.hist) return;
+    const int s = *a.step;
+    if (s < a.steps) {
+        double* d = a.hist + (size_t)s * 6;
+        const double total_charge = r[1];
+        const double integrated = __dmul_rn(rho, a.vol);
+        const double den = r[6] > 1e-12 ? r[6] : 1e-12;
+        const double kin = r[3];
+        const double fe = __dmul_rn(__dmul_rn(0.5, ee), a.vol);
+        d[0] = __ddiv_rn(fabs(__dsub_rn(integrated, total_charge)), den);
+        d[1] = total_charge;
+        d[2] = integrated;
+        d[3] = kin;
+        d[4] = fe;
+        d[5] = __dadd_rn(kin, fe);
+    }
+    *a.step = s + 1;
+}
+
+// partial[block] = (sum of rho, sum of Ex^2 + Ey^2) over a fixed chunk
+__global__ void __launch_bounds__(RED_THREADS) grid_sum_partials(const double* __restrict__ rho,
+                                                                const double* __restrict__ Ex,
+                                                                const double* __restrict__ Ey, size_t g,
+                                                                double* __restrict__ partial) {
+    const size_t chunk = (g + RED_BLOCKS - 1) / RED_BLOCKS;
+    const size_t b = (size_t)blockIdx.x * chunk;
+    const size_t e = b + chunk < g ? b + chunk : g;
+    double s = 0.0, ee = 0.0;
+    for (size_t i = b + threadIdx.x; i < e; i += RED_THREADS) {
+        s = __dadd_rn(s, rho[i]);
+        ee = __dadd_rn(ee, __dadd_rn(__dmul_rn(Ex[i], Ex[i]), __dmul_rn(Ey[i], Ey[i])));
+    }
+    s = block_sum(s);
+    ee = block_sum(ee);
+    if (threadIdx.x == 0) reinterpret_cast<double2*>(partial)[blockIdx.x] = make_double2(s, ee);
 }
 
 // ---- Poisson ---------------------------------------------------------------
-__global__ void rhs_from_rho(const double* __restrict__ rho, double vol, size_t g, double* __restrict__ rhs) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < g) rhs[i] = __dmul_rn(rho[i], vol);  // poisson_fft.cpp:51-55
-}
-
-// spectrum /= k^2 (continuous k, poisson_fft.cpp:23-35), DC = 0 (poisson_fft.cpp:59-62)
-__global__ void k_divide(cufftDoubleComplex* __restrict__ spec, int Nx, int Ny, double Lx, double Ly) {
+// The factor of each frequency, once per context: vol / (k^2 * Nx * Ny) with the
+// continuous k (poisson_fft.cpp:23-35), DC = 0 (poisson_fft.cpp:59-62). It carries
+// the right-hand side's cell volume (poisson_fft.cpp:51-55) and the inverse
+// transform's 1/(Nx*Ny) (poisson_fft.cpp:66-75), so a solve needs no pass of its
+// own for either, and no FP64 division (slow on this part) per element.
+__global__ void make_fft_scale(double* __restrict__ scale, int Nx, int Ny, double Lx, double Ly, double num) {
     const int nh = Nx / 2 + 1;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (size_t)nh * Ny) return;
     const int i = (int)(t % nh), j = (int)(t / nh);
-    if (i == 0 && j == 0) {
-        spec[t].x = 0.0;
-        spec[t].y = 0.0;
-        return;
-    }
     const double twopi = 2.0 * 3.14159265358979323846;
     const int mx = (i <= Nx / 2) ? i : i - Nx;
     const int my = (j <= Ny / 2) ? j : j - Ny;
     const double kx = __ddiv_rn(__dmul_rn(twopi, (double)mx), Lx);
     const double ky = __ddiv_rn(__dmul_rn(twopi, (double)my), Ly);
     const double k2 = __dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky));
-    spec[t].x = __ddiv_rn(spec[t].x, k2);
-    spec[t].y = __ddiv_rn(spec[t].y, k2);
+    scale[t] = t == 0 ? 0.0 : __ddiv_rn(num, k2);
+}
+
+__global__ void k_scale(cufftDoubleComplex* __restrict__ spec, const double* __restrict__ scale, size_t n) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const double f = scale[t];
+    cufftDoubleComplex v = spec[t];
+    v.x = __dmul_rn(v.x, f);
+    v.y = __dmul_rn(v.y, f);
+    spec[t] = v;
 }
 
 __global__ void scale_phi(double* __restrict__ phi, size_t g, double norm) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < g) phi[i] = __dmul_rn(phi[i], norm);  // poisson_fft.cpp:66-75
+    if (i < g) phi[i] = __dmul_rn(phi[i], norm);
 }
 
-// E = -(phi[i+1] - phi[i]) / d (poisson_fft.cpp:77-93, poisson_gs.cpp:48-60); FP32 copies for gather.
-__global__ void efield(const double* __restrict__ phi, int Nx, int Ny, double idx_dx, double idx_dy,
-                       double* __restrict__ Ex, double* __restrict__ Ey, float* __restrict__ Exf,
-                       float* __restrict__ Eyf) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (size_t)Nx * Ny) return;
-    const int i = (int)(t % Nx), j = (int)(t / Nx);
-    const int ip = (i + 1) % Nx, jp = (j + 1) % Ny;
-    const double p = phi[t];
-    const double ex = -__dmul_rn(__dsub_rn(phi[(size_t)j * Nx + ip], p), idx_dx);
-    const double ey = -__dmul_rn(__dsub_rn(phi[(size_t)jp * Nx + i], p), idx_dy);
-    Ex[t] = ex;
-    Ey[t] = ey;
-    Exf[t] = __double2float_rn(ex);
-    Eyf[t] = __double2float_rn(ey);
+// E = -(phi[i+1] - phi[i]) / d (poisson_fft.cpp:77-93, poisson_gs.cpp:48-60); FP32
+// copies for the gather; and the block's sums of rho and E^2, which the step's
+// diagnostics need: no passes over rho and E of their own. A block covers FE_ITEMS
+// rounds of 256 cells.
+constexpr int FE_ITEMS = 4;
+constexpr size_t FE_BLOCK = (size_t)RED_THREADS * FE_ITEMS;
+
+__global__ void __launch_bounds__(RED_THREADS) efield(const double* __restrict__ phi, const double* __restrict__ rho,
+                                                      int Nx, int Ny, double idx_dx, double idx_dy,
+                                                      double* __restrict__ Ex, double* __restrict__ Ey,
+                                                      float* __restrict__ Exf, float* __restrict__ Eyf,
+                                                      double* __restrict__ partial) {
+    const size_t g = (size_t)Nx * Ny;
+    double s = 0.0, ee = 0.0;
+#pragma unroll
+    for (int k = 0; k < FE_ITEMS; ++k) {
+        const size_t t = (size_t)blockIdx.x * FE_BLOCK + k * RED_THREADS + threadIdx.x;
+        if (t < g) {
+            const unsigned j = (unsigned)t / (unsigned)Nx, i = (unsigned)t - j * (unsigned)Nx;  // at most 2^30 cells
+            const double p = phi[t];
+            const size_t xp = i + 1 == (unsigned)Nx ? t - i : t + 1, yp = j + 1 == (unsigned)Ny ? i : t + Nx;
+            const double ex = -__dmul_rn(__dsub_rn(phi[xp], p), idx_dx);
+            const double ey = -__dmul_rn(__dsub_rn(phi[yp], p), idx_dy);
+            Ex[t] = ex;
+            Ey[t] = ey;
+            Exf[t] = __double2float_rn(ex);
+            Eyf[t] = __double2float_rn(ey);
+            s = __dadd_rn(s, rho[t]);
+            ee = __dadd_rn(ee, __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
+        }
+    }
+    s = block_sum(s);
+    ee = block_sum(ee);
+    if (threadIdx.x == 0) reinterpret_cast<double2*>(partial)[blockIdx.x] = make_double2(s, ee);
 }
 
 __global__ void fields_to_f32(const double* __restrict__ Ex, const double* __restrict__ Ey, size_t g,
@@ -232,6 +312,9 @@ int ensure_fields(pic_ctx* c) {
     if (rc) return rc;
     if (!c->red_out) c->red_out = (double*)dalloc(16 * 8, &rc);
     if (rc) return rc;
+    const size_t pairs = (g + FE_BLOCK - 1) / FE_BLOCK;
+    if (!c->grid_partials) c->grid_partials = (double*)dalloc((pairs > RED_BLOCKS ? pairs : RED_BLOCKS) * 16, &rc);
+    if (rc) return rc;
     if (!c->fields_init) {
         PIC_CUDA_TRY(cudaMemsetAsync(c->phi, 0, g * 8, c->stream));
         PIC_CUDA_TRY(cudaMemsetAsync(c->Ex, 0, g * 8, c->stream));
@@ -257,6 +340,11 @@ static int ensure_fft(pic_ctx* c) {
     PIC_CUFFT_TRY(cufftPlan2d(&b, c->Ny, c->Nx, CUFFT_Z2D));
     PIC_CUFFT_TRY(cufftSetStream(f, c->stream));
     PIC_CUFFT_TRY(cufftSetStream(b, c->stream));
+    c->fft_scale = (double*)dalloc(nh * (size_t)c->Ny * 8, &rc);
+    if (rc) return rc;
+    make_fft_scale<<<(unsigned)((nh * c->Ny + 255) / 256), 256, 0, c->stream>>>(
+        c->fft_scale, c->Nx, c->Ny, c->Lx, c->Ly, c->dx * c->dy / (double)c->G);
+    PIC_TRY(check_launch(c, "make_fft_scale"));
     c->fft_fwd = (int)f;
     c->fft_inv = (int)b;
     c->fft_ready = 1;
@@ -270,32 +358,31 @@ void release_fields(pic_ctx* c) {
         c->fft_ready = 0;
     }
     void* ptrs[] = {c->phi, c->Ex, c->Ey, c->Exf, c->Eyf, c->spec, c->fft_rhs, c->red_partials, c->red_out,
-                    c->ke_partials};
+                    c->ke_partials, c->grid_partials, c->fft_scale};
     for (void* p : ptrs) dfree(p);
 }
 
 int efield_from_phi(pic_ctx* c) {
-    const unsigned blocks = (unsigned)((c->G + 255) / 256);
-    efield<<<blocks, 256, 0, c->stream>>>(c->phi, c->Nx, c->Ny, 1.0 / c->dx, 1.0 / c->dy, c->Ex, c->Ey, c->Exf,
-                                          c->Eyf);
-    return check_launch(c, "efield");
+    const unsigned blocks = (unsigned)((c->G + FE_BLOCK - 1) / FE_BLOCK);
+    efield<<<blocks, RED_THREADS, 0, c->stream>>>(c->phi, c->rho, c->Nx, c->Ny, 1.0 / c->dx, 1.0 / c->dy, c->Ex,
+                                                  c->Ey, c->Exf, c->Eyf, c->grid_partials);
+    PIC_TRY(check_launch(c, "efield"));
+    c->grid_sums_ready = 1;
+    return PIC_OK;
 }
 
+// Four FFT launches and two of this library's: the forward transform reads rho
+// itself (an out-of-place real transform leaves its input), k_scale applies the
+// frequency factors, the inverse writes phi, efield follows.
 int poisson_fft(pic_ctx* c) {
     PIC_TRY(ensure_fft(c));
-    const unsigned blocks = (unsigned)((c->G + 255) / 256);
-    rhs_from_rho<<<blocks, 256, 0, c->stream>>>(c->rho, c->dx * c->dy, c->G, c->fft_rhs);
-    PIC_TRY(check_launch(c, "rhs_from_rho"));
     prof_begin(c, "poisson_fft");
-    PIC_CUFFT_TRY(cufftExecD2Z((cufftHandle)c->fft_fwd, c->fft_rhs, (cufftDoubleComplex*)c->spec));
+    PIC_CUFFT_TRY(cufftExecD2Z((cufftHandle)c->fft_fwd, c->rho, (cufftDoubleComplex*)c->spec));
     const size_t ns = (size_t)(c->Nx / 2 + 1) * c->Ny;
-    k_divide<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>((cufftDoubleComplex*)c->spec, c->Nx, c->Ny, c->Lx,
-                                                                   c->Ly);
-    PIC_TRY(check_launch(c, "k_divide"));
+    k_scale<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>((cufftDoubleComplex*)c->spec, c->fft_scale, ns);
+    PIC_TRY(check_launch(c, "k_scale"));
     PIC_CUFFT_TRY(cufftExecZ2D((cufftHandle)c->fft_inv, (cufftDoubleComplex*)c->spec, c->phi));
     prof_end(c);
-    scale_phi<<<blocks, 256, 0, c->stream>>>(c->phi, c->G, 1.0 / (double)c->G);
-    PIC_TRY(check_launch(c, "scale_phi"));
     return efield_from_phi(c);
 }
 
@@ -334,8 +421,9 @@ int solve_discrete_fft(pic_ctx* c, const double* b, double* phi) {
     return check_launch(c, "scale_phi");
 }
 
-// Queues the six diagnostics into c->red_out[0..5] (pic_diag order).
-int diagnostics_async(pic_ctx* c) {
+// Queues the six diagnostics into c->red_out[0..5] (pic_diag order); the last
+// kernel also records them in a time step's history.
+int diagnostics_async(pic_ctx* c, double* hist, int* step, int steps) {
     PIC_TRY(ensure_fields(c));
     SumArgs a{};
     a.st = c->dstats;
@@ -351,8 +439,12 @@ int diagnostics_async(pic_ctx* c) {
         PIC_TRY(device_sum(c, a, c->red_out + 9));
         c->qsum_valid = 1;
     }
-    copy_charge_sums<<<1, 1, 0, c->stream>>>(c->red_out);  // total_charge, sum |q|
-    PIC_TRY(check_launch(c, "copy_charge_sums"));
+    FinalArgs f{};
+    f.r = c->red_out;
+    f.vol = c->dx * c->dy;
+    f.hist = hist;
+    f.step = step;
+    f.steps = steps;
     // kinetic: sum 0.5*m*v^2 in FP64 per particle when masses differ from 1;
     // with unit masses 0.5 * sum v^2 (double-FP32 per thread, FP64 across threads)
     if (a.m) {
@@ -360,25 +452,26 @@ int diagnostics_async(pic_ctx* c) {
         PIC_TRY(device_sum(c, a, c->red_out + 3));
     } else if (c->n > 0 && c->ke_ready) {  // left by the gather that produced these velocities
         c->ke_ready = 0;                     // used once: the next diagnostics recompute unless a gather refills it
-        sum_final<<<1, RED_THREADS, 0, c->stream>>>(c->ke_partials, 0.5, c->red_out + 3, c->ke_count);
-        PIC_TRY(check_launch(c, "sum_final"));
+        f.ke = c->ke_partials;
+        f.ke_count = c->ke_count;
     } else if (c->n > 0) {
         sum_v2_partials<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(c->vx, c->vy, c->n, c->red_partials);
         PIC_TRY(check_launch(c, "sum_v2_partials"));
-        sum_final<<<1, RED_THREADS, 0, c->stream>>>(c->red_partials, 0.5, c->red_out + 3);
-        PIC_TRY(check_launch(c, "sum_final"));
+        f.ke = c->red_partials;
+        f.ke_count = RED_BLOCKS;
     } else {
         PIC_CUDA_TRY(cudaMemsetAsync(c->red_out + 3, 0, sizeof(double), c->stream));
     }
-    SumArgs g{};
-    g.n = c->G;
-    g.kind = SUM_GRID;
-    g.x = c->rho;
-    PIC_TRY(device_sum(c, g, c->red_out + 2));  // sum rho
-    g.kind = SUM_GRID_SQ2;
-    g.x = c->Ex;
-    g.y = c->Ey;
-    return device_sum(c, g, c->red_out + 4);  // sum Ex^2+Ey^2
+    f.grid = c->grid_partials;
+    if (c->grid_sums_ready) {  // left by the solve that produced this E from this rho
+        f.grid_count = (int)((c->G + FE_BLOCK - 1) / FE_BLOCK);
+    } else {
+        grid_sum_partials<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(c->rho, c->Ex, c->Ey, c->G, c->grid_partials);
+        PIC_TRY(check_launch(c, "grid_sum_partials"));
+        f.grid_count = RED_BLOCKS;
+    }
+    diag_final<<<1, RED_THREADS, 0, c->stream>>>(f);
+    return check_launch(c, "diag_final");
 }
 
 int read_diagnostics(pic_ctx* c, pic_diag* d) {
@@ -406,6 +499,7 @@ int pic_gpu_set_rho(pic_ctx* c, const double* rho) {
     if (!c || !rho) return fail(PIC_ERR_ARG, "NULL argument");
     PIC_CUDA_TRY(cudaSetDevice(c->device));
     PIC_CUDA_TRY(cudaMemcpyAsync(c->rho, rho, c->G * 8, cudaMemcpyHostToDevice, c->stream));
+    c->grid_sums_ready = 0;
     return pic_gpu_synchronize(c);
 }
 
@@ -413,6 +507,7 @@ int pic_gpu_set_fields(pic_ctx* c, const double* phi, const double* Ex, const do
     if (!c) return fail(PIC_ERR_ARG, "NULL context");
     PIC_CUDA_TRY(cudaSetDevice(c->device));
     PIC_TRY(ensure_fields(c));
+    c->grid_sums_ready = 0;
     if (phi) PIC_CUDA_TRY(cudaMemcpyAsync(c->phi, phi, c->G * 8, cudaMemcpyHostToDevice, c->stream));
     if (Ex) PIC_CUDA_TRY(cudaMemcpyAsync(c->Ex, Ex, c->G * 8, cudaMemcpyHostToDevice, c->stream));
     if (Ey) PIC_CUDA_TRY(cudaMemcpyAsync(c->Ey, Ey, c->G * 8, cudaMemcpyHostToDevice, c->stream));

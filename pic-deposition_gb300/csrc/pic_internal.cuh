@@ -107,6 +107,7 @@ struct pic_ctx {
     void* spec = nullptr;  // Ny x (Nx/2+1) complex
     double* fft_rhs = nullptr;
     int fft_fwd = 0, fft_inv = 0, fft_ready = 0;
+    double* fft_scale = nullptr;  // per frequency: cell volume / (k^2 * Nx * Ny), DC 0
     // deterministic FP64 reductions
     double* red_partials = nullptr;
     double* red_out = nullptr;
@@ -115,6 +116,10 @@ struct pic_ctx {
     double* ke_partials = nullptr;
     int ke_ready = 0;
     int ke_count = 0;  // entries the last gather filled
+    // per-block sums of rho and of Ex^2 + Ey^2 left by the field kernel of the last
+    // solve; grid_sums_ready: they belong to the current rho and E
+    double* grid_partials = nullptr;
+    int grid_sums_ready = 0;
     // red_out[8], red_out[9] hold sum(q) and sum(|q|) of the current particle set:
     // charges do not change while particles move or are sorted
     int qsum_valid = 0;
@@ -187,7 +192,9 @@ int sort_particles(pic_ctx* ctx, bool perm = false);
 int ensure_fields(pic_ctx* ctx);
 int poisson_fft(pic_ctx* ctx);
 int efield_from_phi(pic_ctx* ctx);
-int diagnostics_async(pic_ctx* ctx);
+// hist, step (both or neither): also write the step's pic_diag into the history
+// and advance the step counter
+int diagnostics_async(pic_ctx* ctx, double* hist = nullptr, int* step = nullptr, int steps = 0);
 int read_diagnostics(pic_ctx* ctx, pic_diag* d);
 void release_fields(pic_ctx* ctx);
 void release_rbgs(pic_ctx* ctx);
@@ -330,7 +337,6 @@ __device__ __forceinline__ bool cell_coord(double x, double d, double inv_d, int
     *off = r;
     return true;
 }
-
 
 // One unit of the int64 charge grid: max|q| * inv_vol * 2^-24 (FP64). The
 // resident charge is stored normalised, qn = q / max|q|, and a particle carries

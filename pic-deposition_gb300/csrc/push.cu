@@ -145,7 +145,9 @@ int move(pic_ctx* c, double dt, bool gather, bool push, bool ke) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     size_t blocks = (c->n + 255) / 256;
     if (blocks > (size_t)sms * 32) blocks = (size_t)sms * 32;
-    if (ke) blocks = MOVE_KE_BLOCKS;  // the partition of the sums does not depend on the device
+    // the partition of the sums depends on the particle count alone; no more blocks
+    // than particles / 256 (4096 nearly empty blocks took 18 us at 65,536 particles)
+    if (ke) blocks = (c->n + 255) / 256 < (size_t)MOVE_KE_BLOCKS ? (c->n + 255) / 256 : (size_t)MOVE_KE_BLOCKS;
     prof_begin(c, gather && push ? "gather_push" : gather ? "gather" : "push");
     if (gather && push)
         ke ? move_particles<true, true, true><<<(unsigned)blocks, 256, 0, c->stream>>>(a)
@@ -159,7 +161,7 @@ int move(pic_ctx* c, double dt, bool gather, bool push, bool ke) {
     PIC_TRY(check_launch(c, "move_particles"));
     if (push) c->sorted = 0;
     c->ke_ready = ke ? 1 : 0;
-    c->ke_count = MOVE_KE_BLOCKS;
+    c->ke_count = (int)blocks;
     return PIC_OK;
 }
 

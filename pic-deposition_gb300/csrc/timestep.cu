@@ -32,27 +32,6 @@ int rbgs_solve_async(pic_ctx* c, double tol, int max_iters, int check_every);
 int ws_warm_guess(pic_ctx* c, int mode);
 int ws_record_solution(pic_ctx* c);
 
-// pic_diag from the raw sums in red_out (same formulas as read_diagnostics).
-__global__ void finalize_diag(const double* __restrict__ r, double vol, double* __restrict__ hist,
-                              int* __restrict__ step, int steps) {
-    const int s = *step;
-    if (s < steps) {
-        double* d = hist + (size_t)s * 6;
-        const double total_charge = r[1];
-        const double integrated = __dmul_rn(r[2], vol);
-        const double den = r[6] > 1e-12 ? r[6] : 1e-12;
-        const double ke = r[3];
-        const double fe = __dmul_rn(__dmul_rn(0.5, r[4]), vol);
-        d[0] = __ddiv_rn(fabs(__dsub_rn(integrated, total_charge)), den);
-        d[1] = total_charge;
-        d[2] = integrated;
-        d[3] = ke;
-        d[4] = fe;
-        d[5] = __dadd_rn(ke, fe);
-    }
-    *step = s + 1;
-}
-
 // moved[s] = the particles the step's deposit found outside their sorted cell
 // (step s = the diagnostics counter: the previous step's diagnostics are done)
 __global__ void take_moved(DevStats* st, unsigned long long* __restrict__ moved, const int* __restrict__ step,
@@ -71,9 +50,7 @@ static int solve(pic_ctx* c, const pic_run_config* cfg) {
 
 // The diagnostics of the step whose gather has just run.
 static int record_step(pic_ctx* c, double* hist, int* step_ctr, int steps) {
-    PIC_TRY(diagnostics_async(c));
-    finalize_diag<<<1, 1, 0, c->stream>>>(c->red_out, c->dx * c->dy, hist, step_ctr, steps);
-    return check_launch(c, "finalize_diag");
+    return diagnostics_async(c, hist, step_ctr, steps);
 }
 
 // One step; `do_sort` selects the variant with the cell sort. For NGP/CIC/TSC

@@ -26,6 +26,7 @@
 // loads), each lane summing its particles' 24 edge values while they share a
 // cell (one rolled copy of the particle body), a segmented warp scan, and int64
 // atomics from the run tails (deposit_current).
+#include "cells.cuh"
 #include "pic_internal.cuh"
 
 namespace picgb {
@@ -257,85 +258,243 @@ __global__ void __launch_bounds__(J_THREADS) deposit_current(JArgs a) {
     }
 }
 
-// Cell-sorted particles: one lane per cell. A CTA owns a 32 x 8 tile of cells;
-// warp w takes the tile rows w, w + 4, and lane l the cell in column l, walking
-// that cell's range of the sorted stream (16-byte loads of 4 particles) and
-// summing its particles' 24 edge values in 32-bit registers (at most 64
-// particles per sum: |sum| <= 64 * 2^24). Each sum goes to the tile's Jx and Jy
-// accumulators in shared memory (low 15 bits and the rest in two 32-bit words,
-// a halo of one node left and below and two right and above), and the tile to
-// the int64 grids once. Integer sums, so the grids equal those of
-// deposit_current bit for bit.
+// Cell-sorted particles. A CTA owns a 32 x 8 tile of cells; its warps walk units of
+// consecutive cells of a row, K lanes per cell, with the stream staged in shared
+// memory (cells.cuh).
+//  * A particle that stays in its cell (0 <= r + d < 1 on both axes) has
+//    DS = (0, -d, d, 0) and its old and new charges on the same 2x2 nodes: of its
+//    24 edge values seven are not zero, and they follow from five numbers that
+//    add up over the cell's particles: W1[1][1], W1[2][1] and the changes of the
+//    row 0, column 0 and diagonal sums of its integer charges. These are summed
+//    in 32-bit registers (at most 64 particles per sum: |sum| <= 64 * 2^24).
+//  * The others are listed (ballot compaction into a queue per warp, appended 32
+//    at a time) for a second kernel, current_listed: 24 edge values in full, one particle per lane,
+//    int64 atomics. Evaluating them in this kernel (queued, 32 at a time) cost it
+//    half of its resident warps in registers.
+// The sums go to the tile's Jx and Jy accumulators in shared memory (low 15 bits
+// and the rest in two 32-bit words, a halo of one node left and below and two right
+// and above), and the tile to the int64 grids once; tiles so full that the words
+// could overflow add straight to the grids. Integer sums, so the grids equal those
+// of deposit_current bit for bit.
+// Bound by the staying particle's arithmetic (two rounded CIC charges and two
+// edge values). One full evaluation per particle, each lane reading its own cell
+// from global memory, took 1.11 ms at 1024^2, 64 particles per cell.
 constexpr int JC_TW = 32, JC_TH = 8, JC_WARPS = 4;
 constexpr int JC_SW = JC_TW + 3, JC_SH = JC_TH + 3, JC_N = JC_SW * JC_SH;
 constexpr int JC_RUN = 64;
 constexpr int JC_SPLIT = 15;
+constexpr unsigned JC_BATCH = 32;  // particles appended to the list at a time (one atomic on its length)
+// A low word holds 2^17 additions; a run of at most JC_RUN particles of one lane
+// adds to a node once, 32 lanes may share a cell, and five cells reach a node.
+constexpr uint32_t JC_RUN_MAX = 1u << 17;  // particles of a tile whose runs use the tile's accumulators
+
+// The listed particles with their values (the sort's spare arrays): reading them
+// back from the particle arrays took a 64-byte DRAM access per value.
+struct JList {
+    unsigned* count;
+    uint32_t *p, *cell;
+    float *xr, *yr, *vx, *vy;
+};
+
+// All 24 edge values of the listed particles (also the Courant check).
+__global__ void __launch_bounds__(J_THREADS) current_listed(JArgs a, JList l) {
+    const unsigned n = *l.count;
+    for (unsigned i = blockIdx.x * J_THREADS + threadIdx.x; i < n; i += gridDim.x * J_THREADS) {
+        const uint32_t p = l.p[i];
+        int v[NJ];
+        if (edge_values(a, l.xr[i], l.yr[i], l.vx[i], l.vy[i], a.qc != 0.0f ? a.qc : a.q[p], p, v))
+            flush_edges(a, l.cell[i], v);
+    }
+}
 
 template <bool QC>
-__global__ void __launch_bounds__(JC_WARPS * 32) current_cells(JArgs a, const uint32_t* __restrict__ offsets,
-                                                                int tiles_x) {
+__global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const uint32_t* __restrict__ offsets,
+                                                                   int tiles_x, int klog, int cap, JList list) {
+    constexpr int NF = QC ? 4 : 5;
+    extern __shared__ __align__(16) uint32_t sbufs[];  // [JC_WARPS][NF][cap]
+    __shared__ uint32_t soff[JC_TH * (JC_TW + 1)];
     __shared__ uint32_t slo[2 * JC_N];
     __shared__ int shi[2 * JC_N];
+    __shared__ uint32_t s_count;
+    __shared__ uint2 squeue[JC_WARPS][JC_BATCH + 32];   // particle, cell
+    __shared__ float4 sqval[JC_WARPS][JC_BATCH + 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
     const int x0 = tx * JC_TW, y0 = ty * JC_TH;
     const int tw = min(JC_TW, a.Nx - x0), th = min(JC_TH, a.Ny - y0);
+    if (threadIdx.x == 0) s_count = 0;
     for (int i = threadIdx.x; i < 2 * JC_N; i += JC_WARPS * 32) {
         slo[i] = 0;
         shi[i] = 0;
     }
+    for (int i = threadIdx.x; i < th * (tw + 1); i += JC_WARPS * 32) {
+        const int r = i / (tw + 1);
+        soff[i] = offsets[(uint32_t)(y0 + r) * (uint32_t)a.Nx + (uint32_t)x0 + (uint32_t)(i - r * (tw + 1))];
+    }
     __syncthreads();
-    int acc[NJ];
-    // adds acc (the cell in column `lane`, tile row r) to the tile accumulators
-    auto flush = [&](int r) {
-#pragma unroll
-        for (int t = 0; t < NJ; ++t) {
-            const int v = acc[t];
-            if (v != 0) {
-                // Jx edge (j, i) = t (j * 3 + i), Jy edge (j, i) = t - 12 (j * 4 + i): local node (lane + i, r + j)
-                const int j = t < 12 ? t / 3 : (t - 12) / 4, i = t < 12 ? t % 3 : (t - 12) % 4;
-                const int idx = (t < 12 ? 0 : JC_N) + (r + j) * JC_SW + lane + i;
-                atomicAdd(slo + idx, (uint32_t)v & ((1u << JC_SPLIT) - 1u));
-                atomicAdd(shi + idx, v >> JC_SPLIT);
-            }
-            acc[t] = 0;
+    if (threadIdx.x < th) atomicAdd(&s_count, soff[threadIdx.x * (tw + 1) + tw] - soff[threadIdx.x * (tw + 1)]);
+    __syncthreads();
+    const bool run_to_grid = s_count >= JC_RUN_MAX;
+    uint2* queue = squeue[warp];
+    float4* qval = sqval[warp];
+    unsigned qn = 0;
+    auto append = [&](unsigned m) {  // the first m queued particles to the list
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(list.count, m);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (unsigned i = (unsigned)lane; i < m; i += 32) {
+            const uint2 id = queue[i];
+            const float4 v = qval[i];
+            list.p[at + i] = id.x;
+            list.cell[at + i] = id.y;
+            list.xr[at + i] = v.x;
+            list.yr[at + i] = v.y;
+            list.vx[at + i] = v.z;
+            list.vy[at + i] = v.w;
         }
     };
-    for (int r = warp; r < th; r += JC_WARPS) {
-        uint32_t beg = 0, end = 0;
-        if (lane < tw) {
-            const uint32_t cell = (uint32_t)(y0 + r) * (uint32_t)a.Nx + (uint32_t)(x0 + lane);
-            beg = offsets[cell];
-            end = offsets[cell + 1];
-        }
-#pragma unroll
-        for (int t = 0; t < NJ; ++t) acc[t] = 0;
-        int cnt = 0;
-        const uint32_t q0 = beg >> 2, q1 = end > beg ? (end + 3u) >> 2 : q0;
+    // one charge: values of +2^24 units, mirrored for a negative charge
+    const int sgn = QC && a.qc < 0.0f ? -1 : 1;
+    uint32_t* sbuf = sbufs + (size_t)warp * NF * cap;
+    CellWalk<NF, JC_WARPS> walk;
+    walk.init(tw, th, klog, cap);
+    walk.soff = soff;
+    walk.buf_addr = (uint32_t)__cvta_generic_to_shared(sbuf);
+    walk.field[0] = reinterpret_cast<const uint32_t*>(a.xr);
+    walk.field[1] = reinterpret_cast<const uint32_t*>(a.yr);
+    walk.field[2] = reinterpret_cast<const uint32_t*>(a.vx);
+    walk.field[3] = reinterpret_cast<const uint32_t*>(a.vy);
+    if constexpr (!QC) walk.field[4] = reinterpret_cast<const uint32_t*>(a.q);
+    CellPiece cw;
+    for (walk.start(cw, warp); !walk.done(cw); walk.advance(cw)) {
+        walk.stage(cw, lane);
+        const float* sb = reinterpret_cast<const float*>(sbuf);
+        const int r = cw.r, col = cw.c0 + (lane >> klog);
+        int m, first;
+        uint32_t ncell;
+        walk.share(cw, lane, first, m, ncell);
+        // cells small enough that 32-bit sums hold all their lanes' particles
+        const bool small = __all_sync(0xffffffffu, ncell <= 127u);
+        // W1[1][1], W1[2][1]; changes of row 0, column 0 and the diagonal of the charges
+        int e1 = 0, e2 = 0, drow = 0, dcol = 0, ddia = 0, cnt = 0;
+        // value k of the cell's seven (edges below) to the tile, or to the grids
+        auto add = [&](int k, long long x) {
+            if (x == 0) return;
+            // edges: Jx (1,1), (2,1), (3,1); Jy (1,1), (2,1), (1,2), (2,2), as (row j, column i)
+            const int j = k == 0 || k == 3 || k == 5 ? 1 : k == 2 ? 3 : 2;
+            const int i = k < 5 ? 1 : 2;
+            if (!run_to_grid) {
+                const int idx = (k < 3 ? 0 : JC_N) + (r + j) * JC_SW + col + i;
+                atomicAdd(slo + idx, (uint32_t)x & ((1u << JC_SPLIT) - 1u));
+                atomicAdd(shi + idx, (int)(x >> JC_SPLIT));
+            } else {
+                const size_t g = (size_t)wrap_i(y0 + r - 1 + j, a.Ny) * a.Nx + wrap_i(x0 + col - 1 + i, a.Nx);
+                atomicAdd((k < 3 ? a.jx : a.jy) + g, (unsigned long long)x);
+            }
+        };
+        auto flush = [&](int from, int step) {
+            // change of node (0,0): exact, as the total does not change
+            const long long d00 = ((long long)drow + dcol + ddia) / 2;
+            const long long w = (long long)dcol - e1 - e2;  // W1[3][1] = -W1[3][2]
+            const long long d01 = drow - d00;               // change of node (0,1)
+            for (int k = from; k < 7; k += step) {
+                const long long x = k == 0 ? -e1 : k == 1 ? -e2 : k == 2 || k == 4 ? -w : k == 3 ? e1 - d00 : k == 5 ? -(d01 + e1) : w;
+                add(k, QC ? sgn * x : x);
+            }
+            e1 = e2 = drow = dcol = ddia = cnt = 0;
+        };
+        // warp-uniform trips of two particles per lane, cyclically from a pair that
+        // differs from cell to cell (bank conflicts, as in deposit_cells)
+        constexpr int UN = 2;
+        const int ng = (m + UN - 1) / UN;
+        const int trips = __reduce_max_sync(0xffffffffu, ng);
+        int g = (lane >> klog) < ng ? lane >> klog : 0;
 #pragma unroll 1
-        for (uint32_t qd = q0; qd < q1; ++qd) {
-            const float4 xr = __ldg(reinterpret_cast<const float4*>(a.xr) + qd);
-            const float4 yr = __ldg(reinterpret_cast<const float4*>(a.yr) + qd);
-            const float4 vx = __ldg(reinterpret_cast<const float4*>(a.vx) + qd);
-            const float4 vy = __ldg(reinterpret_cast<const float4*>(a.vy) + qd);
-            const float4 q = QC ? make_float4(a.qc, a.qc, a.qc, a.qc) : __ldg(reinterpret_cast<const float4*>(a.q) + qd);
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t p = 4u * qd + (uint32_t)k;
-                if (p < beg || p >= end) continue;
-                int v[NJ];
-                if (edge_values(a, f4(xr, k), f4(yr, k), f4(vx, k), f4(vy, k), f4(q, k), p, v)) {
+        for (int t = 0; t < trips; ++t) {
+            const int left = t < ng ? m - g * UN : 0;
+            const int i0 = first + g * UN;
+            g = g + 1 >= ng ? 0 : g + 1;
 #pragma unroll
-                    for (int t = 0; t < NJ; ++t) acc[t] += v[t];
+            for (int k = 0; k < UN; ++k) {
+                const bool valid = k < left;
+                float rx = 0.0f, ry = 0.0f, vx = 0.0f, vy = 0.0f;
+                if (valid) {
+                    rx = sb[i0 + k];
+                    ry = sb[cap + i0 + k];
+                    vx = sb[2 * cap + i0 + k];
+                    vy = sb[3 * cap + i0 + k];
                 }
-                if (++cnt == JC_RUN) {
-                    flush(r);
-                    cnt = 0;
+                const float dx = vx * a.dtdx, dy = vy * a.dtdy;
+                const float ex = rx + dx, ey = ry + dy;
+                // 0 <= e < 1 on both axes: the bits of non-negative floats are in their order
+                const bool stays = fmaxf(fabsf(dx), fabsf(dy)) < 1.0f && max(__float_as_uint(ex), __float_as_uint(ey)) < 0x3F800000u;
+                const unsigned out = __ballot_sync(0xffffffffu, valid && !stays);
+                if (out) {
+                    if (valid && !stays) {
+                        const unsigned at = qn + __popc(out & ((1u << lane) - 1u));
+                        queue[at] = make_uint2(cw.pos + (uint32_t)(i0 + k),
+                                               (uint32_t)(y0 + r) * (uint32_t)a.Nx + (uint32_t)(x0 + col));
+                        qval[at] = make_float4(rx, ry, vx, vy);
+                    }
+                    qn += __popc(out);
+                    __syncwarp();
+                    if (qn >= JC_BATCH) {
+                        append(JC_BATCH);
+                        const uint2 rest = queue[JC_BATCH + lane];
+                        const float4 rval = qval[JC_BATCH + lane];
+                        qn -= JC_BATCH;
+                        __syncwarp();
+                        if ((unsigned)lane < qn) {
+                            queue[lane] = rest;
+                            qval[lane] = rval;
+                        }
+                        __syncwarp();
+                    }
+                }
+                if (valid && stays) {
+                    if constexpr (QC) {
+                        int r0, c0, g0, r1, c1, g1;
+                        cic_unit(rx, ry, r0, c0, g0);
+                        cic_unit(ex, ey, r1, c1, g1);
+                        drow += r1 - r0;
+                        dcol += c1 - c0;
+                        ddia += g1 - g0;
+                        e1 += __float2int_rn((16777216.0f * ((1.0f - ry) - 0.5f * dy)) * -dx);
+                        e2 += __float2int_rn((16777216.0f * (ry + 0.5f * dy)) * -dx);
+                    } else {
+                        const float aq = sb[4 * cap + i0 + k] * 16777216.0f;
+                        const int A = __float2int_rn(aq);
+                        int v0[4], v1[4];
+                        cic_int(aq, A, rx, ry, v0);
+                        cic_int(aq, A, ex, ey, v1);
+                        ddia += v1[0] + v1[3] - v0[0] - v0[3];
+                        drow += v1[0] + v1[1] - v0[0] - v0[1];
+                        dcol += v1[0] + v1[2] - v0[0] - v0[2];
+                        e1 += __float2int_rn((aq * ((1.0f - ry) - 0.5f * dy)) * -dx);
+                        e2 += __float2int_rn((aq * (ry + 0.5f * dy)) * -dx);
+                    }
+                    if (++cnt == JC_RUN && !small) flush(0, 1);
                 }
             }
         }
-        if (cnt) flush(r);
+        if (small) {
+            // the cell's sums over its K lanes, which share the seven values
+            const int K = 1 << klog;
+            for (int o = 1; o < K; o <<= 1) {
+                e1 += __shfl_xor_sync(0xffffffffu, e1, o);
+                e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+                drow += __shfl_xor_sync(0xffffffffu, drow, o);
+                dcol += __shfl_xor_sync(0xffffffffu, dcol, o);
+                ddia += __shfl_xor_sync(0xffffffffu, ddia, o);
+                cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+            }
+            if (cnt) flush(lane & (K - 1), K);
+        } else if (cnt) {
+            flush(0, 1);
+        }
+        __syncwarp();
     }
+    if (qn) append(qn);
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * JC_N; i += JC_WARPS * 32) {
         const long long v = (long long)shi[i] * (1ll << JC_SPLIT) + (long long)slo[i];
@@ -373,7 +532,7 @@ static int ensure_current(pic_ctx* c) {
     if (rc) return rc;
     if (!c->jy) c->jy = (double*)dalloc(c->G * 8, &rc);
     if (rc) return rc;
-    if (!c->junits) c->junits = (double*)dalloc(2 * 8, &rc);
+    if (!c->junits) c->junits = (double*)dalloc(3 * 8, &rc);  // units, and the list's length
     return rc;
 }
 
@@ -401,13 +560,29 @@ int deposit_current_async(pic_ctx* c, double dt) {
     if (c->n && c->sorted) {
         // cell-sorted: one lane per cell over the sort's ranges
         const int tiles_x = (c->Nx + JC_TW - 1) / JC_TW, tiles_y = (c->Ny + JC_TH - 1) / JC_TH;
+        int klog, cap;
+        const bool qc = a.qc != 0.0f;
+        cells_shape(c->n, c->G, qc ? 4 : 5, 1560, &klog, &cap);
+        PIC_TRY(ensure_sort_scratch(c));  // the list takes the sort's spare arrays
+        unsigned* count = reinterpret_cast<unsigned*>(c->junits + 2);
+        PIC_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(unsigned), c->stream));
+        const JList list{count, c->idx_b, c->cell_alt, c->alt[0], c->alt[1], c->alt[2], c->alt[3]};
+        const size_t smem = (size_t)JC_WARPS * (qc ? 4 : 5) * cap * 4;
+        PIC_TRY(opt_in_dynamic_smem(qc ? (const void*)current_cells<true> : (const void*)current_cells<false>, smem));
         prof_begin(c, "current");
-        if (a.qc != 0.0f)
-            current_cells<true><<<(unsigned)(tiles_x * tiles_y), JC_WARPS * 32, 0, c->stream>>>(a, c->offsets, tiles_x);
+        const unsigned tiles = (unsigned)(tiles_x * tiles_y);
+        if (qc)
+            current_cells<true><<<tiles, JC_WARPS * 32, smem, c->stream>>>(a, c->offsets, tiles_x, klog, cap, list);
         else
-            current_cells<false><<<(unsigned)(tiles_x * tiles_y), JC_WARPS * 32, 0, c->stream>>>(a, c->offsets, tiles_x);
-        prof_end(c);
+            current_cells<false><<<tiles, JC_WARPS * 32, smem, c->stream>>>(a, c->offsets, tiles_x, klog, cap, list);
         PIC_TRY(check_launch(c, "current_cells"));
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        size_t blocks = (c->n + J_THREADS - 1) / J_THREADS;
+        if (blocks > (size_t)sms * 4) blocks = (size_t)sms * 4;
+        current_listed<<<(unsigned)blocks, J_THREADS, 0, c->stream>>>(a, list);
+        prof_end(c);
+        PIC_TRY(check_launch(c, "current_listed"));
     } else if (c->n) {
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);

@@ -46,6 +46,7 @@
 //
 // Compiled with --fmad=false: no multiply-add is fused, so every FP32 result
 // equals the oracle's (compiled with -ffp-contract=off).
+#include "cells.cuh"
 #include "pic_internal.cuh"
 
 namespace picgb {
@@ -90,6 +91,7 @@ struct DepArgs {
     float dtf, dtdx, dtdy;
     int tile_w, tile_h, tiles_x;
     float qc;  // nonzero: every particle's stored charge (the charge stream is not read)
+    int klog, cap;  // deposit_cells: log2 lanes per cell, particles of a stage buffer
     DevStats* st;
     // non-null: the kernel deposits only when *gate == gate_when (the choice
     // between the cell kernel and the any-order kernel between sorts is made on
@@ -580,7 +582,8 @@ __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
 // ---------------------------------------------------------------------------
 constexpr uint32_t TSCI_ONE = 1u << 15;
 
-__device__ __forceinline__ void tsci_weights(float rx, float ry, uint32_t (&X)[4], uint32_t (&Y)[4]) {
+// The three weights (left, centre, right) of each axis.
+__device__ __forceinline__ void tsci_weights3(float rx, float ry, uint32_t (&X)[3], uint32_t (&Y)[3]) {
     const bool sx = rx >= 0.5f, sy = ry >= 0.5f;
     float mx, my;
     f2_unpack(f2_add(f2_pack(rx, ry), f2_pack(-1.0f, -1.0f)), mx, my);
@@ -592,17 +595,27 @@ __device__ __forceinline__ void tsci_weights(float rx, float ry, uint32_t (&X)[4
     float lx, ly, rxw, ryw;
     f2_unpack(wl, lx, ly);
     f2_unpack(wr, rxw, ryw);
-    const uint32_t WLx = __float_as_uint(lx) - TSC_MAGIC_BITS, WLy = __float_as_uint(ly) - TSC_MAGIC_BITS;
-    const uint32_t WRx = __float_as_uint(rxw) - TSC_MAGIC_BITS, WRy = __float_as_uint(ryw) - TSC_MAGIC_BITS;
-    const uint32_t WCx = TSCI_ONE - WLx - WRx, WCy = TSCI_ONE - WLy - WRy;
-    X[0] = sx ? 0u : WLx;
-    X[1] = sx ? WLx : WCx;
-    X[2] = sx ? WCx : WRx;
-    X[3] = sx ? WRx : 0u;
-    Y[0] = sy ? 0u : WLy;
-    Y[1] = sy ? WLy : WCy;
-    Y[2] = sy ? WCy : WRy;
-    Y[3] = sy ? WRy : 0u;
+    X[0] = __float_as_uint(lx) - TSC_MAGIC_BITS;
+    Y[0] = __float_as_uint(ly) - TSC_MAGIC_BITS;
+    X[2] = __float_as_uint(rxw) - TSC_MAGIC_BITS;
+    Y[2] = __float_as_uint(ryw) - TSC_MAGIC_BITS;
+    X[1] = TSCI_ONE - X[0] - X[2];
+    Y[1] = TSCI_ONE - Y[0] - Y[2];
+}
+
+// The weights on the 4-node frame of the particle's cell.
+__device__ __forceinline__ void tsci_weights(float rx, float ry, uint32_t (&X)[4], uint32_t (&Y)[4]) {
+    const bool sx = rx >= 0.5f, sy = ry >= 0.5f;
+    uint32_t x[3], y[3];
+    tsci_weights3(rx, ry, x, y);
+    X[0] = sx ? 0u : x[0];
+    X[1] = sx ? x[0] : x[1];
+    X[2] = sx ? x[1] : x[2];
+    X[3] = sx ? x[2] : 0u;
+    Y[0] = sy ? 0u : y[0];
+    Y[1] = sy ? y[0] : y[1];
+    Y[2] = sy ? y[1] : y[2];
+    Y[3] = sy ? y[2] : 0u;
 }
 
 // c + a * b in 64 bits, one multiply-add (a widening multiply followed by a
@@ -763,21 +776,6 @@ __device__ __forceinline__ void particle_to_global(const DepArgs& a, uint32_t ke
     flush_global<S>(a, key, tv);
 }
 
-// Adds a lane's run totals for cell `key` (64-bit values) straight to the global grid.
-template <int NX, int LO, int NV>
-__device__ __forceinline__ void flush_global_ll(const DepArgs& a, uint32_t key, const long long (&tv)[NV]) {
-    const int iy = (int)(key / (uint32_t)a.Nx), ix = (int)(key - (uint32_t)iy * (uint32_t)a.Nx);
-#pragma unroll
-    for (int j = 0; j < NX; ++j) {
-        const size_t row = (size_t)wrap_i(iy + LO + j, a.Ny) * a.Nx;
-#pragma unroll
-        for (int i = 0; i < NX; ++i) {
-            const long long v = tv[j * NX + i];
-            if (v != 0) atomicAdd(a.acc + row + wrap_i(ix + LO + i, a.Nx), (unsigned long long)v);
-        }
-    }
-}
-
 // Fields of a particle staged by the sorted kernel: cell, xr, yr, q (not when
 // one charge is shared), vx, vy (Esirkepov).
 template <int S, bool QC>
@@ -796,15 +794,6 @@ struct StageFields {
 // Denser tiles add their cells' totals straight to the global int64 grid.
 constexpr int TILE_SPLIT = 15;
 constexpr uint32_t TILE_SPLIT_MAX = 1u << 17;  // particles per tile for the split accumulators
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 // Adds a run's exact integer TSC totals for cell `key` straight to the global
 // grid, without integer division (as flush_global_nd).
@@ -958,36 +947,33 @@ __global__ void __launch_bounds__(DEP_THREADS, 4) deposit_runs_tsc(DepArgs a) {
 
 // ---------------------------------------------------------------------------
 // Sorted path, cell form (deposit_cells). One CTA of NW warps per tile of
-// tile_w x tile_h cells; the tile's rows are cut into units of up to 32
-// consecutive cells and warp w walks units w, w+NW, ... Lane l of a unit owns
-// one cell: the contiguous range [offsets[c], offsets[c+1]) of the cell-sorted
-// stream, which it walks in stages of LPP particles.
-//  * Staging: each stage's quads (4 particles, from the 16-byte boundary at or
-//    below the cell's first particle) are copied global -> shared with
-//    cp.async, 16 bytes per lane, field and quad, into [field][quad][lane]
-//    slots (the copies and the lanes' 128-bit reads are conflict-free); two
-//    stage buffers per warp, the next stage -- or the next unit's first -- in
-//    flight while this one is used. A unit takes as many stages as its fullest
-//    cell; lanes whose cell is done idle.
+// tile_w x tile_h cells; the tile's rows are cut into units of U = 32 / K
+// consecutive cells and warp w walks units w, w+NW, ... K lanes share a cell of
+// the unit: its contiguous range [offsets[c], offsets[c+1]) of the cell-sorted
+// stream, every K-th particle each.
+//  * Staging: a unit's particles are one contiguous range, copied to shared memory
+//    coalesced (cells.cuh). Lanes then walk their own cells there, starting at
+//    different particles of the cell, so that cells of equal size do not meet in
+//    one bank. (Per-lane copies of each lane's own cell touched 32 lines per copy
+//    instruction.)
 //  * A lane's particles all belong to its cell, so there are no runs to detect
 //    and no cell keys to read: the offsets name every particle's cell (KEYS =
 //    false, a fresh sort). After particles have moved since the sort (KEYS =
-//    true, between the sorts of a time-stepping loop) the keys are read;
+//    true, between the sorts of a time-stepping loop) the keys are staged too;
 //    particles that left their cell are queued per warp (ballot compaction
-//    into shared memory) and, after the stage, all lanes deposit them straight
-//    to the global grid, one per lane (no divergent per-particle path).
-//  * Sums: per stage in 32 bits (at most LPP particles), added to 64-bit cell
-//    totals at the end of each stage (CellRun); the exact integer TSC form
-//    keeps 9 of its 16 entries and 6 axis sums (see CellRun<S_TSC, true>).
-//  * Each lane writes its cell's totals out once: to the tile's split 32-bit
-//    shared accumulators (adjacent lanes hit different nodes: no same-address
-//    conflicts), or, in a tile of 2^17 particles or more, to the global grid.
+//    into shared memory) and, 32 at a time, deposited by all lanes, one per
+//    lane (no divergent per-particle path).
+//  * Sums: in 32 bits over at most 32 particles, then added to 64-bit cell
+//    totals (CellRun); the exact integer TSC form keeps 9 of its 16 entries and
+//    6 axis sums (see CellRun<S_TSC, true>).
+//  * Each lane writes its totals out once per unit: to the tile's split 32-bit
+//    shared accumulators, or, in a tile of 2^17 particles or more, to the global grid.
 // At the end the tile is added to the global int64 grid once.
 // ---------------------------------------------------------------------------
 template <int S, bool QC>
 struct CellRun {
     static constexpr int NV = Frame<S>::NX * Frame<S>::NX;
-    uint32_t v[NV];   // this stage's sums (TSC: outer entries biased, see tsc_accumulate)
+    uint32_t v[NV];   // sums since the last fold (TSC: outer entries biased, see tsc_accumulate)
     long long T[NV];  // the cell's totals
     __device__ __forceinline__ void zero() {
 #pragma unroll
@@ -997,9 +983,8 @@ struct CellRun {
         }
     }
     __device__ __forceinline__ void end_quad() {}
-    __device__ __forceinline__ void finish() {}
-    // adds the sums of a stage (`cnt` particles) to the totals
-    __device__ __forceinline__ void end_stage(uint32_t cnt, bool) {
+    // adds the sums of `cnt` particles (at most 32) to the totals
+    __device__ __forceinline__ void fold(uint32_t cnt) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
             if constexpr (S == S_TSC)
@@ -1023,9 +1008,9 @@ struct CellRun {
 // follow exactly (integer identities) when the cell is written out. Per
 // particle: 9 32-bit multiply-adds and 6 adds. Bounds: the 8 entries other than
 // A[1][1] are at most 2^12 * 24576 < 2^26.6 per particle, summed in 32 bits for
-// at most 32 particles (32/LPP stages) and then added to 64-bit totals; A[1][1] <=
-// 24576^2 < 2^29.2 per particle is summed in 32 bits for a quad (4 particles);
-// the axis sums are 64-bit totals of 32-bit sums of as many stages.
+// at most 32 particles and then added to 64-bit totals; A[1][1] <= 24576^2 <
+// 2^29.2 per particle is summed in 32 bits for 4 particles; the axis sums are
+// 64-bit totals of 32-bit sums of as many particles.
 template <>
 struct CellRun<S_TSC, true> {
     static constexpr int NV = 16;
@@ -1067,8 +1052,8 @@ struct CellRun<S_TSC, true> {
         C11 += c11;
         c11 = 0;
     }
-    // partial sums -> 64-bit totals (every 4 stages: at most 32 particles, 2^31.6)
-    __device__ __forceinline__ void fold() {
+    // partial sums -> 64-bit totals (at most 32 particles, 2^31.6)
+    __device__ __forceinline__ void fold(uint32_t) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             E[k] += e[k];
@@ -1082,11 +1067,7 @@ struct CellRun<S_TSC, true> {
         SY3 += sy3;
         sx0 = sx1 = sx3 = sy0 = sy1 = sy3 = 0;
     }
-    __device__ __forceinline__ void end_stage(uint32_t, bool fold_now) {
-        if (fold_now) fold();
-    }
-    __device__ __forceinline__ void finish() { fold(); }
-    // the 16 totals of n particles, row-major A[j][i] (after finish)
+    // the 16 totals of n particles, row-major A[j][i] (after fold)
     __device__ __forceinline__ void totals(uint32_t n, long long (&A)[16]) const {
         const long long one = (long long)TSCI_ONE;
         A[0] = (long long)E[0];
@@ -1127,14 +1108,51 @@ struct CellRun<S_NGP, true> {
         nxy += sx & sy;
     }
     __device__ __forceinline__ void end_quad() {}
-    __device__ __forceinline__ void end_stage(uint32_t, bool) {}
-    __device__ __forceinline__ void finish() {}
+    __device__ __forceinline__ void fold(uint32_t) {}
     __device__ __forceinline__ void totals(uint32_t n, long long (&T)[4]) const {
         const long long a = A;
         T[0] = a * ((long long)n - nx - ny + nxy);
         T[1] = a * ((long long)nx - nxy);
         T[2] = a * ((long long)ny - nxy);
         T[3] = a * (long long)nxy;
+    }
+};
+
+// CIC with one charge for all particles: a cell's four node sums follow from
+// its count and three signed sums (cic_unit; linear in the particles), so a
+// particle rounds three products by an FP32 add instead of four by F2I and has
+// no remainder to place. 32-bit sums of at most 32 particles (2^28), then 64-bit totals.
+template <>
+struct CellRun<S_CIC, true> {
+    static constexpr int NV = 4;
+    int sgn;  // sign of the charge
+    int r, c, d;
+    long long R, C, D;
+    __device__ __forceinline__ void zero() {
+        r = c = d = 0;
+        R = C = D = 0;
+    }
+    __device__ __forceinline__ void add(float rx, float ry) {
+        int row0, col0, diag;
+        cic_unit(rx, ry, row0, col0, diag);
+        r += row0;
+        c += col0;
+        d += diag;
+    }
+    __device__ __forceinline__ void end_quad() {}
+    __device__ __forceinline__ void fold(uint32_t) {
+        R += r;
+        C += c;
+        D += d;
+        r = c = d = 0;
+    }
+    __device__ __forceinline__ void totals(uint32_t n, long long (&T)[4]) const {
+        // row 0, column 0 and the diagonal are R, C, D plus n A/2; all four nodes n A
+        const long long h = (long long)n << 23, v = (R + C + D + h) / 2;
+        T[0] = sgn * v;
+        T[1] = sgn * (R + h - v);
+        T[2] = sgn * (C + h - v);
+        T[3] = sgn * (D + h - v);
     }
 };
 
@@ -1165,15 +1183,23 @@ __device__ __noinline__ bool stale_to_tile(const DepArgs& a, uint32_t key, float
     if (cy < -(a.Ny / 2)) cy += a.Ny;
     if (cx < -1 || cx > tw || cy < -1 || cy > th) return false;
     const int lx0 = cx + 2 + LO, ly0 = cy + 2 + LO;  // local node of frame entry (0, 0)
+    if constexpr (S == S_TSC && QC) {  // the nine nodes of the particle's own 3x3 frame
+        uint32_t X3[3], Y3[3];
+        tsci_weights3(rx, ry, X3, Y3);
+        const bool sx = rx >= 0.5f, sy = ry >= 0.5f;
+        const int base = (ly0 + (sy ? 1 : 0)) * SW + lx0 + (sx ? 1 : 0);
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const uint32_t v = X3[i] * Y3[j];  // below 2^30
+                atomicAdd(slo + base + j * SW + i, v & ((1u << TILE_SPLIT) - 1u));
+                atomicAdd(shi + base + j * SW + i, (int)(v >> TILE_SPLIT));
+            }
+        return true;
+    }
     long long tv[NV];
-    if constexpr (S == S_TSC && QC) {
-        uint32_t X[4], Y[4];
-        tsci_weights(rx, ry, X, Y);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) tv[j * 4 + i] = (long long)((unsigned long long)X[i] * Y[j]);
-    } else if constexpr (S == S_TSC) {
+    if constexpr (S == S_TSC) {
         uint32_t val[16];
         tsc_values(rx, ry, qn, val);
 #pragma unroll
@@ -1196,15 +1222,17 @@ __device__ __noinline__ bool stale_to_tile(const DepArgs& a, uint32_t key, float
     return true;
 }
 
-// Shared memory: [stage buffers: NW warps x NBUF x NF fields x LPP/4 quads x
-// 32 lanes x 16 bytes][tile accumulators: low, high words][the tile rows' cell
-// offsets].
-template <int S, int LPP, int NW, bool QC, bool KEYS, int NBUF>
-__host__ __device__ constexpr size_t cells_fixed_bytes() {
-    return (size_t)NW * NBUF * (StageFields<S, QC>::NF - (KEYS ? 0 : 1)) * (LPP / 4) * 512;
+constexpr int CELLS_QUEUE = 32 + 128;  // queued particles (KEYS): below 32 left over, and one step of 4 per lane
+
+// Shared memory: [stage buffers: NW warps x NF fields x cap words][KEYS: a
+// queue per warp][tile accumulators: low, high words][the tile rows' cell offsets].
+template <int S, int NW, bool QC, bool KEYS>
+__host__ __device__ constexpr size_t cells_fixed_bytes(int cap) {
+    return (size_t)NW * (StageFields<S, QC>::NF - (KEYS ? 0 : 1)) * cap * 4 +
+           (KEYS ? (size_t)NW * CELLS_QUEUE * 4 : 0);
 }
 
-template <int S, int LPP, int NW, int MINB, bool QC, bool KEYS, int NBUF>
+template <int S, int NW, int MINB, bool QC, bool KEYS>
 __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
     if (gated_off(a)) return;
     constexpr int NX = Frame<S>::NX, LO = Frame<S>::LO, V = Frame<S>::V;
@@ -1213,11 +1241,9 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
     constexpr int FX = KEYS ? 1 : 0;                            // stage field of xr
     constexpr int FQ = FX + 2;                                  // of q (not QC)
     constexpr int FV = FX + (QC ? 2 : 3);                       // of vx (ESK)
-    constexpr int QL = LPP / 4;                                 // quads per lane per stage
-    constexpr int BUFB = NF * QL * 512;                         // bytes of one stage buffer of a warp
     constexpr bool TSCI = S == S_TSC && QC;                     // exact integer TSC weights
-    static_assert(LPP % 4 == 0 && LPP <= 16, "stage sums of LPP particles stay in 32 bits");
-    constexpr uint32_t FOLD = 32 / LPP;  // stages per fold of the exact TSC partial sums (32 particles)
+    constexpr int FOLD = 32;                                    // particles of a lane between folds
+    constexpr int UN = S == S_ESK ? 1 : 4;                      // particles of a lane in flight
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_count;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1229,15 +1255,14 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
     const int x0 = tx * a.tile_w, y0 = ty * a.tile_h;
     const int tw = min(a.tile_w, a.Nx - x0), th = min(a.tile_h, a.Ny - y0);
     const int nloc = (th + 3 + 2 * PAD) * SW;
-    const int nch = (tw + 31) >> 5;  // units of up to 32 cells per tile row
-    unsigned char* swarp = smem_raw + (size_t)warp * NBUF * BUFB;
-    const uint32_t stage0 = (uint32_t)__cvta_generic_to_shared(swarp) + (uint32_t)(lane * 16);
-    uint32_t* slo = reinterpret_cast<uint32_t*>(smem_raw + cells_fixed_bytes<S, LPP, NW, QC, KEYS, NBUF>());
+    const int cap = a.cap;
+    uint32_t* sbuf = reinterpret_cast<uint32_t*>(smem_raw) + (size_t)warp * NF * cap;
+    uint32_t* squeue = reinterpret_cast<uint32_t*>(smem_raw) + (size_t)NW * NF * cap +
+                       (KEYS ? warp * CELLS_QUEUE : 0);
+    uint32_t* slo = reinterpret_cast<uint32_t*>(smem_raw + cells_fixed_bytes<S, NW, QC, KEYS>(cap));
     int* shi = reinterpret_cast<int*>(slo + nloc);
     uint32_t* soff = reinterpret_cast<uint32_t*>(shi + nloc);  // the tile rows' offsets, th x (tw + 1)
     const int ow = tw + 1;
-    // KEYS: this warp's queue of particles that left their cell (at most a stage)
-    uint32_t* squeue = soff + a.tile_h * (a.tile_w + 1) + warp * 32 * LPP;
     if (threadIdx.x == 0) s_count = 0;
     for (int i = threadIdx.x; i < nloc; i += NW * 32) {
         slo[i] = 0;
@@ -1252,190 +1277,227 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
     __syncthreads();
     const bool dense = s_count >= TILE_SPLIT_MAX;
 
-    const uint32_t* fptr[NF];
-    if constexpr (KEYS) fptr[0] = a.cell;
-    fptr[FX] = reinterpret_cast<const uint32_t*>(a.xr);
-    fptr[FX + 1] = reinterpret_cast<const uint32_t*>(a.yr);
-    if constexpr (!QC) fptr[FQ] = reinterpret_cast<const uint32_t*>(a.q);
+    CellWalk<NF, NW> walk;
+    walk.init(tw, th, a.klog, cap);
+    walk.soff = soff;
+    walk.buf_addr = (uint32_t)__cvta_generic_to_shared(sbuf);
+    if constexpr (KEYS) walk.field[0] = a.cell;
+    walk.field[FX] = reinterpret_cast<const uint32_t*>(a.xr);
+    walk.field[FX + 1] = reinterpret_cast<const uint32_t*>(a.yr);
+    if constexpr (!QC) walk.field[FQ] = reinterpret_cast<const uint32_t*>(a.q);
     if constexpr (S == S_ESK) {
-        fptr[FV] = reinterpret_cast<const uint32_t*>(a.vx);
-        fptr[FV + 1] = reinterpret_cast<const uint32_t*>(a.vy);
+        walk.field[FV] = reinterpret_cast<const uint32_t*>(a.vx);
+        walk.field[FV + 1] = reinterpret_cast<const uint32_t*>(a.vy);
     }
-    // unit u = (tile row, 32-cell chunk); this lane's cell range and quads
-    struct Unit {
-        uint32_t beg, end, q0, q1, nst;  // particles [beg, end), quads [q0, q1), stages of the unit
-        int r, col;                     // tile row, this lane's column in the tile (-1: no cell)
-    };
-    const int nunits = th * nch;
-    auto unit_of = [&](int u) {
-        Unit w;
-        w.r = u / nch;
-        const int col = (u - w.r * nch) * 32 + lane;
-        w.col = col < tw ? col : -1;
-        w.beg = w.end = 0;
-        if (w.col >= 0) {
-            w.beg = soff[w.r * ow + w.col];
-            w.end = soff[w.r * ow + w.col + 1];
-        }
-        w.q0 = w.beg >> 2;
-        w.q1 = w.end > w.beg ? (w.end + 3u) >> 2 : w.q0;
-        const uint32_t st = (w.q1 - w.q0 + QL - 1) / QL;
-        w.nst = __reduce_max_sync(FULL, st);
-        return w;
-    };
-    auto issue = [&](const Unit& w, uint32_t t, int buf) {
-        const uint32_t dst = stage0 + (uint32_t)(buf * BUFB);
-#pragma unroll
-        for (int h = 0; h < QL; ++h) {
-            const uint32_t qd = w.q0 + t * QL + (uint32_t)h;
-            if (qd < w.q1) {
-#pragma unroll
-                for (int f = 0; f < NF; ++f) cp_async16(dst + (uint32_t)((f * QL + h) * 512), fptr[f] + 4u * qd);
-            }
-        }
-        cp_async_commit();
-    };
 
-    // the first non-empty unit at or after u (nunits: none)
-    auto next_unit = [&](int u, Unit& w) {
-        for (; u < nunits; u += NW) {
-            w = unit_of(u);
-            if (w.nst) break;
-        }
-        return u;
-    };
-    // prefetch cursor (stage pt of unit pu), NBUF - 1 stages ahead of the consumer
-    Unit pw{};
-    int pu = next_unit(warp, pw);
-    uint32_t pt = 0;
-    auto issue_next = [&](int buf) {
-        if (pu < nunits) {
-            issue(pw, pt, buf);
-            if (++pt >= pw.nst) {
-                pt = 0;
-                pu = next_unit(pu + NW, pw);
-            }
-        } else {
-            cp_async_commit();  // an empty group keeps the wait counts uniform
-        }
-    };
-#pragma unroll
-    for (int k = 0; k < NBUF - 1; ++k) issue_next(k);
-    Unit cw{};
-    int u = next_unit(warp, cw);
-    uint32_t t = 0;
-    int buf = 0;
-    uint32_t cnt = 0;  // particles of the cell summed (KEYS: those still in it)
+    CellPiece cw;
+    uint32_t cnt = 0;    // particles of the lane's cell summed (KEYS: those still in it)
     uint32_t moved = 0;  // KEYS: particles of this warp's cells that left them (warp-uniform)
+    unsigned qn = 0;     // KEYS: particles in the queue (warp-uniform)
     CellRun<S, QC> run;
     if constexpr (S == S_NGP && QC) run.A = __float2int_rn(a.qc * 16777216.0f);
+    if constexpr (S == S_CIC && QC) run.sgn = a.qc < 0.0f ? -1 : 1;
     run.zero();
-    while (u < nunits) {
-        issue_next(buf == 0 ? NBUF - 1 : buf - 1);  // the buffer consumed last
-        cp_async_wait<NBUF - 1>();
-        __syncwarp();
-        const bool unit_end = t + 1 >= cw.nst;
-
-        const int iy = y0 + cw.r;
-        const uint32_t rowbase = (uint32_t)iy * (uint32_t)a.Nx;
-        const uint32_t mykey = rowbase + (uint32_t)(x0 + cw.col);
-        const unsigned char* sb = swarp + (size_t)buf * BUFB + lane * 16;
-        uint32_t scnt = 0;  // particles summed in this stage
-        uint32_t qn = 0;  // particles of this stage that left their cell (KEYS), queued in squeue
-#pragma unroll
-        for (int h = 0; h < QL; ++h) {
-            const uint32_t qd = cw.q0 + t * QL + (uint32_t)h;
-            const bool qok = qd < cw.q1;
-            if (KEYS || qok) {
-                Quad<S> d;
-                if constexpr (KEYS) d.cell = qok ? *reinterpret_cast<const uint4*>(sb + h * 512) : make_uint4(0, 0, 0, 0);
-                d.xr = *reinterpret_cast<const float4*>(sb + (FX * QL + h) * 512);
-                d.yr = *reinterpret_cast<const float4*>(sb + ((FX + 1) * QL + h) * 512);
-                if constexpr (QC)
-                    d.q = make_float4(a.qc, a.qc, a.qc, a.qc);
-                else
-                    d.q = *reinterpret_cast<const float4*>(sb + (FQ * QL + h) * 512);
-                if constexpr (S == S_ESK) {
-                    d.vx = *reinterpret_cast<const float4*>(sb + (FV * QL + h) * 512);
-                    d.vy = *reinterpret_cast<const float4*>(sb + ((FV + 1) * QL + h) * 512);
-                }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint32_t p = 4u * qd + (uint32_t)k;
-                    bool valid = qok && p - cw.beg < cw.end - cw.beg;
-                    if constexpr (KEYS) {
-                        // a particle that left its cell since the last sort is queued and
-                        // deposited after the stage by all lanes together (no divergent path)
-                        const bool stale = valid && u4(d.cell, k) != mykey;
-                        const unsigned sb_mask = __ballot_sync(FULL, stale);
-                        if (sb_mask) {
-                            if (stale) squeue[qn + __popc(sb_mask & ((1u << lane) - 1u))] = p;
-                            qn += __popc(sb_mask);
-                            valid = valid && !stale;
-                        }
-                    }
-                    if (valid) {
-                        float vxx = 0.0f, vyy = 0.0f;
-                        if constexpr (S == S_ESK) {
-                            vxx = f4(d.vx, k);
-                            vyy = f4(d.vy, k);
-                        }
-                        if constexpr (TSCI || (S == S_NGP && QC)) {
-                            run.add(f4(d.xr, k), f4(d.yr, k));
-                        } else if constexpr (S == S_TSC) {
-                            tsc_accumulate(f4(d.xr, k), f4(d.yr, k), f4(d.q, k), run.v);
-                        } else {
-                            int iv[V];
-                            if (!stencil_values<S>(a, f4(d.xr, k), f4(d.yr, k), f4(d.q, k), vxx, vyy,
-                                                   (int)(mykey - rowbase), iy, p, iv))
-                                continue;  // deposited by the general trajectory path
-#pragma unroll
-                            for (int q = 0; q < NV; ++q) run.v[q] += (uint32_t)iv[q];
-                        }
-                        ++scnt;
-                    }
-                }
-                run.end_quad();
-            }
+    auto drain = [&](unsigned i) {  // one queued particle, read again (from L2: it has just been staged)
+        const uint32_t p = squeue[i];
+        const uint32_t key = a.cell[p];
+        const float rx = a.xr[p], ry = a.yr[p], q = QC ? a.qc : a.q[p];
+        float vxx = 0.0f, vyy = 0.0f;
+        if constexpr (S == S_ESK) {
+            vxx = a.vx[p];
+            vyy = a.vy[p];
         }
-        if constexpr (KEYS) {
-            moved += qn;
-            if (qn) {  // the stage's particles that left their cell, one per lane
-                __syncwarp();
-                for (uint32_t i = (uint32_t)lane; i < qn; i += 32) {
-                    const uint32_t p = squeue[i];
+        if constexpr (PAD > 0) {
+            if (!dense && stale_to_tile<S, QC>(a, key, rx, ry, q, x0, y0, tw, th, SW, slo, shi)) return;
+        }
+        stale_to_global<S, QC>(a, key, rx, ry, q, vxx, vyy, p);
+    };
+    for (walk.start(cw, warp); !walk.done(cw); walk.advance(cw)) {
+        walk.stage(cw, lane);
+        const uint32_t* sb = sbuf;
+        // the lane's share of its cell, walked four particles at a time and cyclically
+        // from a group that differs from cell to cell (cells of equal size would meet
+        // in the same bank)
+        const int cl = lane >> a.klog, iy = y0 + cw.r, col = cw.c0 + cl;
+        const uint32_t mykey = (uint32_t)iy * (uint32_t)a.Nx + (uint32_t)(x0 + col);
+        int m, first;
+        uint32_t ncell;
+        walk.share(cw, lane, first, m, ncell);
+        // CIC with one charge: 32-bit sums are enough for a whole cell of the unit
+        const bool small = S == S_CIC && QC && __all_sync(FULL, ncell <= 127u);
+        const uint32_t fold_at = small ? 0xffffffffu : (uint32_t)(FOLD - UN + 1);
+        uint32_t part = 0;  // particles since the last fold
+        auto sum_one = [&](float rx, float ry, int i) {
+            if constexpr (QC && S != S_ESK) {
+                run.add(rx, ry);
+            } else {
+                const float q = QC ? a.qc : __uint_as_float(sb[FQ * cap + i]);
+                if constexpr (S == S_TSC) {
+                    tsc_accumulate(rx, ry, q, run.v);
+                } else {
                     float vxx = 0.0f, vyy = 0.0f;
                     if constexpr (S == S_ESK) {
-                        vxx = a.vx[p];
-                        vyy = a.vy[p];
+                        vxx = __uint_as_float(sb[FV * cap + i]);
+                        vyy = __uint_as_float(sb[(FV + 1) * cap + i]);
                     }
-                    const uint32_t key = a.cell[p];
-                    const float rx = a.xr[p], ry = a.yr[p], qn = QC ? a.qc : a.q[p];
-                    if constexpr (PAD > 0) {
-                        if (!dense && stale_to_tile<S, QC>(a, key, rx, ry, qn, x0, y0, tw, th, SW, slo, shi)) continue;
-                    }
-                    stale_to_global<S, QC>(a, key, rx, ry, qn, vxx, vyy, p);
+                    int iv[V];
+                    if (!stencil_values<S>(a, rx, ry, q, vxx, vyy, x0 + col, iy, cw.pos + (uint32_t)i, iv))
+                        return;  // deposited by the general trajectory path
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) run.v[k] += (uint32_t)iv[k];
                 }
-                __syncwarp();
+            }
+            ++part;
+        };
+        auto fold = [&]() {
+            run.fold(part);
+            cnt += part;
+            part = 0;
+        };
+        if constexpr (!KEYS) {
+            const int ng = m / UN;  // whole groups; the rest after them
+            int g = cl < ng ? cl : 0;
+            for (int t = 0; t < ng; ++t) {
+                const int i = first + g * UN;
+                float rx[UN], ry[UN];
+#pragma unroll
+                for (int k = 0; k < UN; ++k) {
+                    rx[k] = __uint_as_float(sb[FX * cap + i + k]);
+                    ry[k] = __uint_as_float(sb[(FX + 1) * cap + i + k]);
+                }
+#pragma unroll
+                for (int k = 0; k < UN; ++k) sum_one(rx[k], ry[k], i + k);
+                run.end_quad();
+                if (part >= fold_at) fold();
+                g = g + 1 == ng ? 0 : g + 1;
+            }
+            for (int i = first + ng * UN; i < first + m; ++i)
+                sum_one(__uint_as_float(sb[FX * cap + i]), __uint_as_float(sb[(FX + 1) * cap + i]), i);
+            run.end_quad();
+        } else {
+            // warp-uniform trips: particles that left their cell since the last sort
+            // are queued, and deposited 32 at a time by all lanes together
+            const int ng = (m + UN - 1) / UN;
+            const int trips = __reduce_max_sync(FULL, ng);
+            int g = cl < ng ? cl : 0;
+            for (int t = 0; t < trips; ++t) {
+                const int left = t < ng ? m - g * UN : 0;  // particles of this group
+                const int i = first + g * UN;
+                float rx[UN], ry[UN];
+                bool stale[UN], any = false;
+#pragma unroll
+                for (int k = 0; k < UN; ++k) {
+                    stale[k] = false;
+                    if (k < left) {
+                        stale[k] = sb[i + k] != mykey;
+                        rx[k] = __uint_as_float(sb[FX * cap + i + k]);
+                        ry[k] = __uint_as_float(sb[(FX + 1) * cap + i + k]);
+                    }
+                    any |= stale[k];
+                }
+                if (__any_sync(FULL, any)) {
+#pragma unroll
+                    for (int k = 0; k < UN; ++k) {
+                        const unsigned sm = __ballot_sync(FULL, stale[k]);
+                        if (stale[k]) squeue[qn + __popc(sm & ((1u << lane) - 1u))] = cw.pos + (uint32_t)(i + k);
+                        qn += __popc(sm);
+                        moved += __popc(sm);
+                    }
+                    __syncwarp();
+                    while (qn >= 32) {
+                        qn -= 32;
+                        drain(qn + lane);
+                        __syncwarp();
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < UN; ++k)
+                    if (k < left && !stale[k]) sum_one(rx[k], ry[k], i + k);
+                run.end_quad();
+                if (part >= fold_at) fold();
+                g = g + 1 >= ng ? 0 : g + 1;
             }
         }
-        run.end_stage(scnt, (t + 1u) % FOLD == 0u);
-        cnt += scnt;
-        if (unit_end) {  // the end of the unit: write out this lane's cell
-            if (cnt) {
-                long long tv[NV];
-                run.finish();
-                run.totals(cnt, tv);
-                if (dense) {
-                    flush_global_ll<NX, LO, NV>(a, mykey, tv);
-                } else {
-                    const int lx = cw.col + 1 + LO + PAD;
-                    const int lrow = cw.r + 1 + LO + PAD;
+        if constexpr (S == S_CIC && QC) {
+            if (small && !walk.last(cw)) {
+                cnt += part;
+            } else if (small) {
+                // the cell's sums over its lanes; then a lane writes one node (of 4 / K), all
+                // in 32 bits: a node of at most 127 particles is below 2^31
+                cnt += part;
+                const int K = 1 << a.klog;
+                for (int o = 1; o < K; o <<= 1) {
+                    run.r += __shfl_xor_sync(FULL, run.r, o);
+                    run.c += __shfl_xor_sync(FULL, run.c, o);
+                    run.d += __shfl_xor_sync(FULL, run.d, o);
+                    cnt += __shfl_xor_sync(FULL, cnt, o);
+                }
+                const uint32_t h = cnt << 23;
+                const int v = (int)(((uint32_t)run.r + (uint32_t)run.c + (uint32_t)run.d + h) >> 1);
+                if (cnt) {
+                    for (int q = lane & (K - 1); q < 4; q += K) {
+                        const int other = q == 1 ? run.r : q == 2 ? run.c : run.d;
+                        const int x = run.sgn * (q == 0 ? v : other + (int)h - v);
+                        if (dense) {
+                            const size_t g = (size_t)wrap_i(iy + (q >> 1), a.Ny) * a.Nx + wrap_i(x0 + col + (q & 1), a.Nx);
+                            atomicAdd(a.acc + g, (unsigned long long)(long long)x);
+                        } else {
+                            const int i = (cw.r + 1 + PAD + (q >> 1)) * SW + col + 1 + PAD + (q & 1);
+                            atomicAdd(slo + i, (uint32_t)x & ((1u << TILE_SPLIT) - 1u));
+                            atomicAdd(shi + i, x >> TILE_SPLIT);
+                        }
+                    }
+                }
+                part = 0;
+                cnt = 0;
+                run.zero();
+            } else {
+                fold();
+            }
+        } else {
+            fold();
+        }
+        if (walk.last(cw) && !small) {  // the end of the unit: write out this lane's cell
+            long long tv[NV];
+            run.totals(cnt, tv);
+            int base = 0, keep = NV;  // the lane writes tv[0 .. keep), nodes base ..
+            bool write = cnt != 0;
+            if constexpr ((NV & (NV - 1)) == 0) {
+                // the K lanes of a cell would add to the same nodes: halve the nodes a
+                // lane keeps for each lane it shares the cell with, exchanging the
+                // other half, until it has one; further lanes just add
+                int b = 0;
 #pragma unroll
-                    for (int q = 0; q < NV; ++q) {
-                        const long long x = tv[q];
-                        if (x != 0) {
-                            const int i = (lrow + q / NX) * SW + lx + (q % NX);
+                for (int half = NV / 2; half >= 1; half /= 2) {
+                    if (b < a.klog) {
+                        const bool up = (lane >> b) & 1;
+#pragma unroll
+                        for (int q = 0; q < half; ++q) {
+                            const long long give = up ? tv[q] : tv[half + q];
+                            tv[q] = (up ? tv[half + q] : tv[q]) + __shfl_xor_sync(FULL, give, 1 << b);
+                        }
+                        base += up ? half : 0;
+                        keep = half;
+                        ++b;
+                    }
+                }
+                for (; b < a.klog; ++b) {
+                    tv[0] += __shfl_xor_sync(FULL, tv[0], 1 << b);
+                    if ((lane >> b) & 1) base = -1;
+                }
+                write = base >= 0 && cl < cw.cn;
+            }
+            if (write) {
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    const long long x = tv[k];
+                    if (k < keep && x != 0) {
+                        const int q = base + k;
+                        if (dense) {
+                            const size_t g = (size_t)wrap_i(iy + LO + q / NX, a.Ny) * a.Nx + wrap_i(x0 + col + LO + q % NX, a.Nx);
+                            atomicAdd(a.acc + g, (unsigned long long)x);
+                        } else {
+                            const int i = (cw.r + 1 + LO + PAD + q / NX) * SW + col + 1 + LO + PAD + q % NX;
                             atomicAdd(slo + i, (uint32_t)x & ((1u << TILE_SPLIT) - 1u));
                             atomicAdd(shi + i, (int)(x >> TILE_SPLIT));
                         }
@@ -1446,16 +1508,9 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
             cnt = 0;
         }
         __syncwarp();
-        if (unit_end) {
-            t = 0;
-            u = next_unit(u + NW, cw);
-        } else {
-            ++t;
-        }
-        buf = buf + 1 == NBUF ? 0 : buf + 1;
     }
-    cp_async_wait<0>();
     if constexpr (KEYS) {
+        if ((unsigned)lane < qn) drain((unsigned)lane);
         if (lane == 0 && moved) {
             atomicAdd(&a.st->moved, (unsigned long long)moved);
             atomicAdd(&a.st->moved_dep, (unsigned long long)moved);
@@ -1473,6 +1528,124 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
             atomicAdd(a.acc + (size_t)gy * a.Nx + gx, (unsigned long long)v);
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Trajectory-averaged charge of freshly sorted particles with one charge
+// (PIC_SCHEME_ESIRKEPOV), light path. A particle that moves and stays in its
+// cell on both axes deposits all its A units on its own cell's node
+// (ngp.cpp:36-84: the whole path lies in one cell), so these particles are
+// counted and not summed: the grid starts as A times the cells' counts, which
+// the sort's offsets hold (esk_base), and esk_light streams the particles once
+// with coalesced 16-byte loads, only testing. The others are queued per warp
+// (ballot compaction) and, 32 at a time, deposit their stencil minus the A
+// units already counted straight to the global int64 grid. The sums are the
+// same integers as deposit_cells'. Bound by memory when few particles cross a
+// cell boundary in the move (16 bytes per particle, read once); every one that
+// does costs a few int64 atomics, so a sample decides on the device between this
+// path and deposit_cells (esk_sample), and the one not chosen returns at once.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool esk_stays(float r, float v, float dtf, float dtd) {
+    if (fabsf(v * dtf) < 1e-15f) return false;  // static: CIC weights
+    const float dc = v * dtd;
+    if (!(fabsf(dc) < 1.0f)) return false;
+    const float e = r + dc;
+    return dc > 0.0f ? !(e > 1.0f) : !(e < 0.0f);
+}
+
+constexpr int ESK_SAMPLES = 4096;
+// The light path when fewer than half of the sample leave their cell: at 1024^2 x 64
+// it takes 0.29 ms when 2 % do and about 0.6 ms at 22 %; deposit_cells takes the
+// same at any fraction.
+constexpr unsigned ESK_LIGHT_DENOM = 2;
+
+__global__ void __launch_bounds__(1024) esk_sample(DepArgs a) {
+    __shared__ unsigned s_cross;
+    if (threadIdx.x == 0) s_cross = 0;
+    __syncthreads();
+    const unsigned m = a.n < (size_t)ESK_SAMPLES ? (unsigned)a.n : (unsigned)ESK_SAMPLES;
+    unsigned cross = 0;
+    for (unsigned i = threadIdx.x; i < m; i += 1024) {
+        const size_t p = (size_t)i * (a.n / m);
+        cross += esk_stays(a.xr[p], a.vx[p], a.dtf, a.dtdx) && esk_stays(a.yr[p], a.vy[p], a.dtf, a.dtdy) ? 0u : 1u;
+    }
+    cross = __reduce_add_sync(FULL, cross);
+    if ((threadIdx.x & 31) == 0 && cross) atomicAdd(&s_cross, cross);
+    __syncthreads();
+    if (threadIdx.x == 0) a.st->esk_light = s_cross * ESK_LIGHT_DENOM < m ? 1u : 0u;
+}
+
+// The grid's start: A units per particle of the cell (light path), else zero.
+__global__ void esk_base(DepArgs a, size_t g) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g) return;
+    const long long A = __float2int_rn(a.qc * 16777216.0f);
+    a.acc[i] = a.st->esk_light ? (unsigned long long)(A * (long long)(a.offsets[i + 1] - a.offsets[i])) : 0ull;
+}
+
+constexpr int ESK_QUEUE = 32 + 128;  // left over (below 32) and one step's particles
+
+__global__ void __launch_bounds__(DEP_THREADS) esk_light(DepArgs a) {
+    if (gated_off(a)) return;
+    // the queue holds the particles' values: reading them again took half as many
+    // bytes as the stream itself (32-byte sectors of five arrays per particle)
+    __shared__ uint32_t squeue[DEP_WARPS][ESK_QUEUE];
+    __shared__ float4 sqval[DEP_WARPS][ESK_QUEUE];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t* queue = squeue[warp];
+    float4* qval = sqval[warp];
+    unsigned qn = 0;
+    const uint32_t G = (uint32_t)a.Nx * (uint32_t)a.Ny;
+    const int A = __float2int_rn(a.qc * 16777216.0f);
+    auto deposit = [&](unsigned i) {
+        const uint32_t p = queue[i];
+        const uint32_t key = a.cell[p];
+        if (key >= G) return;  // not in any cell's count either
+        const int iy = (int)(key / (uint32_t)a.Nx), ix = (int)(key - (uint32_t)iy * (uint32_t)a.Nx);
+        int val[Frame<S_ESK>::V];
+        const float4 v = qval[i];
+        stencil_values<S_ESK>(a, v.x, v.y, a.qc, v.z, v.w, ix, iy, p, val);
+        val[4] -= A;  // a move of a cell or more has deposited itself: val is all zero
+        int v9[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v9[k] = val[k];
+        flush_global<S_ESK>(a, key, v9);
+    };
+    const size_t nq = (a.n + 3) / 4, stride = (size_t)gridDim.x * DEP_THREADS;
+    // warp-uniform loop over quads of particles (holding the next quads in registers
+    // as well spilled, and was slower)
+    for (size_t q0 = (size_t)blockIdx.x * DEP_THREADS + warp * 32; q0 < nq; q0 += stride) {
+        const size_t qi = q0 + lane;
+        float4 x = make_float4(0, 0, 0, 0), y = x, u = x, w = x;
+        if (qi < nq) {
+            x = __ldcs(reinterpret_cast<const float4*>(a.xr) + qi);
+            y = __ldcs(reinterpret_cast<const float4*>(a.yr) + qi);
+            u = __ldcs(reinterpret_cast<const float4*>(a.vx) + qi);
+            w = __ldcs(reinterpret_cast<const float4*>(a.vy) + qi);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const size_t p = qi * 4 + k;
+            const bool leaves = p < a.n && !(esk_stays(f4(x, k), f4(u, k), a.dtf, a.dtdx) &&
+                                             esk_stays(f4(y, k), f4(w, k), a.dtf, a.dtdy));
+            const unsigned m = __ballot_sync(FULL, leaves);
+            if (m) {
+                if (leaves) {
+                    const unsigned at = qn + __popc(m & ((1u << lane) - 1u));
+                    queue[at] = (uint32_t)p;
+                    qval[at] = make_float4(f4(x, k), f4(y, k), f4(u, k), f4(w, k));
+                }
+                qn += __popc(m);
+            }
+        }
+        __syncwarp();
+        while (qn >= 32) {
+            deposit(qn - 32 + lane);
+            qn -= 32;
+            __syncwarp();
+        }
+    }
+    if ((unsigned)lane < qn) deposit(lane);
 }
 
 // After a deposit between sorts whose kernel was chosen on the device: once the
@@ -1517,24 +1690,24 @@ __global__ void fixed_to_rho(const long long* __restrict__ acc, size_t g, double
     }
 }
 
-#ifndef CELLS_LPP
-#define CELLS_LPP 8
-#endif
+constexpr int CELLS_NW = 4, CELLS_MINB = 4;  // warps of a CTA, CTAs per SM the registers allow
 
-#ifndef CELLS_NBUF
-#define CELLS_NBUF 2
-#endif
-template <int S, int LPP, int NW, int MINB, bool QC, bool KEYS>
-static int launch_cells(pic_ctx* c, const DepArgs& a, unsigned tiles) {
-    constexpr int NBUF = CELLS_NBUF;
+template <int S, bool QC, bool KEYS>
+static int launch_cells(pic_ctx* c, DepArgs a, unsigned tiles) {
+    constexpr int NW = CELLS_NW, MINB = CELLS_MINB;
     constexpr int PAD = (KEYS && S != S_ESK) ? 1 : 0;  // the kernel's extra halo between sorts
-    const size_t smem = cells_fixed_bytes<S, LPP, NW, QC, KEYS, NBUF>() +
+    // TSC and the trajectory scheme keep four CTAs per SM by their registers: room for
+    // larger units. 1024^2 x 64, one charge, us per call with 1,040 / 2,080 / 3,120
+    // words: CIC 242 / 222 / 221, NGP 202 / 198 / 199, TSC 334 / 285 / 285; a TSC time
+    // step at 100 per cell 2.46 / 2.25 / 2.15 ms, a CIC one at 64 0.46 / 0.44 / 0.45.
+    constexpr int WORDS = S == S_TSC || S == S_ESK ? 3120 : 2080;
+    cells_shape(a.n, c->G, StageFields<S, QC>::NF - (KEYS ? 0 : 1), WORDS, &a.klog, &a.cap);
+    const size_t smem = cells_fixed_bytes<S, NW, QC, KEYS>(a.cap) +
                         (size_t)(a.tile_h + 3 + 2 * PAD) * (a.tile_w + 3 + 2 * PAD) * 2 * sizeof(uint32_t) +
-                        (size_t)a.tile_h * (a.tile_w + 1) * sizeof(uint32_t) +
-                        (KEYS ? (size_t)NW * 32 * LPP * sizeof(uint32_t) : 0);
-    const int rc = opt_in_dynamic_smem((const void*)deposit_cells<S, LPP, NW, MINB, QC, KEYS, NBUF>, smem);
+                        (size_t)a.tile_h * (a.tile_w + 1) * sizeof(uint32_t);
+    const int rc = opt_in_dynamic_smem((const void*)deposit_cells<S, NW, MINB, QC, KEYS>, smem);
     if (rc != PIC_OK) return rc;
-    deposit_cells<S, LPP, NW, MINB, QC, KEYS, NBUF><<<tiles, NW * 32, smem, c->stream>>>(a);
+    deposit_cells<S, NW, MINB, QC, KEYS><<<tiles, NW * 32, smem, c->stream>>>(a);
     return PIC_OK;
 }
 
@@ -1573,29 +1746,50 @@ static int launch_deposit(pic_ctx* c, const DepArgs& a, int kind, bool adaptive)
         ar.gate_when = 1;
         const unsigned tiles = (unsigned)(a.tiles_x * ((c->Ny + a.tile_h - 1) / a.tile_h));
         prof_begin(c, "deposit");
-        int rc = a.qc != 0.0f ? launch_cells<S, CELLS_LPP, 4, 4, true, true>(c, ak, tiles)
-                              : launch_cells<S, CELLS_LPP, 4, 4, false, true>(c, ak, tiles);
+        int rc = a.qc != 0.0f ? launch_cells<S, true, true>(c, ak, tiles)
+                              : launch_cells<S, false, true>(c, ak, tiles);
         if (rc == PIC_OK) rc = check_launch(c, "deposit_cells");
         if (rc == PIC_OK) rc = launch_runs<S>(c, ar);  // fixed_to_rho takes the decision for the next deposit
         prof_end(c);
         return rc;
     }
+    if constexpr (S == S_ESK) {
+        if (kind == 0 && c->sorted && a.qc != 0.0f) {
+            // one charge, freshly sorted: the light path or the cell kernel, chosen on the device
+            DepArgs al = a, ac = a;
+            al.gate = ac.gate = &c->dstats->esk_light;
+            al.gate_when = 1;
+            ac.gate_when = 0;
+            const unsigned tiles = (unsigned)(a.tiles_x * ((c->Ny + a.tile_h - 1) / a.tile_h));
+            int sms = 148;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+            size_t blocks = (a.n + DEP_THREADS * 4 - 1) / (DEP_THREADS * 4);
+            if (blocks > (size_t)sms * 8) blocks = (size_t)sms * 8;
+            esk_sample<<<1, 1024, 0, c->stream>>>(a);
+            PIC_TRY(check_launch(c, "esk_sample"));
+            esk_base<<<(unsigned)((c->G + 255) / 256), 256, 0, c->stream>>>(a, c->G);
+            PIC_TRY(check_launch(c, "esk_base"));
+            prof_begin(c, "deposit");
+            esk_light<<<(unsigned)blocks, DEP_THREADS, 0, c->stream>>>(al);
+            int rc = check_launch(c, "esk_light");
+            if (rc == PIC_OK) rc = launch_cells<S, true, false>(c, ac, tiles);
+            prof_end(c);
+            PIC_TRY(rc);
+            return check_launch(c, "deposit_cells");
+        }
+    }
     if (kind == 0) {
         const unsigned tiles = (unsigned)(a.tiles_x * ((c->Ny + a.tile_h - 1) / a.tile_h));
         prof_begin(c, "deposit");
-        // 8 particles per lane and stage, 4 warps per tile; TSC capped at 96
-        // registers (5 CTAs per SM), measured fastest at 1024^2 x 64 particles/cell.
-        // cp.async staging measured 10 % faster than TMA tensor copies of the
-        // same stages (128-byte swizzle, one lane issuing, mbarrier completion)
         // freshly sorted: the offsets name every particle's cell and the keys are not read
         const bool keys = !c->sorted;
         int rc;
         if (a.qc != 0.0f) {  // one charge for all particles: the charge stream is not staged
-            rc = keys ? launch_cells<S, CELLS_LPP, 4, 4, true, true>(c, a, tiles)
-                      : launch_cells<S, CELLS_LPP, 4, 4, true, false>(c, a, tiles);
+            rc = keys ? launch_cells<S, true, true>(c, a, tiles)
+                      : launch_cells<S, true, false>(c, a, tiles);
         } else {
-            rc = keys ? launch_cells<S, CELLS_LPP, 4, 4, false, true>(c, a, tiles)
-                      : launch_cells<S, CELLS_LPP, 4, 4, false, false>(c, a, tiles);
+            rc = keys ? launch_cells<S, false, true>(c, a, tiles)
+                      : launch_cells<S, false, false>(c, a, tiles);
         }
         prof_end(c);
         if (rc != PIC_OK) return rc;

@@ -26,6 +26,7 @@ struct DevStats {
     float q_first;              // uploads: the first particle's stored charge
     float q_raw0;               // uploads: the first particle's charge before normalisation
     unsigned int any_order;     // between sorts: 1 once most particles have left their sorted cell
+    unsigned int esk_light;     // trajectory charge: 1 when few sampled particles leave their cell in the move
     unsigned long long moved;   // deposits between sorts: particles found outside their sorted cell
     unsigned long long moved_dep;  // the same, for the any_order decision after each deposit
 };
@@ -336,6 +337,34 @@ __device__ __forceinline__ bool cell_coord(double x, double d, double inv_d, int
     *idx = wrap_i(i, n);
     *off = r;
     return true;
+}
+
+// Integer CIC charges of one particle of A = 2^24 units (one charge for every
+// particle; a negative charge is the exact mirror image) at cell offsets x, y,
+// as the general form rounds them: each node rint((A*Y[j])*X[i]), the node of
+// largest weight takes A minus the others. Given as three sums that determine
+// the four nodes, each minus A/2: row 0, column 0 and the diagonal (0,0) + (1,1).
+//  * Only the three smaller node values are rounded. They are at most A/2, so the
+//    FP32 sum of the unscaled product (the scaled one's bits but for the exponent)
+//    and 0.5 lies in [0.5, 1], where floats are 2^-24 apart: its mantissa is the
+//    rounded value, and no float-to-integer conversion is needed.
+//  * With p, q, s the values of the largest node's row mate, its column mate and
+//    the opposite node, row 0 is q + s or A minus that, by the largest node's row;
+//    less A/2 the two are each other's negative, and likewise column 0 (p + s) and
+//    the diagonal (p + q): a sign each, no selects.
+//  * 1 - min(w, 1 - w) is the larger weight exactly as max(w, 1 - w) is: above
+//    1/2 the difference 1 - w is exact.
+__device__ __forceinline__ void cic_unit(float x, float y, int& row0, int& col0, int& diag) {
+    constexpr int BIAS = 2 * 0x3F000000 + (1 << 23);  // twice the bits of 0.5f, and A/2
+    const float xs = fminf(x, 1.0f - x), ys = fminf(y, 1.0f - y);
+    const float xb = 1.0f - xs, yb = 1.0f - ys;
+    const int sx = x > 0.5f ? 1 : -1, sy = y > 0.5f ? 1 : -1;  // + : the largest node is in column / row 1
+    const int p = __float_as_int(yb * xs + 0.5f);
+    const int q = __float_as_int(ys * xb + 0.5f);
+    const int s = __float_as_int(ys * xs + 0.5f);
+    row0 = sy * (q + s - BIAS);
+    col0 = sx * (p + s - BIAS);
+    diag = -sx * sy * (p + q - BIAS);
 }
 
 // One unit of the int64 charge grid: max|q| * inv_vol * 2^-24 (FP64). The

@@ -18,7 +18,8 @@
 // segmented warp scan, one int64 atomic per run of equal cells), a barrier,
 // phase 3 turns the int64 grid into rho (+ background) and clears it. The
 // Poisson solves are one batched cuFFT plan per grid size (runs sorted by
-// size, so equal sizes are contiguous) plus two small kernels. With use_graph
+// size, so equal sizes are contiguous) plus two small kernels, the sizes on
+// streams of their own. With use_graph
 // the whole step is one CUDA graph. Steps with a cell sort run the move, the
 // sort, a tiled deposit and the conversion as separate launches; the tiled
 // deposit's tile shape per (grid size, particles per cell) class is picked by
@@ -554,61 +555,57 @@ __global__ void ens_init_run(InitArgs a) {
     a.q[p] = -1.0f;
 }
 
-// fields.cu k_divide for a batch of equal-size runs: spec /= k^2 (continuous k,
-// L = N), DC = 0.
-__global__ void ens_k_divide(cufftDoubleComplex* __restrict__ spec, int N, int count) {
+// k^2 of every frequency of an N x N run (continuous k, L = N), once per grid size:
+// the solve then divides by it (two FP64 divisions an element instead of four).
+__global__ void ens_make_k2(double* __restrict__ k2, int N) {
     const int nh = N / 2 + 1;
-    const size_t per = (size_t)nh * N;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= per * count) return;
-    const size_t s = t % per;
-    const int i = (int)(s % nh), j = (int)(s / nh);
-    if (i == 0 && j == 0) {
-        spec[t].x = 0.0;
-        spec[t].y = 0.0;
-        return;
-    }
+    if (t >= (size_t)nh * N) return;
+    const int i = (int)(t % nh), j = (int)(t / nh);
     const double twopi = 2.0 * 3.14159265358979323846;
     const int mx = (i <= N / 2) ? i : i - N;
     const int my = (j <= N / 2) ? j : j - N;
     const double L = (double)N;
     const double kx = __ddiv_rn(__dmul_rn(twopi, (double)mx), L);
     const double ky = __ddiv_rn(__dmul_rn(twopi, (double)my), L);
-    const double k2 = __dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky));
-    spec[t].x = __ddiv_rn(spec[t].x, k2);
-    spec[t].y = __ddiv_rn(spec[t].y, k2);
+    k2[t] = __dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky));
 }
 
-// rhs = rho * dV (dV = 1) for the batch's cells
-__global__ void ens_copy_rhs(const double* __restrict__ rho, size_t n, double* __restrict__ rhs) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) rhs[i] = __dmul_rn(rho[i], 1.0);
-}
-
-// phi *= 1/G_run, then E = forward difference (fields.cu scale_phi + efield), per run
-__global__ void ens_scale_efield(const RunDesc* __restrict__ runs, int nruns, uint32_t G, double* __restrict__ phi,
-                                 double* __restrict__ Ex, double* __restrict__ Ey, float* __restrict__ Exf,
-                                 float* __restrict__ Eyf, int phase) {
-    __shared__ uint32_t cbase[MAX_RUNS];
-    for (int i = threadIdx.x; i < nruns; i += blockDim.x) cbase[i] = runs[i].cell_base;
-    __syncthreads();
-    const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    const RunDesc& r = runs[find_run(cbase, nruns, (uint32_t)g)];
-    if (phase == 0) {
-        phi[g] = __dmul_rn(phi[g], 1.0 / (double)r.cells);
-        return;
+// spec /= k^2, DC = 0, for a batch of equal-size runs (blockIdx.y: the run)
+__global__ void ens_k_divide(cufftDoubleComplex* __restrict__ spec, const double* __restrict__ k2, size_t per) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= per) return;
+    cufftDoubleComplex* p = spec + blockIdx.y * per + t;
+    cufftDoubleComplex v = *p;
+    if (t == 0) {
+        v.x = v.y = 0.0;
+    } else {
+        const double k = k2[t];
+        v.x = __ddiv_rn(v.x, k);
+        v.y = __ddiv_rn(v.y, k);
     }
-    const uint32_t local = (uint32_t)g - r.cell_base;
-    const int j = (int)(local / (uint32_t)r.N), i = (int)(local - (uint32_t)j * (uint32_t)r.N);
-    const int ip = (i + 1) % r.N, jp = (j + 1) % r.N;
-    const double p = phi[g];
-    const double ex = -__dmul_rn(__dsub_rn(phi[r.cell_base + (size_t)j * r.N + ip], p), 1.0);
-    const double ey = -__dmul_rn(__dsub_rn(phi[r.cell_base + (size_t)jp * r.N + i], p), 1.0);
-    Ex[g] = ex;
-    Ey[g] = ey;
-    Exf[g] = __double2float_rn(ex);
-    Eyf[g] = __double2float_rn(ey);
+    *p = v;
+}
+
+// phi = raw / N^2 and E = its forward difference (fields.cu efield), for a batch of
+// equal-size runs whose inverse transforms are in raw (blockIdx.y: the run): one
+// pass, since raw and phi are different arrays.
+__global__ void ens_efield(const double* __restrict__ raw, int N, double norm, double* __restrict__ phi,
+                           double* __restrict__ Ex, double* __restrict__ Ey, float* __restrict__ Exf,
+                           float* __restrict__ Eyf) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, cells = (unsigned)N * (unsigned)N;
+    if (t >= cells) return;
+    const size_t b = (size_t)blockIdx.y * cells;
+    const unsigned j = t / (unsigned)N, i = t - j * (unsigned)N;
+    const unsigned xp = i + 1 == (unsigned)N ? t - i : t + 1, yp = j + 1 == (unsigned)N ? i : t + N;
+    const double p = __dmul_rn(raw[b + t], norm);
+    const double ex = -__dmul_rn(__dsub_rn(__dmul_rn(raw[b + xp], norm), p), 1.0);
+    const double ey = -__dmul_rn(__dsub_rn(__dmul_rn(raw[b + yp], norm), p), 1.0);
+    phi[b + t] = p;
+    Ex[b + t] = ex;
+    Ey[b + t] = ey;
+    Exf[b + t] = __double2float_rn(ex);
+    Eyf[b + t] = __double2float_rn(ey);
 }
 
 // Per-run energies of the step into hist[step*nruns + r]: field energy
@@ -759,10 +756,15 @@ struct pic_ens {
         uint32_t cell_base;
         cufftHandle fwd, inv;
         cufftDoubleComplex* spec;
-        double* rhs;
+        double* raw;          // inverse transforms before the 1/N^2
+        double* k2;           // ens_make_k2
+        cudaStream_t stream;  // its solves run beside the other sizes' (the first: the ensemble's stream)
+        cudaEvent_t done;
     };
     std::vector<Batch> batches;
-    double* rhs_all = nullptr;
+    cudaEvent_t rho_ready = nullptr;
+    double* raw_all = nullptr;
+    double* k2_all = nullptr;
     cufftDoubleComplex* spec_all = nullptr;
     // graphs keyed by the particle buffers
     struct G {
@@ -853,25 +855,29 @@ int upload_runs(pic_ens* e) {
     return PIC_OK;
 }
 
+// The batches (one per grid size) are independent chains of five or so small
+// launches; each runs on its own stream, forked from the ensemble's stream once rho
+// is there and joined to it again (in a captured step: parallel branches).
 int poisson(pic_ens* e) {
     pic_ctx* c = e->c;
+    if (e->batches.size() > 1) PIC_CUDA_TRY(cudaEventRecord(e->rho_ready, c->stream));
     for (auto& b : e->batches) {
-        const size_t cells = (size_t)b.count * b.N * b.N;
-        ens_copy_rhs<<<(unsigned)((cells + 255) / 256), 256, 0, c->stream>>>(c->rho + b.cell_base, cells, b.rhs);
-        PIC_TRY(check_launch(c, "ens_copy_rhs"));
-        PIC_TRY(ens_fail_cufft(cufftExecD2Z(b.fwd, b.rhs, b.spec), "cufftExecD2Z"));
-        const size_t ns = (size_t)b.count * b.N * (b.N / 2 + 1);
-        ens_k_divide<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>(b.spec, b.N, b.count);
+        if (b.stream != c->stream) PIC_CUDA_TRY(cudaStreamWaitEvent(b.stream, e->rho_ready, 0));
+        const unsigned count = (unsigned)b.count;
+        // the out-of-place real transform leaves rho (dV = 1) as it is
+        PIC_TRY(ens_fail_cufft(cufftExecD2Z(b.fwd, c->rho + b.cell_base, b.spec), "cufftExecD2Z"));
+        const size_t per = (size_t)b.N * (b.N / 2 + 1), cells = (size_t)b.N * b.N;
+        ens_k_divide<<<dim3((unsigned)((per + 255) / 256), count), 256, 0, b.stream>>>(b.spec, b.k2, per);
         PIC_TRY(check_launch(c, "ens_k_divide"));
-        PIC_TRY(ens_fail_cufft(cufftExecZ2D(b.inv, b.spec, c->phi + b.cell_base), "cufftExecZ2D"));
-        c->launches += 2;
-    }
-    const unsigned blocks = (unsigned)((c->G + 255) / 256);
-    for (int phase = 0; phase < 2; ++phase) {
-        ens_scale_efield<<<blocks, 256, 0, c->stream>>>(e->druns, (int)e->runs.size(), (uint32_t)c->G, c->phi, c->Ex,
-                                                        c->Ey, c->Exf, c->Eyf, phase);
-        PIC_TRY(check_launch(c, "ens_scale_efield"));
-        c->launches++;
+        PIC_TRY(ens_fail_cufft(cufftExecZ2D(b.inv, b.spec, b.raw), "cufftExecZ2D"));
+        ens_efield<<<dim3((unsigned)((cells + 255) / 256), count), 256, 0, b.stream>>>(
+            b.raw, b.N, 1.0 / (double)cells, c->phi + b.cell_base, c->Ex + b.cell_base, c->Ey + b.cell_base,
+            c->Exf + b.cell_base, c->Eyf + b.cell_base);
+        PIC_TRY(check_launch(c, "ens_efield"));
+        if (b.stream != c->stream) {
+            PIC_CUDA_TRY(cudaEventRecord(b.done, b.stream));
+            PIC_CUDA_TRY(cudaStreamWaitEvent(c->stream, b.done, 0));
+        }
     }
     return PIC_OK;
 }
@@ -1105,7 +1111,7 @@ int pic_ens_create(const pic_ens_member* runs_in, int nruns, const pic_ens_confi
         c->qn_uniform = -1.0f;
     }
     // batched FFT plans per grid size
-    size_t spec_total = 0;
+    size_t spec_total = 0, k2_total = 0;
     for (int i = 0; i < nruns && out_rc == PIC_OK;) {
         int j = i;
         while (j + 1 < nruns && e->runs[j + 1].N == e->runs[i].N) ++j;
@@ -1122,20 +1128,40 @@ int pic_ens_create(const pic_ens_member* runs_in, int nruns, const pic_ens_confi
             out_rc = fail(PIC_ERR_CUDA, "cufftPlanMany");
             break;
         }
-        cufftSetStream(b.fwd, c->stream);
-        cufftSetStream(b.inv, c->stream);
+        b.stream = c->stream;
+        if (i > 0) {
+            if (cudaStreamCreateWithFlags(&b.stream, cudaStreamNonBlocking) != cudaSuccess) b.stream = c->stream;
+            if (b.stream != c->stream && cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) != cudaSuccess) {
+                cudaStreamDestroy(b.stream);
+                b.stream = c->stream;
+                b.done = nullptr;
+            }
+            (void)cudaGetLastError();
+        }
+        cufftSetStream(b.fwd, b.stream);
+        cufftSetStream(b.inv, b.stream);
         spec_total += (size_t)b.count * b.N * (b.N / 2 + 1);
+        k2_total += (size_t)b.N * (b.N / 2 + 1);
         e->batches.push_back(b);
         i = j + 1;
     }
     if (out_rc == PIC_OK) {
-        e->rhs_all = (double*)A(G * 8);
+        e->raw_all = (double*)A(G * 8);
+        e->k2_all = (double*)A(k2_total * 8);
         e->spec_all = (cufftDoubleComplex*)A(spec_total * sizeof(cufftDoubleComplex));
-        size_t so = 0;
+        if (out_rc == PIC_OK && cudaEventCreateWithFlags(&e->rho_ready, cudaEventDisableTiming) != cudaSuccess)
+            out_rc = fail(PIC_ERR_CUDA, "cudaEventCreate");
+        size_t so = 0, ko = 0;
         for (auto& b : e->batches) {
-            b.rhs = e->rhs_all ? e->rhs_all + b.cell_base : nullptr;
-            b.spec = e->spec_all ? e->spec_all + so : nullptr;
-            so += (size_t)b.count * b.N * (b.N / 2 + 1);
+            if (out_rc != PIC_OK) break;
+            const size_t per = (size_t)b.N * (b.N / 2 + 1);
+            b.raw = e->raw_all + b.cell_base;
+            b.spec = e->spec_all + so;
+            b.k2 = e->k2_all + ko;
+            so += (size_t)b.count * per;
+            ko += per;
+            ens_make_k2<<<(unsigned)((per + 255) / 256), 256, 0, c->stream>>>(b.k2, b.N);
+            out_rc = check_launch(c, "ens_make_k2");
         }
     }
     if (out_rc == PIC_OK) {
@@ -1159,11 +1185,17 @@ int pic_ens_destroy(pic_ens* e) {
     if (e->c) cudaStreamSynchronize(e->c->stream);
     for (auto& g : e->graphs) cudaGraphExecDestroy(g.exec);
     for (auto& b : e->batches) {
+        if (b.stream != e->c->stream) {
+            cudaStreamSynchronize(b.stream);
+            cudaStreamDestroy(b.stream);
+        }
+        if (b.done) cudaEventDestroy(b.done);
         cufftDestroy(b.fwd);
         cufftDestroy(b.inv);
     }
+    if (e->rho_ready) cudaEventDestroy(e->rho_ready);
     void* ptrs[] = {e->druns, e->dmass, e->bar, e->err, e->step_ctr, e->fe_hist, e->ke_hist, e->en_partial,
-                    e->rhs_all, e->spec_all, e->breaks, e->breaks_ring};
+                    e->raw_all, e->k2_all, e->spec_all, e->breaks, e->breaks_ring};
     for (void* p : ptrs) dfree(p);
     if (e->c) pic_gpu_destroy(e->c);
     delete e;

@@ -93,9 +93,9 @@ static void prof_clear(pic_ctx* ctx, const char* name) {
 }
 
 int check_device_status(pic_ctx* ctx) {
-    DevStats st;
-    PIC_CUDA_TRY(cudaMemcpyAsync(&st, ctx->dstats, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+    PIC_CUDA_TRY(cudaMemcpyAsync(ctx->hstats, ctx->dstats, sizeof(DevStats), cudaMemcpyDeviceToHost, ctx->stream));
     PIC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    const DevStats& st = *ctx->hstats;
     if (st.err == DEV_OK) return PIC_OK;
     // clear so that the context stays usable after the caller handles the error
     PIC_CUDA_TRY(cudaMemsetAsync(&ctx->dstats->err, 0, sizeof(int), ctx->stream));
@@ -222,36 +222,46 @@ int exclusive_scan_u32(pic_ctx* ctx, unsigned int* data, size_t n) {
 // upload: FP64 host SoA -> device cell key + FP32 in-cell offsets
 // ---------------------------------------------------------------------------
 struct ConvertArgs {
-    const double *x, *y, *vx, *vy, *q, *m;  // chunk (device staging or pinned host); vx/vy/m may be null
+    const double *x, *y, *vx, *vy, *q, *m;  // chunk (device staging or host memory); vx/vy/m may be null
     size_t count, first;                    // chunk size and global index of its first particle
     double dx, dy;
     double inv_dx, inv_dy;                  // exact reciprocals when dx / dy are powers of two, else 0
     int Nx, Ny;
     uint32_t* cell;
-    float *xr, *yr, *fvx, *fvy, *fq, *fm;
+    float *xr, *yr, *fvx, *fvy, *fq, *fm;   // fm null: masses are only tested against 1
     DevStats* st;
 };
 
-__global__ void convert_particles(ConvertArgs a) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// The maxima go block by block: a warp's sum to shared memory, then one atomic per
+// maximum that the block raises (three per warp on three words kept 1 M particles
+// at 71 us).
+constexpr int CONVERT_THREADS = 256;
+__global__ void __launch_bounds__(CONVERT_THREADS) convert_particles(ConvertArgs a) {
+    __shared__ unsigned s_max[3];
+    if (threadIdx.x < 3) s_max[threadIdx.x] = 0;
+    __syncthreads();
+    const size_t i = (size_t)blockIdx.x * CONVERT_THREADS + threadIdx.x;
     float aq = 0.0f, avx = 0.0f, avy = 0.0f;
+    bool mass = false;
     if (i < a.count) {
+        // all loads first: they may cross the host link
+        const double x = a.x[i], y = a.y[i], q = a.q[i];
+        const double dvx = a.vx ? a.vx[i] : 0.0, dvy = a.vy ? a.vy[i] : 0.0, m = a.m ? a.m[i] : 1.0;
         int ix = 0, iy = 0;
         float rx = 0.0f, ry = 0.0f;
-        const bool okx = cell_coord(a.x[i], a.dx, a.inv_dx, a.Nx, &ix, &rx);
-        const bool oky = cell_coord(a.y[i], a.dy, a.inv_dy, a.Ny, &iy, &ry);
+        const bool okx = cell_coord(x, a.dx, a.inv_dx, a.Nx, &ix, &rx);
+        const bool oky = cell_coord(y, a.dy, a.inv_dy, a.Ny, &iy, &ry);
         if (!(okx && oky)) set_dev_error(a.st, DEV_BAD_POSITION, (unsigned int)(a.first + i));
         const size_t o = a.first + i;
         a.cell[o] = (uint32_t)iy * (uint32_t)a.Nx + (uint32_t)ix;
         a.xr[o] = rx;
         a.yr[o] = ry;
-        const float fvx = a.vx ? __double2float_rn(a.vx[i]) : 0.0f;
-        const float fvy = a.vy ? __double2float_rn(a.vy[i]) : 0.0f;
-        const float fq = __double2float_rn(a.q[i]);
+        const float fvx = __double2float_rn(dvx), fvy = __double2float_rn(dvy), fq = __double2float_rn(q);
         a.fvx[o] = fvx;
         a.fvy[o] = fvy;
         a.fq[o] = fq;
-        if (a.fm) a.fm[o] = a.m ? __double2float_rn(a.m[i]) : 1.0f;
+        if (a.fm) a.fm[o] = __double2float_rn(m);
+        mass = !(m == 1.0);
         if (o == 0) a.st->q_raw0 = fq;
         aq = fabsf(fq);
         avx = fabsf(fvx);
@@ -263,11 +273,22 @@ __global__ void convert_particles(ConvertArgs a) {
         avx = fmaxf(avx, __shfl_xor_sync(0xffffffffu, avx, o));
         avy = fmaxf(avy, __shfl_xor_sync(0xffffffffu, avy, o));
     }
+    if (__any_sync(0xffffffffu, mass) && (threadIdx.x & 31) == 0) a.st->mass_mixed = 1u;
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(&a.st->maxq_bits, __float_as_uint(aq));
-        atomicMax(&a.st->maxvx_bits, __float_as_uint(avx));
-        atomicMax(&a.st->maxvy_bits, __float_as_uint(avy));
+        atomicMax(&s_max[0], __float_as_uint(aq));
+        atomicMax(&s_max[1], __float_as_uint(avx));
+        atomicMax(&s_max[2], __float_as_uint(avy));
     }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        unsigned* g = threadIdx.x == 0 ? &a.st->maxq_bits : threadIdx.x == 1 ? &a.st->maxvx_bits : &a.st->maxvy_bits;
+        if (s_max[threadIdx.x] > *(volatile unsigned*)g) atomicMax(g, s_max[threadIdx.x]);
+    }
+}
+
+__global__ void convert_masses(const double* __restrict__ m, size_t n, float* __restrict__ fm) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) fm[i] = __double2float_rn(m[i]);
 }
 
 // 1/d when d is a power of two (then x * (1/d) == x / d exactly), else 0.
@@ -393,6 +414,15 @@ int pic_gpu_create(const pic_domain* dom, size_t capacity, int device, pic_ctx**
     c->rho = (double*)A(c->G * 8);
     c->unitbuf = (double*)A(64);
     c->dstats = (DevStats*)A(sizeof(DevStats));
+    if (rc == PIC_OK && cudaHostAlloc((void**)&c->hstats, sizeof(DevStats), cudaHostAllocDefault) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->hstats = nullptr;
+        rc = fail(PIC_ERR_NOMEM, "pinned allocation");
+    }
+    int pageable = 0, tables = 0;
+    cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device);
+    cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device);
+    c->reads_host = pageable && tables;
     if (rc != PIC_OK) {
         pic_gpu_destroy(c);
         return rc;
@@ -417,6 +447,7 @@ int pic_gpu_destroy(pic_ctx* c) {
                     c->alt[0], c->alt[1], c->alt[2], c->alt[3], c->alt[4], c->alt[5], c->counts, c->offsets,
                     c->cellcount, c->scan.partials, c->stage, c->acc, c->rho, c->unitbuf, c->dstats};
     for (void* p : ptrs) dfree(p);
+    if (c->hstats) cudaFreeHost(c->hstats);
     release_fields(c);
     release_rbgs(c);
     release_current(c);
@@ -438,8 +469,7 @@ int pic_gpu_destroy(pic_ctx* c) {
 
 int pic_gpu_synchronize(pic_ctx* c) {
     if (!c) return fail(PIC_ERR_ARG, "NULL context");
-    PIC_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    return check_device_status(c);
+    return check_device_status(c);  // waits for the stream
 }
 
 int pic_gpu_launch_count(pic_ctx* c, long long* out) {
@@ -466,22 +496,48 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
     if (n > c->cap) return fail(PIC_ERR_ARG, "pic_gpu_upload_particles: n exceeds context capacity");
     if (n > 0 && (!x || !y || !q)) return fail(PIC_ERR_ARG, "pic_gpu_upload_particles: x, y, q are required");
     PIC_CUDA_TRY(cudaSetDevice(c->device));
+    // Page-locked arrays are read by the conversion kernel itself over the host link,
+    // and pageable ones too where the GPU uses the host's page tables (a 64^2 upload
+    // of 65,536 particles spent most of its time in five staged copies); other arrays
+    // go through two device staging slots.
+    const double* src[6] = {x, y, vx, vy, q, m};
+    const double* dev_src[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    bool reach[6];  // by the kernel, directly
+    for (int k = 0; k < 6; ++k) {
+        reach[k] = true;
+        if (!src[k] || n == 0) continue;
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, src[k]) != cudaSuccess) {
+            (void)cudaGetLastError();
+            reach[k] = false;
+        } else if (at.type == cudaMemoryTypeHost && at.devicePointer) {
+            dev_src[k] = (const double*)at.devicePointer;
+        } else if (at.type == cudaMemoryTypeUnregistered && c->reads_host) {
+            dev_src[k] = src[k];
+        } else {
+            reach[k] = false;
+        }
+    }
+    bool direct = n > 0 && reach[0] && reach[1] && reach[2] && reach[3] && reach[4];
+    // masses that are not all 1 are stored; a direct upload that reaches them finds
+    // out in its kernel
     bool need_m = false;
-    if (m) {
+    if (m && !(direct && reach[5])) {
         for (size_t i = 0; i < n; ++i)
             if (m[i] != 1.0) {
                 need_m = true;
                 break;
             }
+        if (need_m) direct = false;
     }
-    if (need_m && !c->m) {
-        int rc;
-        c->m = (float*)dalloc(((c->cap ? c->cap : 1) + PARTICLE_PAD) * 4, &rc);
-        if (!c->m) return rc;
-    }
+    auto ensure_mass = [&]() -> int {
+        int rc = PIC_OK;
+        if (!c->m) c->m = (float*)dalloc(((c->cap ? c->cap : 1) + PARTICLE_PAD) * 4, &rc);
+        return rc;
+    };
+    if (need_m) PIC_TRY(ensure_mass());
     c->has_mass = need_m ? 1 : 0;
 
-    const double* src[6] = {x, y, vx, vy, q, need_m ? m : nullptr};
     ConvertArgs a{};
     a.dx = c->dx;
     a.dy = c->dy;
@@ -499,22 +555,6 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
     a.st = c->dstats;
     PIC_CUDA_TRY(cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), c->stream));
 
-    // Page-locked inputs are read by the conversion kernel itself over the
-    // host link (one pass, no staging copy); other inputs go through two device
-    // staging slots, the copy of chunk i+1 overlapping the conversion of chunk i.
-    const double* dev_src[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    bool direct = n > 0;
-    for (int k = 0; k < 6 && direct; ++k) {
-        if (!src[k]) continue;
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, src[k]) != cudaSuccess || at.type != cudaMemoryTypeHost ||
-            !at.devicePointer) {
-            (void)cudaGetLastError();
-            direct = false;
-        } else {
-            dev_src[k] = (const double*)at.devicePointer;
-        }
-    }
     if (direct) {
         a.x = dev_src[0];
         a.y = dev_src[1];
@@ -524,7 +564,7 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
         a.m = dev_src[5];
         a.count = n;
         a.first = 0;
-        convert_particles<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(a);
+        convert_particles<<<(unsigned)((n + CONVERT_THREADS - 1) / CONVERT_THREADS), CONVERT_THREADS, 0, c->stream>>>(a);
         PIC_TRY(check_launch(c, "convert_particles"));
     } else if (n > 0) {
         const size_t chunk = n < ((size_t)1 << 22) ? n : ((size_t)1 << 22);
@@ -548,7 +588,7 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
             double* dst[6];
             for (int k = 0; k < 6; ++k) {
                 dst[k] = s + (size_t)k * chunk;
-                if (src[k])
+                if (src[k] && (k != 5 || need_m))
                     PIC_CUDA_TRY(cudaMemcpyAsync(dst[k], src[k] + first, cnt * sizeof(double),
                                                  cudaMemcpyHostToDevice, c->copy_stream));
             }
@@ -562,7 +602,7 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
             a.m = need_m ? dst[5] : nullptr;
             a.count = cnt;
             a.first = first;
-            convert_particles<<<(unsigned)((cnt + 255) / 256), 256, 0, c->stream>>>(a);
+            convert_particles<<<(unsigned)((cnt + CONVERT_THREADS - 1) / CONVERT_THREADS), CONVERT_THREADS, 0, c->stream>>>(a);
             PIC_TRY(check_launch(c, "convert_particles"));
             PIC_CUDA_TRY(cudaEventRecord(c->ev_converted[slot], c->stream));
         }
@@ -577,14 +617,24 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
         PIC_TRY(check_launch(c, "finish_upload"));
     }
     PIC_TRY(pic_gpu_synchronize(c));
-    DevStats st;
-    PIC_CUDA_TRY(cudaMemcpy(&st, c->dstats, sizeof(st), cudaMemcpyDeviceToHost));
+    const DevStats& st = *c->hstats;
     c->qn_uniform = (n > 0 && st.q_mixed == 0 && st.q_first != 0.0f && std::isfinite(st.q_first)) ? st.q_first : 0.0f;
-    if (st.order_breaks == 0) {
+    const bool in_order = st.order_breaks == 0;
+    if (direct && dev_src[5] && st.mass_mixed) {
+        const int rc = ensure_mass();
+        if (rc != PIC_OK) {
+            c->n = 0;  // the new particles' masses are not there
+            return rc;
+        }
+        convert_masses<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(dev_src[5], n, c->m);
+        PIC_TRY(check_launch(c, "convert_masses"));
+        c->has_mass = 1;
+        PIC_TRY(pic_gpu_synchronize(c));  // the caller's array is read
+    }
+    if (in_order) {
         // already in cell order: offsets make it usable by the tiled kernel without a sort
         PIC_TRY(ensure_sort_scratch(c));
         PIC_TRY(build_offsets(c, c->cell));
-        PIC_TRY(pic_gpu_synchronize(c));
         c->sorted = 1;
         c->part_valid = 1;
     }

@@ -22,6 +22,7 @@ struct DevStats {
     int err;
     unsigned int err_info;
     unsigned int order_breaks;  // uploads: count of i with cell[i] < cell[i-1]
+    unsigned int mass_mixed;    // uploads: nonzero when some mass is not 1
     unsigned int q_mixed;       // uploads: nonzero when the stored charges differ
     float q_first;              // uploads: the first particle's stored charge
     float q_raw0;               // uploads: the first particle's charge before normalisation
@@ -143,6 +144,8 @@ struct pic_ctx {
     long long graph_launches_sort = 0, graph_launches_plain = 0;
 
     picgb::DevStats* dstats = nullptr;
+    picgb::DevStats* hstats = nullptr;  // page-locked copy, filled by check_device_status
+    int reads_host = 0;                 // the GPU reads pageable host memory itself
 
     // tuning
     int order_mode = PIC_ORDER_AUTO;
@@ -167,7 +170,8 @@ namespace picgb {
 int fail(int code, const std::string& msg);
 // Checks a CUDA call; on failure records the message and returns PIC_ERR_CUDA.
 int cuda_fail(cudaError_t e, const char* what);
-// Reads back the device status block; maps a device error to PIC_ERR_*.
+// Waits for the stream and reads back the device status block (into ctx->hstats, one
+// wait for both); maps a device error to PIC_ERR_*.
 int check_device_status(pic_ctx* ctx);
 // Launch-configuration error check after a kernel launch.
 int check_launch(pic_ctx* ctx, const char* what);

@@ -1,0 +1,63 @@
+"""Uploads from page-locked and pageable host arrays, with and without masses:
+the same device layout, charges and masses either way."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("masses", [None, "ones", "last", "mixed"])  # "last": only the last particle's differs from 1
+@pytest.mark.parametrize("n", [1, 255, 257, 70001])
+def test_pageable_equals_page_locked(pg, n, masses):
+    rng = np.random.default_rng(n)
+    a = {"x": rng.random(n) * 20, "y": rng.random(n) * 12, "vx": rng.normal(size=n), "vy": rng.normal(size=n),
+         "q": rng.choice([-1.0, 0.5], n)}
+    if masses:
+        a["m"] = np.ones(n)
+        if masses == "last":
+            a["m"][-1] = 3.0
+        if masses == "mixed":
+            a["m"] = rng.random(n) + 0.5
+    out = []
+    for pinned in (False, True, "m pageable"):
+        hold = {}
+        args = {}
+        for k, v in a.items():
+            if pinned and not (k == "m" and pinned == "m pageable"):
+                hold[k] = pg.PinnedArray(n)
+                hold[k].array[:] = v
+                args[k] = hold[k].array
+            else:
+                args[k] = v
+        with pg.Context(20, 12, 20.0, 12.0, n) as c:
+            c.upload(**args)
+            out.append((c.device_layout(), c.download()))
+        args.clear()
+        for h in hold.values():
+            h.free()
+    for lay, host in out[1:]:
+        for k in lay:
+            assert np.array_equal(lay[k], out[0][0][k])
+        for k in host:
+            assert np.array_equal(host[k], out[0][1][k])
+    want = a.get("m", np.ones(n)).astype(np.float32)
+    assert np.array_equal(out[0][1]["m"], want)
+
+
+def test_mass_set_then_cleared(pg):
+    """A set with masses, then one without: the gather divides by the new set's masses."""
+    n = 1000
+    rng = np.random.default_rng(5)
+    x, y, v = rng.random(n) * 16, rng.random(n) * 16, rng.normal(size=n)
+    e = rng.normal(size=256)
+    got = []
+    for first in (None, rng.random(n) + 0.5):
+        with pg.Context(16, 16, 16.0, 16.0, n) as c:
+            if first is not None:
+                c.upload(x, y, -np.ones(n), v, v, first)
+            c.upload(x, y, -np.ones(n), v, v, np.ones(n))
+            c.set_fields(ex=e, ey=e)
+            c.gather(0.1)
+            got.append(c.device_layout()["vx"])
+            assert np.all(c.download()["m"] == 1.0)
+    assert np.array_equal(*got)

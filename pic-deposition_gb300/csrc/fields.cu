@@ -1,4 +1,4 @@
-// Fields: FFT Poisson solve (cuFFT), forward-difference E, FP64 diagnostics.
+// Fields: FFT Poisson solve, forward-difference E, FP64 diagnostics.
 //
 // PoissonSolverFFT::solve (src/pic/poisson_fft.cpp:45-94) in the reference runs
 // FFTW's R2HC x R2HC transform of rho*dV, divides by the continuous k^2
@@ -7,7 +7,8 @@
 // difference E = -(phi[i+1] - phi[i]) / dx (poisson_fft.cpp:77-93). The
 // separable halfcomplex basis and the complex basis diagonalise the same
 // operator with the same eigenvalue k^2 per frequency, so here the transform is
-// cuFFT's D2Z / Z2D in FP64 with this library's own k-divide and E kernels.
+// this library's FP64 transforms where the sides are powers of two (fft.cu), else
+// cuFFT's D2Z / Z2D in FP64, with this library's own frequency factors and E kernels.
 //
 // Diagnostics (src/pic/field_grid.cpp:24-38, particles_aos.cpp:182-196,
 // diagnostics.cpp:26-51) are FP64 sums computed with a fixed two-level tree
@@ -25,18 +26,31 @@ constexpr int RED_THREADS = 256;
 constexpr int RED_BLOCKS = 1024;  // fixed partition: results do not depend on the device
 
 // ---- deterministic FP64 sums --------------------------------------------
-__device__ __forceinline__ double block_sum(double v) {
-    __shared__ double ws[RED_THREADS / 32];
+// Block sums of K values at once (one exchange); valid in thread 0.
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K]) {
+    __shared__ double ws[K][RED_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
-    if (lane == 0) ws[warp] = v;
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = __dadd_rn(v[k], __shfl_down_sync(0xffffffffu, v[k], o));
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < K; ++k) ws[k][warp] = v[k];
     __syncthreads();
-    double s = 0.0;
     if (threadIdx.x == 0)
-        for (int w = 0; w < RED_THREADS / 32; ++w) s = __dadd_rn(s, ws[w]);
-    __syncthreads();
-    return s;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            double s = 0.0;
+            for (int w = 0; w < RED_THREADS / 32; ++w) s = __dadd_rn(s, ws[k][w]);
+            v[k] = s;
+        }
+}
+__device__ __forceinline__ double block_sum(double v) {
+    double a[1] = {v};
+    block_sums(a);
+    return a[0];
 }
 
 // Per-item quantities summed by the diagnostics.
@@ -142,10 +156,12 @@ __global__ void __launch_bounds__(RED_THREADS) diag_final(FinalArgs a) {
         rho = __dadd_rn(rho, g.x);
         ee = __dadd_rn(ee, g.y);
     }
-    ke = block_sum(ke);
-    rho = block_sum(rho);
-    ee = block_sum(ee);
+    double sums[3] = {ke, rho, ee};
+    block_sums(sums);
     if (threadIdx.x != 0) return;
+    ke = sums[0];
+    rho = sums[1];
+    ee = sums[2];
     double* r = a.r;
     r[1] = r[8];
     r[6] = r[9];
@@ -184,9 +200,9 @@ __global__ void __launch_bounds__(RED_THREADS) grid_sum_partials(const double* _
         s = __dadd_rn(s, rho[i]);
         ee = __dadd_rn(ee, __dadd_rn(__dmul_rn(Ex[i], Ex[i]), __dmul_rn(Ey[i], Ey[i])));
     }
-    s = block_sum(s);
-    ee = block_sum(ee);
-    if (threadIdx.x == 0) reinterpret_cast<double2*>(partial)[blockIdx.x] = make_double2(s, ee);
+    double sums[2] = {s, ee};
+    block_sums(sums);
+    if (threadIdx.x == 0) reinterpret_cast<double2*>(partial)[blockIdx.x] = make_double2(sums[0], sums[1]);
 }
 
 // ---- Poisson ---------------------------------------------------------------
@@ -226,11 +242,15 @@ __global__ void scale_phi(double* __restrict__ phi, size_t g, double norm) {
 
 // E = -(phi[i+1] - phi[i]) / d (poisson_fft.cpp:77-93, poisson_gs.cpp:48-60); FP32
 // copies for the gather; and the block's sums of rho and E^2, which the step's
-// diagnostics need: no passes over rho and E of their own. A block covers FE_ITEMS
-// rounds of 256 cells.
-constexpr int FE_ITEMS = 4;
-constexpr size_t FE_BLOCK = (size_t)RED_THREADS * FE_ITEMS;
+// diagnostics need: no passes over rho and E of their own. A block covers ITEMS
+// rounds of 256 cells: four, or one on a grid too small to give every SM a block.
+static int efield_items(size_t g) { return g < (size_t)RED_THREADS * 4 * 152 ? 1 : 4; }
+static size_t efield_blocks(size_t g) {
+    const size_t per = (size_t)RED_THREADS * efield_items(g);
+    return (g + per - 1) / per;
+}
 
+template <int ITEMS>
 __global__ void __launch_bounds__(RED_THREADS) efield(const double* __restrict__ phi, const double* __restrict__ rho,
                                                       int Nx, int Ny, double idx_dx, double idx_dy,
                                                       double* __restrict__ Ex, double* __restrict__ Ey,
@@ -239,8 +259,8 @@ __global__ void __launch_bounds__(RED_THREADS) efield(const double* __restrict__
     const size_t g = (size_t)Nx * Ny;
     double s = 0.0, ee = 0.0;
 #pragma unroll
-    for (int k = 0; k < FE_ITEMS; ++k) {
-        const size_t t = (size_t)blockIdx.x * FE_BLOCK + k * RED_THREADS + threadIdx.x;
+    for (int k = 0; k < ITEMS; ++k) {
+        const size_t t = ((size_t)blockIdx.x * ITEMS + k) * RED_THREADS + threadIdx.x;
         if (t < g) {
             const unsigned j = (unsigned)t / (unsigned)Nx, i = (unsigned)t - j * (unsigned)Nx;  // at most 2^30 cells
             const double p = phi[t];
@@ -255,9 +275,9 @@ __global__ void __launch_bounds__(RED_THREADS) efield(const double* __restrict__
             ee = __dadd_rn(ee, __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
         }
     }
-    s = block_sum(s);
-    ee = block_sum(ee);
-    if (threadIdx.x == 0) reinterpret_cast<double2*>(partial)[blockIdx.x] = make_double2(s, ee);
+    double sums[2] = {s, ee};
+    block_sums(sums);
+    if (threadIdx.x == 0) reinterpret_cast<double2*>(partial)[blockIdx.x] = make_double2(sums[0], sums[1]);
 }
 
 __global__ void fields_to_f32(const double* __restrict__ Ex, const double* __restrict__ Ey, size_t g,
@@ -312,7 +332,7 @@ int ensure_fields(pic_ctx* c) {
     if (rc) return rc;
     if (!c->red_out) c->red_out = (double*)dalloc(16 * 8, &rc);
     if (rc) return rc;
-    const size_t pairs = (g + FE_BLOCK - 1) / FE_BLOCK;
+    const size_t pairs = efield_blocks(g);
     if (!c->grid_partials) c->grid_partials = (double*)dalloc((pairs > RED_BLOCKS ? pairs : RED_BLOCKS) * 16, &rc);
     if (rc) return rc;
     if (!c->fields_init) {
@@ -326,28 +346,46 @@ int ensure_fields(pic_ctx* c) {
     return PIC_OK;
 }
 
-static int ensure_fft(pic_ctx* c) {
+static int ensure_spec(pic_ctx* c) {
     PIC_TRY(ensure_fields(c));
+    int rc = PIC_OK;
+    if (!c->spec) c->spec = dalloc((size_t)(c->Nx / 2 + 1) * (size_t)c->Ny * sizeof(cufftDoubleComplex), &rc);
+    return rc;
+}
+
+// cuFFT plans: sides that fft.cu does not take, and the discrete solve.
+static int ensure_fft(pic_ctx* c) {
+    PIC_TRY(ensure_spec(c));
     if (c->fft_ready) return PIC_OK;
     int rc = PIC_OK;
-    const size_t nh = (size_t)(c->Nx / 2 + 1);
-    c->spec = dalloc(nh * (size_t)c->Ny * sizeof(cufftDoubleComplex), &rc);
-    if (rc) return rc;
-    c->fft_rhs = (double*)dalloc(c->G * 8, &rc);
+    if (!c->fft_rhs) c->fft_rhs = (double*)dalloc(c->G * 8, &rc);
     if (rc) return rc;
     cufftHandle f, b;
     PIC_CUFFT_TRY(cufftPlan2d(&f, c->Ny, c->Nx, CUFFT_D2Z));
     PIC_CUFFT_TRY(cufftPlan2d(&b, c->Ny, c->Nx, CUFFT_Z2D));
     PIC_CUFFT_TRY(cufftSetStream(f, c->stream));
     PIC_CUFFT_TRY(cufftSetStream(b, c->stream));
-    c->fft_scale = (double*)dalloc(nh * (size_t)c->Ny * 8, &rc);
-    if (rc) return rc;
-    make_fft_scale<<<(unsigned)((nh * c->Ny + 255) / 256), 256, 0, c->stream>>>(
-        c->fft_scale, c->Nx, c->Ny, c->Lx, c->Ly, c->dx * c->dy / (double)c->G);
-    PIC_TRY(check_launch(c, "make_fft_scale"));
     c->fft_fwd = (int)f;
     c->fft_inv = (int)b;
     c->fft_ready = 1;
+    return PIC_OK;
+}
+
+static bool own_fft(const pic_ctx* c) { return own_fft_size(c->Nx) && own_fft_size(c->Ny); }
+
+static int ensure_poisson(pic_ctx* c) {
+    if (c->poisson_ready) return PIC_OK;
+    PIC_TRY(own_fft(c) ? ensure_spec(c) : ensure_fft(c));
+    if (own_fft(c)) PIC_TRY(make_own_fft(c));
+    int rc = PIC_OK;
+    const size_t ns = (size_t)(c->Nx / 2 + 1) * c->Ny;
+    if (!c->fft_scale) c->fft_scale = (double*)dalloc(ns * 8, &rc);
+    if (rc) return rc;
+    const double num = c->dx * c->dy / (double)c->G;
+    make_fft_scale<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>(c->fft_scale, c->Nx, c->Ny, c->Lx, c->Ly,
+                                                                         own_fft(c) ? 0.5 * num : num);
+    PIC_TRY(check_launch(c, "make_fft_scale"));
+    c->poisson_ready = 1;
     return PIC_OK;
 }
 
@@ -358,30 +396,35 @@ void release_fields(pic_ctx* c) {
         c->fft_ready = 0;
     }
     void* ptrs[] = {c->phi, c->Ex, c->Ey, c->Exf, c->Eyf, c->spec, c->fft_rhs, c->red_partials, c->red_out,
-                    c->ke_partials, c->grid_partials, c->fft_scale};
+                    c->ke_partials, c->grid_partials, c->fft_scale, c->fft_tw};
     for (void* p : ptrs) dfree(p);
 }
 
 int efield_from_phi(pic_ctx* c) {
-    const unsigned blocks = (unsigned)((c->G + FE_BLOCK - 1) / FE_BLOCK);
-    efield<<<blocks, RED_THREADS, 0, c->stream>>>(c->phi, c->rho, c->Nx, c->Ny, 1.0 / c->dx, 1.0 / c->dy, c->Ex,
-                                                  c->Ey, c->Exf, c->Eyf, c->grid_partials);
+    const unsigned blocks = (unsigned)efield_blocks(c->G);
+    (efield_items(c->G) == 1 ? efield<1> : efield<4>)<<<blocks, RED_THREADS, 0, c->stream>>>(
+        c->phi, c->rho, c->Nx, c->Ny, 1.0 / c->dx, 1.0 / c->dy, c->Ex, c->Ey, c->Exf, c->Eyf, c->grid_partials);
     PIC_TRY(check_launch(c, "efield"));
     c->grid_sums_ready = 1;
     return PIC_OK;
 }
 
-// Four FFT launches and two of this library's: the forward transform reads rho
-// itself (an out-of-place real transform leaves its input), k_scale applies the
-// frequency factors, the inverse writes phi, efield follows.
+// fft.cu's three kernels, or cuFFT's transforms with k_scale between them; both read
+// rho itself (an out-of-place real transform leaves its input), apply the frequency
+// factors and write phi; efield follows. With cuFFT a 64^2 solve took 50 us in four
+// transform kernels and k_scale, a 512^2 one 130.
 int poisson_fft(pic_ctx* c) {
-    PIC_TRY(ensure_fft(c));
+    PIC_TRY(ensure_poisson(c));
     prof_begin(c, "poisson_fft");
-    PIC_CUFFT_TRY(cufftExecD2Z((cufftHandle)c->fft_fwd, c->rho, (cufftDoubleComplex*)c->spec));
-    const size_t ns = (size_t)(c->Nx / 2 + 1) * c->Ny;
-    k_scale<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>((cufftDoubleComplex*)c->spec, c->fft_scale, ns);
-    PIC_TRY(check_launch(c, "k_scale"));
-    PIC_CUFFT_TRY(cufftExecZ2D((cufftHandle)c->fft_inv, (cufftDoubleComplex*)c->spec, c->phi));
+    if (own_fft(c)) {
+        PIC_TRY(own_fft_solve(c));
+    } else {
+        PIC_CUFFT_TRY(cufftExecD2Z((cufftHandle)c->fft_fwd, c->rho, (cufftDoubleComplex*)c->spec));
+        const size_t ns = (size_t)(c->Nx / 2 + 1) * c->Ny;
+        k_scale<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>((cufftDoubleComplex*)c->spec, c->fft_scale, ns);
+        PIC_TRY(check_launch(c, "k_scale"));
+        PIC_CUFFT_TRY(cufftExecZ2D((cufftHandle)c->fft_inv, (cufftDoubleComplex*)c->spec, c->phi));
+    }
     prof_end(c);
     return efield_from_phi(c);
 }
@@ -464,7 +507,7 @@ int diagnostics_async(pic_ctx* c, double* hist, int* step, int steps) {
     }
     f.grid = c->grid_partials;
     if (c->grid_sums_ready) {  // left by the solve that produced this E from this rho
-        f.grid_count = (int)((c->G + FE_BLOCK - 1) / FE_BLOCK);
+        f.grid_count = (int)efield_blocks(c->G);
     } else {
         grid_sum_partials<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(c->rho, c->Ex, c->Ey, c->G, c->grid_partials);
         PIC_TRY(check_launch(c, "grid_sum_partials"));

@@ -109,7 +109,9 @@ struct pic_ctx {
     void* spec = nullptr;  // Ny x (Nx/2+1) complex
     double* fft_rhs = nullptr;
     int fft_fwd = 0, fft_inv = 0, fft_ready = 0;
-    double* fft_scale = nullptr;  // per frequency: cell volume / (k^2 * Nx * Ny), DC 0
+    double* fft_scale = nullptr;  // per frequency: cell volume / (k^2 * Nx * Ny), DC 0 (half that for fft.cu)
+    void* fft_tw = nullptr;       // fft.cu: twiddles of both sides
+    int poisson_ready = 0;
     // deterministic FP64 reductions
     double* red_partials = nullptr;
     double* red_out = nullptr;
@@ -197,6 +199,10 @@ int sort_particles(pic_ctx* ctx, bool perm = false);
 int ensure_fields(pic_ctx* ctx);
 int poisson_fft(pic_ctx* ctx);
 int efield_from_phi(pic_ctx* ctx);
+// This library's transforms (fft.cu): sides that are powers of two from 8 to 2048.
+bool own_fft_size(int n);
+int make_own_fft(pic_ctx* ctx);
+int own_fft_solve(pic_ctx* ctx);
 // hist, step (both or neither): also write the step's pic_diag into the history
 // and advance the step counter
 int diagnostics_async(pic_ctx* ctx, double* hist = nullptr, int* step = nullptr, int steps = 0);

@@ -660,9 +660,20 @@ __global__ void __launch_bounds__(32) ens_energy_partials(const RunDesc* __restr
                 c[k] = in ? __ldcs(py + i0 + k * STEP) : 0.0f;
             }
         };
+        // lane k brings line k of a later batch into L2 (one of the lines its warp reads)
+        auto prefetch = [&](size_t i0) {
+            const size_t at = i0 - lane + (size_t)lane * STEP;
+            if (at < e) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(px + at));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(py + at));
+            }
+        };
         float kf = 0.0f;
+        prefetch(i + (size_t)EN_UNROLL * STEP);
+        prefetch(i + (size_t)2 * EN_UNROLL * STEP);
         load(i);
         for (; i < e; i += (size_t)EN_UNROLL * STEP) {
+            prefetch(i + (size_t)3 * EN_UNROLL * STEP);
             float t[EN_UNROLL];
 #pragma unroll
             for (int k = 0; k < EN_UNROLL; ++k) t[k] = a[k] * a[k] + c[k] * c[k];

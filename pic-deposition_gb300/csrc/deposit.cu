@@ -1649,7 +1649,7 @@ __global__ void __launch_bounds__(DEP_THREADS) esk_light(DepArgs a) {
 }
 
 // After a deposit between sorts whose kernel was chosen on the device: once the
-// cell kernel has found more than `limit` particles outside their sorted cell,
+// cell kernel has counted more than `limit` particles (any_order_fraction),
 // the any-order kernel takes the following deposits (it is faster when most
 // particles have moved: every mover is a separate frame of atomics in the cell
 // kernel) until the next sort clears the flag. A deposit made in any order
@@ -1711,10 +1711,14 @@ static int launch_cells(pic_ctx* c, DepArgs a, unsigned tiles) {
     return PIC_OK;
 }
 
-// The fraction of the particles above which deposits between sorts switch to
-// the any-order kernel (measured crossover at 1024^2, TSC: the cell kernel takes
-// about 6.7 ms with every particle moved, the any-order kernel 3.0 ms).
-constexpr double ANY_ORDER_FRACTION = 0.4;
+// The fraction of the particles outside their sorted cell above which deposits
+// between sorts switch to the any-order kernel. TSC's nine pairs of shared atomics
+// per mover are cheaper than the any-order kernel's global ones while most movers are
+// near their tile (512^2 x 64, sort every ten steps, 20 steps: moving 0.1 cell a step
+// 12.8 ms at 0.75, 13.8 at 0.6, 15.7 at 0.4; 0.3 cells 18.8, 18.9 and 19.7, 24.5 with
+// no switch). The other schemes' any-order kernels match the tile's atomics earlier
+// (CIC, 0.1 cell: 9.9 ms switching or not; 0.3 cells: 11.3, and 13.5 with no switch).
+static double any_order_fraction(int scheme) { return scheme == PIC_SCHEME_TSC ? 0.75 : 0.4; }
 
 template <int S>
 static int launch_runs(pic_ctx* c, const DepArgs& a) {
@@ -1891,7 +1895,7 @@ int deposit_rho(pic_ctx* c, int scheme, double dt, double background) {
     const bool decide = c->n > 0 && tiled == 0 && adaptive && !c->sorted;
     fixed_to_rho<<<(unsigned)((c->G + 1023) / 1024), 256, 0, c->stream>>>(
         c->acc, c->G, background, inv_vol, scale, c->dstats, c->unitbuf, c->rho,
-        (unsigned long long)(ANY_ORDER_FRACTION * (double)c->n), decide ? (unsigned long long)c->n : 0ull);
+        (unsigned long long)(any_order_fraction(scheme) * (double)c->n), decide ? (unsigned long long)c->n : 0ull);
     PIC_TRY(check_launch(c, "fixed_to_rho"));
     c->grid_sums_ready = 0;
     c->last_scheme = scheme;

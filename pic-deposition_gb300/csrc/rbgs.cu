@@ -211,7 +211,7 @@ static int rb_finish(pic_ctx* c) {
 // equal spacings that are powers of two (unit cells, say) an update is four FP64
 // instructions instead of seven, with the same bits: the products are exact, so
 // (we*s + sn*s + b)*inv is one fused multiply-add of we + sn and b*inv.
-// 256^2, tol 1e-8, 57,920 sweeps from phi = 0: 102 ms in FP64 (1.8 us a sweep), 54 ms
+// 256^2, tol 1e-8, 57,920 sweeps from phi = 0: 92 ms in FP64 (1.6 us a sweep), 54 ms
 // mixed; 515 and 208 ms with 64 x 32 tiles (32 CTAs), seven instructions, an index
 // division per update and a grid-wide barrier per exchange. 64^2, 3,648 sweeps: 3.5
 // ms, from 31. Flags with release and acquire instead of numbered words: 160 ms.
@@ -528,7 +528,7 @@ constexpr int PS_MAX_NPT = 8;
 // neighbours' cells are needed; `step`: the sweeps between checks are a multiple
 // of it, so halo / 2 must divide it.
 static RbTiling rb_tiling(int Nx, int Ny, int max_blocks, int step, size_t bytes, double op_cycles, double min_cycles) {
-    constexpr double EXCHANGE = 2000.0;
+    constexpr double EXCHANGE = 1000.0;  // cycles; 2,000 chose longer halos at 256^2 (101 ms), 500 shorter ones at 222 x 106 (41 against 38)
     RbTiling best;
     double best_cost = 1e300;
     for (int H = 4; H <= 8; H += 4) {

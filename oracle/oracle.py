@@ -37,7 +37,8 @@ def reference_src() -> str | None:
     if not path:
         r = subprocess.run(["make", "-s", "-C", HERE, "print-ref"], capture_output=True, text=True)
         path = r.stdout.strip() if r.returncode == 0 else ""
-    return path if path and os.path.isdir(path) else None
+    # an empty folder is no checkout
+    return path if path and os.path.isdir(os.path.join(path, "src")) else None
 
 NGP, CIC, TSC, ESIRKEPOV = 0, 1, 2, 3
 

@@ -45,6 +45,17 @@ int check_launch(pic_ctx* ctx, const char* what) {
     return PIC_OK;
 }
 
+const void* device_view(const pic_ctx* ctx, const void* p, size_t align) {
+    if ((uintptr_t)p % align) return nullptr;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    if (at.type == cudaMemoryTypeHost && (uintptr_t)at.devicePointer % align == 0) return at.devicePointer;
+    return at.type == cudaMemoryTypeUnregistered && ctx->reads_host ? p : nullptr;
+}
+
 void* dalloc(size_t bytes, int* rc) {
     void* p = nullptr;
     if (bytes == 0) bytes = 16;
@@ -506,17 +517,8 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
     for (int k = 0; k < 6; ++k) {
         reach[k] = true;
         if (!src[k] || n == 0) continue;
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, src[k]) != cudaSuccess) {
-            (void)cudaGetLastError();
-            reach[k] = false;
-        } else if (at.type == cudaMemoryTypeHost && at.devicePointer) {
-            dev_src[k] = (const double*)at.devicePointer;
-        } else if (at.type == cudaMemoryTypeUnregistered && c->reads_host) {
-            dev_src[k] = src[k];
-        } else {
-            reach[k] = false;
-        }
+        dev_src[k] = (const double*)device_view(c, src[k], sizeof(double));
+        reach[k] = dev_src[k] != nullptr;
     }
     bool direct = n > 0 && reach[0] && reach[1] && reach[2] && reach[3] && reach[4];
     // masses that are not all 1 are stored; a direct upload that reaches them finds

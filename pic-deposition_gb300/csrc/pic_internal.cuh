@@ -182,6 +182,10 @@ int check_launch(pic_ctx* ctx, const char* what);
 int opt_in_dynamic_smem(const void* kernel, size_t bytes);
 
 void* dalloc(size_t bytes, int* rc);
+// The address at which kernels read the host array p in place: a page-locked one, or a
+// pageable one where the GPU uses the host's page tables. Null if they cannot, or if p
+// is not a multiple of `align`, the size of an element.
+const void* device_view(const pic_ctx* ctx, const void* p, size_t align);
 void dfree(void* p);
 
 // Device-wide exclusive scan of n u32 values in place (any n >= 0).

@@ -61,3 +61,25 @@ def test_mass_set_then_cleared(pg):
             got.append(c.device_layout()["vx"])
             assert np.all(c.download()["m"] == 1.0)
     assert np.array_equal(*got)
+
+
+@pytest.mark.parametrize("shift", [1, 4, 8])
+def test_upload_from_any_byte_address(pg, shift):
+    """Arrays whose elements do not lie on multiples of their size are copied first."""
+    n = 777
+    rng = np.random.default_rng(shift)
+    a = {"x": rng.random(n) * 16, "y": rng.random(n) * 8, "q": rng.choice([-1.0, 0.5], n), "m": rng.random(n) + 0.5}
+    out = []
+    for s in (0, shift):
+        args = {}
+        for k, v in a.items():
+            raw = np.zeros(n * 8 + 16, np.uint8)
+            off = (-raw.ctypes.data) % 16 + s
+            raw[off : off + n * 8] = np.frombuffer(v.tobytes(), np.uint8)
+            args[k] = raw[off : off + n * 8].view(np.float64)
+        with pg.Context(16, 8, 16.0, 8.0, n) as c:
+            c.upload(**args)
+            out.append((c.device_layout(), c.download()))
+    for i in (0, 1):
+        for k in out[0][i]:
+            assert np.array_equal(out[0][i][k], out[1][i][k])

@@ -83,3 +83,30 @@ def test_upload_from_any_byte_address(pg, shift):
     for i in (0, 1):
         for k in out[0][i]:
             assert np.array_equal(out[0][i][k], out[1][i][k])
+
+
+def test_network_gradient_from_any_host_array(pg):
+    """Loss and gradient of fields that the kernels read in place (pageable, page-locked)
+    and of fields that are copied first (not on a multiple of 4 bytes): the same bits."""
+    nx, ny, batch = 128, 8, 3
+    n = batch * nx * ny
+    rng = np.random.default_rng(2)
+    fields = [rng.normal(size=(batch, ny, nx)).astype(np.float32) for _ in range(2)]
+    hold = [pg.PinnedArray(n // 2) for _ in range(2)]
+    odd = []
+    for h, f in zip(hold, fields):
+        h.array.view(np.float32)[:] = f.reshape(-1)
+        raw = np.zeros(4 * n + 16, np.uint8)
+        off = (-raw.ctypes.data) % 16 + 1
+        raw[off : off + 4 * n] = np.frombuffer(f.tobytes(), np.uint8)
+        odd.append(raw[off : off + 4 * n].view(np.float32).reshape(f.shape))
+    pinned = [h.array.view(np.float32).reshape(batch, ny, nx) for h in hold]
+    with pg.Context(nx, ny, float(nx), float(ny), 16) as c:
+        c.ws_init(seed=3)
+        got = [c.ws_loss_grad(*a) for a in (fields, odd, pinned, (fields[0], odd[1]), (pinned[0], fields[1]))]
+    del pinned
+    for h in hold:
+        h.free()
+    for loss, grad in got[1:]:
+        assert loss == got[0][0]
+        assert np.array_equal(grad, got[0][1])

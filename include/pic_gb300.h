@@ -62,8 +62,8 @@ extern "C" {
 /* ---- deposit ordering modes ---- */
 /* PIC_ORDER_AUTO: the tiled kernel when cell-sorted; between sorts (particles
  * pushed since) the tiled kernel that also finds the particles that left their
- * cell, until one deposit finds more than 40 % of them moved, then the
- * run-aggregating kernel until the next sort (chosen on the device); otherwise
+ * cell, until one deposit finds more than 40 % of them moved (TSC: 75 %), then
+ * the run-aggregating kernel until the next sort (chosen on the device); otherwise
  * the run-aggregating kernel. Every choice gives the same grid bit for bit. */
 #define PIC_ORDER_AUTO 0
 #define PIC_ORDER_SORTED 1   /* tiled kernel; PIC_ERR_STATE unless sorted (or only pushed since) */
@@ -206,7 +206,8 @@ int pic_gpu_get_fields(pic_ctx* ctx, double* phi, double* Ex, double* Ey);
 
 /* ---- Poisson: replaces pic::PoissonSolverFFT::solve (src/pic/poisson_fft.cpp:45-94) ----
  * phi = IFFT(FFT(rho*dV) / k^2) with the continuous k^2 and DC set to 0, then
- * E = -(phi[i+1]-phi[i])/dx. FP64 cuFFT (D2Z/Z2D) plus this library's kernels. */
+ * E = -(phi[i+1]-phi[i])/dx. FP64: this library's transforms where both sides are
+ * powers of two from 8 to 2048, else cuFFT (D2Z/Z2D). */
 int pic_gpu_poisson_fft(pic_ctx* ctx);
 
 /* ---- Poisson by red-black Gauss-Seidel (new; the reference's PoissonSolverGS,

@@ -21,7 +21,8 @@
 // quantities of their own size (no S1 - S0 cancellation): no crossing
 // DS = (0,-d,d,0); crossing up DS = (0, r-1, (1-r)-fr, fr); down DS = (-e, r+e, -r, 0).
 //
-// Kernels: cell-sorted particles, one lane per cell (current_cells); any order,
+// Kernels: cell-sorted particles, the lanes of a cell sum those that stay in it
+// (current_cells) and the rest go through a list (current_listed); any order,
 // the deposit's warp step (128 particles, 4 consecutive per lane via 128-bit
 // loads), each lane summing its particles' 24 edge values while they share a
 // cell (one rolled copy of the particle body), a segmented warp scan, and int64
@@ -558,7 +559,7 @@ int deposit_current_async(pic_ctx* c, double dt) {
     a.jy = reinterpret_cast<unsigned long long*>(c->accjy);
     a.st = c->dstats;
     if (c->n && c->sorted) {
-        // cell-sorted: one lane per cell over the sort's ranges
+        // cell-sorted: each cell's lanes over the sort's range of it
         const int tiles_x = (c->Nx + JC_TW - 1) / JC_TW, tiles_y = (c->Ny + JC_TH - 1) / JC_TH;
         int klog, cap;
         const bool qc = a.qc != 0.0f;

@@ -15,13 +15,13 @@
 //    for bit. TSC with one charge for every particle uses exact integer
 //    weights instead (2^30 units per particle, see tsci_weights).
 //  * Sorted path (deposit_cells). One CTA per tile of tile_w x tile_h cells;
-//    one lane per cell of a 32-cell unit of a tile row walks the cell's
-//    contiguous range of the cell-sorted stream (staged into shared memory with
-//    cp.async), sums its particles' stencil values in registers and adds the
-//    cell's totals to the tile's accumulators in shared memory once (split
-//    into two native 32-bit atomics); at the end the tile is flushed to the
-//    global int64 grid once. A freshly sorted stream needs no cell keys: the
-//    offsets name every particle's cell. Details at the kernel.
+//    K lanes per cell (one where cells hold many particles, up to 32 where the grid
+//    is small) walk the cell's contiguous range of the cell-sorted stream (staged
+//    into shared memory with cp.async), sum its particles' stencil values in
+//    registers and add the cell's totals to the tile's accumulators in shared
+//    memory once (split into two native 32-bit atomics); at the end the tile is
+//    flushed to the global int64 grid once. A freshly sorted stream needs no cell
+//    keys: the offsets name every particle's cell. Details at the kernel.
 //  * Any-order path (deposit_runs): a warp handles 128 consecutive particles
 //    at a time, lane l taking particles 4l..4l+3 (one 128-bit streaming load
 //    per field, the next step's loads issued first); a lane sums its

@@ -12,8 +12,9 @@
 //     deposit(dt) -> + background -> Poisson -> push(dt) -> gather(dt) -> diagnostics.
 // The reference sorts a copy of the particles inside every deposit
 // (deposition.cpp:185-188); here the sort is in place and persists, and between
-// sorts the deposit uses the run-aggregating kernel on the nearly ordered
-// particles. Because the deposit is fixed point (order independent), the sort
+// sorts the deposit takes the nearly ordered particles by cell until too many have
+// moved, then by runs of equal cells (chosen on the device, see
+// any_order_fraction). Because the deposit is fixed point (order independent), the sort
 // interval does not change any result bit.
 //
 // Diagnostics of every step (pic::computeDiagnostics, diagnostics.cpp:42-51)

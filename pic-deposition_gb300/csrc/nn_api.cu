@@ -76,7 +76,7 @@ extern "C" int pic_nn_conv3x3(int op, int batch, int H, int W, int cin, int cout
         if (op <= 1) PIC_CUDA_TRY(cudaMemcpy(db, bias, (size_t)kcout * 4, cudaMemcpyHostToDevice));
         if (op == 2) PIC_CUDA_TRY(cudaMemcpy(dmask, aux, P * kcout * 2, cudaMemcpyHostToDevice));
         PIC_TRY(picnn::build_weight_image(dw, cin, cout, op == 2 ? 1 : 0, img, s));
-        picnn::ConvLaunch a{dx, img, db, dmask, dout, batch, H, W, 8, derr};
+        picnn::ConvLaunch a{dx, img, db, dmask, dout, batch, H, W, derr, 0};
         const int epi = op == 0 ? picnn::EPI_BIAS_RELU : op == 1 ? picnn::EPI_BIAS_OUT : picnn::EPI_MASK;
         PIC_TRY(picnn::launch_conv(a, kcin, kcout, epi, s));
         PIC_CUDA_TRY(cudaDeviceSynchronize());

@@ -1,19 +1,31 @@
 // 3x3 periodic convolutions as implicit GEMMs on the 5th-generation tensor cores.
 //
 // Forward / input-gradient kernel (conv3x3_kernel): one CTA owns a 128-pixel
-// segment of a run of image rows. The GEMM per output row is
-//     D[128 px][cout] = sum over 9 taps of A_tap[128 px][cin] * B_tap[cin][cout]
+// segment of a run of image rows, taken in blocks of 4 output rows. The GEMM of a
+// block is
+//     D[128 px][row r, cout] = sum over input rows m and dx of
+//                              A_(m,dx)[128 px][cin] * B_(m-r,dx)[cin][cout]
 // with D in tensor memory (FP32), issued as tcgen05.mma kind::f16 (BF16 x BF16,
-// M = 128, N = cout, K = 16) by one thread. The input rows are staged in shared
+// M = 128, K = 16, N = cout times the up to three output rows that an input row
+// reaches) by one thread. An MMA of N = 32 spends its time on reading A (64 cycles,
+// measured, where its products are 16), one of N = 96 no more than that: a row at a
+// time takes 18 of them per row (cin = 32), a block 39 per 4 rows. An output's
+// products are added in the same order either way.
+// The input rows are staged in shared
 // memory as "planes" of 8 channels: pixel slot s of plane j holds the 16 bytes of
 // channels 8j..8j+7 of pixel x0-1+s. In the K-major no-swizzle operand layout
 // (8-row core matrices of 16-byte rows, stride between row groups SBO = 128 B,
 // between the two K halves LBO = one plane) row r of A sits at r*16 bytes, so
 // the operand of tap dx is the same staged row with its start moved by
-// (dx+1)*16 bytes: im2col costs nothing. Warp-specialised: one warp stages rows
-// into a ring of 6 slots, one thread issues the MMAs of row y into one TMEM
-// buffer while four warps drain row y-1 from the other (bias + ReLU, or the
+// (dx+1)*16 bytes: im2col costs nothing. The weight image holds the three dy of a
+// dx side by side along N, the last first: output rows r, r+1, .. want m-r, m-r-1, ..
+// Warp-specialised: two warps stage rows
+// into a ring of 9 slots, one thread issues the MMAs of a block into one TMEM
+// buffer while eight warps drain the block before from the other (bias + ReLU, or the
 // ReLU mask of the backward pass), handing over through mbarriers.
+// 32 to 32 channels, 512^2, batch 16: forward 131 us (171 a row at a time), 537 MB;
+// input gradient 152 us (194), 805 MB. Bound by memory and the chain
+// load - MMA - epilogue together: with a quarter of the MMAs 113 and 147 us.
 //
 // Weight-gradient kernel (wgrad_kernel): D[(dy, ci)][(dx, co)] = sum over pixels
 // of x[p + (dy, dx)][ci] * dy[p][co], K = pixels, both operands MN-major as they
@@ -26,6 +38,8 @@
 // on expiry the kernel records an error, skips the remaining work, frees its
 // tensor memory and returns.
 #include <cuda_bf16.h>
+
+#include <climits>
 
 #include "nn_conv.cuh"
 #include "pic_internal.cuh"
@@ -141,44 +155,106 @@ __host__ __device__ constexpr uint32_t tmem_cols(int n) { return n <= 32 ? 32u :
 // ---------------------------------------------------------------------------
 // forward / input gradient
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+
+// Which of the 8 BF16 values are above zero, bit e for value e.
+__device__ __forceinline__ uint32_t positive8(uint4 m) {
+    const uint32_t w[4] = {m.x, m.y, m.z, m.w};
+    uint32_t x = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x |= __vcmpgts2(w[q], 0u) & (1u << (2 * q) | 1u << (17 + 2 * q));
+    return (x | x >> 16) & 0xFFu;
+}
+
+// A warp's 32 pixels of a row, in both directions as one contiguous range of
+// 32 * COUT * 2 bytes: the ReLU mask is loaded 16 bytes per lane, a row ahead, and
+// its signs handed to the pixels' lanes by shuffles; the outputs are put together in
+// shared memory (each lane its pixel, the 16-byte pieces in an order that keeps 8
+// lanes off one another's banks) and stored by one bulk copy. (Each lane loading and
+// storing its own pixel's 64 bytes in four pieces, half a sector each: 231 us against
+// 175 for the input gradient of 32 channels at 512^2, batch 16, 172 against 145
+// forward.)
 template <int COUT, int EPI>
-__device__ __forceinline__ void conv_epilogue(const ConvLaunch& a, int b, int y, int x0, uint32_t taddr,
-                                              const float* sbias, int warp, int lane) {
-    float v[COUT];
-    tmem_load<COUT>(taddr, v);
-    const int px = x0 + warp * 32 + lane;
-    const size_t pix = ((size_t)b * a.H + y) * a.W + px;
-    if (EPI == EPI_BIAS_OUT) {
-        reinterpret_cast<float*>(a.y)[pix] = v[0] + sbias[0];
-        return;
+struct RowEpilogue {
+    static constexpr int P = COUT / 8;         // 16-byte pieces per pixel
+    static constexpr int BYTES = 32 * COUT * 2;
+    uint4 next[P];
+
+    __device__ __forceinline__ void prefetch(const ConvLaunch& a, size_t pix0, int lane) {
+        if (EPI != EPI_MASK) return;
+        const uint4* m = reinterpret_cast<const uint4*>(a.mask + pix0 * COUT);
+#pragma unroll
+        for (int q = 0; q < P; ++q) next[q] = m[q * 32 + lane];
     }
-    if (EPI == EPI_BIAS_RELU) {
+    // The mask of the lane's pixel, bit c for channel c. Piece q * 32 + lane is piece
+    // lane % P of pixel q * 32 / P + lane / P.
+    __device__ __forceinline__ uint32_t mask_bits(int lane) const {
+        uint32_t bits = 0;
 #pragma unroll
-        for (int c = 0; c < COUT; ++c) v[c] = fmaxf(v[c] + sbias[c], 0.0f);
-    } else {
-        const uint4* m = reinterpret_cast<const uint4*>(a.mask + pix * COUT);
+        for (int q = 0; q < P; ++q) {
+            uint32_t v = positive8(next[q]) << (8 * (lane % P));
 #pragma unroll
-        for (int q = 0; q < COUT / 8; ++q) {
-            const uint4 mm = m[q];
-            const uint32_t w[4] = {mm.x, mm.y, mm.z, mm.w};
+            for (int o = 1; o < P; o *= 2) v |= __shfl_xor_sync(0xffffffffu, v, o);
+            v = __shfl_sync(0xffffffffu, v, lane % (32 / P) * P);
+            if (lane / (32 / P) == q) bits = v;
+        }
+        return bits;
+    }
+    // v: the accumulators of the lane's pixel. stage: the warp's buffer of BYTES, free
+    __device__ __forceinline__ void finish(const ConvLaunch& a, size_t pix0, float (&v)[COUT], uint32_t bits, uint8_t* stage,
+                                           const float* sbias, int lane) const {
+        if constexpr (EPI == EPI_BIAS_OUT) {
+            reinterpret_cast<float*>(a.y)[pix0 + lane] = v[0] + sbias[0];
+            return;
+        } else {
+            uint4 o[P];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int16_t bits = (int16_t)((w[e >> 1] >> ((e & 1) * 16)) & 0xFFFFu);
-                if (!(bits > 0)) v[q * 8 + e] = 0.0f;
+            for (int q = 0; q < P; ++q) {
+                uint32_t w[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int c = q * 8 + 2 * e;
+                    if (EPI == EPI_BIAS_RELU)
+                        w[e] = pack_bf16x2(fmaxf(v[c] + sbias[c], 0.0f), fmaxf(v[c + 1] + sbias[c + 1], 0.0f));
+                    else
+                        w[e] = pack_bf16x2(bits >> c & 1u ? v[c] : 0.0f, bits >> (c + 1) & 1u ? v[c + 1] : 0.0f);
+                }
+                o[q] = make_uint4(w[0], w[1], w[2], w[3]);
             }
+            // pieces in the order (q + rot) % P
+            const int rot = lane * P / 8 % P;
+#pragma unroll
+            for (int step = 1; step < P; step *= 2) {
+                uint4 t[P];
+#pragma unroll
+                for (int q = 0; q < P; ++q) {
+                    const uint4 x = o[q], y = o[(q + step) % P];
+                    const bool r = (rot & step) != 0;
+                    t[q] = make_uint4(r ? y.x : x.x, r ? y.y : x.y, r ? y.z : x.z, r ? y.w : x.w);
+                }
+#pragma unroll
+                for (int q = 0; q < P; ++q) o[q] = t[q];
+            }
+            uint4* row = reinterpret_cast<uint4*>(stage) + lane * P;
+#pragma unroll
+            for (int q = 0; q < P; ++q) row[(q + rot) % P] = o[q];
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) bulk_store(reinterpret_cast<uint16_t*>(a.y) + pix0 * COUT, smem_addr(stage), BYTES);
         }
     }
-    uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.y) + pix * COUT);
-#pragma unroll
-    for (int q = 0; q < COUT / 8; ++q) {
-        uint4 o;
-        o.x = pack_bf16x2(v[q * 8 + 0], v[q * 8 + 1]);
-        o.y = pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]);
-        o.z = pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]);
-        o.w = pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]);
-        out[q] = o;
-    }
-}
+};
+
+constexpr int CONV_ROWS = 4;  // output rows per block
+constexpr int NRING = 9;      // staged rows: a block's 6 and three of the next one's 4
+constexpr int AHEAD = 3;      // rows whose copies are in flight behind the newest
 
 template <int CIN, int COUT>
 struct ConvSmem {
@@ -186,42 +262,73 @@ struct ConvSmem {
     static constexpr int SLOT = PLANES * PLANE;
     static constexpr int WBYTES = 9 * CIN * COUT * 2;
     static constexpr int OFF_BIAS = WBYTES;
-    static constexpr int OFF_RING = ((WBYTES + COUT * 4) + 127) / 128 * 128;
-    static constexpr int BYTES = OFF_RING + 6 * SLOT;
+    static constexpr int OFF_OUT = ((WBYTES + COUT * 4) + 127) / 128 * 128;
+    static constexpr int OFF_RING = OFF_OUT + 4 * 2 * 32 * COUT * 2;  // a buffer per epilogue warp
+    // no more CTAs on an SM than its 512 TMEM columns serve at once
+    static constexpr int TCOLS = (int)tmem_cols(2 * CONV_ROWS * COUT);
+    static constexpr int LEAST = 228 * 1024 / (512 / TCOLS + 1) + 1024;
+    static constexpr int BYTES = OFF_RING + NRING * SLOT > LEAST ? OFF_RING + NRING * SLOT : LEAST;
+    static constexpr int CTAS = 227 * 1024 / (BYTES + 1024);
 };
 
 __device__ __forceinline__ void mbar_arrive_cta(uint32_t a) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
 }
 
-// Warp-specialised: warp 4 stages input rows into the ring (cp.async), lane 0
-// of warp 5 issues each output row's MMAs, warps 0-3 (one TMEM lane quarter
-// each) run the epilogue of the previous row from the other TMEM buffer.
-// Barriers: full[s] (32 producer arrivals: the row in slot s has landed),
-// rowfree[s] (an MMA commit: the last output row that reads slot s is done),
-// tfull[b] (an MMA commit: accumulator b holds a row), tempty[b] (128
-// epilogue arrivals: accumulator b has been read). Every wait is bounded and
-// no role waits at a CTA barrier inside the loop.
-constexpr int CONV_THREADS = 192;
-constexpr int NRING = 6;
+// A ring's place: slot and the parity of its present use.
+struct RingPos {
+    int slot = 0;
+    uint32_t parity = 0;
+    __device__ __forceinline__ void advance(int n) {
+        if (++slot == n) {
+            slot = 0;
+            parity ^= 1u;
+        }
+    }
+};
+
+// The persistent CTAs take work items (128 pixels x a.rows output rows of an image)
+// blockIdx.x, blockIdx.x + gridDim.x, ... in one unbroken pipeline: loading the
+// weights, allocating TMEM and filling and draining the pipeline anew for every item
+// took 64 us of 139 at 512^2, batch 16.
+// Warp-specialised: warps 9 and 10 stage input rows into the ring (cp.async), lane 0
+// of warp 8 issues each block's MMAs, warps 0-7 (a TMEM lane quarter and every
+// other row each) run the epilogue of the previous block from the other TMEM buffer.
+// Barriers: full[s] (the producers' arrivals: the row in slot s has landed),
+// rowfree[s] (an MMA commit: the last block that reads slot s is done with it),
+// tfull[b] (an MMA commit: accumulator b holds a block), tempty[b] (the
+// epilogue's arrivals: accumulator b has been read). A block needs staged rows
+// 4i .. 4i+5 of its item; row 4i+5 is handed over once the copies three rows on are
+// issued, into the slot of row 4i-1, which the block before frees. Every wait is
+// bounded and no role waits at a CTA barrier inside the loop.
+constexpr int PRODUCERS = 64;
+constexpr int EPI_WARPS = 8;
+constexpr int CONV_THREADS = EPI_WARPS * 32 + 32 + PRODUCERS;
+
+struct ConvItem {
+    int b, x0, y0, nout;  // image, first pixel and row, output rows (nout + 2 staged rows from y0 - 1)
+};
+__device__ __forceinline__ ConvItem conv_item(const ConvLaunch& a, int k) {
+    const int segs = a.W / 128, runs = (a.H + a.rows - 1) / a.rows;
+    ConvItem it;
+    it.x0 = k % segs * 128;
+    it.y0 = k / segs % runs * a.rows;
+    it.b = k / segs / runs;
+    it.nout = min(a.rows, a.H - it.y0);
+    return it;
+}
 
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(CONV_THREADS) conv3x3_kernel(ConvLaunch a) {
+__global__ void __launch_bounds__(CONV_THREADS, 2) conv3x3_kernel(ConvLaunch a) {
     using L = ConvSmem<CIN, COUT>;
     constexpr int KSTEPS = CIN / 16;
-    constexpr uint32_t IDESC = idesc_bf16(128, COUT);
-    constexpr uint32_t TCOLS = tmem_cols(2 * COUT);
+    constexpr uint32_t TCOLS = (uint32_t)L::TCOLS;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[NRING], rowfree[NRING], tfull[2], tempty[2];
     __shared__ uint32_t tmem_slot;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int x0 = blockIdx.x * 128;
-    const int b = blockIdx.z;
-    const int y_begin = blockIdx.y * a.rows_per_cta;
-    const int y_end = min(a.H, y_begin + a.rows_per_cta);
-    if (y_begin >= y_end) return;
-    const int nout = y_end - y_begin, nrows = nout + 2;  // output rows; staged rows y_begin-1 .. y_end
+    const int items = a.batch * ((a.H + a.rows - 1) / a.rows) * (a.W / 128);
     const uint32_t s_w = smem_addr(smem);
     const uint32_t s_ring = s_w + L::OFF_RING;
     float* sbias = reinterpret_cast<float*>(smem + L::OFF_BIAS);
@@ -233,12 +340,12 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3x3_kernel(ConvLaunch a) {
     fence_async_smem();
     if (tid == 0) {
         for (int i = 0; i < NRING; ++i) {
-            mbar_init(smem_addr(&full[i]), 32);
+            mbar_init(smem_addr(&full[i]), PRODUCERS);
             mbar_init(smem_addr(&rowfree[i]), 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_addr(&tfull[i]), 1);
-            mbar_init(smem_addr(&tempty[i]), 128);
+            mbar_init(smem_addr(&tempty[i]), EPI_WARPS * 32);
         }
     }
     if (warp == 0) tmem_alloc(smem_addr(&tmem_slot), TCOLS);
@@ -246,81 +353,156 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3x3_kernel(ConvLaunch a) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    auto slot_addr = [&](int rr) { return s_ring + (uint32_t)((rr % NRING) * L::SLOT); };
+    auto slot_addr = [&](int slot) { return s_ring + (uint32_t)(slot * L::SLOT); };
 
     int ok = 1;
-    if (warp == 4) {
-        // producer: staged row rr (input row y_begin - 1 + rr) into slot rr % NRING
-        for (int rr = 0; rr < nrows; ++rr) {
-            if (rr >= NRING &&
-                !mbar_wait(smem_addr(&rowfree[rr % NRING]), ((rr / NRING) - 1) & 1)) {
-                ok = 0;
-                break;
-            }
-            constexpr int PLANES = CIN / 8;
-            const int yy = (((y_begin - 1 + rr) % a.H) + a.H) % a.H;
-            const uint16_t* row = a.x + ((size_t)b * a.H + yy) * (size_t)a.W * CIN;
-            const uint32_t dst = slot_addr(rr);
-            for (int t = lane; t < SLOTS * PLANES; t += 32) {
-                const int sl = t / PLANES, j = t - sl * PLANES;
-                int xx = x0 - 1 + sl;
+    if (warp > EPI_WARPS) {
+        // producers: input row y0 - 1 + rr of the item; a thread copies the same
+        // 16-byte pieces of every row
+        constexpr int PLANES = CIN / 8, PIECES = SLOTS * PLANES, PER = (PIECES + PRODUCERS - 1) / PRODUCERS;
+        RingPos put, give;  // the next slot to fill; the next to hand over
+        int filled = 0, given = 0;
+        for (int k = blockIdx.x; k < items && ok; k += gridDim.x) {
+            const ConvItem it = conv_item(a, k);
+            uint32_t src[PER];
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int t = u * PRODUCERS + tid - (EPI_WARPS + 1) * 32, sl = t / PLANES, j = t - sl * PLANES;
+                int xx = it.x0 - 1 + sl;
                 if (xx < 0) xx += a.W;
                 if (xx >= a.W) xx -= a.W;
-                cp_async16(dst + (uint32_t)(j * PLANE + sl * 16), row + (size_t)xx * CIN + j * 8);
+                src[u] = (uint32_t)(xx * CIN + j * 8);
             }
-            cp_async_commit();
-            if (rr >= 1) {  // the previous row's copies have landed: hand it over
-                cp_async_wait_group<1>();
-                fence_async_smem();
-                mbar_arrive_cta(smem_addr(&full[(rr - 1) % NRING]));
+            int yy = it.y0 == 0 ? a.H - 1 : it.y0 - 1;
+            for (int rr = 0; rr < it.nout + 2; ++rr) {
+                if (filled >= NRING && !mbar_wait(smem_addr(&rowfree[put.slot]), put.parity ^ 1u)) {
+                    ok = 0;
+                    break;
+                }
+                const uint16_t* row = a.x + ((size_t)it.b * a.H + yy) * (size_t)a.W * CIN;
+                if (++yy == a.H) yy = 0;
+                const uint32_t slot = slot_addr(put.slot);
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    const int t = u * PRODUCERS + tid - (EPI_WARPS + 1) * 32, sl = t / PLANES, j = t - sl * PLANES;
+                    if (u + 1 < PER || t < PIECES) cp_async16(slot + (uint32_t)(j * PLANE + sl * 16), row + src[u]);
+                }
+                cp_async_commit();
+                put.advance(NRING);
+                if (++filled > AHEAD) {  // that row's copies have landed: hand it over
+                    cp_async_wait_group<AHEAD>();
+                    fence_async_smem();
+                    mbar_arrive_cta(smem_addr(&full[give.slot]));
+                    give.advance(NRING);
+                    ++given;
+                }
             }
         }
         if (ok) {
             cp_async_wait_group<0>();
             fence_async_smem();
-            mbar_arrive_cta(smem_addr(&full[(nrows - 1) % NRING]));
+            for (; given < filled; ++given) {
+                mbar_arrive_cta(smem_addr(&full[give.slot]));
+                give.advance(NRING);
+            }
         }
-    } else if (warp == 5) {
+    } else if (warp == EPI_WARPS) {
         if (lane == 0) {
-            // MMA issuer: output row i reads staged rows i, i+1, i+2
-            for (int i = 0; i < nout && ok; ++i) {
-                for (int rr = (i == 0 ? 0 : i + 2); rr <= i + 2; ++rr)
-                    if (!mbar_wait(smem_addr(&full[rr % NRING]), (rr / NRING) & 1)) ok = 0;
-                if (ok && i >= 2 && !mbar_wait(smem_addr(&tempty[i & 1]), ((i >> 1) - 1) & 1)) ok = 0;
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)((i & 1) * COUT);
-                int k = 0;
+            // MMA issuer: output row r of a block reads its staged rows r, r+1, r+2
+            RingPos top;           // the slot of the block's first staged row
+            int blk = 0;           // blocks issued
+            for (int k = blockIdx.x; k < items && ok; k += gridDim.x) {
+                const int nout = conv_item(a, k).nout;
+                for (int done = 0; done < nout && ok; done += CONV_ROWS, ++blk) {
+                    const int nb = min(CONV_ROWS, nout - done);
+                    const bool last = done + nb == nout;
+                    if (blk >= 2 && !mbar_wait(smem_addr(&tempty[blk & 1]), ((blk >> 1) - 1) & 1)) ok = 0;
+                    const uint32_t d = tmem + (uint32_t)((blk & 1) * CONV_ROWS * COUT);
+                    RingPos at = top;
+                    for (int m = 0; m < nb + 2 && ok; ++m) {
+                        // staged row m, of output rows r0 .. r1
+                        if ((done == 0 || m >= 2) && !mbar_wait(smem_addr(&full[at.slot]), at.parity)) {
+                            ok = 0;
+                            break;
+                        }
+                        tc_fence_after();
+                        const int r0 = max(0, m - 2), r1 = min(m, nb - 1);
+                        // descriptors advance by (bytes >> 4) in their start-address field
+                        const uint64_t ad0 = umma_desc(slot_addr(at.slot), PLANE, 128);
+                        const uint64_t bd0 = umma_desc(s_w + (uint32_t)((2 - m + r0) * COUT * 16), 3 * COUT * 16, 128);
+                        // row m's accumulator starts with its first product
+                        const int old = min(r1 + 1, m) - r0;
 #pragma unroll
-                for (int t = 0; t < 9; ++t) {
-                    const int dy = t / 3, dx = t % 3;  // staged row i + dy, pixel offset dx
-                    const uint32_t arow = slot_addr(i + dy) + dx * 16;
-#pragma unroll
-                    for (int s = 0; s < KSTEPS; ++s, ++k) {
-                        const uint64_t ad = umma_desc(arow + 2 * s * PLANE, PLANE, 128);
-                        const uint64_t bd = umma_desc(s_w + (t * L::PLANES + 2 * s) * COUT * 16, COUT * 16, 128);
-                        mma_bf16(d, ad, bd, IDESC, k > 0 ? 1u : 0u);
+                        for (int q = 0; q < 3 * KSTEPS; ++q) {
+                            const int dx = q / KSTEPS, ks = q % KSTEPS;
+                            const uint64_t ad = ad0 + (uint64_t)(dx + 2 * ks * (PLANE >> 4));
+                            const uint64_t bd = bd0 + (uint64_t)((dx * L::PLANES + 2 * ks) * 3 * COUT);
+                            if (q == 0) {
+                                if (old > 0) mma_bf16(d + r0 * COUT, ad, bd, idesc_bf16(128, old * COUT), 1u);
+                                if (r1 == m) mma_bf16(d + m * COUT, ad, bd + old * COUT, idesc_bf16(128, COUT), 0u);
+                            } else {
+                                mma_bf16(d + r0 * COUT, ad, bd, idesc_bf16(128, (r1 - r0 + 1) * COUT), 1u);
+                            }
+                        }
+                        if (m < CONV_ROWS || last) mma_commit(smem_addr(&rowfree[at.slot]));  // its last reader
+                        at.advance(NRING);
+                        if (m < CONV_ROWS || last) top = at;
                     }
+                    if (ok) mma_commit(smem_addr(&tfull[blk & 1]));
                 }
-                mma_commit(smem_addr(&tfull[i & 1]));
-                mma_commit(smem_addr(&rowfree[i % NRING]));  // staged row i: its last reader
             }
         }
         __syncwarp();
     } else {
-        // epilogue warps 0-3: TMEM lanes 32*warp .. 32*warp + 31 = pixels
-        const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int i = 0; i < nout; ++i) {
-            // the TMEM load below is warp-aligned: the warp decides together
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_addr(&tfull[i & 1]), (i >> 1) & 1))) {
-                ok = 0;
-                break;
+        // epilogue warps: TMEM lanes 32*(warp%4) .. + 31 = pixels, rows warp/4, warp/4 + 2
+        const int quarter = warp & 3, half = warp >> 2;
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+        using E = RowEpilogue<COUT, EPI>;
+        E epi;
+        uint8_t* stage = smem + L::OFF_OUT + warp * E::BYTES;
+        // the warp's first pixel of row y of an item
+        auto pixel = [&](const ConvItem& it, int y) { return ((size_t)it.b * a.H + it.y0 + y) * a.W + it.x0 + quarter * 32; };
+        // first pixel of the warp's first row of item k, if there is one
+        auto first = [&](int k, size_t otherwise) {
+            if (k >= items) return otherwise;
+            const ConvItem it = conv_item(a, k);
+            return half < it.nout ? pixel(it, half) : otherwise;
+        };
+        int blk = 0;
+        size_t held = first(blockIdx.x, 0);  // the pixels whose mask is in registers
+        epi.prefetch(a, held, lane);
+        for (int k = blockIdx.x; k < items && ok; k += gridDim.x) {
+            const ConvItem it = conv_item(a, k);
+            for (int done = 0; done < it.nout; done += CONV_ROWS, ++blk) {
+                // the TMEM load below is warp-aligned: the warp decides together
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_addr(&tfull[blk & 1]), (blk >> 1) & 1))) {
+                    ok = 0;
+                    break;
+                }
+                tc_fence_after();
+                const int nb = min(CONV_ROWS, it.nout - done);
+                for (int r = half; r < nb; r += 2) {
+                    const size_t pix0 = pixel(it, done + r);
+                    float v[COUT];
+                    tmem_load<COUT>(lane_base + (uint32_t)(((blk & 1) * CONV_ROWS + r) * COUT), v);
+                    uint32_t bits = 0;
+                    if (EPI == EPI_MASK) {
+                        if (held != pix0) epi.prefetch(a, pix0, lane);
+                        bits = epi.mask_bits(lane);
+                        held = done + r + 2 < it.nout ? pix0 + 2 * (size_t)a.W : first(k + gridDim.x, pix0);
+                        epi.prefetch(a, held, lane);
+                    }
+                    if (EPI != EPI_BIAS_OUT) {  // the buffer's last copy has been read
+                        if (lane == 0) bulk_wait_read<0>();
+                        __syncwarp();
+                    }
+                    epi.finish(a, pix0, v, bits, stage, sbias, lane);
+                }
+                tc_fence_before();
+                mbar_arrive_cta(smem_addr(&tempty[blk & 1]));
             }
-            tc_fence_after();
-            conv_epilogue<COUT, EPI>(a, b, y_begin + i, x0, lane_base + (i & 1) * COUT, sbias, warp, lane);
-            tc_fence_before();
-            mbar_arrive_cta(smem_addr(&tempty[i & 1]));
         }
+        if (lane == 0) bulk_wait_read<0>();
     }
     cp_async_wait_all();
     ok = __syncthreads_and(ok);
@@ -604,13 +786,15 @@ __global__ void weight_image_kernel(const float* __restrict__ w, int cin, int co
     const int total = 9 * kcin * kcout;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
-    // img[((tap*(kcin/8) + j)*kcout + n)*8 + e] holds kernel weight (tap, out n, in 8j+e)
+    // img[(((dx*(kcin/8) + j)*3 + 2 - dy)*kcout + n)*8 + e] holds kernel weight
+    // (tap 3*dy + dx, out n, in 8j+e)
     const int e = i & 7;
     const int r = i >> 3;
     const int n = r % kcout;
     const int r2 = r / kcout;
-    const int j = r2 % (kcin / 8);
-    const int tap = r2 / (kcin / 8);
+    const int j = r2 / 3 % (kcin / 8);
+    const int dx = r2 / 3 / (kcin / 8);
+    const int tap = 3 * (2 - r2 % 3) + dx;
     const int kc = 8 * j + e;
     const float v = transpose ? w[((size_t)(8 - tap) * cout + kc) * cin + n] : w[((size_t)tap * cout + n) * cin + kc];
     const __nv_bfloat16 h = __float2bfloat16_rn(v);
@@ -648,12 +832,26 @@ __global__ void __launch_bounds__(RW_WARPS * 32) reduce_wgrad_kernel(const float
 }
 
 template <int CIN, int COUT, int EPI>
-int launch_conv_t(const ConvLaunch& a, cudaStream_t s) {
+int launch_conv_t(const ConvLaunch& a0, cudaStream_t s) {
     using L = ConvSmem<CIN, COUT>;
     const int attr = picgb::opt_in_dynamic_smem((const void*)conv3x3_kernel<CIN, COUT, EPI>, L::BYTES);
     if (attr != PIC_OK) return attr;
-    const dim3 grid(a.W / 128, (a.H + a.rows_per_cta - 1) / a.rows_per_cta, a.batch);
-    conv3x3_kernel<CIN, COUT, EPI><<<grid, CONV_THREADS, L::BYTES, s>>>(a);
+    // Rows of an item: a CTA stages two more than it puts out and computes, so long
+    // items are better, unless they leave CTAs without one.
+    const long long segs = (long long)a0.batch * (a0.W / 128), slots = 152 * L::CTAS;
+    ConvLaunch a = a0;
+    long long best = 0, items = 0;
+    for (int rows = CONV_ROWS; rows <= 64; rows += CONV_ROWS) {
+        const long long n = segs * ((a.H + rows - 1) / rows), cost = (n + slots - 1) / slots * (rows + 3);
+        if (best == 0 || cost < best) {
+            best = cost;
+            items = n;
+            a.rows = rows;
+        }
+        if (rows >= a.H) break;
+    }
+    if (items > INT_MAX) return picgb::fail(PIC_ERR_ARG, "convolution: too many pixels");
+    conv3x3_kernel<CIN, COUT, EPI><<<(unsigned)(items < slots ? items : slots), CONV_THREADS, L::BYTES, s>>>(a);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PIC_OK : picgb::cuda_fail(e, "conv3x3_kernel launch");
 }
@@ -731,8 +929,8 @@ int build_weight_image(const float* w_math, int cin, int cout, int transpose, ui
 }
 
 int launch_conv(const ConvLaunch& a, int kcin, int kcout, int epi, cudaStream_t s) {
-    if (a.W % 128 != 0 || a.W <= 0 || a.H <= 0 || a.batch <= 0 || a.rows_per_cta <= 0)
-        return picgb::fail(PIC_ERR_ARG, "convolution needs W a multiple of 128 and H, batch, rows > 0");
+    if (a.W % 128 != 0 || a.W <= 0 || a.H <= 0 || a.batch <= 0)
+        return picgb::fail(PIC_ERR_ARG, "convolution needs W a multiple of 128 and H, batch > 0");
     if (kcin == 16 && kcout == 16) return launch_conv_epi<16, 16>(a, epi, s);
     if (kcin == 16 && kcout == 32) return launch_conv_epi<16, 32>(a, epi, s);
     if (kcin == 32 && kcout == 16) return launch_conv_epi<32, 16>(a, epi, s);

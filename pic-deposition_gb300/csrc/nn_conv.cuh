@@ -28,8 +28,8 @@ struct ConvLaunch {
     const uint16_t* mask;  // NHWC, cout channels (EPI_MASK)
     void* y;               // output
     int batch, H, W;
-    int rows_per_cta;
     int* err;              // set to 1 when a wait on the tensor cores times out
+    int rows;              // output rows of a work item (filled by launch_conv)
 };
 
 struct WgradLaunch {

@@ -248,10 +248,9 @@ int ws_images(pic_ctx* c) {
 // Network forward on act[0] for nb samples -> s->out (FP32, nb*P).
 int ws_forward(pic_ctx* c, int nb) {
     WsState* s = c->ws;
-    const int rows = nb >= 4 ? 16 : 8;
     for (int l = 0; l < NL; ++l) {
         picnn::ConvLaunch a{s->act[l], s->img_f[l], s->params + s->off_b[l], nullptr,
-                            l < NL - 1 ? (void*)s->act[l + 1] : (void*)s->out, nb, s->H, s->W, rows, s->err};
+                            l < NL - 1 ? (void*)s->act[l + 1] : (void*)s->out, nb, s->H, s->W, s->err, 0};
         prof_begin(c, "conv_fwd");
         const int rc = picnn::launch_conv(a, CIN[l], COUT[l], l < NL - 1 ? picnn::EPI_BIAS_RELU : picnn::EPI_BIAS_OUT,
                                           c->stream);
@@ -265,7 +264,6 @@ int ws_forward(pic_ctx* c, int nb) {
 // Backward from dz16 (gradient at the output) into s->grad.
 int ws_backward(pic_ctx* c, int nb) {
     WsState* s = c->ws;
-    const int rows = nb >= 4 ? 16 : 8;
     const long long units = picnn::wgrad_units(nb, s->H, s->W);
     const int grid0 = picnn::wgrad_grid(units);
     const int upc = (int)((units + grid0 - 1) / grid0);
@@ -283,7 +281,7 @@ int ws_backward(pic_ctx* c, int nb) {
         c->launches += 2;
         if (l > 0) {
             uint16_t* next = bufs[l & 1];
-            picnn::ConvLaunch a{g, s->img_b[l], nullptr, s->act[l], next, nb, s->H, s->W, rows, s->err};
+            picnn::ConvLaunch a{g, s->img_b[l], nullptr, s->act[l], next, nb, s->H, s->W, s->err, 0};
             prof_begin(c, "conv_dgrad");
             const int rd = picnn::launch_conv(a, COUT[l], CIN[l], picnn::EPI_MASK, c->stream);
             prof_end(c);

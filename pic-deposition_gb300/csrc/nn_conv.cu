@@ -20,17 +20,16 @@
 // (dx+1)*16 bytes: im2col costs nothing. The weight image holds the three dy of a
 // dx side by side along N, the last first: output rows r, r+1, .. want m-r, m-r-1, ..
 // Warp-specialised: two warps stage rows
-// into a ring of 9 slots, one thread issues the MMAs of a block into one TMEM
+// into a ring of 7 slots or more, one thread issues the MMAs of a block into one TMEM
 // buffer while eight warps drain the block before from the other (bias + ReLU, or the
 // ReLU mask of the backward pass), handing over through mbarriers.
-// 32 to 32 channels, 512^2, batch 16: forward 131 us (171 a row at a time), 537 MB;
-// input gradient 152 us (194), 805 MB. Bound by memory and the chain
-// load - MMA - epilogue together: with a quarter of the MMAs 113 and 147 us.
+// 32 to 32 channels, 512^2, batch 16: forward 104 us (171 a row at a time), 537 MB;
+// input gradient 122 us (194), 805 MB, where a copy of as many bytes takes 80 and 120.
 //
-// Weight-gradient kernel (wgrad_kernel): D[(dy, ci)][(dx, co)] = sum over pixels
-// of x[p + (dy, dx)][ci] * dy[p][co], K = pixels, both operands MN-major as they
-// sit in NHWC memory (see the kernel's comment); the bias gradient is one more
-// MMA per K step against an all-ones operand. Each CTA accumulates its blocks
+// Weight-gradient kernel (wgrad_kernel): D[(x row, ci)][(dy row, co)] = sum over
+// pixels of x[row, px + dx][ci] * dy[row, px][co], K = pixels, both operands MN-major as
+// they sit in NHWC memory (see the kernel's comment); the bias gradient is an
+// MMA against an all-ones operand. Each CTA accumulates its blocks
 // of pixels in TMEM and writes one partial sum; reduce_wgrad adds the partials
 // in a fixed order, so gradients are identical run to run.
 //
@@ -50,7 +49,6 @@ namespace {
 
 constexpr int SLOTS = 130;             // pixels x0-1 .. x0+128
 constexpr int PLANE = SLOTS * 16;      // bytes per 8-channel plane
-constexpr int THREADS = 128;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -67,8 +65,10 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// Through L1 (.ca): the two halves of a 32-byte sector go to different planes, and .cg
+// asks L2 for each (twice the L2 reads; forward 131 us against 112, both with rings of 9).
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -121,6 +121,16 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
         "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// One lane of the warp. The issuing warp computes descriptors in all its lanes and only
+// the MMA itself is the elected lane's: they stay in uniform registers, where the
+// instruction takes them from (an MMA issued from one lane's branch took about 95
+// cycles whatever its size: weight gradient 159 us against 148, with 16 channels on one
+// side 152 against 108 and 120).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r != 0;
+}
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
@@ -133,6 +143,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
 }
+// 16 consecutive columns of this thread's TMEM lane set to zero
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+                 "r"(0)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 template <int N>
@@ -150,7 +167,9 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-__host__ __device__ constexpr uint32_t tmem_cols(int n) { return n <= 32 ? 32u : n <= 64 ? 64u : n <= 128 ? 128u : 256u; }
+__host__ __device__ constexpr uint32_t tmem_cols(int n) {
+    return n <= 32 ? 32u : n <= 64 ? 64u : n <= 128 ? 128u : n <= 256 ? 256u : 512u;
+}
 
 // ---------------------------------------------------------------------------
 // forward / input gradient
@@ -253,11 +272,16 @@ struct RowEpilogue {
 };
 
 constexpr int CONV_ROWS = 4;  // output rows per block
-constexpr int NRING = 9;      // staged rows: a block's 6 and three of the next one's 4
-constexpr int AHEAD = 3;      // rows whose copies are in flight behind the newest
 
 template <int CIN, int COUT>
 struct ConvSmem {
+    // Staged rows: a block's 6 and AHEAD of the next one's 4. AHEAD rows' copies are in
+    // flight behind the newest. Copies go through L1, of which shared memory leaves 60
+    // KB with two CTAs of 7 rows and 28 with more (32 to 32 channels, 512^2, batch 16:
+    // forward 105 us, input gradient 126, with 8 or 9 rows 112 and 154); the 16-channel
+    // outputs' CTAs are smaller (32 to 16: 82 us with 9, 112 with 7).
+    static constexpr int AHEAD = COUT == 32 ? 1 : 3;
+    static constexpr int NRING = 6 + AHEAD;
     static constexpr int PLANES = CIN / 8;
     static constexpr int SLOT = PLANES * PLANE;
     static constexpr int WBYTES = 9 * CIN * COUT * 2;
@@ -298,7 +322,7 @@ struct RingPos {
 // rowfree[s] (an MMA commit: the last block that reads slot s is done with it),
 // tfull[b] (an MMA commit: accumulator b holds a block), tempty[b] (the
 // epilogue's arrivals: accumulator b has been read). A block needs staged rows
-// 4i .. 4i+5 of its item; row 4i+5 is handed over once the copies three rows on are
+// 4i .. 4i+5 of its item; row 4i+5 is handed over once the copies AHEAD rows on are
 // issued, into the slot of row 4i-1, which the block before frees. Every wait is
 // bounded and no role waits at a CTA barrier inside the loop.
 constexpr int PRODUCERS = 64;
@@ -323,11 +347,13 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) conv3x3_kernel(ConvLaunch a) 
     using L = ConvSmem<CIN, COUT>;
     constexpr int KSTEPS = CIN / 16;
     constexpr uint32_t TCOLS = (uint32_t)L::TCOLS;
+    constexpr int NRING = L::NRING, AHEAD = L::AHEAD;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[NRING], rowfree[NRING], tfull[2], tempty[2];
     __shared__ uint32_t tmem_slot;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // the same in all lanes, for the compiler too
     const int items = a.batch * ((a.H + a.rows - 1) / a.rows) * (a.W / 128);
     const uint32_t s_w = smem_addr(smem);
     const uint32_t s_ring = s_w + L::OFF_RING;
@@ -352,7 +378,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) conv3x3_kernel(ConvLaunch a) 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     auto slot_addr = [&](int slot) { return s_ring + (uint32_t)(slot * L::SLOT); };
 
     int ok = 1;
@@ -407,49 +433,48 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) conv3x3_kernel(ConvLaunch a) 
             }
         }
     } else if (warp == EPI_WARPS) {
-        if (lane == 0) {
-            // MMA issuer: output row r of a block reads its staged rows r, r+1, r+2
-            RingPos top;           // the slot of the block's first staged row
-            int blk = 0;           // blocks issued
-            for (int k = blockIdx.x; k < items && ok; k += gridDim.x) {
-                const int nout = conv_item(a, k).nout;
-                for (int done = 0; done < nout && ok; done += CONV_ROWS, ++blk) {
-                    const int nb = min(CONV_ROWS, nout - done);
-                    const bool last = done + nb == nout;
-                    if (blk >= 2 && !mbar_wait(smem_addr(&tempty[blk & 1]), ((blk >> 1) - 1) & 1)) ok = 0;
-                    const uint32_t d = tmem + (uint32_t)((blk & 1) * CONV_ROWS * COUT);
-                    RingPos at = top;
-                    for (int m = 0; m < nb + 2 && ok; ++m) {
-                        // staged row m, of output rows r0 .. r1
-                        if ((done == 0 || m >= 2) && !mbar_wait(smem_addr(&full[at.slot]), at.parity)) {
-                            ok = 0;
-                            break;
-                        }
-                        tc_fence_after();
-                        const int r0 = max(0, m - 2), r1 = min(m, nb - 1);
-                        // descriptors advance by (bytes >> 4) in their start-address field
-                        const uint64_t ad0 = umma_desc(slot_addr(at.slot), PLANE, 128);
-                        const uint64_t bd0 = umma_desc(s_w + (uint32_t)((2 - m + r0) * COUT * 16), 3 * COUT * 16, 128);
-                        // row m's accumulator starts with its first product
-                        const int old = min(r1 + 1, m) - r0;
-#pragma unroll
-                        for (int q = 0; q < 3 * KSTEPS; ++q) {
-                            const int dx = q / KSTEPS, ks = q % KSTEPS;
-                            const uint64_t ad = ad0 + (uint64_t)(dx + 2 * ks * (PLANE >> 4));
-                            const uint64_t bd = bd0 + (uint64_t)((dx * L::PLANES + 2 * ks) * 3 * COUT);
-                            if (q == 0) {
-                                if (old > 0) mma_bf16(d + r0 * COUT, ad, bd, idesc_bf16(128, old * COUT), 1u);
-                                if (r1 == m) mma_bf16(d + m * COUT, ad, bd + old * COUT, idesc_bf16(128, COUT), 0u);
-                            } else {
-                                mma_bf16(d + r0 * COUT, ad, bd, idesc_bf16(128, (r1 - r0 + 1) * COUT), 1u);
-                            }
-                        }
-                        if (m < CONV_ROWS || last) mma_commit(smem_addr(&rowfree[at.slot]));  // its last reader
-                        at.advance(NRING);
-                        if (m < CONV_ROWS || last) top = at;
+        const bool leader = elect_one();
+        // MMA issuer: output row r of a block reads its staged rows r, r+1, r+2
+        RingPos top;           // the slot of the block's first staged row
+        int blk = 0;           // blocks issued
+        for (int k = blockIdx.x; k < items && ok; k += gridDim.x) {
+            const int nout = conv_item(a, k).nout;
+            for (int done = 0; done < nout && ok; done += CONV_ROWS, ++blk) {
+                const int nb = min(CONV_ROWS, nout - done);
+                const bool last = done + nb == nout;
+                if (blk >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_addr(&tempty[blk & 1]), ((blk >> 1) - 1) & 1))) ok = 0;
+                const uint32_t d = tmem + (uint32_t)((blk & 1) * CONV_ROWS * COUT);
+                RingPos at = top;
+                for (int m = 0; m < nb + 2 && ok; ++m) {
+                    // staged row m, of output rows r0 .. r1
+                    if ((done == 0 || m >= 2) && !__all_sync(0xffffffffu, mbar_wait(smem_addr(&full[at.slot]), at.parity))) {
+                        ok = 0;
+                        break;
                     }
-                    if (ok) mma_commit(smem_addr(&tfull[blk & 1]));
+                    tc_fence_after();
+                    const int r0 = max(0, m - 2), r1 = min(m, nb - 1);
+                    // descriptors advance by (bytes >> 4) in their start-address field
+                    const uint64_t ad0 = umma_desc(slot_addr(at.slot), PLANE, 128);
+                    const uint64_t bd0 = umma_desc(s_w + (uint32_t)((2 - m + r0) * COUT * 16), 3 * COUT * 16, 128);
+                    // row m's accumulator starts with its first product
+                    const int old = min(r1 + 1, m) - r0;
+#pragma unroll
+                    for (int q = 0; q < 3 * KSTEPS; ++q) {
+                        const int dx = q / KSTEPS, ks = q % KSTEPS;
+                        const uint64_t ad = ad0 + (uint64_t)(dx + 2 * ks * (PLANE >> 4));
+                        const uint64_t bd = bd0 + (uint64_t)((dx * L::PLANES + 2 * ks) * 3 * COUT);
+                        if (q == 0) {
+                            if (old > 0 && leader) mma_bf16(d + r0 * COUT, ad, bd, idesc_bf16(128, old * COUT), 1u);
+                            if (r1 == m && leader) mma_bf16(d + m * COUT, ad, bd + old * COUT, idesc_bf16(128, COUT), 0u);
+                        } else {
+                            if (leader) mma_bf16(d + r0 * COUT, ad, bd, idesc_bf16(128, (r1 - r0 + 1) * COUT), 1u);
+                        }
+                    }
+                    if ((m < CONV_ROWS || last) && leader) mma_commit(smem_addr(&rowfree[at.slot]));  // its last reader
+                    at.advance(NRING);
+                    if (m < CONV_ROWS || last) top = at;
                 }
+                if (ok && leader) mma_commit(smem_addr(&tfull[blk & 1]));
             }
         }
         __syncwarp();
@@ -518,137 +543,128 @@ __global__ void __launch_bounds__(CONV_THREADS, 2) conv3x3_kernel(ConvLaunch a) 
 // ---------------------------------------------------------------------------
 // weight gradient
 // ---------------------------------------------------------------------------
-// Both operands are MN-major: A[m][k] = x with m = (row offset, channel) and
-// k = pixel, B[k][n] = dy with n = output channel. Staged as 8-channel planes
+// Both operands are MN-major: A[m][k] = x with m = (row, channel) and
+// k = pixel, B[k][n] = dy with n = (row, output channel). Staged as 8-channel planes
 // (16 bytes per pixel slot) they are the canonical MN-major no-swizzle layout:
 // a core matrix is 8 pixels (K, 16 B apart) of 8 channels (MN, contiguous); K
 // core matrices are 128 B apart (LBO), MN core matrices one plane apart (SBO).
-// With the staged x rows of a block one after the other, the 16 MN core
-// matrices of an M = 128 operand starting at row i are rows i .. i + 128/CIN - 1:
-// rows i, i+1, i+2 are the taps dy = -1, 0, 1 of output row i (the rest is
-// discarded), and the tap dx moves the start by one 16-byte pixel slot. The
-// bias gradient is one more MMA per K step, of a constant all-ones A.
+// With the staged rows of a block one after the other, the 16 MN core
+// matrices of an M = 128 operand starting at x row i are rows i .. i + 128/CIN - 1,
+// and those of an N = 2 COUT operand dy rows i and i + 1: with a the x row and b the
+// dy row of the product, a - b = 0, 1, 2 are the taps dy = -1, 0, 1 (the rest is
+// discarded). The tap dx moves A's start by one 16-byte pixel slot.
+// Bias gradient: an all-ones A against all the dy rows of the block, N = 256
+// (COUT = 32). A block is 26 MMAs where one dy row at a time took 64.
+// Planes are an odd number of 16-byte slots apart, so that the core matrices of an
+// operand do not share banks (little matters: 182 to 176 us at 32 x 32 channels,
+// 512^2, batch 16, together with bias MMAs over all rows instead of four).
+// TMEM starts at zero: an odd last row's MMAs write the first dy row's columns alone.
 //
-// Staging: a row of a block is one TMA copy (cp.async.bulk.tensor) of a box of
-// 8 channels x 34 (or 40) pixels x planes through a 5-D view of the NHWC tensor whose
-// pixel stride is the pixel's size and whose plane stride is 16 bytes, so the
-// box lands plane by plane; the periodic row wrap is the row coordinate. The two
-// segments at the ends of an image row, whose pixel halo wraps around, are
-// staged with cp.async by three warps instead.
-constexpr int WG_ROWS = 8;    // output rows per block
-constexpr int WG_PX = 32;     // output pixels per block (one K segment)
-constexpr int WG_SLOTS = 34;  // x pixels used: x0-1 .. x0+32
-constexpr int WG_DPLANE = WG_PX * 16;
-constexpr int WG_NBUF = 2;    // blocks in the shared-memory ring
-constexpr int WG_ONES = 16 * 256;  // all-ones A operand: 16 MN x 2 K core matrices
+// Staging: cp.async, whole 64-byte pixels per four lanes. (TMA boxes of 8 channels x 34
+// pixels x planes read L2 in 16-byte pieces: 2.1 GB of sectors for 0.64 GB.)
+constexpr int WG_ROWS = 8;           // output rows per block
+constexpr int WG_XROWS = WG_ROWS + 2;
+constexpr int WG_PX = 32;            // output pixels per block (one K segment)
+constexpr int WG_SLOTS = 34;         // x pixels: x0-1 .. x0+32
+constexpr int WG_XPLANE = 35 * 16;
+constexpr int WG_DPLANE = 33 * 16;
+constexpr int WG_NBUF = 4;           // blocks in the shared-memory ring
+constexpr int WG_LAG = 1;            // blocks whose copies are in flight behind the newest
+constexpr int WG_ONES = 16 * 256;    // all-ones A operand: 16 MN x 2 K core matrices
+constexpr int WG_THREADS = 256;
+constexpr int WG_PRODUCERS = WG_THREADS - 32;
 
 template <int CIN, int COUT>
 struct WgSmem {
-    static constexpr int G = 128 / CIN;                 // x rows spanned by one M = 128 operand
-    static constexpr int XROWS = WG_ROWS + G - 1;       // staged x rows per block
-    // x pixels per TMA box: the 34 used, or 40 where 34 would leave the rows off
-    // the 128-byte alignment of a TMA destination
-    static constexpr int XBOX = ((CIN / 8) * 34 * 16) % 128 == 0 ? 34 : 40;
-    static constexpr int XPLANE = XBOX * 16;
-    static constexpr int XROW = (CIN / 8) * XPLANE;     // bytes per staged x row
+    static constexpr int XROW = (CIN / 8) * WG_XPLANE;  // bytes per staged x row
     static constexpr int DROW = (COUT / 8) * WG_DPLANE;
-    static constexpr int XBYTES = XROWS * XROW;
+    static constexpr int XBYTES = WG_XROWS * XROW;
     static constexpr int DBYTES = WG_ROWS * DROW;
     static constexpr int BUF = (XBYTES + DBYTES + 127) / 128 * 128;
     static constexpr int OFF_ONES = WG_NBUF * BUF;
-    static constexpr int BYTES = OFF_ONES + WG_ONES;
+    // one CTA on an SM: with 32 channels it takes all 512 TMEM columns
+    static constexpr int BYTES = OFF_ONES + WG_ONES > 116 * 1024 ? OFF_ONES + WG_ONES : 116 * 1024;
+    static constexpr int BIAS_COL = 6 * COUT;           // columns before: 2 * COUT per dx
+    static constexpr int COLS = BIAS_COL + WG_ROWS * COUT;
+    static constexpr uint32_t TCOLS = tmem_cols(COLS);
+    // an M = 128 operand at the last pair's row ends inside the allocation
+    static_assert((WG_ROWS - 2 + 128 / CIN) * XROW <= BUF + WG_ONES, "A operand");
 };
-
-__device__ __forceinline__ void cp_async_wait_all_groups() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive(uint32_t a) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_tx(uint32_t a, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, int c1, int c2, int c3, int c4,
-                                            uint32_t mbar) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
-        "%6}], [%7];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(mbar)
-        : "memory");
-}
 
 // Instruction descriptor of kind::f16 with both operands MN-major.
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n) {
     return idesc_bf16(m, n) | (1u << 15) | (1u << 16);
 }
 
+// A block of the CTA's range: 32-pixel segments fastest, then rows, then images.
 struct WgBlock {
     int b, y0, x0, rows;
-    bool edge;  // the x halo wraps around the image row: staged with cp.async
+    __device__ __forceinline__ WgBlock(const WgradLaunch& a, long long blk) {
+        const int segs = a.W / WG_PX, yblocks = (a.H + WG_ROWS - 1) / WG_ROWS;
+        x0 = (int)(blk % segs) * WG_PX;
+        y0 = (int)(blk / segs % yblocks) * WG_ROWS;
+        b = (int)(blk / segs / yblocks);
+        rows = min(WG_ROWS, a.H - y0);
+    }
+    __device__ __forceinline__ void advance(const WgradLaunch& a) {
+        x0 += WG_PX;
+        if (x0 < a.W) return;
+        x0 = 0;
+        y0 += WG_ROWS;
+        if (y0 >= a.H) {
+            y0 = 0;
+            ++b;
+        }
+        rows = min(WG_ROWS, a.H - y0);
+    }
 };
 
-__device__ __forceinline__ WgBlock wg_block(const WgradLaunch& a, long long blk) {
-    const int segs = a.W / WG_PX, yblocks = (a.H + WG_ROWS - 1) / WG_ROWS;
-    WgBlock k;
-    const int seg = (int)(blk % segs);
-    const long long r2 = blk / segs;
-    k.y0 = (int)(r2 % yblocks) * WG_ROWS;
-    k.b = (int)(r2 / yblocks);
-    k.x0 = seg * WG_PX;
-    k.rows = min(WG_ROWS, a.H - k.y0);
-    k.edge = seg == 0 || seg == segs - 1;
-    return k;
-}
-
-// cp.async staging of a block by the 96 producer threads (pt = 0..95): the same
-// layout as the TMA boxes (slots past 33 of a plane, if any, are not written or read).
+// Copies of a block by producer thread pt: x rows y0 - 1 .. y0 + rows, dy rows y0 ..
 template <int CIN, int COUT>
-__device__ __forceinline__ void wg_stage_cp(const WgradLaunch& a, const WgBlock& k, uint32_t buf, int pt) {
+__device__ __forceinline__ void wg_stage(const WgradLaunch& a, const WgBlock& k, uint32_t buf, int pt) {
     using L = WgSmem<CIN, COUT>;
     constexpr int XP = CIN / 8, DP = COUT / 8;
     const size_t img = (size_t)k.b * a.H;
-    int ystart = (k.y0 - 1) % a.H;
-    if (ystart < 0) ystart += a.H;
-    for (int u = pt; u < XP * WG_SLOTS; u += 96) {
-        const int sl = u / XP, j = u % XP;
+    for (int u = pt; u < (k.rows + 2) * WG_SLOTS * XP; u += WG_PRODUCERS) {
+        const int r = u / (WG_SLOTS * XP), p = u - r * (WG_SLOTS * XP), sl = p / XP, j = p % XP;
         int xx = k.x0 - 1 + sl;
         if (xx < 0) xx += a.W;
         if (xx >= a.W) xx -= a.W;
-        const uint16_t* col = a.x + (size_t)xx * CIN + j * 8;
-        int yy = ystart;
-#pragma unroll
-        for (int r = 0; r < L::XROWS; ++r) {
-            cp_async16(buf + (uint32_t)(r * L::XROW + j * L::XPLANE + sl * 16), col + (img + yy) * (size_t)a.W * CIN);
-            if (++yy == a.H) yy = 0;
-        }
+        int yy = k.y0 - 1 + r;
+        if (yy < 0) yy += a.H;
+        if (yy >= a.H) yy %= a.H;
+        cp_async16(buf + (uint32_t)(r * L::XROW + j * WG_XPLANE + sl * 16),
+                   a.x + ((img + yy) * (size_t)a.W + xx) * CIN + j * 8);
     }
-    for (int u = pt; u < DP * WG_PX; u += 96) {
-        const int sl = u / DP, j = u % DP;
-        const uint16_t* col = a.dy + ((img + k.y0) * a.W + k.x0 + sl) * COUT + j * 8;
-        for (int r = 0; r < k.rows; ++r)
-            cp_async16(buf + (uint32_t)(L::XBYTES + r * L::DROW + j * WG_DPLANE + sl * 16), col + (size_t)r * a.W * COUT);
+    const uint16_t* dy = a.dy + ((img + k.y0) * (size_t)a.W + k.x0) * COUT;
+    for (int u = pt; u < k.rows * WG_PX * DP; u += WG_PRODUCERS) {
+        const int r = u / (WG_PX * DP), p = u % (WG_PX * DP), sl = p / DP, j = p % DP;
+        cp_async16(buf + (uint32_t)(L::XBYTES + r * L::DROW + j * WG_DPLANE + sl * 16), dy + (size_t)r * a.W * COUT + p * 8);
     }
 }
 
-// Warp-specialised pipeline over a ring of WG_NBUF buffers. Warps 1-3 are the
-// producers (lane 0 of warp 1 issues the TMA copies; all three warps stage the
-// edge blocks with cp.async); lane 0 of warp 0 issues the MMAs. full[b] takes one
-// arrival from every producer thread for every block (after its cp.async copies
-// landed; the TMA issuer's arrival carries the expected bytes) and says buffer b
+// One CTA per SM. Warps 1-7 are the producers; lane 0 of warp 0 issues the MMAs.
+// full[b] takes one arrival from every producer thread for every block (after its
+// copies landed, WG_LAG blocks later) and says buffer b
 // holds a block; empty[b] (the MMAs' commit) says the tensor cores are done with
 // it. Every producer thread waits on empty and arrives on full for every block,
 // so no thread is ever more than one phase away from a barrier it waits on (a
 // parity wait needs that), and no producer waits for another, so a wait that
 // runs out cannot strand the rest.
+// 32 x 32 channels, 512^2, batch 16: 148 us, 185 with TMA staging and one dy row per MMA
+// (when the MMAs took 181 us and the staging 172 by themselves; now the MMAs take 98).
+// Bound by staging through L1, 0.6 GB. Four buffers and one block's lag leave L1 more
+// room than five and two (160 us).
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(THREADS) wgrad_kernel(const __grid_constant__ WgradLaunch a) {
+__global__ void __launch_bounds__(WG_THREADS) wgrad_kernel(WgradLaunch a) {
     using L = WgSmem<CIN, COUT>;
-    constexpr uint32_t IDESC = idesc_bf16_mn(128, COUT);
-    constexpr uint32_t TCOLS = tmem_cols(4 * COUT);
     constexpr int MPAD = 9 * CIN + 1;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[WG_NBUF], empty[WG_NBUF];
     __shared__ uint32_t tmem_slot;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // the same in all lanes, for the compiler too
     const long long total = (long long)a.batch * ((a.H + WG_ROWS - 1) / WG_ROWS) * (a.W / WG_PX);
     const long long k_begin = (long long)blockIdx.x * a.units_per_cta;
     const int nk = (int)max(0ll, min(total, k_begin + a.units_per_cta) - k_begin);
@@ -657,86 +673,90 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const __grid_constant__ 
 
     {  // the all-ones operand of the bias MMAs (BF16 1.0)
         uint4* o = reinterpret_cast<uint4*>(smem + L::OFF_ONES);
-        for (int i = tid; i < WG_ONES / 16; i += THREADS) o[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+        for (int i = tid; i < WG_ONES / 16; i += WG_THREADS) o[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
     }
     fence_async_smem();
     if (tid == 0) {
         for (int i = 0; i < WG_NBUF; ++i) {
-            mbar_init(smem_addr(&full[i]), 96);
+            mbar_init(smem_addr(&full[i]), WG_PRODUCERS);
             mbar_init(smem_addr(&empty[i]), 1);
         }
     }
-    if (warp == 0) tmem_alloc(smem_addr(&tmem_slot), TCOLS);
+    if (warp == 0) tmem_alloc(smem_addr(&tmem_slot), L::TCOLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    if (warp < 4) {
+#pragma unroll 4
+        for (int c = 0; c < L::COLS; c += 16) tmem_zero16(lanes + c);
+        tmem_wait_st();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
 
     int ok = 1;
     if (warp > 0) {
         const int pt = tid - 32;
-        for (int k = 0; k < nk; ++k) {
+        WgBlock blk(a, k_begin);
+        for (int k = 0; k < nk; ++k, blk.advance(a)) {
             const int bsel = k % WG_NBUF;
-            const uint32_t buf = s0 + (uint32_t)(bsel * L::BUF);
-            const uint32_t fb = smem_addr(&full[bsel]);
-            const WgBlock blk = wg_block(a, k_begin + k);
             if (k >= WG_NBUF && !mbar_wait(smem_addr(&empty[bsel]), ((k / WG_NBUF) - 1) & 1)) {
                 ok = 0;
                 break;
             }
-            if (blk.edge) {
-                wg_stage_cp<CIN, COUT>(a, blk, buf, pt);
-                cp_async_commit();
-                cp_async_wait_all_groups();
+            wg_stage<CIN, COUT>(a, blk, s0 + (uint32_t)(bsel * L::BUF), pt);
+            cp_async_commit();
+            if (k >= WG_LAG) {
+                cp_async_wait_group<WG_LAG>();
                 fence_async_smem();
-                mbar_arrive(fb);
-            } else if (pt != 0) {
-                mbar_arrive(fb);
-            } else {
-                mbar_arrive_tx(fb, (uint32_t)(L::XROWS * L::XROW + blk.rows * L::DROW));
-                int yy = (blk.y0 - 1) % a.H;
-                if (yy < 0) yy += a.H;
-                for (int r = 0; r < L::XROWS; ++r) {
-                    tma_load_5d(buf + (uint32_t)(r * L::XROW), &a.tmx, blk.x0 - 1, 0, yy, blk.b, fb);
-                    if (++yy == a.H) yy = 0;
-                }
-                for (int r = 0; r < blk.rows; ++r)
-                    tma_load_5d(buf + (uint32_t)(L::XBYTES + r * L::DROW), &a.tmdy, blk.x0, 0, blk.y0 + r, blk.b, fb);
+                mbar_arrive_cta(smem_addr(&full[(k - WG_LAG) % WG_NBUF]));
             }
         }
-    } else if (lane == 0) {
-        bool first = true;
+        if (ok) {
+            cp_async_wait_group<0>();
+            fence_async_smem();
+            for (int k = max(0, nk - WG_LAG); k < nk; ++k) mbar_arrive_cta(smem_addr(&full[k % WG_NBUF]));
+        }
+    } else {
+        const bool leader = elect_one();
         const uint64_t ones = umma_desc(s0 + (uint32_t)L::OFF_ONES, 128, 256);
-        for (int k = 0; k < nk; ++k) {
+        WgBlock blk(a, k_begin);
+        for (int k = 0; k < nk; ++k, blk.advance(a)) {
             const int bsel = k % WG_NBUF;
             const uint32_t buf = s0 + (uint32_t)(bsel * L::BUF);
-            if (!mbar_wait(smem_addr(&full[bsel]), (k / WG_NBUF) & 1)) {
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_addr(&full[bsel]), (k / WG_NBUF) & 1))) {
                 ok = 0;
                 break;
             }
             tc_fence_after();
-            const int rows = wg_block(a, k_begin + k).rows;
+            const int rows = blk.rows;
             // descriptors advance by (bytes >> 4) in their start-address field
-            const uint64_t a0 = umma_desc(buf, 128, L::XPLANE);
+            const uint64_t a0 = umma_desc(buf, 128, WG_XPLANE);
             const uint64_t b0 = umma_desc(buf + (uint32_t)L::XBYTES, 128, WG_DPLANE);
-            for (int i = 0; i < rows; ++i) {
+            for (int i = 0; i < rows; i += 2) {
+                const uint32_t idesc = idesc_bf16_mn(128, i + 1 < rows ? 2 * COUT : COUT);
 #pragma unroll
                 for (int kk = 0; kk < WG_PX / 16; ++kk) {
                     const uint64_t bd = b0 + (uint64_t)((i * L::DROW + 16 * kk * 16) >> 4);
-                    const uint32_t acc = (first && kk == 0) ? 0u : 1u;
 #pragma unroll
                     for (int dx = 0; dx < 3; ++dx) {
                         const uint64_t ad = a0 + (uint64_t)((i * L::XROW + (16 * kk + dx) * 16) >> 4);
-                        mma_bf16(tmem + (uint32_t)(dx * COUT), ad, bd, IDESC, acc);
+                        if (leader) mma_bf16(tmem + (uint32_t)(dx * 2 * COUT), ad, bd, idesc, 1u);
                     }
-                    mma_bf16(tmem + (uint32_t)(3 * COUT), ones, bd, IDESC, acc);
                 }
-                first = false;
             }
-            mma_commit(smem_addr(&empty[bsel]));
+#pragma unroll
+            for (int kk = 0; kk < WG_PX / 16; ++kk)
+                if (leader)
+                    mma_bf16(tmem + (uint32_t)L::BIAS_COL, ones, b0 + (uint64_t)((16 * kk * 16) >> 4),
+                             idesc_bf16_mn(128, rows * COUT), 1u);
+            if (leader) mma_commit(smem_addr(&empty[bsel]));
         }
     }
-    cp_async_wait_all_groups();
+    cp_async_wait_all();
     __syncwarp();
     ok = __syncthreads_and(ok);
     if (ok && nk > 0) {
@@ -744,39 +764,54 @@ __global__ void __launch_bounds__(THREADS) wgrad_kernel(const __grid_constant__ 
         ok = __syncthreads_and(mbar_wait(smem_addr(&empty[last % WG_NBUF]), (last / WG_NBUF) & 1));
         if (ok) {
             tc_fence_after();
-            // TMEM lane m = (row offset dyi, channel ci); column dx * COUT + co;
-            // columns 3 * COUT + co: the bias gradient (every lane the same)
-            if (warp * 32 < 3 * CIN) {
-                const int m = warp * 32 + lane, dyi = m / CIN, ci = m % CIN;
+            // TMEM lane m = (x row a, channel ci), columns dx * 2 COUT + b * COUT + co:
+            // tap row dyi is a = dyi, b = 0 plus a = dyi + 1, b = 1, which goes
+            // through shared memory (the ring is free)
+            float* other = reinterpret_cast<float*>(smem);  // [dyi][ci][co]
+            const int m = warp * 32 + lane, xr = m / CIN, ci = m % CIN;
+            for (int dx = 0; dx < 3; ++dx) {
+                float v[COUT];
+                if (warp * 32 < 4 * CIN) {  // warps of x rows 0 .. 3
+                    tmem_load<COUT>(lanes + (uint32_t)((dx * 2 + 1) * COUT), v);
+                    if (xr >= 1 && xr <= 3) {
 #pragma unroll
-                for (int dx = 0; dx < 3; ++dx) {
-                    float v[COUT];
-                    tmem_load<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dx * COUT), v);
-                    if (dyi < 3) {
-                        float* row = part + (size_t)((dyi * 3 + dx) * CIN + ci) * COUT;
-#pragma unroll
-                        for (int c = 0; c < COUT; ++c) row[c] = v[c];
+                        for (int c = 0; c < COUT; ++c) other[((xr - 1) * CIN + ci) * (COUT + 1) + c] = v[c];
                     }
                 }
+                __syncthreads();
+                if (warp * 32 < 4 * CIN) {
+                    tmem_load<COUT>(lanes + (uint32_t)(dx * 2 * COUT), v);
+                    if (xr < 3) {
+                        float* row = part + (size_t)((xr * 3 + dx) * CIN + ci) * COUT;
+#pragma unroll
+                        for (int c = 0; c < COUT; ++c) row[c] = v[c] + other[(xr * CIN + ci) * (COUT + 1) + c];
+                    }
+                }
+                __syncthreads();
             }
-            if (warp == 0) {
-                float v[COUT];
-                tmem_load<COUT>(tmem + (uint32_t)(3 * COUT), v);
+            if (warp == 0) {  // every lane the same: columns (dy row, channel)
+                float s[COUT] = {};
+                for (int r = 0; r < WG_ROWS; ++r) {
+                    float v[COUT];
+                    tmem_load<COUT>(tmem + (uint32_t)(L::BIAS_COL + r * COUT), v);
+#pragma unroll
+                    for (int c = 0; c < COUT; ++c) s[c] += v[c];
+                }
                 if (lane == 0) {
 #pragma unroll
-                    for (int c = 0; c < COUT; ++c) part[(size_t)9 * CIN * COUT + c] = v[c];
+                    for (int c = 0; c < COUT; ++c) part[(size_t)9 * CIN * COUT + c] = s[c];
                 }
             }
         }
     } else if (ok) {
-        for (int i = tid; i < MPAD * COUT; i += THREADS) part[i] = 0.0f;
+        for (int i = tid; i < MPAD * COUT; i += WG_THREADS) part[i] = 0.0f;
     }
     if (!ok && tid == 0) atomicExch(a.err, 1);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, TCOLS);
+        tmem_dealloc(tmem, L::TCOLS);
     }
 }
 
@@ -856,52 +891,12 @@ int launch_conv_t(const ConvLaunch& a0, cudaStream_t s) {
     return e == cudaSuccess ? PIC_OK : picgb::cuda_fail(e, "conv3x3_kernel launch");
 }
 
-typedef CUresult (*TensorMapEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                           const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                           CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-int tensor_map_encoder(TensorMapEncodeTiledFn* out) {
-    static TensorMapEncodeTiledFn fn = nullptr;
-    if (!fn) {
-        cudaDriverEntryPointQueryResult q;
-        const cudaError_t e =
-            cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void**)&fn, 12000, cudaEnableDefault, &q);
-        if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn) {
-            fn = nullptr;
-            return picgb::fail(PIC_ERR_UNSUPPORTED, "the driver does not provide cuTensorMapEncodeTiled");
-        }
-    }
-    *out = fn;
-    return PIC_OK;
-}
-
-// 5-D view of an NHWC BF16 tensor with C channels: (8 channels, pixel, 8-channel
-// plane, row, image), pixel stride C * 2 bytes and plane stride 16 bytes, and a
-// box of 8 channels x `px` pixels x all planes of one row, which lands in shared
-// memory as planes of `px` 16-byte pixel slots.
-int encode_planes_map(CUtensorMap* m, const uint16_t* base, int C, int batch, int H, int W, int px) {
-    TensorMapEncodeTiledFn enc;
-    PIC_TRY(tensor_map_encoder(&enc));
-    const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)(C / 8), (cuuint64_t)H, (cuuint64_t)batch};
-    const cuuint64_t strides[4] = {(cuuint64_t)C * 2, 16, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    const cuuint32_t box[5] = {8, (cuuint32_t)px, (cuuint32_t)(C / 8), 1, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<uint16_t*>(base), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return picgb::fail(PIC_ERR_CUDA, "cuTensorMapEncodeTiled failed for the weight gradient");
-    return PIC_OK;
-}
-
 template <int CIN, int COUT>
-int launch_wgrad_t(const WgradLaunch& a0, int grid, cudaStream_t s) {
+int launch_wgrad_t(const WgradLaunch& a, int grid, cudaStream_t s) {
     using L = WgSmem<CIN, COUT>;
     const int attr = picgb::opt_in_dynamic_smem((const void*)wgrad_kernel<CIN, COUT>, L::BYTES);
     if (attr != PIC_OK) return attr;
-    WgradLaunch a = a0;
-    PIC_TRY(encode_planes_map(&a.tmx, a.x, CIN, a.batch, a.H, a.W, L::XBOX));
-    PIC_TRY(encode_planes_map(&a.tmdy, a.dy, COUT, a.batch, a.H, a.W, WG_PX));
-    wgrad_kernel<CIN, COUT><<<grid, THREADS, L::BYTES, s>>>(a);
+    wgrad_kernel<CIN, COUT><<<grid, WG_THREADS, L::BYTES, s>>>(a);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PIC_OK : picgb::cuda_fail(e, "wgrad_kernel launch");
 }
@@ -939,7 +934,7 @@ int launch_conv(const ConvLaunch& a, int kcin, int kcout, int epi, cudaStream_t 
 }
 
 int wgrad_grid(long long units) {
-    const long long g = units < 2 * 152 ? units : 2 * 152;
+    const long long g = units < 152 ? units : 152;
     return (int)(g < 1 ? 1 : g);
 }
 

@@ -7,7 +7,6 @@
 //     y[b,y,x,co] = bias[co] + sum_{dy,dx,ci} x[b,(y+dy)%H,(x+dx)%W,ci] * w[tap][co][ci].
 #pragma once
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -39,7 +38,6 @@ struct WgradLaunch {
     int batch, H, W;
     int units_per_cta;   // blocks (8 rows x 32 pixels of one image) per CTA
     int* err;
-    CUtensorMap tmx, tmdy;  // TMA views of x and dy (filled by launch_wgrad)
 };
 
 // Bytes of a weight image for (cin, cout).

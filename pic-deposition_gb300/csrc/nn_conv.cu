@@ -124,8 +124,8 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
 // One lane of the warp. The issuing warp computes descriptors in all its lanes and only
 // the MMA itself is the elected lane's: they stay in uniform registers, where the
 // instruction takes them from (an MMA issued from one lane's branch took about 95
-// cycles whatever its size: weight gradient 159 us against 148, with 16 channels on one
-// side 152 against 108 and 120).
+// cycles whatever its size: weight gradient, with 7 staging warps, 159 us against 148,
+// with 16 channels on one side 152 against 108 and 120).
 __device__ __forceinline__ bool elect_one() {
     uint32_t r;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n}" : "=r"(r));
@@ -568,10 +568,10 @@ constexpr int WG_PX = 32;            // output pixels per block (one K segment)
 constexpr int WG_SLOTS = 34;         // x pixels: x0-1 .. x0+32
 constexpr int WG_XPLANE = 35 * 16;
 constexpr int WG_DPLANE = 33 * 16;
-constexpr int WG_NBUF = 4;           // blocks in the shared-memory ring
+constexpr int WG_NBUF = 3;           // blocks in the shared-memory ring
 constexpr int WG_LAG = 1;            // blocks whose copies are in flight behind the newest
 constexpr int WG_ONES = 16 * 256;    // all-ones A operand: 16 MN x 2 K core matrices
-constexpr int WG_THREADS = 256;
+constexpr int WG_THREADS = 512;
 constexpr int WG_PRODUCERS = WG_THREADS - 32;
 
 template <int CIN, int COUT>
@@ -643,7 +643,7 @@ __device__ __forceinline__ void wg_stage(const WgradLaunch& a, const WgBlock& k,
     }
 }
 
-// One CTA per SM. Warps 1-7 are the producers; lane 0 of warp 0 issues the MMAs.
+// One CTA per SM. Warps 1-15 are the producers; lane 0 of warp 0 issues the MMAs.
 // full[b] takes one arrival from every producer thread for every block (after its
 // copies landed, WG_LAG blocks later) and says buffer b
 // holds a block; empty[b] (the MMAs' commit) says the tensor cores are done with
@@ -651,10 +651,10 @@ __device__ __forceinline__ void wg_stage(const WgradLaunch& a, const WgBlock& k,
 // so no thread is ever more than one phase away from a barrier it waits on (a
 // parity wait needs that), and no producer waits for another, so a wait that
 // runs out cannot strand the rest.
-// 32 x 32 channels, 512^2, batch 16: 148 us, 185 with TMA staging and one dy row per MMA
+// 32 x 32 channels, 512^2, batch 16: 124 us, 185 with TMA staging and one dy row per MMA
 // (when the MMAs took 181 us and the staging 172 by themselves; now the MMAs take 98).
-// Bound by staging through L1, 0.6 GB. Four buffers and one block's lag leave L1 more
-// room than five and two (160 us).
+// Bound by staging through L1, 0.6 GB: 15 producer warps (7: 142 us, 23: 130); three
+// buffers leave L1 more room than four (131 us; with 7 warps 148, five 160).
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(WG_THREADS) wgrad_kernel(WgradLaunch a) {
     using L = WgSmem<CIN, COUT>;

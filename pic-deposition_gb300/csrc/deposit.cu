@@ -47,6 +47,7 @@
 // Compiled with --fmad=false: no multiply-add is fused, so every FP32 result
 // equals the oracle's (compiled with -ffp-contract=off).
 #include "cells.cuh"
+#include "diag.cuh"
 #include "pic_internal.cuh"
 
 namespace picgb {
@@ -1667,10 +1668,17 @@ __device__ void choose_any_order(DevStats* st, unsigned long long limit, unsigne
 // inv_vol * 2^-24, or, for the exact integer TSC form, max|q| * inv_vol * (qn *
 // 2^-30) (scale != 0); each thread forms it, and the first also stores it and,
 // with n > 0, takes the any-order decision of a deposit between sorts: two
-// launches fewer per deposit.
-__global__ void fixed_to_rho(const long long* __restrict__ acc, size_t g, double background, double inv_vol,
+// launches fewer per deposit. In a time step one more block ends the diagnostics of the
+// step before, whose sums this step's move and that step's solve have left: by
+// itself it was a link of the step's chain of launches (64^2, 16 per cell: 54.6 us a
+// step against 52.4; 256^2, TSC: 88.5 against 85.6).
+__global__ void __launch_bounds__(RED_THREADS) fixed_to_rho(const long long* __restrict__ acc, size_t g, double background, double inv_vol,
                              double scale, DevStats* st, double* __restrict__ unit_out, double* __restrict__ rho,
-                             unsigned long long limit, unsigned long long n) {
+                             unsigned long long limit, unsigned long long n, FinalArgs diag) {
+    if (diag.r && blockIdx.x == gridDim.x - 1) {
+        diag_block(diag);
+        return;
+    }
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const double unit = scale == 0.0 ? charge_unit(st, inv_vol)
                                      : __dmul_rn(__dmul_rn((double)load_maxq(st), inv_vol), scale);
@@ -1817,7 +1825,7 @@ static int launch_deposit(pic_ctx* c, const DepArgs& a, int kind, bool adaptive)
     return check_launch(c, "deposit_atomic");
 }
 
-int deposit_rho(pic_ctx* c, int scheme, double dt, double background) {
+int deposit_rho(pic_ctx* c, int scheme, double dt, double background, const FinalArgs* diag) {
     if (scheme < PIC_SCHEME_NGP || scheme > PIC_SCHEME_ESIRKEPOV) return fail(PIC_ERR_ARG, "unknown scheme");
     int tiled;  // kernel kind, see launch_deposit
     if (c->order_mode == PIC_ORDER_SORTED) {
@@ -1893,9 +1901,10 @@ int deposit_rho(pic_ctx* c, int scheme, double dt, double background) {
                              ? (double)c->qn_uniform * 0x1p-30
                              : 0.0;
     const bool decide = c->n > 0 && tiled == 0 && adaptive && !c->sorted;
-    fixed_to_rho<<<(unsigned)((c->G + 1023) / 1024), 256, 0, c->stream>>>(
+    fixed_to_rho<<<(unsigned)((c->G + 1023) / 1024) + (diag ? 1 : 0), RED_THREADS, 0, c->stream>>>(
         c->acc, c->G, background, inv_vol, scale, c->dstats, c->unitbuf, c->rho,
-        (unsigned long long)(any_order_fraction(scheme) * (double)c->n), decide ? (unsigned long long)c->n : 0ull);
+        (unsigned long long)(any_order_fraction(scheme) * (double)c->n), decide ? (unsigned long long)c->n : 0ull,
+        diag ? *diag : FinalArgs{});
     PIC_TRY(check_launch(c, "fixed_to_rho"));
     c->grid_sums_ready = 0;
     c->last_scheme = scheme;

@@ -209,13 +209,16 @@ int make_own_fft(pic_ctx* ctx);
 int own_fft_solve(pic_ctx* ctx);
 // hist, step (both or neither): also write the step's pic_diag into the history
 // and advance the step counter
+struct FinalArgs;  // diag.cuh
 int diagnostics_async(pic_ctx* ctx, double* hist = nullptr, int* step = nullptr, int steps = 0);
+int diagnostics_partials(pic_ctx* ctx, double* hist, int* step, int steps, FinalArgs* out);
 int read_diagnostics(pic_ctx* ctx, pic_diag* d);
 void release_fields(pic_ctx* ctx);
 void release_rbgs(pic_ctx* ctx);
 void release_current(pic_ctx* ctx);
 // Deposit (deposit.cu).
-int deposit_rho(pic_ctx* ctx, int scheme, double dt, double background);
+// diag: the last stage of the diagnostics, for the deposit's last kernel to run
+int deposit_rho(pic_ctx* ctx, int scheme, double dt, double background, const FinalArgs* diag = nullptr);
 // Red-black Gauss-Seidel pieces (rbgs.cu): right-hand side b = rho*dV - mean into
 // the solver's buffer; r = b - A phi; the 5-point operator's coefficients; a
 // solve from the phi in the context.

@@ -23,6 +23,7 @@
 // step with and without the sort are captured as CUDA graphs and replayed.
 #include <vector>
 
+#include "diag.cuh"
 #include "pic_internal.cuh"
 
 namespace picgb {
@@ -59,7 +60,8 @@ static int record_step(pic_ctx* c, double* hist, int* step_ctr, int steps) {
 // the previous step's gather runs fused with this step's push (kick of step
 // s-1 and drift of step s in one pass over the particles, push.cu's fused
 // kernel), then the previous step's diagnostics (the push leaves the velocities
-// unchanged); the last step's gather runs after the loop.
+// unchanged), whose last stage the deposit's last kernel runs; the last step's gather
+// runs after the loop.
 static int one_step(pic_ctx* c, const pic_run_config* cfg, bool do_sort, double* hist, int* step_ctr, int steps,
                     bool head, unsigned long long* moved) {
     auto count_moved = [&]() -> int {
@@ -75,14 +77,15 @@ static int one_step(pic_ctx* c, const pic_run_config* cfg, bool do_sort, double*
         PIC_TRY(move(c, cfg->dt, true, false, true));
         return record_step(c, hist, step_ctr, steps);
     }
+    FinalArgs diag;
     if (head) {
         PIC_TRY(move(c, cfg->dt, true, true, true));
-        PIC_TRY(record_step(c, hist, step_ctr, steps));
+        PIC_TRY(diagnostics_partials(c, hist, step_ctr, steps, &diag));
     } else {
         PIC_TRY(move(c, cfg->dt, false, true));
     }
     if (do_sort) PIC_TRY(sort_particles(c));
-    PIC_TRY(deposit_rho(c, cfg->scheme, cfg->dt, cfg->background));
+    PIC_TRY(deposit_rho(c, cfg->scheme, cfg->dt, cfg->background, head ? &diag : nullptr));
     PIC_TRY(count_moved());
     return solve(c, cfg);
 }

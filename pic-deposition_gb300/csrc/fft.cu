@@ -7,10 +7,10 @@
 //     (fields.cu fft_scale: volume / k^2 / (nx ny)), inverse transform;
 //   fft_rows_inverse: the two rows' frequencies back into one complex transform,
 //     its real and imaginary parts the two rows of phi.
-// A transform is the autosorting (Stockham) radix-8 form of Govindaraju et al.,
-// "High performance discrete Fourier transforms on graphics processors", SC 2008:
-// thread j of n/8 holds elements j + m n/8, a step is a radix-8 butterfly in
-// registers and an exchange through shared memory, and a last step of radix 2 or 4
+// A transform is the autosorting (Stockham) form of Govindaraju et al.,
+// "High performance discrete Fourier transforms on graphics processors", SC 2008, of
+// radix E = 8 or 4: thread j of n/E holds elements j + m n/E, a step is a butterfly in
+// registers and an exchange through shared memory, and a last step of a smaller radix
 // completes n. Twiddles come from a table of exp(-2 pi i k / n).
 //
 // Bound by FP64 arithmetic, of which an SM does two multiply-adds per cycle: about
@@ -80,40 +80,43 @@ __device__ __forceinline__ void eight(C2 (&v)[8]) {
 __device__ __forceinline__ int padded(int i) { return i + (i >> 3); }
 __host__ __device__ constexpr int region(int n) { return n + n / 8 + 2; }
 
-// N-point transform of the elements j + m N/8 in v (N/8 threads, j < N/8), in natural
-// order in the same places; NS: what the steps so far cover. sm: this transform's
-// region (free when the call begins).
-template <int N, bool INV, int NS = 1>
-__device__ __forceinline__ void transform(C2 (&v)[8], int j, double2* sm, const double2* __restrict__ tw) {
-    constexpr int T = N / 8;
-    if constexpr (N / NS >= 8) {
+// N-point transform of the elements j + m N/E in v (N/E threads, j < N/E; E is 8 or 4,
+// the radix), in natural order in the same places; NS: what the steps so far cover. sm:
+// this transform's region (free when the call begins).
+template <int N, bool INV, int NS = 1, int E>
+__device__ __forceinline__ void transform(C2 (&v)[E], int j, double2* sm, const double2* __restrict__ tw) {
+    constexpr int T = N / E;
+    if constexpr (N / NS >= E) {
         if constexpr (NS > 1) {
-            const int step = (j & (NS - 1)) * (N / (NS * 8));
+            const int step = (j & (NS - 1)) * (N / (NS * E));
 #pragma unroll
-            for (int r = 1; r < 8; ++r) {
+            for (int r = 1; r < E; ++r) {
                 double2 w = __ldg(tw + step * r);
                 if (INV) w.y = -w.y;
                 v[r] = cmul(v[r], w);
             }
         }
-        eight<INV>(v);
-        if constexpr (NS * 8 < N) {
-            const int base = (j / NS) * NS * 8 + (j & (NS - 1));
+        if constexpr (E == 8)
+            eight<INV>(v);
+        else
+            four<INV>(v[0], v[1], v[2], v[3]);
+        if constexpr (NS * E < N) {
+            const int base = (j / NS) * NS * E + (j & (NS - 1));
             __syncthreads();
 #pragma unroll
-            for (int r = 0; r < 8; ++r) sm[padded(base + r * NS)] = make_double2(v[r].x, v[r].y);
+            for (int r = 0; r < E; ++r) sm[padded(base + r * NS)] = make_double2(v[r].x, v[r].y);
             __syncthreads();
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
+            for (int m = 0; m < E; ++m) {
                 const double2 e = sm[padded(j + m * T)];
                 v[m] = {e.x, e.y};
             }
-            transform<N, INV, NS * 8>(v, j, sm, tw);
+            transform<N, INV, NS * E>(v, j, sm, tw);
         }
     } else {
-        // radix 4 (two butterflies per thread) or 2 (four): butterfly j + b N/8 of
-        // elements v[b + r 8/R], back into the same places
-        constexpr int R = N / NS, B = 8 / R;
+        // radix 4 (two butterflies per thread) or 2 (four, of E = 4 two): butterfly
+        // j + b N/E of elements v[b + r E/R], back into the same places
+        constexpr int R = N / NS, B = E / R;
 #pragma unroll
         for (int b = 0; b < B; ++b) {
 #pragma unroll
@@ -130,26 +133,36 @@ __device__ __forceinline__ void transform(C2 (&v)[8], int j, double2* sm, const 
     }
 }
 
+// Where the transforms are few (up to four per SM) and of at most 1024 elements, each is
+// a block of its own with four elements per thread, radix 4: a warp's FP64 instruction
+// takes its SM 16 cycles however many of its lanes work, a transform's chain of them is
+// the kernel's time, and in radix 8 with fewer threads the chain is twice as long. Many
+// transforms fill the SMs either way and radix 8 has less to do. us per step, radix 8
+// against radix 4: 64^2 53 and 44, 256^2 (TSC) 86 and 71, 512^2 121 and 105, 64 x 1024 90
+// and 67; with sides of 2048 taking it too, or more transforms, 100 and 102 at 2048 x 64,
+// 98 and 99 at 64 x 2048.
+constexpr int SMALL_MAX = 1024, SMALL_COUNT = 608;
+
 // transforms of a block: whole warps of small ones
 __host__ __device__ constexpr int row_batch(int n) { return n / 8 >= 32 ? 1 : 32 / (n / 8); }
 
-template <int N>
-__global__ void __launch_bounds__(row_batch(N) * (N / 8)) fft_rows_forward(const double* __restrict__ in, int pairs,
+template <int N, int E, int RB>
+__global__ void __launch_bounds__(RB * (N / E)) fft_rows_forward(const double* __restrict__ in, int pairs,
                                                                            const double2* __restrict__ tw,
                                                                            double2* __restrict__ spec) {
-    constexpr int T = N / 8, NH = N / 2 + 1;
-    __shared__ double2 smem[row_batch(N) * region(N)];
-    const int j = threadIdx.x % T, f = blockIdx.x * row_batch(N) + threadIdx.x / T;
+    constexpr int T = N / E, NH = N / 2 + 1;
+    __shared__ double2 smem[RB * region(N)];
+    const int j = threadIdx.x % T, f = blockIdx.x * RB + threadIdx.x / T;
     double2* sm = smem + (threadIdx.x / T) * region(N);
     const bool on = f < pairs;
     const double* r0 = in + (size_t)f * 2 * N;
-    C2 v[8];
+    C2 v[E];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) v[m] = on ? C2{r0[j + m * T], r0[N + j + m * T]} : C2{0.0, 0.0};
+    for (int m = 0; m < E; ++m) v[m] = on ? C2{r0[j + m * T], r0[N + j + m * T]} : C2{0.0, 0.0};
     transform<N, false>(v, j, sm, tw);
     __syncthreads();
 #pragma unroll
-    for (int m = 0; m < 8; ++m) sm[padded(j + m * T)] = make_double2(v[m].x, v[m].y);
+    for (int m = 0; m < E; ++m) sm[padded(j + m * T)] = make_double2(v[m].x, v[m].y);
     __syncthreads();
     if (!on) return;
     // twice the rows' frequencies: Z[k] + conj Z[-k] and -i (Z[k] - conj Z[-k]); the
@@ -162,19 +175,19 @@ __global__ void __launch_bounds__(row_batch(N) * (N / 8)) fft_rows_forward(const
     }
 }
 
-template <int N>
-__global__ void __launch_bounds__(row_batch(N) * (N / 8)) fft_rows_inverse(const double2* __restrict__ spec, int pairs,
+template <int N, int E, int RB>
+__global__ void __launch_bounds__(RB * (N / E)) fft_rows_inverse(const double2* __restrict__ spec, int pairs,
                                                                            const double2* __restrict__ tw,
                                                                            double* __restrict__ out) {
-    constexpr int T = N / 8, NH = N / 2 + 1;
-    __shared__ double2 smem[row_batch(N) * region(N)];
-    const int j = threadIdx.x % T, f = blockIdx.x * row_batch(N) + threadIdx.x / T;
+    constexpr int T = N / E, NH = N / 2 + 1;
+    __shared__ double2 smem[RB * region(N)];
+    const int j = threadIdx.x % T, f = blockIdx.x * RB + threadIdx.x / T;
     double2* sm = smem + (threadIdx.x / T) * region(N);
     const bool on = f < pairs;
     const double2* s0 = spec + (size_t)f * 2 * NH;
-    C2 v[8];
+    C2 v[E];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
+    for (int m = 0; m < E; ++m) {
         const int k = j + m * T, kk = k <= N / 2 ? k : N - k;
         double2 a = make_double2(0.0, 0.0), b = a;
         if (on) {
@@ -189,7 +202,7 @@ __global__ void __launch_bounds__(row_batch(N) * (N / 8)) fft_rows_inverse(const
     if (!on) return;
     double* r0 = out + (size_t)f * 2 * N;
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
+    for (int m = 0; m < E; ++m) {
         r0[j + m * T] = v[m].x;
         r0[N + j + m * T] = v[m].y;
     }
@@ -198,32 +211,32 @@ __global__ void __launch_bounds__(row_batch(N) * (N / 8)) fft_rows_inverse(const
 // columns of a block: 64-byte row segments, less where a transform needs 128 threads or more
 __host__ __device__ constexpr int col_batch(int n) { return n <= 512 ? 4 : n <= 1024 ? 2 : 1; }
 
-template <int N>
-__global__ void __launch_bounds__(col_batch(N) * (N / 8)) fft_columns(double2* __restrict__ spec, int nh,
+template <int N, int E, int CB>
+__global__ void __launch_bounds__(CB * (N / E)) fft_columns(double2* __restrict__ spec, int nh,
                                                                       const double2* __restrict__ tw,
                                                                       const double* __restrict__ scale) {
-    constexpr int T = N / 8, CB = col_batch(N);
+    constexpr int T = N / E;
     extern __shared__ double2 csm[];
     const int c = threadIdx.x % CB, j = threadIdx.x / CB, col = blockIdx.x * CB + c;
     double2* sm = csm + c * region(N);
     const bool on = col < nh;
     double2* s = spec + col;
-    C2 v[8];
+    C2 v[E];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
+    for (int m = 0; m < E; ++m) {
         const double2 e = on ? s[(size_t)(j + m * T) * nh] : make_double2(0.0, 0.0);
         v[m] = {e.x, e.y};
     }
-    double f[8];
+    double f[E];
 #pragma unroll
-    for (int m = 0; m < 8; ++m) f[m] = on ? scale[(size_t)(j + m * T) * nh + col] : 0.0;
+    for (int m = 0; m < E; ++m) f[m] = on ? scale[(size_t)(j + m * T) * nh + col] : 0.0;
     transform<N, false>(v, j, sm, tw);
 #pragma unroll
-    for (int m = 0; m < 8; ++m) v[m] = {__dmul_rn(v[m].x, f[m]), __dmul_rn(v[m].y, f[m])};
+    for (int m = 0; m < E; ++m) v[m] = {__dmul_rn(v[m].x, f[m]), __dmul_rn(v[m].y, f[m])};
     transform<N, true>(v, j, sm, tw);
     if (!on) return;
 #pragma unroll
-    for (int m = 0; m < 8; ++m) s[(size_t)(j + m * T) * nh] = make_double2(v[m].x, v[m].y);
+    for (int m = 0; m < E; ++m) s[(size_t)(j + m * T) * nh] = make_double2(v[m].x, v[m].y);
 }
 
 __global__ void make_twiddles(double2* __restrict__ tw, int n) {
@@ -234,25 +247,36 @@ __global__ void make_twiddles(double2* __restrict__ tw, int n) {
     tw[k] = make_double2(c, -s);
 }
 
-template <int N>
-int rows(pic_ctx* c, const double2* tw, const double* in, double2* spec, double* out) {
+template <int N, int E, int RB>
+int rows_as(pic_ctx* c, const double2* tw, const double* in, double2* spec, double* out) {
     const int pairs = c->Ny / 2;
-    const unsigned blocks = (unsigned)((pairs + row_batch(N) - 1) / row_batch(N));
+    const unsigned blocks = (unsigned)((pairs + RB - 1) / RB);
     if (in)
-        fft_rows_forward<N><<<blocks, row_batch(N) * (N / 8), 0, c->stream>>>(in, pairs, tw, spec);
+        fft_rows_forward<N, E, RB><<<blocks, RB * (N / E), 0, c->stream>>>(in, pairs, tw, spec);
     else
-        fft_rows_inverse<N><<<blocks, row_batch(N) * (N / 8), 0, c->stream>>>(spec, pairs, tw, out);
+        fft_rows_inverse<N, E, RB><<<blocks, RB * (N / E), 0, c->stream>>>(spec, pairs, tw, out);
     return check_launch(c, in ? "fft_rows_forward" : "fft_rows_inverse");
 }
+template <int N>
+int rows(pic_ctx* c, const double2* tw, const double* in, double2* spec, double* out) {
+    if constexpr (N <= SMALL_MAX)
+        if (c->Ny / 2 <= SMALL_COUNT) return rows_as<N, 4, 1>(c, tw, in, spec, out);
+    return rows_as<N, 8, row_batch(N)>(c, tw, in, spec, out);
+}
 
+template <int N, int E, int CB>
+int columns_as(pic_ctx* c, const double2* tw, double2* spec) {
+    const int nh = c->Nx / 2 + 1;
+    const size_t smem = (size_t)CB * region(N) * sizeof(double2);
+    PIC_TRY(opt_in_dynamic_smem((const void*)fft_columns<N, E, CB>, smem));
+    fft_columns<N, E, CB><<<(unsigned)((nh + CB - 1) / CB), CB * (N / E), smem, c->stream>>>(spec, nh, tw, c->fft_scale);
+    return check_launch(c, "fft_columns");
+}
 template <int N>
 int columns(pic_ctx* c, const double2* tw, double2* spec) {
-    const int nh = c->Nx / 2 + 1;
-    const size_t smem = (size_t)col_batch(N) * region(N) * sizeof(double2);
-    PIC_TRY(opt_in_dynamic_smem((const void*)fft_columns<N>, smem));
-    fft_columns<N><<<(unsigned)((nh + col_batch(N) - 1) / col_batch(N)), col_batch(N) * (N / 8), smem, c->stream>>>(
-        spec, nh, tw, c->fft_scale);
-    return check_launch(c, "fft_columns");
+    if constexpr (N <= SMALL_MAX)
+        if (c->Nx / 2 + 1 <= SMALL_COUNT) return columns_as<N, 4, 1>(c, tw, spec);
+    return columns_as<N, 8, col_batch(N)>(c, tw, spec);
 }
 
 #define PIC_FFT_SIZES(X) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048)

@@ -371,8 +371,12 @@ int pic_gpu_ws_study(pic_ctx* ctx, int steps, double dt, double background, int 
  * Particles are generated on the device (counter-based random numbers, seed per
  * run): x from the density 1 + amplitude*cos(2*pi*x/N), y uniform, Maxwellian v
  * of thermal speed vth; charge -1/ppc and mass 1/ppc per particle (mean charge
- * density -1, omega_p = 1). Each run's state equals that of the same run
- * advanced alone through pic_gpu_run (scheme CIC, FFT Poisson, background 1). */
+ * density -1, omega_p = 1). Each run advances as the same run alone through
+ * pic_gpu_run (scheme CIC, FFT Poisson, background 1) does: from equal fields the
+ * particles, the int64 charge and rho are equal bit for bit. The solves round
+ * differently (here cuFFT, a division by k^2 and a factor 1/N^2; there see
+ * pic_gpu_poisson_fft), so phi agrees to FP64 rounding and later steps as far as
+ * the plasma does not amplify that. */
 typedef struct pic_ens pic_ens;
 typedef struct pic_ens_member {
     int N;          /* grid N x N (even) */

@@ -25,9 +25,12 @@
 // deposit's tile shape per (grid size, particles per cell) class is picked by
 // timing candidate shapes on the first sorted step (the autotuner).
 //
-// Every arithmetic operation on a particle or a cell is the one the single-run
-// path performs (push.cu, deposit.cu, fields.cu), so each run's particles and
-// fields equal, bit for bit, those of the same run advanced alone.
+// Every arithmetic operation on a particle, on the charge grid and from phi to E is
+// the one the single-run path performs (push.cu, deposit.cu, fields.cu efield): from
+// equal fields a step's particles, int64 charge and rho equal, bit for bit, those of
+// the same run advanced alone. The solve is not: a batched cuFFT plan, a division by
+// k^2 and a multiplication by 1/N^2 here, fft.cu's transforms or cuFFT and one factor
+// vol/(k^2 N^2) there, so phi agrees to FP64 rounding.
 #include <cuda_runtime.h>
 #include <cufft.h>
 

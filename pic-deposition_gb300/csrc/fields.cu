@@ -384,10 +384,28 @@ int solve_discrete_fft(pic_ctx* c, const double* b, double* phi) {
     return check_launch(c, "scale_phi");
 }
 
+// The particle set's charge sums (total charge, sum |q|) into red_out[8], red_out[9]:
+// they change only with the set, so once per set. A time step that is captured must
+// find them done: four kernels over the charges would be replayed with every step.
+int ensure_charge_sums(pic_ctx* c) {
+    PIC_TRY(ensure_fields(c));
+    if (c->qsum_valid) return PIC_OK;
+    SumArgs a{};
+    a.st = c->dstats;
+    a.q = c->q;
+    a.n = c->n;
+    a.kind = SUM_Q;
+    PIC_TRY(device_sum(c, a, c->red_out + 8));
+    a.kind = SUM_ABS_Q;
+    PIC_TRY(device_sum(c, a, c->red_out + 9));
+    c->qsum_valid = 1;
+    return PIC_OK;
+}
+
 // Queues the six diagnostics into c->red_out[0..5] (pic_diag order) but for their last
 // stage, which the caller launches: it also records them in a time step's history.
 int diagnostics_partials(pic_ctx* c, double* hist, int* step, int steps, FinalArgs* out) {
-    PIC_TRY(ensure_fields(c));
+    PIC_TRY(ensure_charge_sums(c));
     SumArgs a{};
     a.st = c->dstats;
     a.q = c->q;
@@ -395,13 +413,6 @@ int diagnostics_partials(pic_ctx* c, double* hist, int* step, int steps, FinalAr
     a.vy = c->vy;
     a.m = c->has_mass ? c->m : nullptr;
     a.n = c->n;
-    if (!c->qsum_valid) {  // total charge and sum |q| change only with the particle set
-        a.kind = SUM_Q;
-        PIC_TRY(device_sum(c, a, c->red_out + 8));
-        a.kind = SUM_ABS_Q;
-        PIC_TRY(device_sum(c, a, c->red_out + 9));
-        c->qsum_valid = 1;
-    }
     FinalArgs f{};
     f.r = c->red_out;
     f.vol = c->dx * c->dy;

@@ -213,6 +213,7 @@ struct FinalArgs;  // diag.cuh
 int diagnostics_async(pic_ctx* ctx, double* hist = nullptr, int* step = nullptr, int steps = 0);
 int diagnostics_partials(pic_ctx* ctx, double* hist, int* step, int steps, FinalArgs* out);
 int read_diagnostics(pic_ctx* ctx, pic_diag* d);
+int ensure_charge_sums(pic_ctx* ctx);
 void release_fields(pic_ctx* ctx);
 void release_rbgs(pic_ctx* ctx);
 void release_current(pic_ctx* ctx);

@@ -50,11 +50,6 @@ static int solve(pic_ctx* c, const pic_run_config* cfg) {
     return cfg->rbgs_warm > 0 ? ws_record_solution(c) : PIC_OK;
 }
 
-// The diagnostics of the step whose gather has just run.
-static int record_step(pic_ctx* c, double* hist, int* step_ctr, int steps) {
-    return diagnostics_async(c, hist, step_ctr, steps);
-}
-
 // One step; `do_sort` selects the variant with the cell sort. For NGP/CIC/TSC
 // the step ends after its Poisson solve with its gather pending: with `head`,
 // the previous step's gather runs fused with this step's push (kick of step
@@ -75,7 +70,7 @@ static int one_step(pic_ctx* c, const pic_run_config* cfg, bool do_sort, double*
         PIC_TRY(solve(c, cfg));
         PIC_TRY(move(c, cfg->dt, false, true));
         PIC_TRY(move(c, cfg->dt, true, false, true));
-        return record_step(c, hist, step_ctr, steps);
+        return diagnostics_async(c, hist, step_ctr, steps);
     }
     FinalArgs diag;
     if (head) {
@@ -219,7 +214,7 @@ int run_steps(pic_ctx* c, const pic_run_config* cfg, int steps, pic_diag* histor
     rc = [&]() -> int {
         PIC_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(int), c->stream));
         PIC_CUDA_TRY(cudaMemsetAsync(&c->dstats->moved, 0, sizeof(unsigned long long), c->stream));
-        PIC_TRY(ensure_fields(c));
+        PIC_TRY(ensure_charge_sums(c));  // before any capture
         const int k = cfg->sort_interval;
         // the Gauss-Seidel stop is decided on the host, so those steps run eagerly
         const bool graph = cfg->use_graph && cfg->poisson == 0;
@@ -262,7 +257,14 @@ int run_steps(pic_ctx* c, const pic_run_config* cfg, int steps, pic_diag* histor
                 StepGraph sg;
                 sg.do_sort = do_sort;
                 sg.before = now;
-                PIC_TRY(capture(c, cfg, do_sort, hist, ctr, steps, head, moved, &sg.exec));
+                const int ke_ready = c->ke_ready, grid_ready = c->grid_sums_ready;
+                const int cap = capture(c, cfg, do_sort, hist, ctr, steps, head, moved, &sg.exec);
+                if (cap != PIC_OK) {  // nothing of the step has run: what the host side set is taken back
+                    set_buffers(c, now);
+                    c->ke_ready = ke_ready;
+                    c->grid_sums_ready = grid_ready;
+                    return cap;
+                }
                 sg.after = buffers_of(c);  // the capture ran the host side: pointers as the graph leaves them
                 sg.kernels = do_sort ? c->graph_launches_sort : c->graph_launches_plain;
                 graphs.push_back(sg);
@@ -275,7 +277,7 @@ int run_steps(pic_ctx* c, const pic_run_config* cfg, int steps, pic_diag* histor
         }
         if (!esk) {  // the last step's gather and diagnostics
             PIC_TRY(move(c, cfg->dt, true, false, true));
-            PIC_TRY(record_step(c, hist, ctr, steps));
+            PIC_TRY(diagnostics_async(c, hist, ctr, steps));
         }
         if (history)
             PIC_CUDA_TRY(cudaMemcpyAsync(history, hist, (size_t)steps * 6 * sizeof(double), cudaMemcpyDeviceToHost,

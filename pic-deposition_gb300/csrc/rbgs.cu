@@ -724,6 +724,12 @@ static int rbgs_solve_mixed(pic_ctx* c, const RbArgs& a, double tol, int max_ite
         res = s[2] > 0.0 ? std::sqrt(s[1] / s[2]) : std::sqrt(s[1]);
         if (outer == 0) c->first_rbgs_resid = res;
         if (res <= tol || it >= max_iters) break;
+        const int left = max_iters - it;
+        if (left < 4) {  // the FP32 sweeps come in fours, as the check interval does: the last few in FP64
+            PIC_TRY(rb_sweeps(c, a, left));
+            it += left;
+            continue;
+        }
         rb_residual_field<<<gb, 256, 0, c->stream>>>(a, c->phi, r64);
         PIC_TRY(check_launch(c, "rb_residual_field"));
         rb_to_f32<<<gb, 256, 0, c->stream>>>(r64, c->G, r32, e32);
@@ -738,20 +744,20 @@ static int rbgs_solve_mixed(pic_ctx* c, const RbArgs& a, double tol, int max_ite
             int it64 = 0;
             double r64v = 0.0;
             const double first = c->first_rbgs_resid;
-            const int prc = rbgs_solve_persistent(c, a, tol, (max_iters - it) & ~1, check_every & ~1 ? check_every & ~1 : 2,
+            const int prc = rbgs_solve_persistent(c, a, tol, left & ~1, check_every & ~1 ? check_every & ~1 : 2,
                                                   &it64, &r64v);
             c->first_rbgs_resid = first;
             if (prc == PIC_OK) {
                 it += it64;
                 res = r64v;
-                break;
+                if (res <= tol || it >= max_iters) break;
+                continue;
             }
             if (prc != PIC_ERR_UNSUPPORTED) return prc;
         }
         prev_res = res;
-        // sweeps come in fours, as the check interval does
         const PsArgs<float> p{e32, r32, xb32, c->Nx, c->Ny, t.ntx, t.nty, (float)a.ix2, (float)a.iy2,
-                              (float)a.inv_denom, (float)a.denom, (double)(float)itol, (max_iters - it + 3) & ~3, ce,
+                              (float)a.inv_denom, (float)a.denom, (double)(float)itol, left & ~3, ce,
                               c->rb_ps, bar, err, out, -1, PS_WAIT_NS};
         PIC_TRY(rb_launch<float>(c, t, p, pow2));
         rb_add_correction<<<gb, 256, 0, c->stream>>>(c->phi, e32, c->G);

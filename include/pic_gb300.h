@@ -258,7 +258,8 @@ typedef struct pic_run_config {
     int poisson;           /* 0: FFT (PoissonSolverFFT), 1: red-black Gauss-Seidel warm-started from phi */
     double dt;             /* Domain::dt; also the Esirkepov path length v*dt */
     double background;     /* added to rho after each deposit (applyBackgroundIfNeeded, simulation.cpp:52-59) */
-    int sort_interval;     /* in-place cell sort every k steps (0: never); results do not depend on it */
+    int sort_interval;     /* in-place cell sort every k steps (0: never); results do not depend on it.
+                              Steps of the Esirkepov rho do not sort: the particles keep their order */
     int use_graph;         /* replay the step as a CUDA graph (FFT Poisson only) */
     double rbgs_tol;       /* poisson == 1: relative residual target */
     int rbgs_max_iters;    /* poisson == 1: sweep limit per solve */

@@ -179,7 +179,9 @@ int run_steps(pic_ctx* c, const pic_run_config* cfg, int steps, pic_diag* histor
         return fail(PIC_ERR_ARG, "sort_moved_fraction must be in [0, 1]");
     if (steps == 0) return PIC_OK;
     int rc = PIC_OK;
-    const bool by_moved = cfg->sort_moved_fraction > 0.0;
+    // the trajectory scheme's steps do not sort (its particles keep their order)
+    const bool esk = cfg->scheme == PIC_SCHEME_ESIRKEPOV;
+    const bool by_moved = !esk && cfg->sort_moved_fraction > 0.0;
     double* hist = (double*)dalloc((size_t)steps * 6 * sizeof(double), &rc);
     if (!hist) return rc;
     int* ctr = (int*)dalloc(sizeof(int), &rc);
@@ -218,11 +220,10 @@ int run_steps(pic_ctx* c, const pic_run_config* cfg, int steps, pic_diag* histor
         const int k = cfg->sort_interval;
         // the Gauss-Seidel stop is decided on the host, so those steps run eagerly
         const bool graph = cfg->use_graph && cfg->poisson == 0;
-        const bool esk = cfg->scheme == PIC_SCHEME_ESIRKEPOV;
         const double limit = cfg->sort_moved_fraction * (double)c->n;
         int last_sort = -1;
         for (int s = 0; s < steps; ++s) {
-            bool do_sort = k > 0 && (s % k) == 0;
+            bool do_sort = !esk && k > 0 && (s % k) == 0;
             if (by_moved) {
                 // interval: steps since the last sort; step 0 sorts unless already in order
                 do_sort = (s == 0 && !c->sorted) || (k > 0 && last_sort >= 0 && s - last_sort >= k);

@@ -185,6 +185,12 @@ int pic_gpu_deposit(pic_ctx* ctx, int scheme, double dt, double background, doub
 int pic_gpu_get_rho_fixed(pic_ctx* ctx, int64_t* acc_out, double* unit_out);
 int pic_gpu_get_rho(pic_ctx* ctx, double* rho_out);
 
+/* Test hook: what the last deposits chose on the device. esk_light: the trajectory charge
+ * of sorted particles with one charge took the light path; current_full: the sorted
+ * current evaluated every particle in full; any_order: deposits between sorts have
+ * switched to the run-aggregating kernel. Any pointer may be NULL. */
+int pic_gpu_test_device_choices(pic_ctx* ctx, int* esk_light, int* current_full, int* any_order);
+
 /* ---- Esirkepov current (new; the reference's "Esirkepov" deposits charge only,
  *      src/deposition/ngp.cpp:13-84) ----
  * First-order charge-conserving current (Esirkepov 2001) of the move x -> x + v*dt

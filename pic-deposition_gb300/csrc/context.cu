@@ -736,6 +736,15 @@ int pic_gpu_charge_uniform(pic_ctx* c, float* out) {
     return PIC_OK;
 }
 
+int pic_gpu_test_device_choices(pic_ctx* c, int* esk_light, int* current_full, int* any_order) {
+    if (!c) return fail(PIC_ERR_ARG, "NULL context");
+    PIC_TRY(pic_gpu_synchronize(c));
+    if (esk_light) *esk_light = (int)c->hstats->esk_light;
+    if (current_full) *current_full = (int)c->hstats->j_full;
+    if (any_order) *any_order = (int)c->hstats->any_order;
+    return PIC_OK;
+}
+
 int pic_gpu_profile_enable(pic_ctx* c, int enable) {
     if (!c) return fail(PIC_ERR_ARG, "NULL context");
     c->prof_enabled = enable ? 1 : 0;

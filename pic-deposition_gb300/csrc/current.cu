@@ -27,6 +27,8 @@
 // loads), each lane summing its particles' 24 edge values while they share a
 // cell (one rolled copy of the particle body), a segmented warp scan, and int64
 // atomics from the run tails (deposit_current).
+#include <cmath>
+
 #include "cells.cuh"
 #include "pic_internal.cuh"
 
@@ -259,7 +261,8 @@ __global__ void __launch_bounds__(J_THREADS) deposit_current(JArgs a) {
     }
 }
 
-// Cell-sorted particles. A CTA owns a 32 x 8 tile of cells; its warps walk units of
+// Cell-sorted particles. A CTA owns a tile of 32 x tile_h cells (8 rows, fewer on grids
+// that would not fill the SMs); its warps walk units of
 // consecutive cells of a row, K lanes per cell, with the stream staged in shared
 // memory (cells.cuh).
 //  * A particle that stays in its cell (0 <= r + d < 1 on both axes) has
@@ -278,16 +281,60 @@ __global__ void __launch_bounds__(J_THREADS) deposit_current(JArgs a) {
 // could overflow add straight to the grids. Integer sums, so the grids equal those
 // of deposit_current bit for bit.
 // Bound by the staying particle's arithmetic (two rounded CIC charges and two
-// edge values). One full evaluation per particle, each lane reading its own cell
-// from global memory, took 1.11 ms at 1024^2, 64 particles per cell.
+// edge values). Where many particles leave their cell the list's atomics cost more than
+// evaluating every particle in full: current_begin looks at a sample, and current_full
+// takes the particles instead.
 constexpr int JC_TW = 32, JC_TH = 8, JC_WARPS = 4;
 constexpr int JC_SW = JC_TW + 3, JC_SH = JC_TH + 3, JC_N = JC_SW * JC_SH;
 constexpr int JC_RUN = 64;
+constexpr int JC_FULL_CTAS = 10;  // current_full's CTAs per SM: two rounds of those that fit
 constexpr int JC_SPLIT = 15;
 constexpr unsigned JC_BATCH = 32;  // particles appended to the list at a time (one atomic on its length)
 // A low word holds 2^17 additions; a run of at most JC_RUN particles of one lane
 // adds to a node once, 32 lanes may share a cell, and five cells reach a node.
 constexpr uint32_t JC_RUN_MAX = 1u << 17;  // particles of a tile whose runs use the tile's accumulators
+
+// The particle stays in its cell. 0 <= e < 1 on both axes: the bits of non-negative
+// floats are in their order.
+__device__ __forceinline__ bool j_stays(float rx, float ry, float dx, float dy) {
+    const float ex = rx + dx, ey = ry + dy;
+    return fmaxf(fabsf(dx), fabsf(dy)) < 1.0f && max(__float_as_uint(ex), __float_as_uint(ey)) < 0x3F800000u;
+}
+
+// Zeroes the grids and the list, and chooses the kernel from a sample of the particles:
+// current_full when at least `many` of them leave their cell in the move.
+constexpr int J_SAMPLES = 4;  // per thread of the first block
+__global__ void __launch_bounds__(J_THREADS) current_begin(JArgs a, size_t g, float many, unsigned* __restrict__ count) {
+    if (blockIdx.x == 0) {
+        const size_t step = a.n / (J_SAMPLES * J_THREADS) ? a.n / (J_SAMPLES * J_THREADS) : 1;
+        float x[J_SAMPLES], y[J_SAMPLES], u[J_SAMPLES], w[J_SAMPLES];
+        bool in[J_SAMPLES];
+#pragma unroll
+        for (int k = 0; k < J_SAMPLES; ++k) {
+            const size_t p = (size_t)(k * J_THREADS + threadIdx.x) * step;
+            in[k] = p < a.n;
+            x[k] = y[k] = u[k] = w[k] = 0.0f;
+            if (in[k]) {
+                x[k] = a.xr[p];
+                y[k] = a.yr[p];
+                u[k] = a.vx[p];
+                w[k] = a.vy[p];
+            }
+        }
+        int leave = 0, all = 0;
+#pragma unroll
+        for (int k = 0; k < J_SAMPLES; ++k) {
+            leave += __syncthreads_count(in[k] && !j_stays(x[k], y[k], u[k] * a.dtdx, w[k] * a.dtdy));
+            all += __syncthreads_count(in[k]);
+        }
+        if (threadIdx.x == 0) {
+            a.st->j_full = (float)leave >= many * (float)all ? 1u : 0u;
+            *count = 0;
+        }
+    }
+    for (size_t i = (size_t)blockIdx.x * J_THREADS + threadIdx.x; i < g; i += (size_t)gridDim.x * J_THREADS)
+        a.jx[i] = a.jy[i] = 0ull;
+}
 
 // The listed particles with their values (the sort's spare arrays): reading them
 // back from the particle arrays took a 64-byte DRAM access per value.
@@ -308,9 +355,118 @@ __global__ void __launch_bounds__(J_THREADS) current_listed(JArgs a, JList l) {
     }
 }
 
+constexpr uint32_t JC_FULL_MAX = 1u << 21;  // particles of a tile whose sums use its accumulators in current_full
+
+// A tile's accumulators to the grids.
+__device__ __forceinline__ void tile_to_grids(const JArgs& a, const uint32_t* slo, const int* shi, int x0, int y0) {
+    for (int i = threadIdx.x; i < 2 * JC_N; i += JC_WARPS * 32) {
+        const long long v = (long long)shi[i] * (1ll << JC_SPLIT) + (long long)slo[i];
+        if (v != 0) {
+            const int li = i < JC_N ? i : i - JC_N;
+            const int ly = li / JC_SW, lx = li - ly * JC_SW;
+            const size_t g = (size_t)wrap_i(y0 - 1 + ly, a.Ny) * a.Nx + wrap_i(x0 - 1 + lx, a.Nx);
+            atomicAdd((i < JC_N ? a.jx : a.jy) + g, (unsigned long long)v);
+        }
+    }
+}
+
+// All 24 edge values of every particle: one lane per cell of a tile row walks the cell's
+// range (16-byte loads of 4 particles) and sums them in registers (at most 64 particles:
+// |sum| <= 64 * 2^24), then adds the sums to the tile's accumulators, or to the grids in a
+// tile whose high words could overflow (2^16 sums of 2^15 each). Takes the same time
+// whatever the particles do. The CTAs walk the tiles: a launch that is not wanted costs
+// little.
+template <bool QC>
+__global__ void __launch_bounds__(JC_WARPS * 32) current_full(JArgs a, const uint32_t* __restrict__ offsets, int tiles_x,
+                                                               int tiles, int tile_h) {
+    if (!a.st->j_full) return;
+    __shared__ uint32_t slo[2 * JC_N];
+    __shared__ int shi[2 * JC_N];
+    __shared__ uint32_t s_count;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int tx = tile % tiles_x, ty = tile / tiles_x;
+        const int x0 = tx * JC_TW, y0 = ty * tile_h;
+        const int tw = min(JC_TW, a.Nx - x0), th = min(tile_h, a.Ny - y0);
+        for (int i = threadIdx.x; i < 2 * JC_N; i += JC_WARPS * 32) {
+            slo[i] = 0;
+            shi[i] = 0;
+        }
+        if (threadIdx.x == 0) s_count = 0;
+        __syncthreads();
+        if ((int)threadIdx.x < th) {
+            const uint32_t* row = offsets + (uint32_t)(y0 + (int)threadIdx.x) * (uint32_t)a.Nx + (uint32_t)x0;
+            atomicAdd(&s_count, row[tw] - row[0]);
+        }
+        __syncthreads();
+        const bool to_grids = s_count >= JC_FULL_MAX;
+        int acc[NJ];
+        // adds acc (the cell in column `lane`, tile row r) to the tile accumulators
+        auto flush = [&](int r) {
+            if (to_grids) {
+                flush_edges(a, (uint32_t)(y0 + r) * (uint32_t)a.Nx + (uint32_t)(x0 + lane), acc);
+#pragma unroll
+                for (int t = 0; t < NJ; ++t) acc[t] = 0;
+                return;
+            }
+#pragma unroll
+            for (int t = 0; t < NJ; ++t) {
+                const int v = acc[t];
+                if (v != 0) {
+                    // Jx edge (j, i) = t (j * 3 + i), Jy edge (j, i) = t - 12 (j * 4 + i): local node (lane + i, r + j)
+                    const int j = t < 12 ? t / 3 : (t - 12) / 4, i = t < 12 ? t % 3 : (t - 12) % 4;
+                    const int idx = (t < 12 ? 0 : JC_N) + (r + j) * JC_SW + lane + i;
+                    atomicAdd(slo + idx, (uint32_t)v & ((1u << JC_SPLIT) - 1u));
+                    atomicAdd(shi + idx, v >> JC_SPLIT);
+                }
+                acc[t] = 0;
+            }
+        };
+        for (int r = warp; r < th; r += JC_WARPS) {
+            uint32_t beg = 0, end = 0;
+            if (lane < tw) {
+                const uint32_t cell = (uint32_t)(y0 + r) * (uint32_t)a.Nx + (uint32_t)(x0 + lane);
+                beg = offsets[cell];
+                end = offsets[cell + 1];
+            }
+#pragma unroll
+            for (int t = 0; t < NJ; ++t) acc[t] = 0;
+            int cnt = 0;
+            const uint32_t q0 = beg >> 2, q1 = end > beg ? (end + 3u) >> 2 : q0;
+#pragma unroll 1
+            for (uint32_t qd = q0; qd < q1; ++qd) {
+                const float4 xr = __ldg(reinterpret_cast<const float4*>(a.xr) + qd);
+                const float4 yr = __ldg(reinterpret_cast<const float4*>(a.yr) + qd);
+                const float4 vx = __ldg(reinterpret_cast<const float4*>(a.vx) + qd);
+                const float4 vy = __ldg(reinterpret_cast<const float4*>(a.vy) + qd);
+                const float4 q = QC ? make_float4(a.qc, a.qc, a.qc, a.qc) : __ldg(reinterpret_cast<const float4*>(a.q) + qd);
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t p = 4u * qd + (uint32_t)k;
+                    if (p < beg || p >= end) continue;
+                    int v[NJ];
+                    if (edge_values(a, f4(xr, k), f4(yr, k), f4(vx, k), f4(vy, k), f4(q, k), p, v)) {
+#pragma unroll
+                        for (int t = 0; t < NJ; ++t) acc[t] += v[t];
+                    }
+                    if (++cnt == JC_RUN) {
+                        flush(r);
+                        cnt = 0;
+                    }
+                }
+            }
+            if (cnt) flush(r);
+        }
+        __syncthreads();
+        tile_to_grids(a, slo, shi, x0, y0);
+        __syncthreads();
+    }
+}
+
 template <bool QC>
 __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const uint32_t* __restrict__ offsets,
-                                                                   int tiles_x, int klog, int cap, JList list) {
+                                                                   int tiles_x, int tile_h, int klog, int cap, JList list) {
+    if (a.st->j_full) return;
     constexpr int NF = QC ? 4 : 5;
     extern __shared__ __align__(16) uint32_t sbufs[];  // [JC_WARPS][NF][cap]
     __shared__ uint32_t soff[JC_TH * (JC_TW + 1)];
@@ -321,8 +477,8 @@ __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const
     __shared__ float4 sqval[JC_WARPS][JC_BATCH + 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
-    const int x0 = tx * JC_TW, y0 = ty * JC_TH;
-    const int tw = min(JC_TW, a.Nx - x0), th = min(JC_TH, a.Ny - y0);
+    const int x0 = tx * JC_TW, y0 = ty * tile_h;
+    const int tw = min(JC_TW, a.Nx - x0), th = min(tile_h, a.Ny - y0);
     if (threadIdx.x == 0) s_count = 0;
     for (int i = threadIdx.x; i < 2 * JC_N; i += JC_WARPS * 32) {
         slo[i] = 0;
@@ -427,8 +583,7 @@ __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const
                 }
                 const float dx = vx * a.dtdx, dy = vy * a.dtdy;
                 const float ex = rx + dx, ey = ry + dy;
-                // 0 <= e < 1 on both axes: the bits of non-negative floats are in their order
-                const bool stays = fmaxf(fabsf(dx), fabsf(dy)) < 1.0f && max(__float_as_uint(ex), __float_as_uint(ey)) < 0x3F800000u;
+                const bool stays = j_stays(rx, ry, dx, dy);
                 const unsigned out = __ballot_sync(0xffffffffu, valid && !stays);
                 if (out) {
                     if (valid && !stays) {
@@ -497,30 +652,30 @@ __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const
     }
     if (qn) append(qn);
     __syncthreads();
-    for (int i = threadIdx.x; i < 2 * JC_N; i += JC_WARPS * 32) {
-        const long long v = (long long)shi[i] * (1ll << JC_SPLIT) + (long long)slo[i];
-        if (v != 0) {
-            const int li = i < JC_N ? i : i - JC_N;
-            const int ly = li / JC_SW, lx = li - ly * JC_SW;
-            const size_t g = (size_t)wrap_i(y0 - 1 + ly, a.Ny) * a.Nx + wrap_i(x0 - 1 + lx, a.Nx);
-            atomicAdd((i < JC_N ? a.jx : a.jy) + g, (unsigned long long)v);
+    tile_to_grids(a, slo, shi, x0, y0);
+}
+
+// The grids as FP64, four cells per thread: each thread forms the units (FP64
+// multiplications are slow on this part: 7 us at 1024^2 with a cell per thread), the first
+// also stores them.
+__global__ void __launch_bounds__(256) current_to_f64(const long long* __restrict__ jx, const long long* __restrict__ jy,
+                                                      size_t g, double inv_vol, double dxdt, double dydt,
+                                                      const DevStats* st, double* __restrict__ units,
+                                                      double* __restrict__ ox, double* __restrict__ oy) {
+    const size_t i0 = (size_t)blockIdx.x * 1024 + threadIdx.x;
+    const double u = charge_unit(st, inv_vol), ux = __dmul_rn(u, dxdt), uy = __dmul_rn(u, dydt);
+    if (i0 == 0) {
+        units[0] = ux;
+        units[1] = uy;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const size_t i = i0 + k * 256;
+        if (i < g) {
+            ox[i] = __dmul_rn((double)jx[i], ux);
+            oy[i] = __dmul_rn((double)jy[i], uy);
         }
     }
-}
-
-__global__ void current_to_f64(const long long* __restrict__ jx, const long long* __restrict__ jy, size_t g,
-                               const double* __restrict__ units, double* __restrict__ ox, double* __restrict__ oy) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < g) {
-        ox[i] = __dmul_rn((double)jx[i], units[0]);
-        oy[i] = __dmul_rn((double)jy[i], units[1]);
-    }
-}
-
-__global__ void current_units(double inv_vol, double dxdt, double dydt, const DevStats* st, double* units) {
-    const double u = charge_unit(st, inv_vol);
-    units[0] = __dmul_rn(u, dxdt);
-    units[1] = __dmul_rn(u, dydt);
 }
 
 static int ensure_current(pic_ctx* c) {
@@ -540,8 +695,6 @@ static int ensure_current(pic_ctx* c) {
 int deposit_current_async(pic_ctx* c, double dt) {
     if (!(dt > 0.0)) return fail(PIC_ERR_ARG, "deposit_current: dt must be > 0");
     PIC_TRY(ensure_current(c));
-    PIC_CUDA_TRY(cudaMemsetAsync(c->accjx, 0, c->G * 8, c->stream));
-    PIC_CUDA_TRY(cudaMemsetAsync(c->accjy, 0, c->G * 8, c->stream));
     JArgs a;
     a.cell = c->cell;
     a.xr = c->xr;
@@ -558,46 +711,70 @@ int deposit_current_async(pic_ctx* c, double dt) {
     a.jx = reinterpret_cast<unsigned long long*>(c->accjx);
     a.jy = reinterpret_cast<unsigned long long*>(c->accjy);
     a.st = c->dstats;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     if (c->n && c->sorted) {
-        // cell-sorted: each cell's lanes over the sort's range of it
-        const int tiles_x = (c->Nx + JC_TW - 1) / JC_TW, tiles_y = (c->Ny + JC_TH - 1) / JC_TH;
-        int klog, cap;
         const bool qc = a.qc != 0.0f;
+        const int tiles_x = (c->Nx + JC_TW - 1) / JC_TW;
+        // at least two tiles for every SM where the rows allow: a warp takes its units one
+        // after the other (33 x 9: 48 us with tiles of 8 rows)
+        int th = JC_TH;
+        while (th > 1 && (long long)tiles_x * ((c->Ny + th - 1) / th) < 2 * sms) th /= 2;
+        int klog, cap;
         cells_shape(c->n, c->G, qc ? 4 : 5, 1560, &klog, &cap);
         PIC_TRY(ensure_sort_scratch(c));  // the list takes the sort's spare arrays
         unsigned* count = reinterpret_cast<unsigned*>(c->junits + 2);
-        PIC_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(unsigned), c->stream));
         const JList list{count, c->idx_b, c->cell_alt, c->alt[0], c->alt[1], c->alt[2], c->alt[3]};
         const size_t smem = (size_t)JC_WARPS * (qc ? 4 : 5) * cap * 4;
         PIC_TRY(opt_in_dynamic_smem(qc ? (const void*)current_cells<true> : (const void*)current_cells<false>, smem));
+        // current_full where each scheduler gets a warp of 32 cells (on smaller grids its
+        // serial cells lose at any fraction: 64^2 x 64, 0.62 leaving: 107 us against 49) and
+        // enough particles leave their cell; denser cells list more of them. Where the two
+        // take the same time: above 0.63 leaving at 1 per cell, 0.38 at 4, 0.27 at 16, 0.2 at
+        // 64 and 0.12 at 200 (512^2 and 1024^2). 1024^2 x 64, 0.62 leaving: 1.36 ms, 3.5 with
+        // the list.
+        const bool may_full = c->G >= (size_t)32 * 4 * sms;
+        const float many = may_full ? (float)(0.1 + 0.58 / std::sqrt((double)c->n / (double)c->G)) : 2.0f;
+        size_t zero = (c->G + J_THREADS * 4 - 1) / (J_THREADS * 4);
+        if (zero > (size_t)sms * 8) zero = (size_t)sms * 8;
+        current_begin<<<(unsigned)zero, J_THREADS, 0, c->stream>>>(a, c->G, many, count);
+        PIC_TRY(check_launch(c, "current_begin"));
         prof_begin(c, "current");
-        const unsigned tiles = (unsigned)(tiles_x * tiles_y);
+        const unsigned tiles = (unsigned)(tiles_x * ((c->Ny + th - 1) / th));
         if (qc)
-            current_cells<true><<<tiles, JC_WARPS * 32, smem, c->stream>>>(a, c->offsets, tiles_x, klog, cap, list);
+            current_cells<true><<<tiles, JC_WARPS * 32, smem, c->stream>>>(a, c->offsets, tiles_x, th, klog, cap, list);
         else
-            current_cells<false><<<tiles, JC_WARPS * 32, smem, c->stream>>>(a, c->offsets, tiles_x, klog, cap, list);
+            current_cells<false><<<tiles, JC_WARPS * 32, smem, c->stream>>>(a, c->offsets, tiles_x, th, klog, cap, list);
         PIC_TRY(check_launch(c, "current_cells"));
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
         size_t blocks = (c->n + J_THREADS - 1) / J_THREADS;
         if (blocks > (size_t)sms * 4) blocks = (size_t)sms * 4;
         current_listed<<<(unsigned)blocks, J_THREADS, 0, c->stream>>>(a, list);
-        prof_end(c);
         PIC_TRY(check_launch(c, "current_listed"));
-    } else if (c->n) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        size_t blocks = (c->n + J_THREADS * 4 - 1) / (J_THREADS * 4);
-        if (blocks > (size_t)sms * 8) blocks = (size_t)sms * 8;
-        prof_begin(c, "current");
-        deposit_current<<<(unsigned)blocks, J_THREADS, 0, c->stream>>>(a);
+        if (may_full) {
+            const int fh = th < JC_WARPS ? JC_WARPS : th;  // a row for every warp
+            const int ftiles = tiles_x * ((c->Ny + fh - 1) / fh);
+            const unsigned ctas = (unsigned)(ftiles < sms * JC_FULL_CTAS ? ftiles : sms * JC_FULL_CTAS);
+            if (qc)
+                current_full<true><<<ctas, JC_WARPS * 32, 0, c->stream>>>(a, c->offsets, tiles_x, ftiles, fh);
+            else
+                current_full<false><<<ctas, JC_WARPS * 32, 0, c->stream>>>(a, c->offsets, tiles_x, ftiles, fh);
+            PIC_TRY(check_launch(c, "current_full"));
+        }
         prof_end(c);
-        PIC_TRY(check_launch(c, "deposit_current"));
+    } else {
+        PIC_CUDA_TRY(cudaMemsetAsync(c->accjx, 0, c->G * 8, c->stream));
+        PIC_CUDA_TRY(cudaMemsetAsync(c->accjy, 0, c->G * 8, c->stream));
+        if (c->n) {
+            size_t blocks = (c->n + J_THREADS * 4 - 1) / (J_THREADS * 4);
+            if (blocks > (size_t)sms * 8) blocks = (size_t)sms * 8;
+            prof_begin(c, "current");
+            deposit_current<<<(unsigned)blocks, J_THREADS, 0, c->stream>>>(a);
+            prof_end(c);
+            PIC_TRY(check_launch(c, "deposit_current"));
+        }
     }
-    current_units<<<1, 1, 0, c->stream>>>(1.0 / (c->dx * c->dy), c->dx / dt, c->dy / dt, c->dstats, c->junits);
-    PIC_TRY(check_launch(c, "current_units"));
-    current_to_f64<<<(unsigned)((c->G + 255) / 256), 256, 0, c->stream>>>(c->accjx, c->accjy, c->G, c->junits, c->jx,
-                                                                           c->jy);
+    current_to_f64<<<(unsigned)((c->G + 1023) / 1024), 256, 0, c->stream>>>(
+        c->accjx, c->accjy, c->G, 1.0 / (c->dx * c->dy), c->dx / dt, c->dy / dt, c->dstats, c->junits, c->jx, c->jy);
     PIC_TRY(check_launch(c, "current_to_f64"));
     c->has_current = 1;
     return PIC_OK;

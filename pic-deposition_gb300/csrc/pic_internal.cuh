@@ -27,6 +27,7 @@ struct DevStats {
     float q_first;              // uploads: the first particle's stored charge
     float q_raw0;               // uploads: the first particle's charge before normalisation
     unsigned int any_order;     // between sorts: 1 once most particles have left their sorted cell
+    unsigned int j_full;        // sorted current: 1 when many sampled particles leave their cell in the move
     unsigned int esk_light;     // trajectory charge: 1 when few sampled particles leave their cell in the move
     unsigned long long moved;   // deposits between sorts: particles found outside their sorted cell
     unsigned long long moved_dep;  // the same, for the any_order decision after each deposit

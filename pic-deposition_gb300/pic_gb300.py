@@ -229,6 +229,7 @@ class GenConfig(C.Structure):
 _SIGS.append(("pic_gpu_generate", [_vp, C.POINTER(GenConfig)]))
 _SIGS.append(("pic_gpu_set_rbgs_precision", [_vp, C.c_int]))
 _SIGS.append(("pic_gpu_test_rbgs_barrier_timeout", [_vp, C.c_int, C.c_double]))
+_SIGS.append(("pic_gpu_test_device_choices", [_vp] + [C.POINTER(C.c_int)] * 3))
 
 
 class EnsMember(C.Structure):
@@ -548,6 +549,12 @@ class Context:
         ux, uy = C.c_double(), C.c_double()
         _check(lib().pic_gpu_get_current_fixed(self.h, _ptr(jx), _ptr(jy), C.byref(ux), C.byref(uy)))
         return jx, jy, ux.value, uy.value
+
+    def test_device_choices(self) -> dict:
+        """What the last deposits chose on the device (pic_gpu_test_device_choices)."""
+        v = [C.c_int() for _ in range(3)]
+        _check(lib().pic_gpu_test_device_choices(self.h, *[C.byref(k) for k in v]))
+        return dict(zip(("esk_light", "current_full", "any_order"), (k.value for k in v)))
 
     def set_rbgs_precision(self, mixed: bool):
         """False: FP64 sweeps; True: FP32 sweeps on FP64-refined corrections."""

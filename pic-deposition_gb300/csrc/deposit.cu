@@ -46,6 +46,8 @@
 //
 // Compiled with --fmad=false: no multiply-add is fused, so every FP32 result
 // equals the oracle's (compiled with -ffp-contract=off).
+#include <cmath>
+
 #include "cells.cuh"
 #include "diag.cuh"
 #include "pic_internal.cuh"
@@ -1537,14 +1539,14 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
 // cell on both axes deposits all its A units on its own cell's node
 // (ngp.cpp:36-84: the whole path lies in one cell), so these particles are
 // counted and not summed: the grid starts as A times the cells' counts, which
-// the sort's offsets hold (esk_base), and esk_light streams the particles once
+// the sort's offsets hold (esk_begin), and esk_light streams the particles once
 // with coalesced 16-byte loads, only testing. The others are queued per warp
 // (ballot compaction) and, 32 at a time, deposit their stencil minus the A
 // units already counted straight to the global int64 grid. The sums are the
 // same integers as deposit_cells'. Bound by memory when few particles cross a
 // cell boundary in the move (16 bytes per particle, read once); every one that
 // does costs a few int64 atomics, so a sample decides on the device between this
-// path and deposit_cells (esk_sample), and the one not chosen returns at once.
+// path and deposit_cells (esk_begin), and the one not chosen returns at once.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ bool esk_stays(float r, float v, float dtf, float dtd) {
     if (fabsf(v * dtf) < 1e-15f) return false;  // static: CIC weights
@@ -1554,34 +1556,37 @@ __device__ __forceinline__ bool esk_stays(float r, float v, float dtf, float dtd
     return dc > 0.0f ? !(e > 1.0f) : !(e < 0.0f);
 }
 
-constexpr int ESK_SAMPLES = 4096;
-// The light path when fewer than half of the sample leave their cell: at 1024^2 x 64
-// it takes 0.29 ms when 2 % do and about 0.6 ms at 22 %; deposit_cells takes the
-// same at any fraction.
-constexpr unsigned ESK_LIGHT_DENOM = 2;
-
-__global__ void __launch_bounds__(1024) esk_sample(DepArgs a) {
-    __shared__ unsigned s_cross;
-    if (threadIdx.x == 0) s_cross = 0;
-    __syncthreads();
-    const unsigned m = a.n < (size_t)ESK_SAMPLES ? (unsigned)a.n : (unsigned)ESK_SAMPLES;
-    unsigned cross = 0;
-    for (unsigned i = threadIdx.x; i < m; i += 1024) {
-        const size_t p = (size_t)i * (a.n / m);
-        cross += esk_stays(a.xr[p], a.vx[p], a.dtf, a.dtdx) && esk_stays(a.yr[p], a.vy[p], a.dtf, a.dtdy) ? 0u : 1u;
+// Starts the grid and chooses: every block looks at the same sample, so each knows
+// whether its cells begin with A units per particle (light path) or at zero, without a
+// launch between the sample and the grid.
+constexpr int ESK_SAMPLES = 4;  // per thread
+__global__ void __launch_bounds__(DEP_THREADS) esk_begin(DepArgs a, size_t g, float light) {
+    const size_t step = a.n / (ESK_SAMPLES * DEP_THREADS) ? a.n / (ESK_SAMPLES * DEP_THREADS) : 1;
+    float x[ESK_SAMPLES], y[ESK_SAMPLES], u[ESK_SAMPLES], w[ESK_SAMPLES];
+    bool in[ESK_SAMPLES];
+#pragma unroll
+    for (int k = 0; k < ESK_SAMPLES; ++k) {
+        const size_t p = (size_t)(k * DEP_THREADS + threadIdx.x) * step;
+        in[k] = p < a.n;
+        x[k] = y[k] = u[k] = w[k] = 0.0f;
+        if (in[k]) {
+            x[k] = a.xr[p];
+            y[k] = a.yr[p];
+            u[k] = a.vx[p];
+            w[k] = a.vy[p];
+        }
     }
-    cross = __reduce_add_sync(FULL, cross);
-    if ((threadIdx.x & 31) == 0 && cross) atomicAdd(&s_cross, cross);
-    __syncthreads();
-    if (threadIdx.x == 0) a.st->esk_light = s_cross * ESK_LIGHT_DENOM < m ? 1u : 0u;
-}
-
-// The grid's start: A units per particle of the cell (light path), else zero.
-__global__ void esk_base(DepArgs a, size_t g) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g) return;
+    int leave = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < ESK_SAMPLES; ++k) {
+        leave += __syncthreads_count(in[k] && !(esk_stays(x[k], u[k], a.dtf, a.dtdx) && esk_stays(y[k], w[k], a.dtf, a.dtdy)));
+        all += __syncthreads_count(in[k]);
+    }
+    const bool on = (float)leave < light * (float)all;
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.st->esk_light = on ? 1u : 0u;
     const long long A = __float2int_rn(a.qc * 16777216.0f);
-    a.acc[i] = a.st->esk_light ? (unsigned long long)(A * (long long)(a.offsets[i + 1] - a.offsets[i])) : 0ull;
+    for (size_t i = (size_t)blockIdx.x * DEP_THREADS + threadIdx.x; i < g; i += (size_t)gridDim.x * DEP_THREADS)
+        a.acc[i] = on ? (unsigned long long)(A * (long long)(a.offsets[i + 1] - a.offsets[i])) : 0ull;
 }
 
 constexpr int ESK_QUEUE = 32 + 128;  // left over (below 32) and one step's particles
@@ -1747,6 +1752,9 @@ static int launch_runs(pic_ctx* c, const DepArgs& a) {
     return check_launch(c, "deposit_runs");
 }
 
+// The trajectory charge of freshly sorted particles with one charge: esk_begin starts the grid.
+static bool esk_chosen(const pic_ctx* c, int kind) { return kind == 0 && c->sorted && c->n > 0 && c->qn_uniform != 0.0f; }
+
 template <int S>
 // kernel choice: 0 tiled (cell-sorted), 1 run-aggregating (any order), 2 one thread per particle;
 // `adaptive`: between sorts, the device picks the tiled or the any-order kernel (choose_any_order)
@@ -1766,7 +1774,7 @@ static int launch_deposit(pic_ctx* c, const DepArgs& a, int kind, bool adaptive)
         return rc;
     }
     if constexpr (S == S_ESK) {
-        if (kind == 0 && c->sorted && a.qc != 0.0f) {
+        if (esk_chosen(c, kind)) {
             // one charge, freshly sorted: the light path or the cell kernel, chosen on the device
             DepArgs al = a, ac = a;
             al.gate = ac.gate = &c->dstats->esk_light;
@@ -1777,10 +1785,16 @@ static int launch_deposit(pic_ctx* c, const DepArgs& a, int kind, bool adaptive)
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
             size_t blocks = (a.n + DEP_THREADS * 4 - 1) / (DEP_THREADS * 4);
             if (blocks > (size_t)sms * 8) blocks = (size_t)sms * 8;
-            esk_sample<<<1, 1024, 0, c->stream>>>(a);
-            PIC_TRY(check_launch(c, "esk_sample"));
-            esk_base<<<(unsigned)((c->G + 255) / 256), 256, 0, c->stream>>>(a, c->G);
-            PIC_TRY(check_launch(c, "esk_base"));
+            size_t start = (c->G + DEP_THREADS * 4 - 1) / (DEP_THREADS * 4);
+            if (start > (size_t)sms * 4) start = (size_t)sms * 4;
+            // The light path below this fraction that leaves: every leaving particle costs it
+            // atomics, the more of them the denser the cells; deposit_cells takes nearly the same
+            // at any fraction. Where the two take the same time: above 0.63 at 1 to 10 per cell,
+            // 0.56 at 16, 0.37 to 0.43 at 64, 0.36 at 200. 1024^2 x 64: 0.32 ms light when 3 %
+            // leave, 0.70 at 28 % and 1.23 at 62 %, where deposit_cells takes 0.85.
+            const float light = (float)std::fmax(0.37, 0.3 + 0.8 / std::sqrt((double)c->n / (double)c->G));
+            esk_begin<<<(unsigned)start, DEP_THREADS, 0, c->stream>>>(a, c->G, light);
+            PIC_TRY(check_launch(c, "esk_begin"));
             prof_begin(c, "deposit");
             esk_light<<<(unsigned)blocks, DEP_THREADS, 0, c->stream>>>(al);
             int rc = check_launch(c, "esk_light");
@@ -1842,7 +1856,8 @@ int deposit_rho(pic_ctx* c, int scheme, double dt, double background, const Fina
         // another cell on their own; otherwise the run-aggregating kernel
         tiled = (c->sorted || c->part_valid) ? 0 : 1;
     }
-    PIC_CUDA_TRY(cudaMemsetAsync(c->acc, 0, c->G * sizeof(long long), c->stream));
+    if (!(scheme == PIC_SCHEME_ESIRKEPOV && esk_chosen(c, tiled)))
+        PIC_CUDA_TRY(cudaMemsetAsync(c->acc, 0, c->G * sizeof(long long), c->stream));
     DepArgs a;
     a.cell = c->cell;
     a.xr = c->xr;

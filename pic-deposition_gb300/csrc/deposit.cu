@@ -1790,9 +1790,11 @@ static int launch_deposit(pic_ctx* c, const DepArgs& a, int kind, bool adaptive)
             // The light path below this fraction that leaves: every leaving particle costs it
             // atomics, the more of them the denser the cells; deposit_cells takes nearly the same
             // at any fraction. Where the two take the same time: above 0.63 at 1 to 10 per cell,
-            // 0.56 at 16, 0.37 to 0.43 at 64, 0.36 at 200. 1024^2 x 64: 0.32 ms light when 3 %
+            // 0.56 at 16, 0.37 to 0.43 at 64, 0.36 at 200; on grids too small for a warp of 32
+            // cells on every scheduler 0.41 (16^2 x 4000) and more. 1024^2 x 64: 0.32 ms light when 3 %
             // leave, 0.70 at 28 % and 1.23 at 62 %, where deposit_cells takes 0.85.
-            const float light = (float)std::fmax(0.37, 0.3 + 0.8 / std::sqrt((double)c->n / (double)c->G));
+            const double least = c->G < (size_t)32 * 4 * sms ? 0.45 : 0.37;
+            const float light = (float)std::fmax(least, 0.3 + 0.8 / std::sqrt((double)c->n / (double)c->G));
             esk_begin<<<(unsigned)start, DEP_THREADS, 0, c->stream>>>(a, c->G, light);
             PIC_TRY(check_launch(c, "esk_begin"));
             prof_begin(c, "deposit");

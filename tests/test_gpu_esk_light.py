@@ -18,13 +18,13 @@ def stays(r, d):
 @pytest.mark.parametrize("vth,ppc,light", [(0.05, 40, 1), (0.25, 40, 1), (0.45, 40, 0), (0.9, 40, 0), (0.35, 6, 1),
                                            (0.9, 6, 0), (0.9, 1, 1), (0.0, 40, 0)])
 @pytest.mark.parametrize("charge", [1.5, -0.25])
-@pytest.mark.parametrize("nx,ny", [(70, 34), (128, 40)])
+@pytest.mark.parametrize("nx,ny", [(70, 34), (128, 40), (210, 130)])
 def test_path_and_grid(pg, nx, ny, charge, vth, ppc, light):
     rng = np.random.default_rng(nx + ppc)
     n = nx * ny * ppc
     x, y = rng.random(n) * nx, rng.random(n) * ny
     vx, vy = np.clip(rng.normal(0, 1, (2, n)), -2, 2) * vth
-    line = max(0.37, 0.3 + 0.8 / ppc**0.5)
+    line = max(0.45 if nx * ny < 16384 else 0.37, 0.3 + 0.8 / ppc**0.5)
     leave = 1.0 - np.mean(stays(x % 1.0, vx) & stays(y % 1.0, vy))
     assert abs(leave - line) > 3 * 0.5 / 1024**0.5 and light == (leave < line)
     with pg.Context(nx, ny, float(nx), float(ny), n) as c:

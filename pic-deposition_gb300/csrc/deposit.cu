@@ -1713,7 +1713,11 @@ static int launch_cells(pic_ctx* c, DepArgs a, unsigned tiles) {
     // larger units. 1024^2 x 64, one charge, us per call with 1,040 / 2,080 / 3,120
     // words: CIC 242 / 222 / 221, NGP 202 / 198 / 199, TSC 334 / 285 / 285; a TSC time
     // step at 100 per cell 2.46 / 2.25 / 2.15 ms, a CIC one at 64 0.46 / 0.44 / 0.45.
-    constexpr int WORDS = S == S_TSC || S == S_ESK ? 3120 : 2080;
+    // The trajectory scheme between sorts stages up to six fields: with 3,120 words three CTAs
+    // fit an SM, and 512 tiles of a 256^2 grid take a second round (mixed charges, 64 per
+    // cell: 213 us against 132 with 2,600, 183 in the form without staged units; 1024^2 x 64
+    // 1.92 and 1.56 ms).
+    constexpr int WORDS = S == S_ESK && KEYS ? 2600 : S == S_TSC || S == S_ESK ? 3120 : 2080;
     cells_shape(a.n, c->G, StageFields<S, QC>::NF - (KEYS ? 0 : 1), WORDS, &a.klog, &a.cap);
     const size_t smem = cells_fixed_bytes<S, NW, QC, KEYS>(a.cap) +
                         (size_t)(a.tile_h + 3 + 2 * PAD) * (a.tile_w + 3 + 2 * PAD) * 2 * sizeof(uint32_t) +

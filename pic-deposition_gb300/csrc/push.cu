@@ -48,9 +48,11 @@ struct MoveArgs {
 // rate at 40 bytes per particle (0.80 with one at a time and the next one's values
 // prefetched). Four at a time spread a warp's field reads over more cells: 10 % slower
 // when the particles are out of order.
-template <bool GATHER, bool PUSH, bool KE = false>
+// Few particles are one wave of threads either way, and two per thread only lengthen each
+// one's chain: NP = 1 there (not with the kinetic sums, whose chains would change).
+template <int NP, bool GATHER, bool PUSH, bool KE = false>
 __global__ void __launch_bounds__(256, 5) move_particles(MoveArgs a) {
-    constexpr int NP = 2;
+    static_assert(NP == 2 || (NP == 1 && !KE), "");
     float ke_hi = 0.0f, ke_lo = 0.0f;
     const float maxq = load_maxq(a.st);
     const float inv_nx = 1.0f / (float)a.Nx;
@@ -58,12 +60,24 @@ __global__ void __launch_bounds__(256, 5) move_particles(MoveArgs a) {
     for (size_t qi = (size_t)blockIdx.x * blockDim.x + threadIdx.x; qi < nq; qi += stride) {
         const size_t p = qi * NP;
         const int cnt = a.n - p < NP ? (int)(a.n - p) : NP;
-        // the arrays are aligned and padded past the last particle
-        const uint2 kv = *reinterpret_cast<const uint2*>(a.cell + p);
-        const float2 xv = *reinterpret_cast<const float2*>(a.xr + p), yv = *reinterpret_cast<const float2*>(a.yr + p);
-        const float2 uv = *reinterpret_cast<const float2*>(a.vx + p), wv = *reinterpret_cast<const float2*>(a.vy + p);
-        uint32_t key[NP] = {kv.x, kv.y};
-        float rx[NP] = {xv.x, xv.y}, ry[NP] = {yv.x, yv.y}, vx[NP] = {uv.x, uv.y}, vy[NP] = {wv.x, wv.y};
+        uint32_t key[NP];
+        float rx[NP], ry[NP], vx[NP], vy[NP];
+        if constexpr (NP == 2) {  // the arrays are aligned and padded past the last particle
+            const uint2 kv = *reinterpret_cast<const uint2*>(a.cell + p);
+            const float2 xv = *reinterpret_cast<const float2*>(a.xr + p), yv = *reinterpret_cast<const float2*>(a.yr + p);
+            const float2 uv = *reinterpret_cast<const float2*>(a.vx + p), wv = *reinterpret_cast<const float2*>(a.vy + p);
+            key[0] = kv.x, key[1] = kv.y;
+            rx[0] = xv.x, rx[1] = xv.y;
+            ry[0] = yv.x, ry[1] = yv.y;
+            vx[0] = uv.x, vx[1] = uv.y;
+            vy[0] = wv.x, vy[1] = wv.y;
+        } else {
+            key[0] = a.cell[p];
+            rx[0] = a.xr[p];
+            ry[0] = a.yr[p];
+            vx[0] = a.vx[p];
+            vy[0] = a.vy[p];
+        }
         int ix[NP], iy[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
@@ -104,15 +118,15 @@ __global__ void __launch_bounds__(256, 5) move_particles(MoveArgs a) {
                 key[k] = (uint32_t)iy[k] * (uint32_t)a.Nx + (uint32_t)ix[k];
             }
         }
-        if (cnt == NP) {
+        if (NP == 2 && cnt == NP) {
             if constexpr (GATHER) {
-                *reinterpret_cast<float2*>(a.vx + p) = make_float2(vx[0], vx[1]);
-                *reinterpret_cast<float2*>(a.vy + p) = make_float2(vy[0], vy[1]);
+                *reinterpret_cast<float2*>(a.vx + p) = make_float2(vx[0], vx[NP - 1]);
+                *reinterpret_cast<float2*>(a.vy + p) = make_float2(vy[0], vy[NP - 1]);
             }
             if constexpr (PUSH) {
-                *reinterpret_cast<float2*>(a.xr + p) = make_float2(rx[0], rx[1]);
-                *reinterpret_cast<float2*>(a.yr + p) = make_float2(ry[0], ry[1]);
-                *reinterpret_cast<uint2*>(a.cell + p) = make_uint2(key[0], key[1]);
+                *reinterpret_cast<float2*>(a.xr + p) = make_float2(rx[0], rx[NP - 1]);
+                *reinterpret_cast<float2*>(a.yr + p) = make_float2(ry[0], ry[NP - 1]);
+                *reinterpret_cast<uint2*>(a.cell + p) = make_uint2(key[0], key[NP - 1]);
             }
         } else {
             if constexpr (GATHER) {
@@ -175,15 +189,19 @@ int move(pic_ctx* c, double dt, bool gather, bool push, bool ke) {
     // the partition of the sums depends on the particle count alone; no more blocks
     // than the particles fill (4096 nearly empty blocks took 18 us at 65,536 particles)
     if (ke) blocks = filled < (size_t)MOVE_KE_BLOCKS ? filled : (size_t)MOVE_KE_BLOCKS;
+    // One particle per thread up to the counts where two become as fast: 256 per SM for a
+    // push alone, 4,096 where fields are gathered (262,144 particles out of order on 512^2,
+    // gather: 10.3 us against 11.3; 1,001: 4.1 against 6.2).
+    const bool one = !ke && c->n <= (size_t)sms * (gather ? 4096 : 256);
+    if (one) blocks = (c->n + 255) / 256;
+    auto launch = [&](auto kernel) { kernel<<<(unsigned)blocks, 256, 0, c->stream>>>(a); };
     prof_begin(c, gather && push ? "gather_push" : gather ? "gather" : "push");
     if (gather && push)
-        ke ? move_particles<true, true, true><<<(unsigned)blocks, 256, 0, c->stream>>>(a)
-           : move_particles<true, true><<<(unsigned)blocks, 256, 0, c->stream>>>(a);
+        launch(ke ? move_particles<2, true, true, true> : one ? move_particles<1, true, true> : move_particles<2, true, true>);
     else if (gather)
-        ke ? move_particles<true, false, true><<<(unsigned)blocks, 256, 0, c->stream>>>(a)
-           : move_particles<true, false><<<(unsigned)blocks, 256, 0, c->stream>>>(a);
+        launch(ke ? move_particles<2, true, false, true> : one ? move_particles<1, true, false> : move_particles<2, true, false>);
     else
-        move_particles<false, true><<<(unsigned)blocks, 256, 0, c->stream>>>(a);
+        launch(one ? move_particles<1, false, true> : move_particles<2, false, true>);
     prof_end(c);
     PIC_TRY(check_launch(c, "move_particles"));
     if (push) c->sorted = 0;

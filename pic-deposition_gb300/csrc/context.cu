@@ -521,10 +521,12 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
         reach[k] = dev_src[k] != nullptr;
     }
     bool direct = n > 0 && reach[0] && reach[1] && reach[2] && reach[3] && reach[4];
-    // masses that are not all 1 are stored; a direct upload that reaches them finds
-    // out in its kernel
-    bool need_m = false;
-    if (m && !(direct && reach[5])) {
+    // Masses that are not all 1 are stored. A direct upload that reaches them finds out in
+    // its kernel, which stores them as it goes where the first one says so or there is an
+    // array for them already; else a second pass does.
+    const bool scan = m && !(direct && reach[5]);
+    bool need_m = m && n > 0 && !scan && m[0] != 1.0;
+    if (scan) {
         for (size_t i = 0; i < n; ++i)
             if (m[i] != 1.0) {
                 need_m = true;
@@ -538,6 +540,7 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
         return rc;
     };
     if (need_m) PIC_TRY(ensure_mass());
+    const bool store_m = need_m || (m && !scan && c->m);
     c->has_mass = need_m ? 1 : 0;
 
     ConvertArgs a{};
@@ -553,7 +556,7 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
     a.fvx = c->vx;
     a.fvy = c->vy;
     a.fq = c->q;
-    a.fm = need_m ? c->m : nullptr;
+    a.fm = store_m ? c->m : nullptr;
     a.st = c->dstats;
     PIC_CUDA_TRY(cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), c->stream));
 
@@ -622,7 +625,9 @@ int pic_gpu_upload_particles(pic_ctx* c, const double* x, const double* y, const
     const DevStats& st = *c->hstats;
     c->qn_uniform = (n > 0 && st.q_mixed == 0 && st.q_first != 0.0f && std::isfinite(st.q_first)) ? st.q_first : 0.0f;
     const bool in_order = st.order_breaks == 0;
-    if (direct && dev_src[5] && st.mass_mixed) {
+    if (direct && store_m) {
+        c->has_mass = st.mass_mixed ? 1 : 0;
+    } else if (direct && dev_src[5] && st.mass_mixed) {
         const int rc = ensure_mass();
         if (rc != PIC_OK) {
             c->n = 0;  // the new particles' masses are not there

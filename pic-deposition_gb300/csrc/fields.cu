@@ -161,8 +161,9 @@ __global__ void scale_phi(double* __restrict__ phi, size_t g, double norm) {
 }
 
 // E = -(phi[i+1] - phi[i]) / d (poisson_fft.cpp:77-93, poisson_gs.cpp:48-60); FP32
-// copies for the gather; and the block's sums of rho and E^2, which the step's
-// diagnostics need: no passes over rho and E of their own. A block covers ITEMS
+// copies for the gather; and, in a time step (SUMS), the block's sums of rho and E^2,
+// which the step's diagnostics need: no passes over rho and E of their own. (A solve by
+// itself leaves them out: FP64 arithmetic of 60 us at 2048^2.) A block covers ITEMS
 // rounds of 256 cells: four, or one on a grid too small to give every SM a block.
 static int efield_items(size_t g) { return g < (size_t)RED_THREADS * 4 * 152 ? 1 : 4; }
 static size_t efield_blocks(size_t g) {
@@ -170,7 +171,7 @@ static size_t efield_blocks(size_t g) {
     return (g + per - 1) / per;
 }
 
-template <int ITEMS>
+template <int ITEMS, bool SUMS>
 __global__ void __launch_bounds__(RED_THREADS) efield(const double* __restrict__ phi, const double* __restrict__ rho,
                                                       int Nx, int Ny, double idx_dx, double idx_dy,
                                                       double* __restrict__ Ex, double* __restrict__ Ey,
@@ -191,10 +192,13 @@ __global__ void __launch_bounds__(RED_THREADS) efield(const double* __restrict__
             Ey[t] = ey;
             Exf[t] = __double2float_rn(ex);
             Eyf[t] = __double2float_rn(ey);
-            s = __dadd_rn(s, rho[t]);
-            ee = __dadd_rn(ee, __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
+            if constexpr (SUMS) {
+                s = __dadd_rn(s, rho[t]);
+                ee = __dadd_rn(ee, __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
+            }
         }
     }
+    if constexpr (!SUMS) return;
     double sums[2] = {s, ee};
     block_sums(sums);
     if (threadIdx.x == 0) reinterpret_cast<double2*>(partial)[blockIdx.x] = make_double2(sums[0], sums[1]);
@@ -322,10 +326,12 @@ void release_fields(pic_ctx* c) {
 
 int efield_from_phi(pic_ctx* c) {
     const unsigned blocks = (unsigned)efield_blocks(c->G);
-    (efield_items(c->G) == 1 ? efield<1> : efield<4>)<<<blocks, RED_THREADS, 0, c->stream>>>(
-        c->phi, c->rho, c->Nx, c->Ny, 1.0 / c->dx, 1.0 / c->dy, c->Ex, c->Ey, c->Exf, c->Eyf, c->grid_partials);
+    const bool one = efield_items(c->G) == 1;
+    auto kernel = c->in_run ? (one ? efield<1, true> : efield<4, true>) : (one ? efield<1, false> : efield<4, false>);
+    kernel<<<blocks, RED_THREADS, 0, c->stream>>>(c->phi, c->rho, c->Nx, c->Ny, 1.0 / c->dx, 1.0 / c->dy, c->Ex, c->Ey,
+                                                  c->Exf, c->Eyf, c->grid_partials);
     PIC_TRY(check_launch(c, "efield"));
-    c->grid_sums_ready = 1;
+    c->grid_sums_ready = c->in_run;
     return PIC_OK;
 }
 

@@ -125,6 +125,7 @@ struct pic_ctx {
     // solve; grid_sums_ready: they belong to the current rho and E
     double* grid_partials = nullptr;
     int grid_sums_ready = 0;
+    int in_run = 0;  // pic_gpu_run is stepping: its solves leave those sums
     // red_out[8], red_out[9] hold sum(q) and sum(|q|) of the current particle set:
     // charges do not change while particles move or are sorted
     int qsum_valid = 0;

@@ -213,6 +213,7 @@ int run_steps(pic_ctx* c, const pic_run_config* cfg, int steps, pic_diag* histor
         cleanup();
         return rc;
     }
+    c->in_run = 1;
     rc = [&]() -> int {
         PIC_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(int), c->stream));
         PIC_CUDA_TRY(cudaMemsetAsync(&c->dstats->moved, 0, sizeof(unsigned long long), c->stream));
@@ -287,6 +288,7 @@ int run_steps(pic_ctx* c, const pic_run_config* cfg, int steps, pic_diag* histor
         c->sorted = 0;  // conservative: the last step pushed the particles
         return check_device_status(c);
     }();
+    c->in_run = 0;
     cleanup();
     return rc;
 }

@@ -111,6 +111,11 @@ int pic_gpu_get_stream(pic_ctx* ctx, void** stream_out);
 int pic_gpu_profile_enable(pic_ctx* ctx, int enable);
 int pic_gpu_profile_read(pic_ctx* ctx, const char* kernel, double* total_ms, long long* launches);
 
+/* Test hook of the paths that a full device takes: the calling thread's further device
+ * allocations through this library may take `bytes` in all, and fail with PIC_ERR_NOMEM
+ * beyond that (cuFFT's own are not counted). ULLONG_MAX: no limit, as at the start. */
+int pic_gpu_test_alloc_budget(unsigned long long bytes);
+
 /* Page-locked host buffers for fast uploads/downloads (cudaHostAlloc / cudaFreeHost). */
 int pic_gpu_host_alloc(size_t bytes, void** out);
 int pic_gpu_host_free(void* p);
@@ -231,7 +236,8 @@ int pic_gpu_poisson_rbgs(pic_ctx* ctx, double tol, int max_iters, int warm_start
  * 0 (default) FP64 sweeps; 1 FP32 sweeps on a correction equation, refined in FP64
  * (r = b - A phi in FP64, A e = r relaxed in FP32, phi += e, until the FP64
  * relative residual meets tol). Both stop on the same FP64 test; mode 1 needs a
- * grid that tiles into 64x32 (or smaller power-of-two) tiles, else it runs mode 0. */
+ * grid that tiles into 64x32 (or smaller power-of-two) tiles, and room for its buffers
+ * (48 bytes per cell), else it runs mode 0. */
 int pic_gpu_set_rbgs_precision(pic_ctx* ctx, int mixed);
 
 /* Test hook of the bounded device waits (no counterpart in the reference): runs

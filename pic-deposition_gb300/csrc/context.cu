@@ -56,9 +56,17 @@ const void* device_view(const pic_ctx* ctx, const void* p, size_t align) {
     return at.type == cudaMemoryTypeUnregistered && ctx->reads_host ? p : nullptr;
 }
 
+// What pic_gpu_test_alloc_budget leaves this thread; the largest value: no limit.
+static thread_local unsigned long long g_alloc_budget = ~0ull;
+
 void* dalloc(size_t bytes, int* rc) {
     void* p = nullptr;
     if (bytes == 0) bytes = 16;
+    if (bytes > g_alloc_budget) {
+        *rc = fail(PIC_ERR_NOMEM, "allocation of " + std::to_string(bytes) + " bytes: beyond pic_gpu_test_alloc_budget");
+        return nullptr;
+    }
+    if (g_alloc_budget != ~0ull) g_alloc_budget -= bytes;
     const cudaError_t e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess) {
         *rc = fail(PIC_ERR_NOMEM, std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
@@ -738,6 +746,11 @@ int pic_gpu_is_sorted(pic_ctx* c, int* out) {
 int pic_gpu_charge_uniform(pic_ctx* c, float* out) {
     if (!c || !out) return fail(PIC_ERR_ARG, "NULL argument");
     *out = c->qn_uniform;
+    return PIC_OK;
+}
+
+int pic_gpu_test_alloc_budget(unsigned long long bytes) {
+    g_alloc_budget = bytes;
     return PIC_OK;
 }
 

@@ -605,12 +605,15 @@ static int rb_launch(pic_ctx* c, const RbTiling& t, const PsArgs<T>& p, bool pow
     return PIC_OK;
 }
 
-// Device words of the one-launch solves: partial sums, then out[0..3], the
-// barrier and the error flag.
-static int ensure_ps(pic_ctx* c) {
+// Buffers of the one-launch solves: partial sums, out[0..3], the barrier and the error
+// flag; the exchange buffers; with `mixed` the residuals and the correction. False when the
+// device has no room for them: the launches per colour need none.
+static bool ensure_ps(pic_ctx* c, bool mixed) {
     int rc = PIC_OK;
     if (!c->rb_ps) c->rb_ps = (double*)dalloc((4 * PS_MAX_BLOCKS + 8) * sizeof(double), &rc);
-    return rc;
+    if (!rc && !c->rb_xb) c->rb_xb = dalloc(2 * c->G * 2 * sizeof(double), &rc);
+    if (!rc && mixed && !c->rb_mix) c->rb_mix = (double*)dalloc(c->G * (8 + 4 + 4), &rc);
+    return rc == PIC_OK;
 }
 
 static int sm_count(pic_ctx* c) {
@@ -625,8 +628,8 @@ static int largest_divisor_tile(int n, const int* cand, int ncand) {
     return 0;
 }
 
-// Solves in one cooperative launch when the tiles fit the SMs' shared memory;
-// returns PIC_ERR_UNSUPPORTED (nothing queued) otherwise.
+// Solves in one cooperative launch when the tiles fit the SMs' shared memory and its
+// buffers the device's; returns PIC_ERR_UNSUPPORTED (nothing queued) otherwise.
 // absent_block >= 0 makes that CTA leave before its first barrier, so that every
 // other CTA's wait runs out after wait_ns (the timeout test hook; -1 in solves).
 static int rbgs_solve_persistent(pic_ctx* c, const RbArgs& a, double tol, int max_iters, int check_every, int* it,
@@ -636,10 +639,7 @@ static int rbgs_solve_persistent(pic_ctx* c, const RbArgs& a, double tol, int ma
     const int step = (check_every % 4 == 0 && max_iters % 4 == 0) ? 4 : 2;
     const RbTiling t = rb_tiling(c->Nx, c->Ny, sm_count(c), step, sizeof(double), pow2 ? 64.0 : 112.0, 400.0);
     if (!t.ntx) return PIC_ERR_UNSUPPORTED;
-    PIC_TRY(ensure_ps(c));
-    int rc = PIC_OK;
-    if (!c->rb_xb) c->rb_xb = dalloc(2 * c->G * 2 * sizeof(double), &rc);
-    if (rc) return rc;
+    if (!ensure_ps(c, false)) return PIC_ERR_UNSUPPORTED;
     double* out = c->rb_ps + 4 * PS_MAX_BLOCKS;
     unsigned* bar = reinterpret_cast<unsigned*>(out + 4);
     int* err = reinterpret_cast<int*>(out + 5);
@@ -697,12 +697,7 @@ static int rbgs_solve_mixed(pic_ctx* c, const RbArgs& a, double tol, int max_ite
     const bool pow2 = rb_pow2(a);
     const RbTiling t = rb_tiling(c->Nx, c->Ny, sm_count(c), 4, sizeof(float), 14.0, 200.0);
     if (!t.ntx) return PIC_ERR_UNSUPPORTED;
-    PIC_TRY(ensure_ps(c));
-    int rc = PIC_OK;
-    if (!c->rb_mix) c->rb_mix = (double*)dalloc(c->G * (8 + 4 + 4), &rc);
-    if (rc) return rc;
-    if (!c->rb_xb) c->rb_xb = dalloc(2 * c->G * 2 * sizeof(double), &rc);
-    if (rc) return rc;
+    if (!ensure_ps(c, true)) return PIC_ERR_UNSUPPORTED;
     double* r64 = c->rb_mix;
     float* r32 = reinterpret_cast<float*>(r64 + c->G);
     float* e32 = r32 + c->G;

@@ -17,6 +17,7 @@ compiled library and a CUDA device and raises if either is missing.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import enum
 import os
@@ -188,6 +189,19 @@ def run_ensemble_ranks(runs, steps: int, rank: int = 0, world_size: int = 1, ens
     return out_fe, out_ke
 
 
+@contextlib.contextmanager
+def test_alloc_budget(nbytes: int):
+    """Device allocations of this thread's calls may take `nbytes` in all (pic_gpu_test_alloc_budget)."""
+    _check(lib().pic_gpu_test_alloc_budget(int(nbytes)))
+    try:
+        yield
+    finally:
+        _check(lib().pic_gpu_test_alloc_budget(2**64 - 1))
+
+
+test_alloc_budget.__test__ = False
+
+
 def nn_conv3x3(op: int, x: np.ndarray, weight=None, bias=None, aux=None, cin: int = 32, cout: int = 32):
     """One tensor-core convolution layer on host arrays (pic_nn_conv3x3).
 
@@ -229,6 +243,7 @@ class GenConfig(C.Structure):
 _SIGS.append(("pic_gpu_generate", [_vp, C.POINTER(GenConfig)]))
 _SIGS.append(("pic_gpu_set_rbgs_precision", [_vp, C.c_int]))
 _SIGS.append(("pic_gpu_test_rbgs_barrier_timeout", [_vp, C.c_int, C.c_double]))
+_SIGS.append(("pic_gpu_test_alloc_budget", [C.c_ulonglong]))
 _SIGS.append(("pic_gpu_test_device_choices", [_vp] + [C.POINTER(C.c_int)] * 3))
 
 

@@ -281,9 +281,6 @@ static int ensure_spec(pic_ctx* c) {
 static int ensure_fft(pic_ctx* c) {
     PIC_TRY(ensure_spec(c));
     if (c->fft_ready) return PIC_OK;
-    int rc = PIC_OK;
-    if (!c->fft_rhs) c->fft_rhs = (double*)dalloc(c->G * 8, &rc);
-    if (rc) return rc;
     cufftHandle f, b;
     PIC_CUFFT_TRY(cufftPlan2d(&f, c->Ny, c->Nx, CUFFT_D2Z));
     PIC_CUFFT_TRY(cufftPlan2d(&b, c->Ny, c->Nx, CUFFT_Z2D));
@@ -377,6 +374,9 @@ __global__ void k_divide_discrete(cufftDoubleComplex* __restrict__ spec, int Nx,
 
 int solve_discrete_fft(pic_ctx* c, const double* b, double* phi) {
     PIC_TRY(ensure_fft(c));
+    int rc = PIC_OK;
+    if (!c->fft_rhs) c->fft_rhs = (double*)dalloc(c->G * 8, &rc);
+    if (rc) return rc;
     double ix2, iy2, denom;
     rbgs_operator(c, &ix2, &iy2, &denom);
     PIC_CUDA_TRY(cudaMemcpyAsync(c->fft_rhs, b, c->G * 8, cudaMemcpyDeviceToDevice, c->stream));

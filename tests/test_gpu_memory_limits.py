@@ -1,5 +1,6 @@
 """Solves on a device that has no room for more: the one-launch Gauss-Seidel solve's
-buffers are optional."""
+buffers are optional, and an FFT solve takes no more memory than its spectrum and one
+grid."""
 import numpy as np
 import pytest
 
@@ -23,6 +24,19 @@ def test_gauss_seidel_without_its_exchange_buffers(pg, nx, ny, room, mixed):
         assert all(np.array_equal(a, b) for a, b in zip(got[1], want[1]))
         it, _ = c.poisson_rbgs(tol=0.0, max_iters=40, warm_start=False, check_every=8)  # with room again
         assert it == 40
+
+
+@pytest.mark.parametrize("nx,ny", [(96, 160), (64, 64), (77, 33)])
+def test_fft_solve_within_spectrum_and_one_grid(pg, nx, ny):
+    rho = np.random.default_rng(nx).normal(size=nx * ny)
+    with pg.Context(nx, ny, float(nx), float(ny), 1) as c, pg.Context(nx, ny, float(nx), float(ny), 1) as free:
+        for k in (c, free):
+            k.set_rho(rho)
+            k.fields()  # phi and E
+        with pg.test_alloc_budget(16 * (nx // 2 + 1) * ny + 8 * nx * ny):
+            c.poisson_fft()
+        free.poisson_fft()
+        assert all(np.array_equal(a, b) for a, b in zip(c.fields(), free.fields()))
 
 
 def test_the_budget_fails_with_nomem(pg):

@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const
     for (walk.start(cw, warp); !walk.done(cw); walk.advance(cw)) {
         walk.stage(cw, lane);
         const float* sb = reinterpret_cast<const float*>(sbuf);
-        const int r = cw.r, col = cw.c0 + (lane >> klog);
+        const int r = cw.r, col = cw.c0 + (lane >> cw.klog);
         int m, first;
         uint32_t ncell;
         walk.share(cw, lane, first, m, ncell);
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const
         constexpr int UN = 2;
         const int ng = (m + UN - 1) / UN;
         const int trips = __reduce_max_sync(0xffffffffu, ng);
-        int g = (lane >> klog) < ng ? lane >> klog : 0;
+        int g = (lane >> cw.klog) < ng ? lane >> cw.klog : 0;
 #pragma unroll 1
         for (int t = 0; t < trips; ++t) {
             const int left = t < ng ? m - g * UN : 0;
@@ -635,7 +635,7 @@ __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const
         }
         if (small) {
             // the cell's sums over its K lanes, which share the seven values
-            const int K = 1 << klog;
+            const int K = 1 << cw.klog;
             for (int o = 1; o < K; o <<= 1) {
                 e1 += __shfl_xor_sync(0xffffffffu, e1, o);
                 e2 += __shfl_xor_sync(0xffffffffu, e2, o);
@@ -720,8 +720,9 @@ int deposit_current_async(pic_ctx* c, double dt) {
         // after the other (33 x 9: 48 us with tiles of 8 rows)
         int th = JC_TH;
         while (th > 1 && (long long)tiles_x * ((c->Ny + th - 1) / th) < 2 * sms) th /= 2;
+        const unsigned tiles = (unsigned)(tiles_x * ((c->Ny + th - 1) / th));
         int klog, cap;
-        cells_shape(c->n, c->G, qc ? 4 : 5, 1560, &klog, &cap);
+        cells_shape(c->n, c->G, qc ? 4 : 5, 1560, (size_t)tiles * JC_WARPS, &klog, &cap);
         PIC_TRY(ensure_sort_scratch(c));  // the list takes the sort's spare arrays
         unsigned* count = reinterpret_cast<unsigned*>(c->junits + 2);
         const JList list{count, c->idx_b, c->cell_alt, c->alt[0], c->alt[1], c->alt[2], c->alt[3]};
@@ -740,7 +741,6 @@ int deposit_current_async(pic_ctx* c, double dt) {
         current_begin<<<(unsigned)zero, J_THREADS, 0, c->stream>>>(a, c->G, many, count);
         PIC_TRY(check_launch(c, "current_begin"));
         prof_begin(c, "current");
-        const unsigned tiles = (unsigned)(tiles_x * ((c->Ny + th - 1) / th));
         if (qc)
             current_cells<true><<<tiles, JC_WARPS * 32, smem, c->stream>>>(a, c->offsets, tiles_x, th, klog, cap, list);
         else

@@ -1321,7 +1321,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
         // the lane's share of its cell, walked four particles at a time and cyclically
         // from a group that differs from cell to cell (cells of equal size would meet
         // in the same bank)
-        const int cl = lane >> a.klog, iy = y0 + cw.r, col = cw.c0 + cl;
+        const int cl = lane >> cw.klog, iy = y0 + cw.r, col = cw.c0 + cl;
         const uint32_t mykey = (uint32_t)iy * (uint32_t)a.Nx + (uint32_t)(x0 + col);
         int m, first;
         uint32_t ncell;
@@ -1422,13 +1422,11 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
             }
         }
         if constexpr (S == S_CIC && QC) {
-            if (small && !walk.last(cw)) {
-                cnt += part;
-            } else if (small) {
+            if (small) {
                 // the cell's sums over its lanes; then a lane writes one node (of 4 / K), all
                 // in 32 bits: a node of at most 127 particles is below 2^31
                 cnt += part;
-                const int K = 1 << a.klog;
+                const int K = 1 << cw.klog;
                 for (int o = 1; o < K; o <<= 1) {
                     run.r += __shfl_xor_sync(FULL, run.r, o);
                     run.c += __shfl_xor_sync(FULL, run.c, o);
@@ -1460,19 +1458,37 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
         } else {
             fold();
         }
-        if (walk.last(cw) && !small) {  // the end of the unit: write out this lane's cell
-            long long tv[NV];
-            run.totals(cnt, tv);
-            int base = 0, keep = NV;  // the lane writes tv[0 .. keep), nodes base ..
-            bool write = cnt != 0;
-            if constexpr ((NV & (NV - 1)) == 0) {
+        if (!small) {  // the end of the piece: write out this lane's cell
+            long long t[NV];
+            run.totals(cnt, t);
+            auto put = [&](int q, long long x) {  // x to node q of the lane's cell
+                if (x == 0) return;
+                if (dense) {
+                    const size_t g = (size_t)wrap_i(iy + LO + q / NX, a.Ny) * a.Nx + wrap_i(x0 + col + LO + q % NX, a.Nx);
+                    atomicAdd(a.acc + g, (unsigned long long)x);
+                } else {
+                    const int i = (cw.r + 1 + LO + PAD + q / NX) * SW + col + 1 + LO + PAD + q % NX;
+                    atomicAdd(slo + i, (uint32_t)x & ((1u << TILE_SPLIT) - 1u));
+                    atomicAdd(shi + i, (int)(x >> TILE_SPLIT));
+                }
+            };
+            if (NV == 9 && cw.klog == 0) {
+                if (cnt) {
+#pragma unroll
+                    for (int q = 0; q < NV; ++q) put(q, t[q]);
+                }
+            } else {
                 // the K lanes of a cell would add to the same nodes: halve the nodes a
                 // lane keeps for each lane it shares the cell with, exchanging the
                 // other half, until it has one; further lanes just add
-                int b = 0;
+                constexpr int NP = NV <= 4 ? 4 : 16;  // NV, rounded up to a power of two
+                long long tv[NP];
 #pragma unroll
-                for (int half = NV / 2; half >= 1; half /= 2) {
-                    if (b < a.klog) {
+                for (int q = 0; q < NP; ++q) tv[q] = q < NV ? t[q < NV ? q : 0] : 0;
+                int base = 0, keep = NV, b = 0;  // the lane writes tv[0 .. keep), nodes base ..
+#pragma unroll
+                for (int half = NP / 2; half >= 1; half /= 2) {
+                    if (b < cw.klog) {
                         const bool up = (lane >> b) & 1;
 #pragma unroll
                         for (int q = 0; q < half; ++q) {
@@ -1484,27 +1500,14 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
                         ++b;
                     }
                 }
-                for (; b < a.klog; ++b) {
+                for (; b < cw.klog; ++b) {
                     tv[0] += __shfl_xor_sync(FULL, tv[0], 1 << b);
                     if ((lane >> b) & 1) base = -1;
                 }
-                write = base >= 0 && cl < cw.cn;
-            }
-            if (write) {
+                if (base >= 0 && ncell != 0) {
 #pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    const long long x = tv[k];
-                    if (k < keep && x != 0) {
-                        const int q = base + k;
-                        if (dense) {
-                            const size_t g = (size_t)wrap_i(iy + LO + q / NX, a.Ny) * a.Nx + wrap_i(x0 + col + LO + q % NX, a.Nx);
-                            atomicAdd(a.acc + g, (unsigned long long)x);
-                        } else {
-                            const int i = (cw.r + 1 + LO + PAD + q / NX) * SW + col + 1 + LO + PAD + q % NX;
-                            atomicAdd(slo + i, (uint32_t)x & ((1u << TILE_SPLIT) - 1u));
-                            atomicAdd(shi + i, (int)(x >> TILE_SPLIT));
-                        }
-                    }
+                    for (int k = 0; k < NV; ++k)
+                        if (k < keep) put(base + k, tv[k]);
                 }
             }
             run.zero();
@@ -1718,7 +1721,7 @@ static int launch_cells(pic_ctx* c, DepArgs a, unsigned tiles) {
     // cell: 213 us against 132 with 2,600, 183 in the form without staged units; 1024^2 x 64
     // 1.92 and 1.56 ms).
     constexpr int WORDS = S == S_ESK && KEYS ? 2600 : S == S_TSC || S == S_ESK ? 3120 : 2080;
-    cells_shape(a.n, c->G, StageFields<S, QC>::NF - (KEYS ? 0 : 1), WORDS, &a.klog, &a.cap);
+    cells_shape(a.n, c->G, StageFields<S, QC>::NF - (KEYS ? 0 : 1), WORDS, (size_t)tiles * NW, &a.klog, &a.cap);
     const size_t smem = cells_fixed_bytes<S, NW, QC, KEYS>(a.cap) +
                         (size_t)(a.tile_h + 3 + 2 * PAD) * (a.tile_w + 3 + 2 * PAD) * 2 * sizeof(uint32_t) +
                         (size_t)a.tile_h * (a.tile_w + 1) * sizeof(uint32_t);

@@ -161,9 +161,10 @@ __global__ void scale_phi(double* __restrict__ phi, size_t g, double norm) {
 }
 
 // E = -(phi[i+1] - phi[i]) / d (poisson_fft.cpp:77-93, poisson_gs.cpp:48-60); FP32
-// copies for the gather; and, in a time step (SUMS), the block's sums of rho and E^2,
-// which the step's diagnostics need: no passes over rho and E of their own. (A solve by
-// itself leaves them out: FP64 arithmetic of 60 us at 2048^2.) A block covers ITEMS
+// copies for the gather; and (SUMS) the block's sums of rho and E^2, which the step's
+// diagnostics need: no passes over rho and E of their own (11 us less for a solve and its
+// diagnostics at 64^2). Gauss-Seidel solves of large grids outside a time step leave them
+// out: FP64 arithmetic of 60 us at 2048^2. A block covers ITEMS
 // rounds of 256 cells: four, or one on a grid too small to give every SM a block.
 static int efield_items(size_t g) { return g < (size_t)RED_THREADS * 4 * 152 ? 1 : 4; }
 static size_t efield_blocks(size_t g) {
@@ -321,14 +322,14 @@ void release_fields(pic_ctx* c) {
     for (void* p : ptrs) dfree(p);
 }
 
-int efield_from_phi(pic_ctx* c) {
+int efield_from_phi(pic_ctx* c, bool sums) {
     const unsigned blocks = (unsigned)efield_blocks(c->G);
     const bool one = efield_items(c->G) == 1;
-    auto kernel = c->in_run ? (one ? efield<1, true> : efield<4, true>) : (one ? efield<1, false> : efield<4, false>);
+    auto kernel = sums ? (one ? efield<1, true> : efield<4, true>) : (one ? efield<1, false> : efield<4, false>);
     kernel<<<blocks, RED_THREADS, 0, c->stream>>>(c->phi, c->rho, c->Nx, c->Ny, 1.0 / c->dx, 1.0 / c->dy, c->Ex, c->Ey,
                                                   c->Exf, c->Eyf, c->grid_partials);
     PIC_TRY(check_launch(c, "efield"));
-    c->grid_sums_ready = c->in_run;
+    c->grid_sums_ready = sums;
     return PIC_OK;
 }
 

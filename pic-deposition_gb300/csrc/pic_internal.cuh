@@ -125,7 +125,7 @@ struct pic_ctx {
     // solve; grid_sums_ready: they belong to the current rho and E
     double* grid_partials = nullptr;
     int grid_sums_ready = 0;
-    int in_run = 0;  // pic_gpu_run is stepping: its solves leave those sums
+    int in_run = 0;  // pic_gpu_run is stepping: every solve leaves those sums
     // red_out[8], red_out[9] hold sum(q) and sum(|q|) of the current particle set:
     // charges do not change while particles move or are sorted
     int qsum_valid = 0;
@@ -204,7 +204,7 @@ int sort_particles(pic_ctx* ctx, bool perm = false);
 // Fields, Poisson and diagnostics (fields.cu).
 int ensure_fields(pic_ctx* ctx);
 int poisson_fft(pic_ctx* ctx);
-int efield_from_phi(pic_ctx* ctx);
+int efield_from_phi(pic_ctx* ctx, bool sums = true);
 // This library's transforms (fft.cu): sides that are powers of two from 8 to 2048.
 bool own_fft_size(int n);
 int make_own_fft(pic_ctx* ctx);

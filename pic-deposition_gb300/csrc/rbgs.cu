@@ -183,7 +183,7 @@ static int rb_finish(pic_ctx* c) {
     PIC_TRY(check_launch(c, "rb_final"));
     rb_sub_mean<<<blocks, 256, 0, c->stream>>>(c->phi, c->G, c->rb_scalars + 3);
     PIC_TRY(check_launch(c, "rb_sub_mean"));
-    return efield_from_phi(c);
+    return efield_from_phi(c, c->in_run || c->G <= (size_t)1 << 20);
 }
 
 // ---- one cooperative launch per solve ---------------------------------------

@@ -18,7 +18,7 @@ def check(c, nx, ny):
 
 
 @pytest.mark.parametrize("solve", ["poisson_fft", "poisson_rbgs"])
-@pytest.mark.parametrize("nx,ny", [(16, 8), (30, 22), (512, 330)])
+@pytest.mark.parametrize("nx,ny", [(16, 8), (30, 22), (512, 330), (1200, 900)])
 def test_sums_follow_the_grids(pg, nx, ny, solve):
     rng = np.random.default_rng(nx)
     n = 4000

@@ -655,19 +655,25 @@ __global__ void __launch_bounds__(JC_WARPS * 32, 5) current_cells(JArgs a, const
     tile_to_grids(a, slo, shi, x0, y0);
 }
 
-// The grids as FP64, four cells per thread: each thread forms the units (FP64
-// multiplications are slow on this part: 7 us at 1024^2 with a cell per thread), the first
-// also stores them.
+// The grids as FP64, four cells per thread: each block's first thread forms the units (FP64
+// multiplications are slow on this part), the first block's also stores them.
 __global__ void __launch_bounds__(256) current_to_f64(const long long* __restrict__ jx, const long long* __restrict__ jy,
                                                       size_t g, double inv_vol, double dxdt, double dydt,
                                                       const DevStats* st, double* __restrict__ units,
                                                       double* __restrict__ ox, double* __restrict__ oy) {
     const size_t i0 = (size_t)blockIdx.x * 1024 + threadIdx.x;
-    const double u = charge_unit(st, inv_vol), ux = __dmul_rn(u, dxdt), uy = __dmul_rn(u, dydt);
-    if (i0 == 0) {
-        units[0] = ux;
-        units[1] = uy;
+    __shared__ double s_units[2];
+    if (threadIdx.x == 0) {
+        const double u = charge_unit(st, inv_vol);
+        s_units[0] = __dmul_rn(u, dxdt);
+        s_units[1] = __dmul_rn(u, dydt);
+        if (i0 == 0) {
+            units[0] = s_units[0];
+            units[1] = s_units[1];
+        }
     }
+    __syncthreads();
+    const double ux = s_units[0], uy = s_units[1];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const size_t i = i0 + k * 256;

@@ -1674,9 +1674,10 @@ __device__ void choose_any_order(DevStats* st, unsigned long long limit, unsigne
 
 // The int64 grid as FP64 rho, four cells per thread. One unit (FP64) is max|q| *
 // inv_vol * 2^-24, or, for the exact integer TSC form, max|q| * inv_vol * (qn *
-// 2^-30) (scale != 0); each thread forms it, and the first also stores it and,
-// with n > 0, takes the any-order decision of a deposit between sorts: two
-// launches fewer per deposit. In a time step one more block ends the diagnostics of the
+// 2^-30) (scale != 0); each block's first thread forms it (FP64 multiplications are slow
+// on this part: formed by every thread, 3 M cells took 5 us more), and the first block's
+// also stores it and, with n > 0, takes the any-order decision of a deposit between sorts:
+// two launches fewer per deposit. In a time step one more block ends the diagnostics of the
 // step before, whose sums this step's move and that step's solve have left: by
 // itself it was a link of the step's chain of launches (64^2, 16 per cell: 54.6 us a
 // step against 52.4; 256^2, TSC: 88.5 against 85.6).
@@ -1687,13 +1688,17 @@ __global__ void __launch_bounds__(RED_THREADS) fixed_to_rho(const long long* __r
         diag_block(diag);
         return;
     }
+    __shared__ double s_unit;
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    const double unit = scale == 0.0 ? charge_unit(st, inv_vol)
-                                     : __dmul_rn(__dmul_rn((double)load_maxq(st), inv_vol), scale);
-    if (i == 0) {
-        *unit_out = unit;
-        if (n) choose_any_order(st, limit, n);
+    if (threadIdx.x == 0) {
+        s_unit = scale == 0.0 ? charge_unit(st, inv_vol) : __dmul_rn(__dmul_rn((double)load_maxq(st), inv_vol), scale);
+        if (i == 0) {
+            *unit_out = s_unit;
+            if (n) choose_any_order(st, limit, n);
+        }
     }
+    __syncthreads();
+    const double unit = s_unit;
     if (i + 3 < g) {  // 32-byte aligned: the grids start on 256 bytes
         const longlong2 a = *reinterpret_cast<const longlong2*>(acc + i);
         const longlong2 b = *reinterpret_cast<const longlong2*>(acc + i + 2);

@@ -28,7 +28,7 @@ struct CellPiece {
     int r, ch;          // tile row, unit of the row
     int c0, cn, klog;   // the piece's first column, columns, log2 lanes per cell
     uint32_t pos, end;  // first particle staged, end of the unit's range
-    bool pieces;        // the range is longer than the buffer
+    bool pieces;        // the range is longer than the buffer, and of several cells
 };
 
 // NF fields of 4 bytes per particle; field f of the buffer's particle i is word
@@ -68,7 +68,7 @@ struct CellWalk {
             const uint32_t beg = soff[w.r * (tw + 1) + w.c0];
             w.end = soff[w.r * (tw + 1) + w.c0 + w.cn];
             w.pos = beg & ~3u;
-            w.pieces = w.end - w.pos > (uint32_t)cap;
+            w.pieces = klog < 5 && w.end - w.pos > (uint32_t)cap;  // a unit of one cell has all lanes already
             if (w.end > beg) return;
         }
     }
@@ -86,6 +86,11 @@ struct CellWalk {
         w.cn = 32 - __clz(m) - first;
         w.klog = w.cn == 1 ? 5 : __clz(w.cn - 1) - 27;  // 32 over the next power of two
     }
+    // all lanes are at one cell, and so they are in the next piece: their sums may go on
+    __device__ __forceinline__ bool same_cell(const CellPiece& w) const {
+        if (__builtin_expect(w.cn != 1 || w.end - w.pos <= (uint32_t)cap, 1)) return false;
+        return soff[w.r * (tw + 1) + w.c0 + 1] >= min(w.end, w.pos + 2u * (uint32_t)cap);
+    }
     __device__ __forceinline__ void advance(CellPiece& w) const {
         w.pos += (uint32_t)cap;
         if (w.pos >= w.end) {
@@ -95,7 +100,7 @@ struct CellWalk {
     }
     // copies the piece; returns when it has arrived, in every lane
     __device__ __forceinline__ void stage(CellPiece& w, int lane) const {
-        if (w.pieces) narrow(w);
+        if (__builtin_expect(w.pieces, 0)) narrow(w);
         const uint32_t n4 = (min(w.end - w.pos, (uint32_t)cap) + 3u) >> 2;
         for (uint32_t i = (uint32_t)lane; i < n4; i += 32)
 #pragma unroll
@@ -117,7 +122,7 @@ struct CellWalk {
         const uint32_t b = max(soff[o], w.pos), e = min(soff[o + 1], min(w.end, w.pos + (uint32_t)cap));
         if (e <= b) return;
         int per = (int)(e - b + (1u << w.klog) - 1u) >> w.klog;
-        if (w.klog != klog) per |= 1;  // many lanes of one cell start in different banks
+        per |= w.pieces ? 1 : 0;  // many lanes of one cell start in different banks
         first = (int)(b - w.pos) + sub * per;
         m = max(0, min(per, (int)(e - b) - sub * per));
     }

@@ -719,7 +719,10 @@ int deposit_current_async(pic_ctx* c, double dt) {
     a.st = c->dstats;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    if (c->n && c->sorted) {
+    // Sets of less than a particle per two cells take the any-order kernel also when sorted:
+    // a walk of empty cells costs more (2048^2, 0.01 per cell: 68 us against 190, 150 with one
+    // lane per cell; 0.5: 207 to 297 against 293 to 366; 1.0: 348 to 518 against 316 to 496).
+    if (c->sorted && 2 * c->n >= c->G && c->n) {
         const bool qc = a.qc != 0.0f;
         const int tiles_x = (c->Nx + JC_TW - 1) / JC_TW;
         // at least two tiles for every SM where the rows allow: a warp takes its units one

@@ -1458,7 +1458,9 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
         } else {
             fold();
         }
-        if (!small) {  // the end of the piece: write out this lane's cell
+        // the end of the piece: write out this lane's cell, unless the lanes stay at it (TSC always
+        // writes: its many sums, carried on, cost every unit 1.4 %, 1024^2 x 100 between sorts)
+        if (!small && (S == S_TSC || !walk.same_cell(cw))) {
             long long t[NV];
             run.totals(cnt, t);
             auto put = [&](int q, long long x) {  // x to node q of the lane's cell
@@ -1472,28 +1474,19 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
                     atomicAdd(shi + i, (int)(x >> TILE_SPLIT));
                 }
             };
-            if (NV == 9 && cw.klog == 0) {
-                if (cnt) {
-#pragma unroll
-                    for (int q = 0; q < NV; ++q) put(q, t[q]);
-                }
-            } else {
+            if constexpr ((NV & (NV - 1)) == 0) {
                 // the K lanes of a cell would add to the same nodes: halve the nodes a
                 // lane keeps for each lane it shares the cell with, exchanging the
                 // other half, until it has one; further lanes just add
-                constexpr int NP = NV <= 4 ? 4 : 16;  // NV, rounded up to a power of two
-                long long tv[NP];
+                int base = 0, keep = NV, b = 0;  // the lane writes t[0 .. keep), nodes base ..
 #pragma unroll
-                for (int q = 0; q < NP; ++q) tv[q] = q < NV ? t[q < NV ? q : 0] : 0;
-                int base = 0, keep = NV, b = 0;  // the lane writes tv[0 .. keep), nodes base ..
-#pragma unroll
-                for (int half = NP / 2; half >= 1; half /= 2) {
+                for (int half = NV / 2; half >= 1; half /= 2) {
                     if (b < cw.klog) {
                         const bool up = (lane >> b) & 1;
 #pragma unroll
                         for (int q = 0; q < half; ++q) {
-                            const long long give = up ? tv[q] : tv[half + q];
-                            tv[q] = (up ? tv[half + q] : tv[q]) + __shfl_xor_sync(FULL, give, 1 << b);
+                            const long long give = up ? t[q] : t[half + q];
+                            t[q] = (up ? t[half + q] : t[q]) + __shfl_xor_sync(FULL, give, 1 << b);
                         }
                         base += up ? half : 0;
                         keep = half;
@@ -1501,14 +1494,17 @@ __global__ void __launch_bounds__(NW * 32, MINB) deposit_cells(DepArgs a) {
                     }
                 }
                 for (; b < cw.klog; ++b) {
-                    tv[0] += __shfl_xor_sync(FULL, tv[0], 1 << b);
+                    t[0] += __shfl_xor_sync(FULL, t[0], 1 << b);
                     if ((lane >> b) & 1) base = -1;
                 }
                 if (base >= 0 && ncell != 0) {
 #pragma unroll
                     for (int k = 0; k < NV; ++k)
-                        if (k < keep) put(base + k, tv[k]);
+                        if (k < keep) put(base + k, t[k]);
                 }
+            } else if (cnt) {  // trajectory scheme: few of the nine are not zero
+#pragma unroll
+                for (int q = 0; q < NV; ++q) put(q, t[q]);
             }
             run.zero();
             cnt = 0;
@@ -1711,11 +1707,17 @@ __global__ void __launch_bounds__(RED_THREADS) fixed_to_rho(const long long* __r
     }
 }
 
-constexpr int CELLS_NW = 4, CELLS_MINB = 4;  // warps of a CTA, CTAs per SM the registers allow
+constexpr int CELLS_NW = 4;  // warps of a CTA
+// CTAs per SM the registers allow: NGP with one charge needs little more than the 72 of
+// seven (six: 1024^2 x 1 47 us, seven: 39).
+template <int S, bool QC, bool KEYS>
+constexpr int cells_minb() {
+    return S == S_NGP && QC && !KEYS ? 7 : 4;
+}
 
 template <int S, bool QC, bool KEYS>
 static int launch_cells(pic_ctx* c, DepArgs a, unsigned tiles) {
-    constexpr int NW = CELLS_NW, MINB = CELLS_MINB;
+    constexpr int NW = CELLS_NW, MINB = cells_minb<S, QC, KEYS>();
     constexpr int PAD = (KEYS && S != S_ESK) ? 1 : 0;  // the kernel's extra halo between sorts
     // TSC and the trajectory scheme keep four CTAs per SM by their registers: room for
     // larger units. 1024^2 x 64, one charge, us per call with 1,040 / 2,080 / 3,120

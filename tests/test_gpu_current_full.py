@@ -83,3 +83,17 @@ def test_a_move_of_a_cell_is_refused_either_way(pg):
             with pytest.raises(pg.PicError) as e:
                 c.deposit_current(1.0)
             assert e.value.code == -6  # PIC_ERR_COURANT
+
+
+@pytest.mark.parametrize("nx,ny", [(300, 211), (64, 40)])
+def test_sparse_sets(pg, nx, ny):
+    """Less than a particle per two cells: the any-order kernel, sorted or not. With
+    particles of no charge up to a particle per cell the cell kernels take the same set."""
+    rng = np.random.default_rng(4)
+    m, n = nx * ny // 3, nx * ny
+    x, y = rng.random(n) * nx, rng.random(n) * ny
+    q = np.where(np.arange(n) < m, rng.choice([-1.0, 2.0], n), 0.0)
+    vx, vy = np.clip(rng.normal(0, 0.4, (2, n)), -0.95, 0.95)
+    few, _ = current(pg, nx, ny, (x[:m], y[:m], q[:m], vx[:m], vy[:m]), True)
+    all_, _ = current(pg, nx, ny, (x, y, q, vx, vy), True)
+    assert np.array_equal(few[0], all_[0]) and np.array_equal(few[1], all_[1])

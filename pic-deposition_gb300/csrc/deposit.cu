@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(DEP_THREADS, 4) deposit_runs_tsc(DepArgs a) {
 // tile_w x tile_h cells; the tile's rows are cut into units of U = 32 / K
 // consecutive cells and warp w walks units w, w+NW, ... K lanes share a cell of
 // the unit: its contiguous range [offsets[c], offsets[c+1]) of the cell-sorted
-// stream, every K-th particle each.
+// stream, a stretch of it each.
 //  * Staging: a unit's particles are one contiguous range, copied to shared memory
 //    coalesced (cells.cuh). Lanes then walk their own cells there, starting at
 //    different particles of the cell, so that cells of equal size do not meet in

@@ -12,11 +12,11 @@
 //
 // One step (every run): gather + push, [cell sort], CIC deposit in fixed point,
 // + background, FFT Poisson per run, E. The particle work of a step is ONE
-// persistent cooperative launch (ens_step_kernel): phase 1 moves every particle
-// of every run, a grid-wide barrier, phase 2 deposits them (the run-aggregating
-// warp step: 4 consecutive particles per lane, register sums per cell,
-// segmented warp scan, one int64 atomic per run of equal cells), a barrier,
-// phase 3 turns the int64 grid into rho (+ background) and clears it. The
+// persistent cooperative launch (ens_step_kernel): it moves every particle
+// of every run and deposits each warp's moved particles from registers (the
+// run-aggregating warp step: 4 consecutive particles per lane, register sums per cell,
+// segmented warp scan, one int64 atomic per run of equal cells); then, after a grid-wide
+// barrier, it turns the int64 grid into rho (+ background) and clears it. The
 // Poisson solves are one batched cuFFT plan per grid size (runs sorted by
 // size, so equal sizes are contiguous) plus two small kernels, the sizes on
 // streams of their own. With use_graph

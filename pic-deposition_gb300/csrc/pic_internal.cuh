@@ -45,7 +45,7 @@ enum DevErr : int {
 // the sorted deposit reads four consecutive particles with one 128-bit load
 // from a 4-aligned index below n, which may reach up to 3 elements past n.
 constexpr size_t PARTICLE_PAD = 32;
-constexpr int MOVE_KE_BLOCKS = 4096;  // fixed grid of a gather that sums the kinetic energy
+constexpr int MOVE_KE_BLOCKS = 4096;  // most blocks of a gather that sums the kinetic energy
 
 struct WsState;
 
@@ -116,7 +116,7 @@ struct pic_ctx {
     // deterministic FP64 reductions
     double* red_partials = nullptr;
     double* red_out = nullptr;
-    // per-block sums of vx^2 + vy^2 left by a time step's gather (MOVE_KE_BLOCKS
+    // per-block sums of vx^2 + vy^2 left by a time step's gather (at most MOVE_KE_BLOCKS
     // entries); ke_ready: they belong to the current velocities
     double* ke_partials = nullptr;
     int ke_ready = 0;

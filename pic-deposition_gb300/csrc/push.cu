@@ -40,8 +40,8 @@ struct MoveArgs {
 // KE (with GATHER, every mass 1): the sum of vx^2 + vy^2 of the updated
 // velocities in the arithmetic of fields.cu's sum_v2_partials (exact FP32
 // squares, double-FP32 per thread, FP64 across the block in a fixed order),
-// one partial per block of a fixed grid: the time step's kinetic energy
-// without another pass over the velocities.
+// one partial per block (as many as the particles fill, at most MOVE_KE_BLOCKS): the time
+// step's kinetic energy without another pass over the velocities.
 // A thread takes two consecutive particles at a time: 8-byte loads and stores, and
 // both particles' field reads in flight together. Bound by memory: 0.75 ms for 105 M
 // particles on 1024^2 with gather, push and kinetic sums, 0.84 of the measured copy
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256, 5) move_particles(MoveArgs a) {
 }
 
 // ke: with the gather and unit masses, also leave the kinetic sums of the
-// updated velocities in c->ke_partials (fixed grid of MOVE_KE_BLOCKS blocks).
+// updated velocities in c->ke_partials (c->ke_count blocks' sums).
 int move(pic_ctx* c, double dt, bool gather, bool push, bool ke) {
     c->ke_ready = 0;
     if (c->n == 0) return PIC_OK;

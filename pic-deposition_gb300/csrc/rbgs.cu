@@ -205,9 +205,11 @@ static int rb_finish(pic_ctx* c) {
 // the partials in the same order and takes the same decision. Waits give up
 // after about one second (PIC_ERR_TIMEOUT).
 //
-// Bound by FP64 arithmetic (a warp's FP64 instruction takes the SM 16 cycles) and
-// by the exchange's latency, a store and a load through L2.
-// rb_tiling picks tile counts and halo for the smallest sum of the two. With
+// Bound by the exchange's latency (stores and loads through L2, a thread's halo words one
+// after the other) and by FP64 arithmetic (a warp's FP64 instruction takes the SM 16
+// cycles). rb_tiling picks tile counts and halo for the smallest sum of a model of the two;
+// the model ranks the cuts, it does not give their times (256^2: 1,750 cycles a sweep,
+// measured 3,300). With
 // equal spacings that are powers of two (unit cells, say) an update is four FP64
 // instructions instead of seven, with the same bits: the products are exact, so
 // (we*s + sn*s + b)*inv is one fused multiply-add of we + sn and b*inv.
@@ -528,7 +530,7 @@ constexpr int PS_MAX_NPT = 8;
 // neighbours' cells are needed; `step`: the sweeps between checks are a multiple
 // of it, so halo / 2 must divide it.
 static RbTiling rb_tiling(int Nx, int Ny, int max_blocks, int step, size_t bytes, double op_cycles, double min_cycles) {
-    constexpr double EXCHANGE = 1000.0;  // cycles; 2,000 chose longer halos at 256^2 (101 ms), 500 shorter ones at 222 x 106 (41 against 38)
+    constexpr double EXCHANGE = 1000.0;  // fitted, not measured: 2,000 chose longer halos at 256^2 (101 ms), 500 shorter ones at 222 x 106 (41 against 38)
     RbTiling best;
     double best_cost = 1e300;
     for (int H = 4; H <= 8; H += 4) {
@@ -654,7 +656,7 @@ static int rbgs_solve_persistent(pic_ctx* c, const RbArgs& a, double tol, int ma
     PIC_CUDA_TRY(cudaStreamSynchronize(c->stream));
     int herr = 0;
     std::memcpy(&herr, &h[5], sizeof(int));
-    if (herr) return fail(PIC_ERR_TIMEOUT, "red-black Gauss-Seidel: a grid-wide barrier timed out");
+    if (herr) return fail(PIC_ERR_TIMEOUT, "red-black Gauss-Seidel: a neighbour's exchange or the grid-wide barrier timed out");
     *it = (int)h[0];
     *res = h[1];
     c->first_rbgs_resid = h[2];
@@ -762,7 +764,7 @@ static int rbgs_solve_mixed(pic_ctx* c, const RbArgs& a, double tol, int max_ite
         PIC_CUDA_TRY(cudaStreamSynchronize(c->stream));
         int herr = 0;
         std::memcpy(&herr, &h[5], sizeof(int));
-        if (herr) return fail(PIC_ERR_TIMEOUT, "red-black Gauss-Seidel: a grid-wide barrier timed out");
+        if (herr) return fail(PIC_ERR_TIMEOUT, "red-black Gauss-Seidel: a neighbour's exchange or the grid-wide barrier timed out");
         const int sw = (int)h[0];
         it += sw > 0 ? sw : 1;  // a pass that made no sweep still counts, so the loop ends
     }
